@@ -459,7 +459,9 @@ int tag_fp64_peak(double* flops_per_s);
  * 5 and 6: the halved form of kind 2 with one mean's pair (x[q], y[q]) and
  * the other's (1, 1), so that the two means take different forms
  * (5: ln_mean of the pair in out1; 6: inv_ln_mean of the pair in out2).
- * out1 = ln_mean (kind 4: the Stolarsky mean), out2 = inv_ln_mean. */
+ * out1 = ln_mean (kind 4: the Stolarsky mean), out2 = inv_ln_mean.
+ * 7: out1 = 1/x, out2 = 1/sqrt(y); 8: out1 = x^gamma, out2 = exp(y), in the
+ * kernels' integer-pipe forms. */
 int tag_eval_means(int32_t kind, int64_t n, double cp, double cv, const double* x,
                    const double* y, double* out1, double* out2);
 

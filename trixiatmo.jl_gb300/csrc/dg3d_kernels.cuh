@@ -178,31 +178,6 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
   }
   __syncthreads();
 
-  // per element: can a node pair leave the series range of the logarithmic
-  // means?  If so, the per-node logarithms are computed (once per node)
-  if (Phys::kNodeLogs) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = (nthr + 31) >> 5;
-    for (int el = warp; el < ne; el += nwarps) {
-      const bool logs = element_needs_logs(base + el * S::per_elem + S::oQ, nnn, NQ, Phys::kRho,
-                                           Phys::kBeta, Phys::kLogRange);
-      if (lane == 0) base[el * S::per_elem + S::oL] = logs ? 1.0 : 0.0;
-    }
-    __syncthreads();
-  }
-  if (Phys::kNodeLogs) for (int t = threadIdx.x; t < ne * nnn; t += nthr) {
-    const int el = t / nnn, node = t % nnn;
-    double* eb = base + el * S::per_elem;
-    double* q = eb + S::oQ + node * NQ;
-    if (eb[S::oL] != 0.0) {
-      q[Phys::kLogRho] = log(q[Phys::kRho]);
-      q[Phys::kLogBeta] = log(q[Phys::kBeta]);
-    } else {
-      q[Phys::kLogRho] = 0.0;
-      q[Phys::kLogBeta] = 0.0;
-    }
-  }
-  if (Phys::kNodeLogs) __syncthreads();
-
   // volume integral: each warp takes whole lines (LPW lines of one element,
   // S slots each) and runs their R rounds with only __syncwarp between rounds:
   // the pairs of one line meet the same nodes only across rounds, the lines of
@@ -263,7 +238,8 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
               sfv + ((((size_t)(e_first + el) * 6 + 2 * d + end) * n + p2) * n + p1) * NA;
           double* c = eb + S::oA + (d * nnn + nd) * NA;
 #pragma unroll
-          for (int v = 0; v < NA; ++v) c[v] = fma(sf[v], w, c[v]);
+          for (int v = 0; v < NA; ++v)
+            c[v] = fma(sf[v], Phys::kLastHalved && v == NA - 1 ? 0.5 * w : w, c[v]);
         }
       }
     }
@@ -280,7 +256,8 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
     const double acc = eb[S::oA + (0 * nnn + node) * NA + v] +
                        eb[S::oA + (1 * nnn + node) * NA + v] + eb[S::oA + (2 * nnn + node) * NA + v];
     const size_t gq = (size_t)e * nnn + node;
-    const double dv = acc * (-invJ[gq]) + Phys::source(Pp, eb + S::oU + node * NV, v);
+    const double ij = Phys::kLastHalved && v == NA - 1 ? 2.0 * invJ[gq] : invJ[gq];
+    const double dv = acc * (-ij) + Phys::source(Pp, eb + S::oU + node * NV, v);
     if (not_finite(dv)) bad |= TAG_S_NAN;
     if (MODE == kModeRhs) {
       du[gq * NV + v] = dv;

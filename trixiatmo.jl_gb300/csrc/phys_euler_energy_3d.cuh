@@ -11,19 +11,15 @@ namespace tag {
 struct PhysEnergy3D {
   static constexpr int NV = 6;
   static constexpr int NA = 5;
-  // rho/2, v1/2, v2/2, v3/2, p/2, phi/2, beta/2 = rho/(2p), log(rho/2),
-  // log(beta/2) (odd stride); the halved rho and beta feed ln_mean_pair_halved
+  // rho/2, v1/2, v2/2, v3/2, p/2, phi/4, theta = (p/rho) / (4 (gamma - 1)),
+  // log2(rho), log2(p/rho) (log2_fixed words; odd stride)
   static constexpr int NQ = 9;
-  static constexpr int kRho = 0, kBeta = 6, kLogRho = 7, kLogBeta = 8;
-  // the polynomial forms up to f2 = 0.09 keep every pair of a tall shell element (km-sized
-  // vertical node spacing) out of the logarithms; only elements whose values
-  // spread further take logarithms, once per node
-  static constexpr bool kNodeLogs = true;
-  static constexpr double kLogRange = kLongLogRange;
+  // volume_pair returns half the energy flux (the kernel doubles the node sums)
+  static constexpr bool kLastHalved = true;
   static constexpr bool kHasSources = true;  // Coriolis, added per (node, variable)
 
   struct Params {
-    double gamma, gm1, inv_gm1, c_lmars, quarter_c, inv_c, omega, half_inv_gm1;
+    double gamma, gm1, inv_gm1, c_lmars, quarter_c, inv_c, omega, quarter_inv_gm1;
   };
 
   static Params make_params(const double* p) {
@@ -31,7 +27,7 @@ struct PhysEnergy3D {
     q.gamma = p[0] / p[1];
     q.gm1 = q.gamma - 1.0;
     q.inv_gm1 = 1.0 / (q.gamma - 1.0);
-    q.half_inv_gm1 = 0.5 * q.inv_gm1;
+    q.quarter_inv_gm1 = 0.25 * q.inv_gm1;
     q.c_lmars = p[3];
     q.quarter_c = 0.25 * p[3];
     q.inv_c = 1.0 / p[3];
@@ -39,48 +35,53 @@ struct PhysEnergy3D {
     return q;
   }
 
-  // cons2prim (:568-578) once per node with one reciprocal: rho p =
-  // (gamma - 1)(rho E - |rho v|^2 / 2) needs no division, and r = 1/(rho^2 p)
-  // gives 1/(2 rho) = (rho p) r / 2 and rho/(2p) = rho^3 r / 2.
+  // cons2prim (:568-578) once per node, the reciprocal and both logarithms on
+  // the integer pipe.
   TAG_DEV static void node_prims(const Params& P, const double* u, double* q, unsigned& bad) {
     const double rho = u[0];
+    const double ir = int_rcp(rho), hir = 0.5 * ir;
     const double m2 = fma(u[3], u[3], fma(u[2], u[2], u[1] * u[1]));
-    const double rp = P.gm1 * fma(rho, u[4], -0.5 * m2);
-    const double r = 1.0 / (rho * rp);
-    const double hirho = 0.5 * (rp * r);
+    const double p = P.gm1 * fma(-hir, m2, u[4]);
+    const double pr = p * ir;
     q[0] = 0.5 * rho;
-    q[1] = u[1] * hirho;
-    q[2] = u[2] * hirho;
-    q[3] = u[3] * hirho;
-    q[4] = rp * hirho;
-    q[5] = 0.5 * u[5];
-    q[6] = q[0] * rho * (rho * r);
+    q[1] = u[1] * hir;
+    q[2] = u[2] * hir;
+    q[3] = u[3] * hir;
+    q[4] = 0.5 * p;
+    q[5] = 0.25 * u[5];
+    q[6] = pr * P.quarter_inv_gm1;
+    q[7] = f64_from((u64)log2_fixed(rho));
+    q[8] = f64_from((u64)log2_fixed(pr));
     if (not_positive(rho)) bad |= TAG_S_NEG_DENSITY;
-    if (not_positive(q[4])) bad |= TAG_S_NEG_PRESSURE;
+    if (not_positive(p)) bad |= TAG_S_NEG_PRESSURE;
   }
 
   // flux_ranocha (3D, :382-415) + half of flux_nonconservative_waruszewski_etal
   // (3D, :135-159) for one symmetric pair; see PhysEnergy2D::volume_pair.
-  // nrm is the average of the two nodes' contravariant vectors.  With h the
-  // gravity term rho_mean (phi_b - phi_a) / 2, the momentum fluxes of the two
-  // sides are f1 v + n (p_avg +- h), and the energy fluxes 2 E +- h vn with
-  // E = f1 (v_a.v_b / 4 + inv_beta_mean / (2 (gamma - 1))) + (p_a vn_b + p_b vn_a) / 4
-  // (node values halved, so E is half of flux_ranocha's energy flux).
+  // nrm is twice the average of the two nodes' contravariant vectors (D_split
+  // is halved).  p_ll p_rr inv_ln_mean(rho_ll p_rr, rho_rr p_ll) is
+  // inv_ln_mean(rho_ll/p_ll, rho_rr/p_rr), the mean of the reciprocals of the
+  // node values p/rho.  With g = (phi_b - phi_a) / 4 the momentum fluxes of the
+  // two sides are f1 v + n (p_avg +- 2 rho_mean g), and half the energy fluxes
+  //   f1 (v_a.v_b / 4 + mean(p/rho) / (2 (gamma - 1)) +- g) + (p_a vn_b + p_b vn_a) / 4.
+  // The FP64 pipe bounds the kernel, so the reciprocal and the two series of
+  // the means go to the integer pipe (int_math.cuh): the right-hand side of
+  // the 2,654,208-node shell at polydeg 5 went from 3.48 to 2.37 ms.
   TAG_DEV static void volume_pair(const Params& P, const double* qa, const double* qb,
                                   const double* nrm, double* Fa, double* Fb) {
-    double rho_mean, inv_rho_p_mean;
-    ln_mean_pair_halved(qa[0], qb[0], qa[6], qb[6], qa[7], qb[7], qa[8], qb[8], rho_mean,
-                        inv_rho_p_mean);
+    double R, Q;
+    mean_factors(qa[0], qb[0], qa[6], qb[6], (i64)(f64_bits(qb[7]) - f64_bits(qa[7])),
+                 (i64)(f64_bits(qb[8]) - f64_bits(qa[8])), R, Q);
+    const double rho_mean = (qa[0] + qb[0]) * R;
     const double n1 = nrm[0], n2 = nrm[1], n3 = nrm[2];
     const double v1 = qa[1] + qb[1], v2 = qa[2] + qb[2], v3 = qa[3] + qb[3];
     // halved normal velocities of both nodes: vn = 0.5 (vn_a + vn_b)
     const double vna = fma(qa[3], n3, fma(qa[2], n2, qa[1] * n1));
     const double vnb = fma(qb[3], n3, fma(qb[2], n2, qb[1] * n1));
-    const double vn = vna + vnb;
-    const double f1 = rho_mean * vn;
-    const double h = rho_mean * (qb[5] - qa[5]);
-    const double p_avg = qa[4] + qb[4];
-    const double pp = p_avg + h, pm = p_avg - h;
+    const double f1 = rho_mean * (vna + vnb);
+    const double g = qb[5] - qa[5];
+    const double p_avg = qa[4] + qb[4], r2 = twice(rho_mean);
+    const double pp = fma(r2, g, p_avg), pm = fma(-r2, g, p_avg);
     const double t1 = f1 * v1, t2 = f1 * v2, t3 = f1 * v3;
     Fa[0] = f1;
     Fb[0] = f1;
@@ -91,11 +92,10 @@ struct PhysEnergy3D {
     Fa[3] = fma(n3, pp, t3);
     Fb[3] = fma(n3, pm, t3);
     const double vv = fma(qa[3], qb[3], fma(qa[2], qb[2], qa[1] * qb[1]));
-    const double x = fma(inv_rho_p_mean, P.half_inv_gm1, vv);
+    const double x = fma(qa[6] + qb[6], Q, vv);
     const double e = fma(f1, x, fma(qa[4], vnb, qb[4] * vna));
-    const double hv = h * vn;
-    Fa[4] = fma(2.0, e, hv);
-    Fb[4] = fma(2.0, e, -hv);
+    Fa[4] = fma(f1, g, e);
+    Fb[4] = fma(-f1, g, e);
   }
 
   // FluxLMARS (3D, :430-466) for the (unnormalised) normal n:
@@ -108,7 +108,7 @@ struct PhysEnergy3D {
                             double* F) {
     const double rho_ll = ul[0], rho_rr = ur[0];
     const double srho = rho_ll + rho_rr, prho = rho_ll * rho_rr;
-    const double r = 1.0 / (prho * srho);
+    const double r = int_rcp(prho * srho);
     const double irl = (rho_rr * srho) * r, irr = (rho_ll * srho) * r, isum = prho * r;
     const double ml = fma(ul[3], ul[3], fma(ul[2], ul[2], ul[1] * ul[1]));
     const double mr = fma(ur[3], ur[3], fma(ur[2], ur[2], ur[1] * ur[1]));
@@ -117,7 +117,7 @@ struct PhysEnergy3D {
     const double vl = fma(ul[3], n[2], fma(ul[2], n[1], ul[1] * n[0])) * irl;
     const double vr = fma(ur[3], n[2], fma(ur[2], n[1], ur[1] * n[0])) * irr;
     const double nsq = fma(n[2], n[2], fma(n[1], n[1], n[0] * n[0]));
-    const double inorm = rsqrt(nsq), norm_ = nsq * inorm;
+    const double inorm = int_rsqrt(nsq), norm_ = nsq * inorm;
     const double p = 0.5 * (pl + pr) - P.quarter_c * srho * (vr - vl) * inorm;
     const double v = 0.5 * (vl + vr) - P.inv_c * (pr - pl) * norm_ * isum;
     const double* us = v >= 0.0 ? ul : ur;
@@ -136,7 +136,7 @@ struct PhysEnergy3D {
 
   // boundary_condition_slip_wall (3D), :93-116, with the outward normal n.
   TAG_DEV static void boundary_flux(const Params& P, const double* ui, const double* n, double* F) {
-    const double inn = rsqrt(fma(n[2], n[2], fma(n[1], n[1], n[0] * n[0])));
+    const double inn = int_rsqrt(fma(n[2], n[2], fma(n[1], n[1], n[0] * n[0])));
     const double e0 = n[0] * inn, e1 = n[1] * inn, e2 = n[2] * inn;
     const double un = e0 * ui[1] + e1 * ui[2] + e2 * ui[3];
     const double ub[6] = {ui[0], ui[1] - 2.0 * un * e0, ui[2] - 2.0 * un * e1,
@@ -152,10 +152,10 @@ struct PhysEnergy3D {
   }
 
   TAG_DEV static void max_speeds(const Params& P, const double* u, double* l) {
-    const double irho = 1.0 / u[0];
+    const double irho = int_rcp(u[0]);
     const double v1 = u[1] * irho, v2 = u[2] * irho, v3 = u[3] * irho;
     const double p = P.gm1 * (u[4] - 0.5 * (u[1] * v1 + u[2] * v2 + u[3] * v3));
-    const double c = sqrt(P.gamma * p * irho);
+    const double c = int_sqrt(P.gamma * p * irho);
     l[0] = fabs(v1) + c;
     l[1] = fabs(v2) + c;
     l[2] = fabs(v3) + c;

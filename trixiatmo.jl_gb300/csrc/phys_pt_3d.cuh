@@ -19,9 +19,7 @@ struct PhysPT3D {
   // rho, v1/2, v2/2, v3/2, p/2, phi/2, rho_theta, sigma = rho/rho_theta,
   // rho_theta^gamma, rho_theta^(gamma-1), rho^gamma, rho^(gamma-1), pad (odd stride)
   static constexpr int NQ = 13;
-  static constexpr int kRho = 0, kBeta = 0, kLogRho = 0, kLogBeta = 0;
-  static constexpr bool kNodeLogs = false;
-  static constexpr double kLogRange = kLogMeanRange;
+  static constexpr bool kLastHalved = false;
   static constexpr bool kHasSources = true;  // Coriolis, per (node, variable)
 
   struct Params {

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "../../include/trixiatmo_gpu.h"
+#include "int_math.cuh"
 
 #define TAG_DEV __device__ __forceinline__
 
@@ -235,6 +236,35 @@ TAG_DEV void ln_mean_pair_halved(double hxa, double hxb, double hya, double hyb,
   inv_beta_mean = isy * Q;
 }
 
+// Factors of the two means of a node pair with values (xa, xb) and (ya, yb),
+// from the differences dx, dy of their log2_fixed node logarithms:
+//   ln_mean(xa, xb) = (xa + xb)/2 R,  inv_ln_mean(1/ya, 1/yb) = (ya + yb)/2 Q.
+// Values within a factor of two (every pair of an element that resolves its
+// stratification) take the integer series, whatever their size: no reciprocal,
+// no logarithm, no branch that splits a warp.  The out-of-line branch takes
+// logarithms for the mean that needs them.
+static __device__ __noinline__ void mean_factors_log(double xa, double xb, double ya, double yb,
+                                                     u64 ax, u64 ay, double& R, double& Q) {
+  if (series_in_range(ax))
+    R = ln_mean_factor(log_square(ax));
+  else
+    R = 2.0 * (xb - xa) / (log(xb / xa) * (xa + xb));
+  if (series_in_range(ay))
+    Q = inv_ln_mean_factor(log_square(ay));
+  else
+    Q = 2.0 * ya * yb * log(yb / ya) / ((yb - ya) * (ya + yb));
+}
+TAG_DEV void mean_factors(double xa, double xb, double ya, double yb, i64 dx, i64 dy, double& R,
+                          double& Q) {
+  const u64 ax = magnitude(dx), ay = magnitude(dy);
+  if (!series_in_range(ax | ay)) {
+    mean_factors_log(xa, xb, ya, yb, ax, ay, R, Q);
+    return;
+  }
+  R = ln_mean_factor(log_square(ax));
+  Q = inv_ln_mean_factor(log_square(ay));
+}
+
 // One logarithmic mean (or its inverse) with its own reciprocal: the series of
 // ln_mean_pair in the common range, the reference's (y-x)/log(y/x) outside.
 TAG_DEV double ln_mean_single(double x, double y) {
@@ -261,6 +291,10 @@ TAG_DEV bool not_finite(double x) {
   return ((unsigned long long)__double_as_longlong(x) & 0x7ff0000000000000ull) ==
          0x7ff0000000000000ull;
 }
+
+// 2 x of a normal number with a normal double (an exponent increment on the
+// integer pipe); zero becomes 2^-1022, which any product or sum absorbs.
+TAG_DEV double twice(double x) { return f64_from(f64_bits(x) + (1ull << 52)); }
 
 // Whether the values of one element can push a node pair out of the series
 // range of ln_mean_pair.

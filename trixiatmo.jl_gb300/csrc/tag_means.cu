@@ -26,6 +26,7 @@ int mfail(int code, const std::string& msg) {
 // kind 4: Stolarsky mean of the potential-temperature kernels (out2 unused)
 // kind 5: ln_mean_pair_halved with the pair as the ln_mean pair and (1, 1) as
 //         the inv_ln_mean pair; kind 6 the other way round
+// kind 7: int_rcp(x) and int_rsqrt(y); kind 8: int_pow(x, gamma) and int_exp(y)
 // out1 = ln_mean(x, y) (kind 4: the Stolarsky mean), out2 = inv_ln_mean(x, y);
 // kinds 5 and 6 return the means of their (x, y) and (1, 1) pairs.
 __global__ void k_eval_means(int kind, long n, const double* __restrict__ x,
@@ -54,6 +55,12 @@ __global__ void k_eval_means(int kind, long n, const double* __restrict__ x,
   } else if (kind == 3) {
     m = ln_mean_single(a, b);
     im = inv_ln_mean_single(a, b);
+  } else if (kind == 7) {
+    m = int_rcp(a);
+    im = int_rsqrt(b);
+  } else if (kind == 8) {
+    m = int_pow(a, pt.gamma, (u64)(pt.gamma * 2305843009213693952.0));
+    im = int_exp(b);
   } else {
     const double ag = pow(a, pt.gamma), bg = pow(b, pt.gamma);
     m = PhysPT2D::stolarsky(pt, a, b, ag, ag / a, bg, bg / b);
@@ -68,7 +75,7 @@ extern "C" {
 
 int tag_eval_means(int32_t kind, int64_t n, double gamma_cp, double gamma_cv, const double* x,
                    const double* y, double* out1, double* out2) {
-  if (kind < 0 || kind > 6 || n < 0 || (n > 0 && (!x || !y || !out1 || !out2)))
+  if (kind < 0 || kind > 8 || n < 0 || (n > 0 && (!x || !y || !out1 || !out2)))
     return mfail(TAG_E_INVALID, "tag_eval_means: bad argument");
   if (n == 0) return TAG_OK;
   const double pp[8] = {gamma_cp, gamma_cv, 9.81, 340.0, 0.0, 0.0, 0.0, 1.0};
