@@ -180,8 +180,8 @@ struct ElemSmem {
   static constexpr int oU = 0;
   static constexpr int oQ = oU + nn * NV;
   static constexpr int oJa = oQ + nn * NQ;
-  static constexpr int oC = oJa + nn * 4;        // slots [2][nn][n][NA]
-  static constexpr int oL = oC + 2 * nn * n * NA; // CFL speeds [2][nn]
+  static constexpr int oC = oJa + nn * 4;        // slots [2][nn][n - 1][NA], one per partner
+  static constexpr int oL = oC + 2 * nn * (n - 1) * NA;  // CFL speeds [2][nn]
   static constexpr int oS = oL + 2 * nn;          // sources [nn][NA]
   static constexpr int per_elem = oS + (Phys::kHasSources ? nn * NA : 0);
   static size_t bytes(int epb) { return sizeof(double) * (size_t)per_elem * epb + sizeof(BasisDev); }
@@ -223,46 +223,13 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
   }
   __syncthreads();
 
-  // --- phase 1: per-node primitives; zero the self slots
+  // --- phase 1: per-node primitives
   for (int t = threadIdx.x; t < ne * nn; t += nthr) {
     const int el = t / nn, node = t % nn;
     double* eb = base + el * S::per_elem;
     Phys::node_prims(Pp, eb + S::oU + node * NV, eb + S::oQ + node * NQ, bad);
-    const int i = node % n, j = node / n;
-    if constexpr (VOL == kVolFluxDiff) {
-#pragma unroll
-      for (int v = 0; v < NA; ++v) {
-        eb[S::oC + ((0 * nn + node) * n + i) * NA + v] = 0.0;
-        eb[S::oC + ((1 * nn + node) * n + j) * NA + v] = 0.0;
-      }
-    }
   }
   __syncthreads();
-
-  // per element: can a node pair leave the series range of the logarithmic
-  // means?  If so, the per-node logarithms are computed (once per node)
-  if (Phys::kNodeLogs) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = (nthr + 31) >> 5;
-    for (int el = warp; el < ne; el += nwarps) {
-      const bool logs = element_needs_logs(base + el * S::per_elem + S::oQ, nn, NQ, Phys::kRho,
-                                           Phys::kBeta, kLogMeanRange);
-      if (lane == 0) base[el * S::per_elem + S::oL] = logs ? 1.0 : 0.0;
-    }
-    __syncthreads();
-  }
-  if (Phys::kNodeLogs) for (int t = threadIdx.x; t < ne * nn; t += nthr) {
-    const int el = t / nn, node = t % nn;
-    double* eb = base + el * S::per_elem;
-    double* q = eb + S::oQ + node * NQ;
-    if (eb[S::oL] != 0.0) {
-      q[Phys::kLogRho] = log(q[Phys::kRho]);
-      q[Phys::kLogBeta] = log(q[Phys::kBeta]);
-    } else {
-      q[Phys::kLogRho] = 0.0;
-      q[Phys::kLogBeta] = 0.0;
-    }
-  }
-  if (Phys::kNodeLogs) __syncthreads();
 
   // --- phase 2 (weak form): contravariant fluxes per node,
   //     F~_d = f(u, Ja^d) into slot 0 of direction d
@@ -275,7 +242,7 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
       double F[NA];
       Phys::flux(Pp, eb + S::oU + node * NV, 2.0 * ja[0], 2.0 * ja[1], F);
 #pragma unroll
-      for (int v = 0; v < NA; ++v) eb[S::oC + ((d * nn + node) * n + 0) * NA + v] = F[v];
+      for (int v = 0; v < NA; ++v) eb[S::oC + (d * nn + node) * (n - 1) * NA + v] = F[v];
     }
   }
   // --- phase 2: one thread per symmetric pair (a < b) on a line, ordered by
@@ -301,8 +268,8 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
     double Fa[NA], Fb[NA];
     Phys::volume_pair(Pp, eb + S::oQ + na_ * NQ, eb + S::oQ + nb_ * NQ, n1, n2, Fa, Fb);
     // raw pair fluxes; the D_split weights are applied in the slot reduction
-    double* ca = eb + S::oC + ((d * nn + na_) * n + b) * NA;
-    double* cb = eb + S::oC + ((d * nn + nb_) * n + a) * NA;
+    double* ca = eb + S::oC + ((d * nn + na_) * (n - 1) + b - 1) * NA;  // b > a
+    double* cb = eb + S::oC + ((d * nn + nb_) * (n - 1) + a) * NA;
 #pragma unroll
     for (int v = 0; v < NA; ++v) {
       ca[v] = Fa[v];
@@ -336,28 +303,39 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
     double* eb = base + el * S::per_elem;
     double acc = 0.0;
     if constexpr (VOL == kVolFluxDiff) {
+      // slot s of node a holds the flux with partner s (s < a) or s + 1
 #pragma unroll
-      for (int b = 0; b < n; ++b)
-        acc = fma(sb->Ds[i * n + b], eb[S::oC + ((0 * nn + node) * n + b) * NA + v], acc);
+      for (int s = 0; s < n - 1; ++s)
+        acc = fma(sb->Ds[i * n + s + (s >= i)],
+                  eb[S::oC + ((0 * nn + node) * (n - 1) + s) * NA + v], acc);
 #pragma unroll
-      for (int b = 0; b < n; ++b)
-        acc = fma(sb->Ds[j * n + b], eb[S::oC + ((1 * nn + node) * n + b) * NA + v], acc);
+      for (int s = 0; s < n - 1; ++s)
+        acc = fma(sb->Ds[j * n + s + (s >= j)],
+                  eb[S::oC + ((1 * nn + node) * (n - 1) + s) * NA + v], acc);
     } else {
       // weak form: du(i, j) = sum_b D_hat[i, b] F~_1(b, j) + D_hat[j, b] F~_2(i, b)
 #pragma unroll
       for (int b = 0; b < n; ++b)
-        acc = fma(sb->Dh[i * n + b], eb[S::oC + ((0 * nn + j * n + b) * n + 0) * NA + v], acc);
+        acc = fma(sb->Dh[i * n + b], eb[S::oC + (0 * nn + j * n + b) * (n - 1) * NA + v], acc);
 #pragma unroll
       for (int b = 0; b < n; ++b)
-        acc = fma(sb->Dh[j * n + b], eb[S::oC + ((1 * nn + b * n + i) * n + 0) * NA + v], acc);
+        acc = fma(sb->Dh[j * n + b], eb[S::oC + (1 * nn + b * n + i) * (n - 1) * NA + v], acc);
     }
-    const double* se = sfv + (size_t)e * 4 * n * NA;
-    if (i == 0) acc += se[(0 * n + j) * NA + v] * sb->winv0;
-    if (i == n - 1) acc += se[(1 * n + j) * NA + v] * sb->winvN;
-    if (j == 0) acc += se[(2 * n + i) * NA + v] * sb->winv0;
-    if (j == n - 1) acc += se[(3 * n + i) * NA + v] * sb->winvN;
+    // surface terms: one multiply-add per direction (a node lies on at most
+    // one of a direction's two faces)
+    const double* se = sfv + (size_t)e * 4 * n * NA + v;
+    const bool halved = VOL == kVolFluxDiff && Phys::kLastHalved && v == NA - 1;
+    if (i == 0 || i == n - 1) {
+      const double w = i == 0 ? sb->winv0 : sb->winvN;
+      acc = fma(se[((i == 0 ? 0 : 1) * n + j) * NA], halved ? half_of(w) : w, acc);
+    }
+    if (j == 0 || j == n - 1) {
+      const double w = j == 0 ? sb->winv0 : sb->winvN;
+      acc = fma(se[((j == 0 ? 2 : 3) * n + i) * NA], halved ? half_of(w) : w, acc);
+    }
     const size_t gq = (size_t)e * nn + node;
-    double dv = acc * (-invJ[gq]);
+    const double ij = halved ? twice(invJ[gq]) : invJ[gq];
+    double dv = acc * (-ij);
     if constexpr (Phys::kHasSources) dv += eb[S::oS + node * NA + v];
     if (not_finite(dv)) bad |= TAG_S_NAN;
     if (MODE == kModeRhs) {

@@ -239,7 +239,7 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
           double* c = eb + S::oA + (d * nnn + nd) * NA;
 #pragma unroll
           for (int v = 0; v < NA; ++v)
-            c[v] = fma(sf[v], Phys::kLastHalved && v == NA - 1 ? 0.5 * w : w, c[v]);
+            c[v] = fma(sf[v], Phys::kLastHalved && v == NA - 1 ? half_of(w) : w, c[v]);
         }
       }
     }
@@ -256,7 +256,7 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
     const double acc = eb[S::oA + (0 * nnn + node) * NA + v] +
                        eb[S::oA + (1 * nnn + node) * NA + v] + eb[S::oA + (2 * nnn + node) * NA + v];
     const size_t gq = (size_t)e * nnn + node;
-    const double ij = Phys::kLastHalved && v == NA - 1 ? 2.0 * invJ[gq] : invJ[gq];
+    const double ij = Phys::kLastHalved && v == NA - 1 ? twice(invJ[gq]) : invJ[gq];
     const double dv = acc * (-ij) + Phys::source(Pp, eb + S::oU + node * NV, v);
     if (not_finite(dv)) bad |= TAG_S_NAN;
     if (MODE == kModeRhs) {

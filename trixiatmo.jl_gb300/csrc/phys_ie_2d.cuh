@@ -16,8 +16,7 @@ struct PhysIE2D {
   static constexpr int NA = 4;
   // rho, v1/2, v2/2, p/2, phi/2, beta = rho/p, (unused logs), pad (odd stride)
   static constexpr int NQ = 9;
-  static constexpr int kRho = 0, kBeta = 5, kLogRho = 6, kLogBeta = 7;
-  static constexpr bool kNodeLogs = false;
+  static constexpr bool kLastHalved = false;
   static constexpr bool kHasSources = false;
   static constexpr bool kSurfaceNoncons = true;
 

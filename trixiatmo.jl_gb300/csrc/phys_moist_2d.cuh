@@ -12,8 +12,7 @@ struct PhysMoist2D {
   static constexpr int NA = 6;
   // rho_qd, rho_qv, rho_ql, v1/2, v2/2, 1/T, (v1^2 + v2^2)/4 (odd stride)
   static constexpr int NQ = 7;
-  static constexpr int kRho = 0, kBeta = 0, kLogRho = 0, kLogBeta = 0;
-  static constexpr bool kNodeLogs = false;
+  static constexpr bool kLastHalved = false;
   static constexpr bool kHasSources = true;
   static constexpr bool kSurfaceNoncons = false;  // surface flux only (flux_zero)
 

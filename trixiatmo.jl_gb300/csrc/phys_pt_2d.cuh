@@ -21,8 +21,7 @@ struct PhysPT2D {
   // rho, v1/2, v2/2, p/2, phi/2, rho_theta, sigma = rho/rho_theta,
   // rho_theta^gamma, rho_theta^(gamma-1), rho^gamma, rho^(gamma-1) (odd stride)
   static constexpr int NQ = 11;
-  static constexpr int kRho = 0, kBeta = 0, kLogRho = 0, kLogBeta = 0;
-  static constexpr bool kNodeLogs = false;
+  static constexpr bool kLastHalved = false;
   // MountainWaveSetup's Rayleigh damping when set (Params::mountain)
   static constexpr bool kHasSources = true;
   // surface flux (FluxLMARS(c), flux_zero) or (flux_ec, a nonconservative

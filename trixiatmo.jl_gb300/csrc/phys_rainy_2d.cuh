@@ -60,8 +60,7 @@ struct PhysRainy2D {
   // rho_d, rho_m, rho_r, v1/2, v2/2, rho_vapour, rho_cloud, T, 1/T,
   // v_rain(rho_vapour + rho_cloud, rho_r), (v1^2 + v2^2)/4
   static constexpr int NQ = 11;
-  static constexpr int kRho = 0, kBeta = 0, kLogRho = 0, kLogBeta = 0;
-  static constexpr bool kNodeLogs = false;
+  static constexpr bool kLastHalved = false;
   static constexpr bool kHasSources = true;
   static constexpr bool kSurfaceNoncons = false;  // surface flux only (flux_zero)
 

@@ -236,34 +236,33 @@ TAG_DEV void ln_mean_pair_halved(double hxa, double hxb, double hya, double hyb,
   inv_beta_mean = isy * Q;
 }
 
-// Factors of the two means of a node pair with values (xa, xb) and (ya, yb),
-// from the differences dx, dy of their log2_fixed node logarithms:
+// Factors of the logarithmic means of a node pair, from the difference d of
+// their log2_fixed node logarithms (b minus a):
 //   ln_mean(xa, xb) = (xa + xb)/2 R,  inv_ln_mean(1/ya, 1/yb) = (ya + yb)/2 Q.
 // Values within a factor of two (every pair of an element that resolves its
 // stratification) take the integer series, whatever their size: no reciprocal,
-// no logarithm, no branch that splits a warp.  The out-of-line branch takes
-// logarithms for the mean that needs them.
-static __device__ __noinline__ void mean_factors_log(double xa, double xb, double ya, double yb,
-                                                     u64 ax, u64 ay, double& R, double& Q) {
-  if (series_in_range(ax))
-    R = ln_mean_factor(log_square(ax));
-  else
-    R = 2.0 * (xb - xa) / (log(xb / xa) * (xa + xb));
-  if (series_in_range(ay))
-    Q = inv_ln_mean_factor(log_square(ay));
-  else
-    Q = 2.0 * ya * yb * log(yb / ya) / ((yb - ya) * (ya + yb));
+// no logarithm, no branch that splits a warp.  Beyond it d itself is the
+// logarithm: |d| >= 1, so its 2^-52 is a relative error of the same size.
+TAG_DEV double log_of_difference(i64 d) { return (double)d * 1.539095918623324e-16; }  // ln2 2^-52
+
+static __device__ __noinline__ double ln_factor_far(double xa, double xb, i64 d) {
+  return int_div(2.0 * (xb - xa), log_of_difference(d) * (xa + xb));
 }
-TAG_DEV void mean_factors(double xa, double xb, double ya, double yb, i64 dx, i64 dy, double& R,
-                          double& Q) {
-  const u64 ax = magnitude(dx), ay = magnitude(dy);
-  if (!series_in_range(ax | ay)) {
-    mean_factors_log(xa, xb, ya, yb, ax, ay, R, Q);
-    return;
-  }
-  R = ln_mean_factor(log_square(ax));
-  Q = inv_ln_mean_factor(log_square(ay));
+static __device__ __noinline__ double inv_ln_factor_far(double ya, double yb, i64 d) {
+  return int_div(2.0 * ya * yb * log_of_difference(d), (yb - ya) * (ya + yb));
 }
+TAG_DEV double ln_factor(double xa, double xb, i64 d) {
+  const u64 a = magnitude(d);
+  return series_in_range(a) ? ln_mean_factor(log_square(a)) : ln_factor_far(xa, xb, d);
+}
+TAG_DEV double inv_ln_factor(double ya, double yb, i64 d) {
+  const u64 a = magnitude(d);
+  return series_in_range(a) ? inv_ln_mean_factor(log_square(a)) : inv_ln_factor_far(ya, yb, d);
+}
+
+// Node logarithms are kept among the other node quantities as raw words.
+TAG_DEV double log_word(double x) { return f64_from((u64)log2_fixed(x)); }
+TAG_DEV i64 log_difference(double wa, double wb) { return (i64)(f64_bits(wb) - f64_bits(wa)); }
 
 // One logarithmic mean (or its inverse) with its own reciprocal: the series of
 // ln_mean_pair in the common range, the reference's (y-x)/log(y/x) outside.
@@ -295,6 +294,8 @@ TAG_DEV bool not_finite(double x) {
 // 2 x of a normal number with a normal double (an exponent increment on the
 // integer pipe); zero becomes 2^-1022, which any product or sum absorbs.
 TAG_DEV double twice(double x) { return f64_from(f64_bits(x) + (1ull << 52)); }
+// x / 2 of a normal number with a normal half
+TAG_DEV double half_of(double x) { return f64_from(f64_bits(x) - (1ull << 52)); }
 
 // Whether the values of one element can push a node pair out of the series
 // range of ln_mean_pair.
