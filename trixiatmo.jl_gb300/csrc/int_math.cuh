@@ -310,23 +310,46 @@ TAG_HD double pack_exp2(int i, u64 g) {
 TAG_SLOW double slow_pow(double x, double y) { return pow(x, y); }
 TAG_SLOW double slow_exp(double x) { return exp(x); }
 
-// x^y for an exponent y in (0, 4) given as y_q61 = y 2^61 rounded (a gas
-// constant's ratio, converted once on the host).
-TAG_HD double int_pow(double x, double y, u64 y_q61) {
+// x^y from y as a word with F fraction bits (below 2^63), for normal x whose
+// power is normal too; ok is cleared otherwise.  y log2 x = y t + y l with t the
+// exponent and l the log2 of the significand.
+template <int F>
+TAG_HD double int_pow_word(double x, u64 yq, bool& ok) {
   const u64 b = f64_bits(x);
   const u32 e = (u32)(b >> 52);
-  if (!normal_exponent(e)) return slow_pow(x, y);
-  // y log2 x = y t + y l with t the exponent and l = log2 of the significand
+  ok = normal_exponent(e) && yq != 0;
   const i64 t = (i64)e - 1023;
-  i64 l = log2_significand(significand(b));  // Q.63
+  i64 l = log2_significand(significand(b));                  // Q.63
   l = l < 0 ? 0 : l;
-  const u64 yl = mulhi64(y_q61, (u64)l << 1);                    // y l, Q.61
-  const i64 ti = smulhi64(t << 3, (i64)y_q61);                   // floor(y t) from t y 2^64
-  const u64 tf = ((u64)(t << 3) * y_q61) >> 3;                   // its fraction, Q.61
-  const u64 s = tf + yl;                                         // < 2^61 + 2^63
-  const int i = (int)ti + (int)(s >> 61);
-  if (i < -1020 || i > 1020) return slow_pow(x, y);
-  return pack_exp2(i, s << 3);
+  const u64 yl = mulhi64(yq, (u64)l << 1);                   // y l, Q.F
+  const i64 ti = smulhi64(t << (64 - F), (i64)yq);           // floor(y t)
+  const u64 tf = ((u64)(t << (64 - F)) * yq) >> (64 - F);    // its fraction, Q.F
+  const u64 s = tf + yl;
+  const int i = (int)ti + (int)(s >> F);
+  ok = ok && i >= -1020 && i <= 1020;
+  return pack_exp2(ok ? i : 0, s << (64 - F));
+}
+
+// An exponent y in (0, 4) as Q2.61 for int_pow; 0 (the out-of-line branch)
+// for any other.
+inline u64 pow_exponent(double y) {
+  return y > 0.0 && y < 4.0 ? (u64)(y * 2305843009213693952.0) : 0;
+}
+
+// x^y for a fixed exponent y (a ratio of gas constants), y_q61 = pow_exponent(y).
+TAG_HD double int_pow(double x, double y, u64 y_q61) {
+  bool ok;
+  const double r = int_pow_word<61>(x, y_q61, ok);
+  return ok ? r : slow_pow(x, y);
+}
+
+// x^y for an exponent in [1/64, 16), which Q4.58 holds exactly.
+TAG_HD double int_pow(double x, double y) {
+  const u64 b = f64_bits(y);
+  const int sh = (int)(b >> 52) - 1023;
+  bool ok = sh >= -6 && sh <= 3;
+  const double r = int_pow_word<58>(x, ok ? (significand(b) >> 5) >> -(sh < 0 ? sh : 0) << (sh > 0 ? sh : 0) : 0, ok);
+  return ok ? r : slow_pow(x, y);
 }
 
 // e^x for |x| < 512: x log2 e in fixed point, its integer part the exponent.
@@ -410,6 +433,70 @@ TAG_HD double inv_ln_mean_factor(u64 z) {
   p = TAG_INV_A1 - mulhi64(z, p);
   p = TAG_INV_A0 - mulhi64(z, p);
   return one_minus(mulhi64(z, p));
+}
+
+// A mean's factor 1 - z (a0 + z (a1 + ...)) with coefficients of run-time
+// parameters, in the same form (any signs; seven Q0.63 words, six binary32).
+// ok: the fixed-point form holds (the factor stays within (1/2, 1]).
+struct EvenSeries {
+  i64 a[7];
+  float b[6];
+  int ok;
+};
+TAG_HD double even_factor(const EvenSeries& s, u64 z) {
+  const i64 zq = (i64)(z >> 1);  // Q0.63
+  const float zf = (float)(u32)(z >> 32) * 2.3283064365386963e-10f;
+  float P = s.b[5];
+#pragma unroll
+  for (int k = 4; k >= 0; --k) P = fmaf(zf, P, s.b[k]);
+  i64 p = (i64)f32_to_int(P * 1.152921504606847e18f) << 3;  // Q.60 -> Q.63
+#pragma unroll
+  for (int k = 6; k >= 0; --k) p = s.a[k] + (smulhi64(zq, p) << 1);
+  return one_minus((u64)(smulhi64(zq, p) << 2));
+}
+
+// The Stolarsky mean S(u, v) = (g-1)/g (v^g - u^g)/(v^(g-1) - u^(g-1)) is
+// (u + v)/2 times sinh(g x) (g-1)/g / (sinh((g-1) x) cosh(x)), x = log(v/u)/2:
+// the coefficients of that factor in z = d^2, x = d ln2/2, from the quotient of
+// the three Taylor series.
+inline EvenSeries stolarsky_series(double gamma) {
+  constexpr int T = 14;
+  using R = long double;
+  const R g = gamma, ln2h = 0.346573590279972654708616060729088284L, x2 = ln2h * ln2h;
+  R num[T], den[T], sb[T], ch[T];
+  R p = 1, q = 1, r = 1;
+  for (int k = 0; k < T; ++k) {  // sinh(gx)/(gx), sinh((g-1)x)/((g-1)x), cosh(x)
+    num[k] = p;
+    sb[k] = q;
+    ch[k] = r;
+    p *= g * g * x2 / ((2 * k + 2) * (R)(2 * k + 3));
+    q *= (g - 1) * (g - 1) * x2 / ((2 * k + 2) * (R)(2 * k + 3));
+    r *= x2 / ((2 * k + 1) * (R)(2 * k + 2));
+  }
+  R w[T];
+  for (int k = 0; k < T; ++k) {
+    den[k] = 0;
+    for (int i = 0; i <= k; ++i) den[k] += sb[i] * ch[k - i];
+  }
+  for (int k = 0; k < T; ++k) {
+    w[k] = num[k];
+    for (int i = 1; i <= k; ++i) w[k] -= den[i] * w[k - i];
+  }
+  EvenSeries s{};
+  s.ok = gamma > 1.0 && gamma < 2.0;
+  R at1 = 0;
+  for (int k = 0; k < 13; ++k) {
+    const R a = -w[k + 1];
+    at1 += a;
+    if (k < 7)
+      s.a[k] = (i64)llroundl(a * 9223372036854775808.0L);
+    else
+      s.b[k - 7] = (float)a;
+    if (k == 0 && !(a >= 0 && a < 0.25L)) s.ok = 0;
+    if (k == 7 && !(fabsl(a) < 1e-9L)) s.ok = 0;
+  }
+  if (!(at1 >= 0 && at1 < 0.25L)) s.ok = 0;
+  return s;
 }
 
 }  // namespace tag

@@ -70,6 +70,7 @@ def main():
     for k in (4, 5, 6):
         print("#define TAG_EXP2_C%d %sf" % (k, mp.nstr(LN2 ** k / mp.factorial(k), 10)))
     print("#define TAG_LOG2E_Q62 %dll" % fix(1 / LN2, 62))
+    print("#define TAG_RAINY_LOG2_REF %dll" % fix(mp.log(mp.mpf("273.15"), 2), 58))
     print("#define TAG_LN2_Q64 %dull" % fix(LN2, 64))
     print("}  // namespace tag")
 

@@ -6,10 +6,9 @@
 // (or Artiano et al., Souza et al.); surface flux (FluxLMARS(c), flux_zero).
 //
 // The Stolarsky mean S(x, y) = (gamma-1)/gamma (y^g - x^g) / (y^(g-1) - x^(g-1))
-// (Winters et al. 2020) is evaluated as (x+y)/2 R(f^2), f = (y-x)/(x+y), with the
-// first eight terms of its series in f^2 when f^2 < 1e-2 (coefficients from the
-// binomial expansions of (1 +- f)^a, computed on the host per gamma), else from
-// per-node powers x^g, x^(g-1) with one division per pair.
+// (Winters et al. 2020) is (x+y)/2 times an even function of log(y/x), evaluated
+// as its series on the integer pipe for values within a factor of two
+// (int_math.cuh); beyond that, and for gamma outside (1, 2), from powers.
 #pragma once
 #include "tag_common.cuh"
 
@@ -18,9 +17,10 @@ namespace tag {
 struct PhysPT2D {
   static constexpr int NV = 5;
   static constexpr int NA = 4;
-  // rho, v1/2, v2/2, p/2, phi/2, rho_theta, sigma = rho/rho_theta,
-  // rho_theta^gamma, rho_theta^(gamma-1), rho^gamma, rho^(gamma-1) (odd stride)
-  static constexpr int NQ = 11;
+  // rho/2, v1/2, v2/2, p/2, phi/2, rho_theta/2, the third mean's half value
+  // (flux_ec: theta = rho_theta/rho, flux_etec: 1/theta), log2(rho),
+  // log2(rho_theta) (log2_fixed words; odd stride)
+  static constexpr int NQ = 9;
   static constexpr bool kLastHalved = false;
   // MountainWaveSetup's Rayleigh damping when set (Params::mountain)
   static constexpr bool kHasSources = true;
@@ -30,7 +30,9 @@ struct PhysPT2D {
 
   struct Params {
     double gamma, K, c_lmars, stol_fac;  // stol_fac = (gamma - 1) / gamma
-    double sc[8];                        // Stolarsky series coefficients
+    double sc[8];                        // Stolarsky series in f^2 (gamma outside (1, 2))
+    EvenSeries stol;                     // Stolarsky factor of the logarithms' difference
+    u64 gamma_q61;                       // gamma as int_pow takes it
     int volume;                          // 0 flux_tec, 1 flux_ec, 2 flux_etec,
                                          // 3 flux_kennedy_gruber (3D only)
     int nc;                              // 0 waruszewski, 1 artiano, 2 souza
@@ -51,6 +53,8 @@ struct PhysPT2D {
     q.K = 100000.0 * pow(R / 100000.0, q.gamma);
     q.c_lmars = p[3];
     q.stol_fac = (q.gamma - 1.0) / q.gamma;
+    q.stol = stolarsky_series(q.gamma);
+    q.gamma_q61 = pow_exponent(q.gamma);
     q.nc = (int)p[4];
     q.volume = (int)p[5];
     q.surface = (int)p[6];
@@ -76,42 +80,82 @@ struct PhysPT2D {
     return q;
   }
 
-  TAG_DEV static void node_prims(const Params& P, const double* u, double* q, unsigned& bad) {
-    const double rho = u[0];
-    const double irho = 1.0 / rho;
-    const double tg = pow(u[3], P.gamma);  // rho_theta^gamma
-    q[0] = rho;
-    q[1] = 0.5 * u[1] * irho;
-    q[2] = 0.5 * u[2] * irho;
-    q[3] = 0.5 * (P.K * tg);
-    q[4] = 0.5 * u[4];
-    q[5] = u[3];
-    q[6] = rho / u[3];
-    q[7] = tg;
-    q[8] = tg / u[3];
-    if (P.nc == 1) {
-      const double rg = pow(rho, P.gamma);
-      q[9] = rg;
-      q[10] = rg * irho;
-    } else {
-      q[9] = q[10] = 0.0;
-    }
-    if (!(rho > 0.0)) bad |= TAG_S_NEG_DENSITY;
-    if (!(u[3] > 0.0)) bad |= TAG_S_NEG_PRESSURE;
+  TAG_DEV static double pressure(const Params& P, double rho_theta) {
+    return P.K * int_pow(rho_theta, P.gamma, P.gamma_q61);
   }
 
-  // Stolarsky mean of x, y with per-node powers (x^g, x^(g-1)), (y^g, y^(g-1))
-  TAG_DEV static double stolarsky(const Params& P, double x, double y, double xg, double xg1,
-                                  double yg, double yg1) {
+  // the third mean's half node value (volume 3: flux_kennedy_gruber's theta)
+  TAG_DEV static double third_value(const Params& P, double rho, double rho_theta, double irho) {
+    if (P.volume == 0) return 0.0;
+    return P.volume == 2 ? 0.5 * rho * int_rcp(rho_theta) : 0.5 * rho_theta * irho;
+  }
+
+  TAG_DEV static void node_prims(const Params& P, const double* u, double* q, unsigned& bad) {
+    const double rho = u[0];
+    const double irho = int_rcp(rho), hir = 0.5 * irho;
+    q[0] = 0.5 * rho;
+    q[1] = u[1] * hir;
+    q[2] = u[2] * hir;
+    q[3] = 0.5 * pressure(P, u[3]);
+    q[4] = 0.5 * u[4];
+    q[5] = 0.5 * u[3];
+    q[6] = third_value(P, rho, u[3], irho);
+    q[7] = log_word(rho);
+    q[8] = log_word(u[3]);
+    if (not_positive(rho)) bad |= TAG_S_NEG_DENSITY;
+    if (not_positive(u[3])) bad |= TAG_S_NEG_PRESSURE;
+  }
+
+  // Stolarsky mean over the arithmetic mean, from the values themselves: the
+  // series in f^2 where they nearly agree, else powers
+  static __device__ __noinline__ double stolarsky_factor_far(const Params& P, double x, double y) {
     const double s = x + y, d = y - x;
     const double t = d / s, f2 = t * t;
     if (f2 < 1e-2) {
       double r = P.sc[7];
-#pragma unroll
       for (int k = 6; k >= 0; --k) r = fma(r, f2, P.sc[k]);
-      return 0.5 * s * r;
+      return r;
     }
-    return P.stol_fac * (yg - xg) / (yg1 - xg1);
+    const double xg = pow(x, P.gamma), yg = pow(y, P.gamma);
+    return 2.0 * (P.stol_fac * (yg - xg) / (yg / y - xg / x)) / s;
+  }
+  // x, y: the values or their halves (the factor is homogeneous)
+  TAG_DEV static double stolarsky_factor(const Params& P, double x, double y, i64 d) {
+    const u64 a = magnitude(d);
+    return series_in_range(a) && P.stol.ok ? even_factor(P.stol, log_square(a))
+                                           : stolarsky_factor_far(P, x, y);
+  }
+  TAG_DEV static double stolarsky(const Params& P, double x, double y) {
+    return 0.5 * (x + y) * stolarsky_factor(P, x, y, log2_fixed(y) - log2_fixed(x));
+  }
+
+  // The mass flux f1, the rho_theta flux f and the density average of the
+  // gravity term for the averaged normal velocity vn, from the node values
+  // rho/2, rho_theta/2, the third value and the logarithms' differences.
+  TAG_DEV static void mean_fluxes(const Params& P, double ra, double rb, double ta, double tb,
+                                  double xa, double xb, i64 dr, i64 dt, double vn, double& f1,
+                                  double& f, double& ravg) {
+    const double rs = ra + rb;
+    double rho_ln = 0.0;
+    if (P.volume == 1) {
+      rho_ln = rs * ln_factor(ra, rb, dr);
+      f1 = rho_ln * vn;
+      f = f1 * ((xa + xb) * inv_ln_factor(xa, xb, dt - dr));
+    } else if (P.volume == 3) {
+      f1 = rs * vn;
+      f = f1 * (xa + xb);
+    } else {
+      f = (ta + tb) * stolarsky_factor(P, ta, tb, dt) * vn;
+      if (P.volume == 0) {
+        rho_ln = rs * ln_factor(ra, rb, dr);
+        f1 = rho_ln * vn;
+      } else {
+        f1 = f * ((xa + xb) * ln_factor(xa, xb, dr - dt));
+      }
+    }
+    if (P.nc == 0) ravg = P.volume >= 2 ? rs * ln_factor(ra, rb, dr) : rho_ln;
+    else if (P.nc == 1) ravg = rs * stolarsky_factor(P, ra, rb, dr);
+    else ravg = rs;
   }
 
   // One symmetric pair: the two-point flux F plus half the nonconservative
@@ -120,60 +164,32 @@ struct PhysPT2D {
                                   double n2, double* Fa, double* Fb) {
     const double v1 = a[1] + b[1], v2 = a[2] + b[2];
     const double vn = n1 * v1 + n2 * v2;
+    double f1, f4, ravg;
+    mean_fluxes(P, a[0], b[0], a[5], b[5], a[6], b[6], log_difference(a[7], b[7]),
+                log_difference(a[8], b[8]), vn, f1, f4, ravg);
     const double pa = a[3] + b[3];
-    double rho_ln = 0.0, f1, f4;
-    if (P.volume == 1) {
-      double inv_sig;
-      ln_mean_pair<false>(a[0], b[0], a[6], b[6], 0.0, 0.0, 0.0, 0.0, rho_ln, inv_sig);
-      f1 = rho_ln * vn;
-      f4 = f1 * inv_sig;
-    } else {
-      f4 = stolarsky(P, a[5], b[5], a[7], a[8], b[7], b[8]) * vn;
-      if (P.volume == 0) {
-        rho_ln = ln_mean_single(a[0], b[0]);
-        f1 = rho_ln * vn;
-      } else {
-        f1 = f4 * ln_mean_single(a[6], b[6]);
-      }
-    }
-    double ravg;
-    if (P.nc == 0) ravg = (P.volume == 2) ? ln_mean_single(a[0], b[0]) : rho_ln;
-    else if (P.nc == 1) ravg = stolarsky(P, a[0], b[0], a[9], a[10], b[9], b[10]);
-    else ravg = 0.5 * (a[0] + b[0]);
-    const double jump = 2.0 * (b[4] - a[4]);  // phi_b - phi_a (stored halved)
-    const double g1 = 0.5 * n1 * ravg * jump, g2 = 0.5 * n2 * ravg * jump;
-    const double F2 = f1 * v1 + pa * n1, F3 = f1 * v2 + pa * n2;
+    const double g = b[4] - a[4];  // (phi_b - phi_a) / 2
+    const double pp = fma(ravg, g, pa), pm = fma(-ravg, g, pa);
+    const double t1 = f1 * v1, t2 = f1 * v2;
     Fa[0] = Fb[0] = f1;
-    Fa[1] = F2 + g1;
-    Fb[1] = F2 - g1;
-    Fa[2] = F3 + g2;
-    Fb[2] = F3 - g2;
+    Fa[1] = fma(n1, pp, t1);
+    Fb[1] = fma(n1, pm, t1);
+    Fa[2] = fma(n2, pp, t2);
+    Fb[2] = fma(n2, pm, t2);
     Fa[3] = Fb[3] = f4;
-  }
-
-  // flux(u, normal_direction), :84-98 (pressure() = K exp(gamma log rho_theta))
-  TAG_DEV static void flux(const Params& P, const double* u, double n1, double n2, double* f) {
-    const double v1 = u[1] / u[0], v2 = u[2] / u[0];
-    const double vn = v1 * n1 + v2 * n2;
-    const double rvn = u[0] * vn;
-    const double p = P.K * exp(P.gamma * log(u[3]));
-    f[0] = rvn;
-    f[1] = rvn * v1 + p * n1;
-    f[2] = rvn * v2 + p * n2;
-    f[3] = u[3] * vn;
   }
 
   // FluxLMARS (:171-193)
   TAG_DEV static void lmars(const Params& P, const double* ul, const double* ur, double n1,
                             double n2, double* F) {
     const double a = P.c_lmars;
-    const double p_l = P.K * pow(ul[3], P.gamma), p_r = P.K * pow(ur[3], P.gamma);
-    const double v_l = (ul[1] / ul[0]) * n1 + (ul[2] / ul[0]) * n2;
-    const double v_r = (ur[1] / ur[0]) * n1 + (ur[2] / ur[0]) * n2;
-    const double nrm = sqrt(n1 * n1 + n2 * n2);
-    const double rho = 0.5 * (ul[0] + ur[0]);
-    const double p_int = 0.5 * (p_l + p_r) - 0.5 * a * rho * (v_r - v_l) / nrm;
-    const double v_int = 0.5 * (v_l + v_r) - 1.0 / (2.0 * a * rho) * (p_r - p_l) * nrm;
+    const double p_l = pressure(P, ul[3]), p_r = pressure(P, ur[3]);
+    const double v_l = fma(ul[2], n2, ul[1] * n1) * int_rcp(ul[0]);
+    const double v_r = fma(ur[2], n2, ur[1] * n1) * int_rcp(ur[0]);
+    const double nsq = fma(n2, n2, n1 * n1), inorm = int_rsqrt(nsq), nrm = nsq * inorm;
+    const double rs = ul[0] + ur[0];  // 2 rho
+    const double p_int = 0.5 * (p_l + p_r) - 0.25 * a * rs * (v_r - v_l) * inorm;
+    const double v_int = 0.5 * (v_l + v_r) - int_rcp(a * rs) * (p_r - p_l) * nrm;
     const double* us = v_int > 0.0 ? ul : ur;
     F[0] = us[0] * v_int;
     F[1] = us[1] * v_int + p_int * n1;
@@ -184,15 +200,12 @@ struct PhysPT2D {
   // flux_ec (:290-321) of full states
   TAG_DEV static void flux_ec(const Params& P, const double* ul, const double* ur, double n1,
                               double n2, double* F) {
-    const double irl = 1.0 / ul[0], irr = 1.0 / ur[0];
+    const double irl = int_rcp(ul[0]), irr = int_rcp(ur[0]);
     const double v1l = ul[1] * irl, v2l = ul[2] * irl, v1r = ur[1] * irr, v2r = ur[2] * irr;
-    const double pl = P.K * pow(ul[3], P.gamma), pr = P.K * pow(ur[3], P.gamma);
     const double vn = 0.5 * ((v1l * n1 + v2l * n2) + (v1r * n1 + v2r * n2));
-    const double pa = 0.5 * (pl + pr);
-    double rho_ln, inv_sig;
-    ln_mean_pair<false>(ul[0], ur[0], ul[0] / ul[3], ur[0] / ur[3], 0.0, 0.0, 0.0, 0.0, rho_ln,
-                        inv_sig);
-    const double f1 = rho_ln * vn;
+    const double pa = 0.5 * (pressure(P, ul[3]) + pressure(P, ur[3]));
+    const double f1 = ln_mean_of(ul[0], ur[0]) * vn;
+    const double inv_sig = inv_ln_mean_of_reciprocals(ul[3] * irl, ur[3] * irr);
     F[0] = f1;
     F[1] = f1 * 0.5 * (v1l + v1r) + pa * n1;
     F[2] = f1 * 0.5 * (v2l + v2r) + pa * n2;
@@ -220,20 +233,21 @@ struct PhysPT2D {
     const double rate = P.mw[7], zs = P.mw[3], ze = P.mw[4], xs = P.mw[5], xe = P.mw[6];
     double dv = 0.0, dr = 0.0, dl = 0.0;
     if (x[1] > zs) {
-      const double r = sinpi(0.5 * (x[1] - zs) / (ze - zs));
+      const double r = sinpi(int_div(0.5 * (x[1] - zs), ze - zs));
       dv = rate * (r * r);
     }
     if (!(x[0] < xs)) {
-      const double r = sinpi(0.5 * (x[0] - xs) / (xe - xs));
+      const double r = sinpi(int_div(0.5 * (x[0] - xs), xe - xs));
       dr = rate * (r * r);
     }
     if (!(x[0] > -xs)) {
-      const double r = sinpi(0.5 * (x[0] + xs) / (-xe + xs));
+      const double r = sinpi(int_div(0.5 * (x[0] + xs), -xe + xs));
       dl = rate * (r * r);
     }
     const double damping = -(dv + dr + dl);
-    const double v1 = u[1] / u[0], theta = u[3] / u[0];
-    const double theta_b = P.mw[0] * exp(P.mw[2] * P.mw[2] / P.g * x[1]);
+    const double irho = int_rcp(u[0]);
+    const double v1 = u[1] * irho, theta = u[3] * irho;
+    const double theta_b = P.mw[0] * int_exp(int_div(P.mw[2] * P.mw[2], P.g) * x[1]);
     s[1] = u[0] * (v1 - P.mw[1]) * damping;
     s[2] = u[2] * damping;
     s[3] = u[0] * (theta - theta_b) * damping;
@@ -245,10 +259,9 @@ struct PhysPT2D {
     if (P.snc < 0) return;
     double ra;
     if (P.snc == 0) {
-      ra = ln_mean_single(ul[0], ur[0]);
+      ra = ln_mean_of(ul[0], ur[0]);
     } else if (P.snc == 1) {
-      const double xg = pow(ul[0], P.gamma), yg = pow(ur[0], P.gamma);
-      ra = stolarsky(P, ul[0], ur[0], xg, xg / ul[0], yg, yg / ur[0]);
+      ra = stolarsky(P, ul[0], ur[0]);
     } else {
       ra = 0.5 * (ul[0] + ur[0]);
     }
@@ -273,8 +286,8 @@ struct PhysPT2D {
         F[0] = -F[0]; F[1] = -F[1]; F[2] = -F[2]; F[3] = -F[3];
       }
     } else {
-      const double nn = sqrt(n1 * n1 + n2 * n2);
-      const double nx = n1 / nn, ny = n2 / nn;
+      const double inn = int_rsqrt(n1 * n1 + n2 * n2);
+      const double nx = n1 * inn, ny = n2 * inn;
       const double un = nx * ui[1] + ny * ui[2];
       const double ub[5] = {ui[0], ui[1] - 2.0 * un * nx, ui[2] - 2.0 * un * ny, ui[3], ui[4]};
       surface_flux(P, ui, ub, n1, n2, F);
@@ -283,10 +296,9 @@ struct PhysPT2D {
 
   // max_abs_speeds
   TAG_DEV static void max_speeds(const Params& P, const double* u, double& l1, double& l2) {
-    const double rho = u[0];
-    const double v1 = u[1] / rho, v2 = u[2] / rho;
-    const double p = P.K * pow(u[3], P.gamma);
-    const double c = sqrt(P.gamma * p / rho);
+    const double irho = int_rcp(u[0]);
+    const double v1 = u[1] * irho, v2 = u[2] * irho;
+    const double c = int_sqrt(P.gamma * pressure(P, u[3]) * irho);
     l1 = fabs(v1) + c;
     l2 = fabs(v2) + c;
   }

@@ -6,8 +6,7 @@
 // flux_tec / flux_ec / flux_etec (:428-533) with the nonconservative gravity
 // term of Waruszewski et al. (or Artiano et al., Souza et al.; :146-211);
 // surface flux (FluxLMARS(c), flux_zero) (:213-256); slip walls (:83-107).
-// The Stolarsky mean as in phys_pt_2d.cuh (series below f^2 = 1e-2, per-node
-// powers above).
+// The means as in phys_pt_2d.cuh.
 #pragma once
 #include "phys_pt_2d.cuh"
 
@@ -16,9 +15,9 @@ namespace tag {
 struct PhysPT3D {
   static constexpr int NV = 6;
   static constexpr int NA = 5;
-  // rho, v1/2, v2/2, v3/2, p/2, phi/2, rho_theta, sigma = rho/rho_theta,
-  // rho_theta^gamma, rho_theta^(gamma-1), rho^gamma, rho^(gamma-1), pad (odd stride)
-  static constexpr int NQ = 13;
+  // rho/2, v1/2, v2/2, v3/2, p/2, phi/2, rho_theta/2, the third mean's half
+  // value (phys_pt_2d.cuh), log2(rho), log2(rho_theta), (pad: odd stride)
+  static constexpr int NQ = 11;
   static constexpr bool kLastHalved = false;
   static constexpr bool kHasSources = true;  // Coriolis, per (node, variable)
 
@@ -42,71 +41,44 @@ struct PhysPT3D {
   TAG_DEV static void node_prims(const Params& Q, const double* u, double* q, unsigned& bad) {
     const PhysPT2D::Params& P = Q.pt;
     const double rho = u[0];
-    const double irho = 1.0 / rho;
-    const double tg = pow(u[4], P.gamma);  // rho_theta^gamma
-    q[0] = rho;
-    q[1] = 0.5 * u[1] * irho;
-    q[2] = 0.5 * u[2] * irho;
-    q[3] = 0.5 * u[3] * irho;
-    q[4] = 0.5 * (P.K * tg);
+    const double irho = int_rcp(rho), hir = 0.5 * irho;
+    q[0] = 0.5 * rho;
+    q[1] = u[1] * hir;
+    q[2] = u[2] * hir;
+    q[3] = u[3] * hir;
+    q[4] = 0.5 * PhysPT2D::pressure(P, u[4]);
     q[5] = 0.5 * u[5];
-    q[6] = u[4];
-    q[7] = rho / u[4];
-    q[8] = tg;
-    q[9] = tg / u[4];
-    if (P.nc == 1) {
-      const double rg = pow(rho, P.gamma);
-      q[10] = rg;
-      q[11] = rg * irho;
-    } else {
-      q[10] = q[11] = 0.0;
-    }
-    q[12] = P.volume == 3 ? 0.5 * u[4] * irho : 0.0;  // theta / 2 (flux_kennedy_gruber)
-    if (!(rho > 0.0)) bad |= TAG_S_NEG_DENSITY;
-    if (!(u[4] > 0.0)) bad |= TAG_S_NEG_PRESSURE;
+    q[6] = 0.5 * u[4];
+    q[7] = PhysPT2D::third_value(P, rho, u[4], irho);
+    q[8] = log_word(rho);
+    q[9] = log_word(u[4]);
+    if (not_positive(rho)) bad |= TAG_S_NEG_DENSITY;
+    if (not_positive(u[4])) bad |= TAG_S_NEG_PRESSURE;
   }
 
   // One symmetric pair: the two-point flux F plus half the nonconservative
   // term G (antisymmetric in the pair): Fa = F + G/2, Fb = F - G/2.
+  // (flux_kennedy_gruber, :333-359: arithmetic means of rho, v, p and theta)
   TAG_DEV static void volume_pair(const Params& Q, const double* a, const double* b,
                                   const double* nrm, double* Fa, double* Fb) {
     const PhysPT2D::Params& P = Q.pt;
     const double n1 = nrm[0], n2 = nrm[1], n3 = nrm[2];
     const double v1 = a[1] + b[1], v2 = a[2] + b[2], v3 = a[3] + b[3];
     const double vn = n1 * v1 + n2 * v2 + n3 * v3;
+    double f1, f5, ravg;
+    PhysPT2D::mean_fluxes(P, a[0], b[0], a[6], b[6], a[7], b[7], log_difference(a[8], b[8]),
+                          log_difference(a[9], b[9]), vn, f1, f5, ravg);
     const double pa = a[4] + b[4];
-    double rho_ln = 0.0, f1, f5;
-    if (P.volume == 1) {
-      double inv_sig;
-      ln_mean_pair<false>(a[0], b[0], a[7], b[7], 0.0, 0.0, 0.0, 0.0, rho_ln, inv_sig);
-      f1 = rho_ln * vn;
-      f5 = f1 * inv_sig;
-    } else if (P.volume == 3) {
-      // flux_kennedy_gruber (:333-359): arithmetic means of rho, v, p and theta
-      f1 = 0.5 * (a[0] + b[0]) * vn;
-      f5 = f1 * (a[12] + b[12]);
-    } else {
-      f5 = PhysPT2D::stolarsky(P, a[6], b[6], a[8], a[9], b[8], b[9]) * vn;
-      if (P.volume == 0) {
-        rho_ln = ln_mean_single(a[0], b[0]);
-        f1 = rho_ln * vn;
-      } else {
-        f1 = f5 * ln_mean_single(a[7], b[7]);
-      }
-    }
-    double ravg;
-    if (P.nc == 0) ravg = (P.volume >= 2) ? ln_mean_single(a[0], b[0]) : rho_ln;
-    else if (P.nc == 1) ravg = PhysPT2D::stolarsky(P, a[0], b[0], a[10], a[11], b[10], b[11]);
-    else ravg = 0.5 * (a[0] + b[0]);
-    const double h = ravg * (b[5] - a[5]);  // (phi_b - phi_a) / 2 rho_avg (stored halved)
-    const double F2 = f1 * v1 + pa * n1, F3 = f1 * v2 + pa * n2, F4 = f1 * v3 + pa * n3;
+    const double g = b[5] - a[5];  // (phi_b - phi_a) / 2
+    const double pp = fma(ravg, g, pa), pm = fma(-ravg, g, pa);
+    const double t1 = f1 * v1, t2 = f1 * v2, t3 = f1 * v3;
     Fa[0] = Fb[0] = f1;
-    Fa[1] = F2 + n1 * h;
-    Fb[1] = F2 - n1 * h;
-    Fa[2] = F3 + n2 * h;
-    Fb[2] = F3 - n2 * h;
-    Fa[3] = F4 + n3 * h;
-    Fb[3] = F4 - n3 * h;
+    Fa[1] = fma(n1, pp, t1);
+    Fb[1] = fma(n1, pm, t1);
+    Fa[2] = fma(n2, pp, t2);
+    Fb[2] = fma(n2, pm, t2);
+    Fa[3] = fma(n3, pp, t3);
+    Fb[3] = fma(n3, pm, t3);
     Fa[4] = Fb[4] = f5;
   }
 
@@ -115,13 +87,14 @@ struct PhysPT3D {
                             double* F) {
     const PhysPT2D::Params& P = Q.pt;
     const double a = P.c_lmars;
-    const double p_l = P.K * pow(ul[4], P.gamma), p_r = P.K * pow(ur[4], P.gamma);
-    const double v_l = (ul[1] / ul[0]) * n[0] + (ul[2] / ul[0]) * n[1] + (ul[3] / ul[0]) * n[2];
-    const double v_r = (ur[1] / ur[0]) * n[0] + (ur[2] / ur[0]) * n[1] + (ur[3] / ur[0]) * n[2];
-    const double nrm = sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
-    const double rho = 0.5 * (ul[0] + ur[0]);
-    const double p_int = 0.5 * (p_l + p_r) - 0.5 * a * rho * (v_r - v_l) / nrm;
-    const double v_int = 0.5 * (v_l + v_r) - 1.0 / (2.0 * a * rho) * (p_r - p_l) * nrm;
+    const double p_l = PhysPT2D::pressure(P, ul[4]), p_r = PhysPT2D::pressure(P, ur[4]);
+    const double v_l = fma(ul[3], n[2], fma(ul[2], n[1], ul[1] * n[0])) * int_rcp(ul[0]);
+    const double v_r = fma(ur[3], n[2], fma(ur[2], n[1], ur[1] * n[0])) * int_rcp(ur[0]);
+    const double nsq = fma(n[2], n[2], fma(n[1], n[1], n[0] * n[0]));
+    const double inorm = int_rsqrt(nsq), nrm = nsq * inorm;
+    const double rs = ul[0] + ur[0];  // 2 rho
+    const double p_int = 0.5 * (p_l + p_r) - 0.25 * a * rs * (v_r - v_l) * inorm;
+    const double v_int = 0.5 * (v_l + v_r) - int_rcp(a * rs) * (p_r - p_l) * nrm;
     const double* us = v_int > 0.0 ? ul : ur;
     F[0] = us[0] * v_int;
     F[1] = us[1] * v_int + p_int * n[0];
@@ -137,8 +110,8 @@ struct PhysPT3D {
 
   // boundary_condition_slip_wall (:83-107) with the outward normal n
   TAG_DEV static void boundary_flux(const Params& Q, const double* ui, const double* n, double* F) {
-    const double nn = sqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
-    const double e0 = n[0] / nn, e1 = n[1] / nn, e2 = n[2] / nn;
+    const double inn = int_rsqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
+    const double e0 = n[0] * inn, e1 = n[1] * inn, e2 = n[2] * inn;
     const double un = e0 * ui[1] + e1 * ui[2] + e2 * ui[3];
     const double ub[6] = {ui[0], ui[1] - 2.0 * un * e0, ui[2] - 2.0 * un * e1,
                           ui[3] - 2.0 * un * e2, ui[4], ui[5]};
@@ -155,10 +128,9 @@ struct PhysPT3D {
   // max_abs_speeds (:695-700)
   TAG_DEV static void max_speeds(const Params& Q, const double* u, double* l) {
     const PhysPT2D::Params& P = Q.pt;
-    const double irho = 1.0 / u[0];
+    const double irho = int_rcp(u[0]);
     const double v1 = u[1] * irho, v2 = u[2] * irho, v3 = u[3] * irho;
-    const double p = P.K * pow(u[4], P.gamma);
-    const double c = sqrt(P.gamma * p / u[0]);
+    const double c = int_sqrt(P.gamma * PhysPT2D::pressure(P, u[4]) * irho);
     l[0] = fabs(v1) + c;
     l[1] = fabs(v2) + c;
     l[2] = fabs(v3) + c;

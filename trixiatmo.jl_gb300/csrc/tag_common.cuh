@@ -245,7 +245,11 @@ TAG_DEV void ln_mean_pair_halved(double hxa, double hxb, double hya, double hyb,
 // logarithm: |d| >= 1, so its 2^-52 is a relative error of the same size.
 TAG_DEV double log_of_difference(i64 d) { return (double)d * 1.539095918623324e-16; }  // ln2 2^-52
 
+// (Values of opposite sign, which a moisture density may have, give NaN: the
+// logarithm of their ratio.)
+TAG_DEV bool opposite_signs(double a, double b) { return (i64)(f64_bits(a) ^ f64_bits(b)) < 0; }
 static __device__ __noinline__ double ln_factor_far(double xa, double xb, i64 d) {
+  if (opposite_signs(xa, xb)) return f64_from(0x7ff8000000000000ull);
   return int_div(2.0 * (xb - xa), log_of_difference(d) * (xa + xb));
 }
 static __device__ __noinline__ double inv_ln_factor_far(double ya, double yb, i64 d) {
@@ -260,8 +264,24 @@ TAG_DEV double inv_ln_factor(double ya, double yb, i64 d) {
   return series_in_range(a) ? inv_ln_mean_factor(log_square(a)) : inv_ln_factor_far(ya, yb, d);
 }
 
+// The means of two values themselves (interface kernels): ln_mean(x, y), and
+// inv_ln_mean(1/x, 1/y) from the reciprocals' own values.
+TAG_DEV double ln_mean_of(double x, double y) {
+  return 0.5 * (x + y) * ln_factor(x, y, log2_fixed(y) - log2_fixed(x));
+}
+TAG_DEV double inv_ln_mean_of_reciprocals(double x, double y) {
+  return 0.5 * (x + y) * inv_ln_factor(x, y, log2_fixed(y) - log2_fixed(x));
+}
+
 // Node logarithms are kept among the other node quantities as raw words.
 TAG_DEV double log_word(double x) { return f64_from((u64)log2_fixed(x)); }
+// The same of |x|, with an offset that separates the signs: pairs of one sign
+// see the difference of the logarithms, pairs of two signs leave the series.
+TAG_DEV double log_word_signed(double x) {
+  const u64 b = f64_bits(x);
+  return f64_from((u64)log2_fixed(f64_from(b & 0x7fffffffffffffffull)) + ((b >> 63) << 62));
+}
+TAG_DEV bool is_zero(double x) { return (f64_bits(x) << 1) == 0; }
 TAG_DEV i64 log_difference(double wa, double wb) { return (i64)(f64_bits(wb) - f64_bits(wa)); }
 
 // One logarithmic mean (or its inverse) with its own reciprocal: the series of

@@ -59,11 +59,10 @@ __global__ void k_eval_means(int kind, long n, const double* __restrict__ x,
     m = int_rcp(a);
     im = int_rsqrt(b);
   } else if (kind == 8) {
-    m = int_pow(a, pt.gamma, (u64)(pt.gamma * 2305843009213693952.0));
+    m = int_pow(a, pt.gamma, pt.gamma_q61);
     im = int_exp(b);
   } else {
-    const double ag = pow(a, pt.gamma), bg = pow(b, pt.gamma);
-    m = PhysPT2D::stolarsky(pt, a, b, ag, ag / a, bg, bg / b);
+    m = PhysPT2D::stolarsky(pt, a, b);
   }
   out1[q] = m;
   out2[q] = im;
