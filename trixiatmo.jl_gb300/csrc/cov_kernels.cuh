@@ -29,25 +29,6 @@ enum CovPack : int {
   kPC111, kPC112, kPC122, kPC211, kPC212, kPC222, kPF, kPInvJ, kPack = 16
 };
 
-struct CovGroup {
-  int n;         // nodes per direction
-  int e0, ne;    // elements [e0, e0 + ne)
-  long node0;    // first node of element e0
-  long sf0;      // first double of element e0 in the surface-flux array
-  int if0, nif;  // interfaces [if0, if0 + nif)
-  int epb;       // elements per CTA
-  int blk0;      // first CTA of the group in the element launch
-  int iblk0;     // first CTA of the group in the interface launch
-  int basis;     // offset of the group's BasisDev in the basis array
-};
-
-constexpr int kCovMaxGroups = 64;
-
-struct CovGroups {
-  int count;
-  CovGroup g[kCovMaxGroups];
-};
-
 TAG_DEV int cov_find_group(const CovGroups& G, int blk, bool iface) {
   int lo = 0;
   for (int k = 1; k < G.count; ++k)

@@ -12,17 +12,8 @@
 
 #include <nvtx3/nvToolsExt.h>
 
-#include "dg2d_kernels.cuh"
 #include "cov_kernels.cuh"
-#include "dg3d_kernels.cuh"
-#include "newton_rainy.cuh"
-#include "phys_euler_energy_2d.cuh"
-#include "phys_euler_energy_3d.cuh"
-#include "phys_moist_2d.cuh"
-#include "phys_pt_2d.cuh"
-#include "phys_pt_3d.cuh"
-#include "phys_ie_2d.cuh"
-#include "phys_rainy_2d.cuh"
+#include "handle.cuh"
 #include "tag_analysis.cuh"
 #include "output_kernels.cuh"
 
@@ -47,331 +38,11 @@ namespace {
 
 thread_local std::string g_last_error;
 
-int fail(int code, const std::string& msg) {
-  g_last_error = msg;
-  return code;
-}
-
-#define TAG_CUDA(call)                                                                    \
-  do {                                                                                    \
-    cudaError_t err_ = (call);                                                            \
-    if (err_ != cudaSuccess)                                                              \
-      return fail(TAG_E_CUDA, std::string(#call) + ": " + cudaGetErrorString(err_));      \
-  } while (0)
-
-struct Ops;
-
 }  // namespace
 
 void tag::set_last_error(const std::string& msg) { g_last_error = msg; }
 
-// Threads of an element-kernel CTA: `items` work items split `div` ways,
-// rounded up to whole warps.
-inline int cta_threads(int items, int div) { return ((items + div - 1) / div + 31) / 32 * 32; }
-
-struct tag_handle_s {
-  int eq = 0, n = 0, nelem = 0, nif = 0, nbd = 0, nv = 0, na = 0;
-  int dim = 2, npe = 0, nface = 4, jpn = 4;  // nodes per element, faces, Ja doubles per node
-  long nodes = 0;                            // solution nodes (all elements)
-  int dt_n = 0;                              // n in dt = cfl 2 / (n max_speed); 1 when
-                                             // the kernels reduce n-scaled speeds
-  // covariant equations: element groups, geometry, packed element data
-  CovParams p_cov{};
-
-  CovGroups h_groups{};
-  CovGroups* d_groups = nullptr;
-  BasisDev* d_bases = nullptr;
-  double *d_aux = nullptr, *d_pk = nullptr;
-  int cov_blocks = 0, cov_iblocks = 0, cov_threads = 0;
-  size_t cov_smem = 0;
-  PhysEnergy2D::Params p_energy{};
-  PhysEnergy3D::Params p_energy3d{};
-  PhysRainy2D::Params p_rainy{};
-  PhysMoist2D::Params p_moist{};
-  PhysPT2D::Params p_pt{};
-  PhysPT3D::Params p_pt3d{};
-  PhysIE2D::Params p_ie{};
-  // rainy: Newton stage limiter settings, MLP parameters, statistics counters
-  bool has_limiter = false;
-  int scheme = TAG_RK_CK2N54;  // time integrator of tag_rk_steps
-  NewtonArgs newton{0, 20, 0, 0, 8, 1e-9, nullptr, nullptr, nullptr};
-  float* d_mlp = nullptr;
-  unsigned long long* d_counters = nullptr;
-  int* d_iters = nullptr;
-  // the stage limiter inside tag_rk_steps: its start (NewtonArgs::learned)
-  // and counters accumulated over the run ([0] updates, [1] fallbacks,
-  // [2] not converged), with the number of node solves they cover
-  int newton_start = 0;
-  unsigned long long* d_run_counters = nullptr;
-  long long run_node_solves = 0;
-  BasisDev basis{};
-  cudaStream_t stream = nullptr;
-  double *d_u = nullptr, *d_k = nullptr, *d_Ja = nullptr, *d_invJ = nullptr, *d_xy = nullptr,
-         *d_sfv = nullptr, *d_tmp_u = nullptr, *d_tmp_du = nullptr;
-  // adaptive SSPRK43: the stage value entering the last stage, error partials
-  double *d_u3 = nullptr, *d_err = nullptr;
-  int *d_if_e = nullptr, *d_if_f = nullptr, *d_if_flip = nullptr, *d_bd_e = nullptr,
-      *d_bd_f = nullptr, *d_bd_kind = nullptr;
-  // states of the TAG_BC_DIRICHLET faces [B][n][nv] (allocated when the mesh has
-  // such faces; the interface kernel reads them)
-  double* d_bvals = nullptr;
-  bool need_bvals = false, bvals_set = false;
-  int nmembers = 1;
-  int* d_member = nullptr;        // [E] or null
-  double* d_mscal = nullptr;      // [3 * nmembers]: t, dt, max_speed
-  StepCtl* d_ctl = nullptr;
-  double* h_pin = nullptr;        // pinned staging, 3 * nmembers + 2 doubles
-  unsigned* d_status = nullptr;
-  cudaGraphExec_t graph = nullptr;
-  int graph_epb = -1;
-  // 3D: mapped host array that the last stage of every tag_rk_steps step also
-  // stores the new state into (tag_set_state_sink); armed only while the step
-  // graph is captured, so that no other stage sequence writes it
-  double* sink = nullptr;
-  double* graph_sink = nullptr;
-  bool capturing_steps = false;
-  bool speed_valid = false;
-  int epb = 0;
-  // threads of a CTA = its elements' work items / tile_div, rounded up to
-  // whole warps (1 or 2: one or two items per thread and phase)
-  int tile_div = 1;
-  const Ops* ops = nullptr;
-  // analysis (allocated by the first analysis call)
-  bool an_ready = false;
-  int an_m = 0, an_chunks = 0;
-  long an_chunk = 0;
-  double *d_an_wj = nullptr, *d_an_V = nullptr, *d_an_wa = nullptr, *d_an_rows = nullptr,
-         *d_an_erows = nullptr, *d_an_out = nullptr, *d_an_uex = nullptr, *d_an_x = nullptr;
-  long* d_an_rng = nullptr;  // [4][nmembers]: node begin, node end, element begin, element end
-  size_t an_uex_cap = 0;
-};
-
 namespace {
-
-// Launchers for one (physics, n) instantiation.
-struct Ops {
-  int (*interface)(tag_handle h, const double* u);
-  int (*element)(tag_handle h, int mode, double* u, double* du, int stage, bool last, double t);
-  int (*max_speed)(tag_handle h, const double* u);
-  // optional: u from mapped host memory into d_u with the CFL speeds reduced
-  int (*load_state)(tag_handle h, const double* u_mapped);
-  int (*init)(int max_smem);
-  size_t (*smem_bytes)(int epb);
-  int threads_per_element;
-  int (*max_threads)();  // per-CTA thread limit of the element kernels (registers)
-};
-
-// Largest multiple of 32 threads both element kernels (stage and rhs mode) of
-// one instantiation can be launched with.
-template <class K1, class K2>
-int launch_thread_cap(K1 k1, K2 k2, int& cap) {
-  cudaFuncAttributes a, b;
-  TAG_CUDA(cudaFuncGetAttributes(&a, k1));
-  TAG_CUDA(cudaFuncGetAttributes(&b, k2));
-  cap = (std::min(a.maxThreadsPerBlock, b.maxThreadsPerBlock) / 32) * 32;
-  return TAG_OK;
-}
-
-template <class Phys>
-const typename Phys::Params& params_of(tag_handle h);
-template <>
-const PhysEnergy2D::Params& params_of<PhysEnergy2D>(tag_handle h) {
-  return h->p_energy;
-}
-template <>
-const PhysEnergy3D::Params& params_of<PhysEnergy3D>(tag_handle h) {
-  return h->p_energy3d;
-}
-template <>
-const PhysRainy2D::Params& params_of<PhysRainy2D>(tag_handle h) {
-  return h->p_rainy;
-}
-template <>
-const PhysMoist2D::Params& params_of<PhysMoist2D>(tag_handle h) {
-  return h->p_moist;
-}
-template <>
-const PhysPT2D::Params& params_of<PhysPT2D>(tag_handle h) {
-  return h->p_pt;
-}
-template <>
-const PhysPT3D::Params& params_of<PhysPT3D>(tag_handle h) {
-  return h->p_pt3d;
-}
-template <>
-const PhysIE2D::Params& params_of<PhysIE2D>(tag_handle h) {
-  return h->p_ie;
-}
-
-template <class Phys, int n, int VOL = kVolFluxDiff>
-struct OpsImpl {
-  using S = ElemSmem<Phys, n>;
-  static int interface(tag_handle h, const double* u) {
-    const int total = (h->nif + h->nbd) * n;
-    if (total == 0) return TAG_OK;
-    const int threads = 256;
-    if (h->need_bvals && !h->bvals_set)
-      return fail(TAG_E_INVALID, "Dirichlet boundary faces without states (tag_set_boundary_values)");
-    k_interface<Phys, n><<<(total + threads - 1) / threads, threads, 0, h->stream>>>(
-        params_of<Phys>(h), u, h->d_Ja, h->d_invJ, h->d_if_e, h->d_if_f, h->d_if_flip, h->nif,
-        h->d_bd_e, h->d_bd_f, h->d_bd_kind, h->nbd, h->d_sfv, h->d_bvals);
-    TAG_CUDA(cudaGetLastError());
-    return TAG_OK;
-  }
-  static int element(tag_handle h, int mode, double* u, double* du, int stage, bool last,
-                     double t) {
-    const int epb = h->epb > 0 ? h->epb : 4;
-    const int blocks = (h->nelem + epb - 1) / epb;
-    const int threads = std::min(cap(), cta_threads(epb * S::TPE, h->tile_div));
-    const size_t smem = S::bytes(epb);
-    StageArgs st{};
-    st.member = h->d_member;
-    st.xy = h->d_xy;
-    st.t_rhs = t;
-    if (mode == kModeStage) {
-      set_stage(st, h->scheme, stage);
-      st.t_member = h->d_mscal;
-      st.dt = h->d_mscal + h->nmembers;
-      st.max_speed = last ? h->d_mscal + 2 * h->nmembers : nullptr;
-      st.sink = last && h->capturing_steps ? h->sink : nullptr;
-      k_element<Phys, n, kModeStage, VOL><<<blocks, threads, smem, h->stream>>>(
-          params_of<Phys>(h), h->basis, u, du, h->d_k, h->d_Ja, h->d_invJ, h->d_sfv, h->nelem,
-          epb, st, h->d_status);
-    } else {
-      k_element<Phys, n, kModeRhs, VOL><<<blocks, threads, smem, h->stream>>>(
-          params_of<Phys>(h), h->basis, u, du, h->d_k, h->d_Ja, h->d_invJ, h->d_sfv, h->nelem,
-          epb, st, h->d_status);
-    }
-    TAG_CUDA(cudaGetLastError());
-    return TAG_OK;
-  }
-  static int max_speed(tag_handle h, const double* u) {
-    using K = MaxSpeedTile<n>;
-    k_max_speed<Phys, n><<<(h->nelem + K::EPB - 1) / K::EPB, K::T, 0, h->stream>>>(
-        params_of<Phys>(h), u, h->d_Ja, h->d_invJ, h->nelem, h->d_member,
-        h->d_mscal + 2 * h->nmembers);
-    TAG_CUDA(cudaGetLastError());
-    return TAG_OK;
-  }
-  // opt the element kernels into the device's full dynamic shared memory once,
-  // outside any stream capture
-  static int init(int max_smem) {
-    TAG_CUDA(cudaFuncSetAttribute(k_element<Phys, n, kModeStage, VOL>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
-    TAG_CUDA(cudaFuncSetAttribute(k_element<Phys, n, kModeRhs, VOL>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
-    return launch_thread_cap(k_element<Phys, n, kModeStage, VOL>, k_element<Phys, n, kModeRhs, VOL>,
-                             cap());
-  }
-  static int& cap() {
-    static int c = 1024;
-    return c;
-  }
-  static int max_threads() { return cap(); }
-  static size_t smem_bytes(int epb) { return S::bytes(epb); }
-  static const Ops* get() {
-    static const Ops ops{&interface, &element, &max_speed, nullptr, &init, &smem_bytes,
-                         S::TPE, &max_threads};
-    return &ops;
-  }
-};
-
-template <class Phys, int VOL = kVolFluxDiff>
-const Ops* ops_for_n(int n) {
-  switch (n) {
-    case 2: return OpsImpl<Phys, 2, VOL>::get();
-    case 3: return OpsImpl<Phys, 3, VOL>::get();
-    case 4: return OpsImpl<Phys, 4, VOL>::get();
-    case 5: return OpsImpl<Phys, 5, VOL>::get();
-    case 6: return OpsImpl<Phys, 6, VOL>::get();
-    case 7: return OpsImpl<Phys, 7, VOL>::get();
-    case 8: return OpsImpl<Phys, 8, VOL>::get();
-    default: return nullptr;
-  }
-}
-
-template <class Phys, int n>
-struct OpsImpl3D {
-  using S = ElemSmem3D<Phys, n>;
-  static int interface(tag_handle h, const double* u) {
-    const int total = (h->nif + h->nbd) * n * n;
-    if (total == 0) return TAG_OK;
-    k_interface3d<Phys, n><<<(total + 255) / 256, 256, 0, h->stream>>>(
-        params_of<Phys>(h), u, h->d_Ja, h->d_invJ, h->d_if_e, h->d_if_f, h->d_if_flip, h->nif,
-        h->d_bd_e, h->d_bd_f, h->nbd, h->d_sfv);
-    TAG_CUDA(cudaGetLastError());
-    return TAG_OK;
-  }
-  static int element(tag_handle h, int mode, double* u, double* du, int stage, bool last,
-                     double) {
-    const int epb = h->epb > 0 ? h->epb : 1;
-    const int blocks = (h->nelem + epb - 1) / epb;
-    const int threads = std::min(cap(), cta_threads(epb * S::TPE, h->tile_div));
-    const size_t smem = S::bytes(epb);
-    StageArgs st{};
-    st.member = h->d_member;
-    if (mode == kModeStage) {
-      set_stage(st, h->scheme, stage);
-      st.dt = h->d_mscal + h->nmembers;
-      st.max_speed = last ? h->d_mscal + 2 * h->nmembers : nullptr;
-      st.sink = last && h->capturing_steps ? h->sink : nullptr;
-      k_element3d<Phys, n, kModeStage><<<blocks, threads, smem, h->stream>>>(
-          params_of<Phys>(h), h->basis, u, du, h->d_k, h->d_Ja, h->d_invJ, h->d_sfv, h->nelem,
-          epb, st, h->d_status);
-    } else {
-      k_element3d<Phys, n, kModeRhs><<<blocks, threads, smem, h->stream>>>(
-          params_of<Phys>(h), h->basis, u, du, h->d_k, h->d_Ja, h->d_invJ, h->d_sfv, h->nelem,
-          epb, st, h->d_status);
-    }
-    TAG_CUDA(cudaGetLastError());
-    return TAG_OK;
-  }
-  static int max_speed(tag_handle h, const double* u) { return speeds(h, u, nullptr); }
-  // the state from mapped host memory into the device copy, speeds on the way
-  static int load_state(tag_handle h, const double* u_mapped) {
-    return speeds(h, u_mapped, h->d_u);
-  }
-  static int speeds(tag_handle h, const double* u, double* copy_to) {
-    const int threads = 256, warps = threads / 32;  // one warp per element
-    k_max_speed3d<Phys, n><<<(h->nelem + warps - 1) / warps, threads, 0, h->stream>>>(
-        params_of<Phys>(h), u, h->d_Ja, h->d_invJ, h->nelem, h->d_member,
-        h->d_mscal + 2 * h->nmembers, copy_to);
-    TAG_CUDA(cudaGetLastError());
-    return TAG_OK;
-  }
-  static int init(int max_smem) {
-    TAG_CUDA(cudaFuncSetAttribute(k_element3d<Phys, n, kModeStage>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
-    TAG_CUDA(cudaFuncSetAttribute(k_element3d<Phys, n, kModeRhs>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
-    return launch_thread_cap(k_element3d<Phys, n, kModeStage>, k_element3d<Phys, n, kModeRhs>,
-                             cap());
-  }
-  static int& cap() {
-    static int c = 1024;
-    return c;
-  }
-  static int max_threads() { return cap(); }
-  static size_t smem_bytes(int epb) { return S::bytes(epb); }
-  static const Ops* get() {
-    static const Ops ops{&interface, &element, &max_speed, &load_state, &init, &smem_bytes,
-                         S::TPE, &max_threads};
-    return &ops;
-  }
-};
-
-template <class Phys>
-const Ops* ops3d_for_n(int n) {
-  switch (n) {
-    case 3: return OpsImpl3D<Phys, 3>::get();
-    case 4: return OpsImpl3D<Phys, 4>::get();
-    case 5: return OpsImpl3D<Phys, 5>::get();
-    case 6: return OpsImpl3D<Phys, 6>::get();
-    case 7: return OpsImpl3D<Phys, 7>::get();
-    case 8: return OpsImpl3D<Phys, 8>::get();
-    default: return nullptr;
-  }
-}
 
 template <class T>
 int upload(T** dst, const T* src, size_t count, cudaStream_t s) {
@@ -1081,8 +752,7 @@ int tag_create(const tag_config* cfg, tag_handle* out) {
     h->nv = PhysRainy2D::NV;
     h->na = PhysRainy2D::NA;
     h->p_rainy = PhysRainy2D::make_params(cfg->params, cfg->surface_flux);
-    h->ops = cfg->volume_flux == TAG_VF_WEAK_FORM ? ops_for_n<PhysRainy2D, kVolWeak>(n)
-                                                  : ops_for_n<PhysRainy2D, kVolFluxDiff>(n);
+    h->ops = ops_rainy2d(n, cfg->volume_flux == TAG_VF_WEAK_FORM);
     h->has_limiter = true;
   } else if (cfg->equations == TAG_EQ_POTENTIAL_TEMPERATURE_2D) {
     h->nv = PhysPT2D::NV;
@@ -1093,19 +763,18 @@ int tag_create(const tag_config* cfg, tag_handle* out) {
     pp[6] = cfg->surface_flux == TAG_SF_PT_EC ? 1 : 0;
     if (cfg->surface_flux != TAG_SF_PT_EC) pp[7] = 0;  // flux_zero
     h->p_pt = PhysPT2D::make_params(pp);
-    h->ops = ops_for_n<PhysPT2D, kVolFluxDiff>(n);
+    h->ops = ops_pt2d(n);
   } else if (moist) {
     h->nv = PhysMoist2D::NV;
     h->na = PhysMoist2D::NA;
     h->p_moist = PhysMoist2D::make_params(cfg->params);
     h->p_moist.surface = cfg->surface_flux;
-    h->ops = cfg->volume_flux == TAG_VF_WEAK_FORM ? ops_for_n<PhysMoist2D, kVolWeak>(n)
-                                                  : ops_for_n<PhysMoist2D, kVolFluxDiff>(n);
+    h->ops = ops_moist2d(n, cfg->volume_flux == TAG_VF_WEAK_FORM);
   } else if (cfg->equations == TAG_EQ_INTERNAL_ENERGY_2D) {
     h->nv = PhysIE2D::NV;
     h->na = PhysIE2D::NA;
     h->p_ie = PhysIE2D::make_params(cfg->params);
-    h->ops = ops_for_n<PhysIE2D, kVolFluxDiff>(n);
+    h->ops = ops_ie2d(n);
   } else if (cfg->equations == TAG_EQ_POTENTIAL_TEMPERATURE_3D) {
     h->nv = PhysPT3D::NV;
     h->na = PhysPT3D::NA;
@@ -1116,17 +785,17 @@ int tag_create(const tag_config* cfg, tag_handle* out) {
             : cfg->volume_flux == TAG_VF_PT_KG ? 3
                                                : 2;
     h->p_pt3d = PhysPT3D::make_params(pp);
-    h->ops = ops3d_for_n<PhysPT3D>(n);
+    h->ops = ops_pt3d(n);
   } else if (dim == 3) {
     h->nv = PhysEnergy3D::NV;
     h->na = PhysEnergy3D::NA;
     h->p_energy3d = PhysEnergy3D::make_params(cfg->params);
-    h->ops = ops3d_for_n<PhysEnergy3D>(n);
+    h->ops = ops_energy3d(n);
   } else {
     h->nv = PhysEnergy2D::NV;
     h->na = PhysEnergy2D::NA;
     h->p_energy = PhysEnergy2D::make_params(cfg->params);
-    h->ops = ops_for_n<PhysEnergy2D>(n);
+    h->ops = ops_energy2d(n);
   }
   load_basis(h->basis, cfg->derivative_split, cfg->weights, n);
   auto cleanup = [&](int rc) {
