@@ -14,7 +14,8 @@ namespace tag {
 struct PhysIE2D {
   static constexpr int NV = 5;
   static constexpr int NA = 4;
-  // rho, v1/2, v2/2, p/2, phi/2, beta = rho/p, (unused logs), pad (odd stride)
+  // rho/2, v1/2, v2/2, p/2, phi/2, theta = (p/rho) / (2 (gamma - 1)),
+  // log2(rho), log2(p/rho) (log2_fixed words), pad (odd stride)
   static constexpr int NQ = 9;
   static constexpr bool kLastHalved = false;
   static constexpr bool kHasSources = false;
@@ -35,53 +36,45 @@ struct PhysIE2D {
 
   TAG_DEV static void node_prims(const Params& P, const double* u, double* q, unsigned& bad) {
     const double rho = u[0];
-    const double irho = 1.0 / rho;
+    const double irho = int_rcp(rho), hir = 0.5 * irho;
     const double p = P.gm1 * u[3];
-    q[0] = rho;
-    q[1] = 0.5 * u[1] * irho;
-    q[2] = 0.5 * u[2] * irho;
+    const double pr = p * irho;
+    q[0] = 0.5 * rho;
+    q[1] = u[1] * hir;
+    q[2] = u[2] * hir;
     q[3] = 0.5 * p;
     q[4] = 0.5 * u[4];
-    q[5] = rho / p;
-    q[6] = q[7] = q[8] = 0.0;
-    if (!(rho > 0.0)) bad |= TAG_S_NEG_DENSITY;
-    if (!(p > 0.0)) bad |= TAG_S_NEG_PRESSURE;
+    q[5] = 0.5 * pr * P.inv_gm1;
+    q[6] = log_word(rho);
+    q[7] = log_word(pr);
+    if (not_positive(rho)) bad |= TAG_S_NEG_DENSITY;
+    if (not_positive(p)) bad |= TAG_S_NEG_PRESSURE;
   }
 
   // flux_conservative_etec + half of flux_nonconservative_etec (antisymmetric)
   // on the halved node quantities; p_ll p_rr inv_ln_mean(rho_ll p_rr, rho_rr p_ll)
-  // is evaluated as the equal inv_ln_mean(rho_ll/p_ll, rho_rr/p_rr).
+  // is evaluated as the equal inv_ln_mean(rho_ll/p_ll, rho_rr/p_rr), the mean
+  // of the reciprocals of p/rho.
   TAG_DEV static void volume_pair(const Params& P, const double* qa, const double* qb, double n1,
                                   double n2, double* Fa, double* Fb) {
-    double rho_mean, inv_rho_p_mean;
-    ln_mean_pair<false>(qa[0], qb[0], qa[5], qb[5], 0.0, 0.0, 0.0, 0.0, rho_mean, inv_rho_p_mean);
+    const double rho_mean = (qa[0] + qb[0]) * ln_factor(qa[0], qb[0], log_difference(qa[6], qb[6]));
+    const double e_mean = (qa[5] + qb[5]) * inv_ln_factor(qa[5], qb[5], log_difference(qa[7], qb[7]));
     const double v1 = qa[1] + qb[1], v2 = qa[2] + qb[2];  // averages
     const double vn = n1 * v1 + n2 * v2;                    // 0.5 (vn_a + vn_b)
     const double p_avg = qa[3] + qb[3];
     const double f1 = rho_mean * vn;
-    const double f2 = f1 * v1 + p_avg * n1;
-    const double f3 = f1 * v2 + p_avg * n2;
-    const double f4 = f1 * inv_rho_p_mean * P.inv_gm1 + p_avg * vn;
-    const double gr = rho_mean * (qb[4] - qa[4]);   // rho_mean (phi_b - phi_a) / 2
-    const double gp = -vn * (qb[3] - qa[3]);         // -vn_avg (p_b - p_a) / 2
+    const double g = qb[4] - qa[4];                  // (phi_b - phi_a) / 2
+    const double pp = fma(rho_mean, g, p_avg), pm = fma(-rho_mean, g, p_avg);
+    const double t1 = f1 * v1, t2 = f1 * v2;
+    const double f4 = fma(f1, e_mean, p_avg * vn);
+    const double dp = qb[3] - qa[3];                 // gp = -vn_avg (p_b - p_a) / 2
     Fa[0] = Fb[0] = f1;
-    Fa[1] = f2 + gr * n1;
-    Fb[1] = f2 - gr * n1;
-    Fa[2] = f3 + gr * n2;
-    Fb[2] = f3 - gr * n2;
-    Fa[3] = f4 + gp;
-    Fb[3] = f4 - gp;
-  }
-
-  // Trixi's flux (conservative part) for the weak form and consistency
-  TAG_DEV static void flux(const Params& P, const double* u, double n1, double n2, double* f) {
-    const double v1 = u[1] / u[0], v2 = u[2] / u[0];
-    const double p = P.gm1 * u[3];
-    const double vn = v1 * n1 + v2 * n2;
-    f[0] = u[0] * vn;
-    f[1] = u[1] * vn + p * n1;
-    f[2] = u[2] * vn + p * n2;
-    f[3] = (u[3] + p) * vn;
+    Fa[1] = fma(n1, pp, t1);
+    Fb[1] = fma(n1, pm, t1);
+    Fa[2] = fma(n2, pp, t2);
+    Fb[2] = fma(n2, pm, t2);
+    Fa[3] = fma(-vn, dp, f4);
+    Fb[3] = fma(vn, dp, f4);
   }
 
   // interface speed of sound and normal velocity of the es pair
@@ -91,13 +84,13 @@ struct PhysIE2D {
     const double rl = ul[0], rr = ur[0];
     pl = P.gm1 * ul[3];
     pr = P.gm1 * ur[3];
-    vnl = (ul[1] / rl) * n1 + (ul[2] / rl) * n2;
-    vnr = (ur[1] / rr) * n1 + (ur[2] / rr) * n2;
-    const double cl = sqrt(P.gamma * pl / rl), cr = sqrt(P.gamma * pr / rr);
+    const double irl = int_rcp(rl), irr = int_rcp(rr);
+    vnl = fma(ul[2], n2, ul[1] * n1) * irl;
+    vnr = fma(ur[2], n2, ur[1] * n1) * irr;
+    const double cl = int_sqrt(P.gamma * pl * irl), cr = int_sqrt(P.gamma * pr * irr);
     a = 0.5 * (cl + cr);
-    nrm = sqrt(n1 * n1 + n2 * n2);
-    const double rho_avg = 0.5 * (rl + rr);
-    return 0.5 * (vnl + vnr) - 1.0 / (2.0 * a * rho_avg) * (pr - pl) * nrm;
+    nrm = int_sqrt(n1 * n1 + n2 * n2);
+    return 0.5 * (vnl + vnr) - int_rcp(a * (rl + rr)) * (pr - pl) * nrm;
   }
 
   // flux_conservative_es
@@ -106,9 +99,9 @@ struct PhysIE2D {
     double vnl, vnr, pl, pr, a, nrm;
     const double v_int = v_interface(P, ul, ur, n1, n2, vnl, vnr, pl, pr, a, nrm);
     const double rl = ul[0], rr = ur[0];
-    const double rho_mean = ln_mean_single(rl, rr);
+    const double rho_mean = ln_mean_of(rl, rr);
     const double rho_avg = 0.5 * (rl + rr);
-    const double p_int = 0.5 * (pl + pr) - 0.5 * a * rho_avg * (vnr - vnl) / nrm;
+    const double p_int = 0.5 * (pl + pr) - 0.5 * a * rho_avg * (vnr - vnl) * int_rcp(nrm);
     const double p_avg = 0.5 * (pl + pr);
     double rho_up, f2, f3;
     if (v_int >= 0.0) {
@@ -120,7 +113,8 @@ struct PhysIE2D {
       f2 = ur[1] * v_int;
       f3 = ur[2] * v_int;
     }
-    const double inv_rho_p_mean = inv_ln_mean_single(rl / pl, rr / pr);
+    const double inv_rho_p_mean =
+        inv_ln_mean_of_reciprocals(pl * int_rcp(rl), pr * int_rcp(rr));
     const double f1 = rho_up * v_int;
     F[0] = f1;
     F[1] = f2 + p_int * n1;
@@ -141,8 +135,8 @@ struct PhysIE2D {
   // flux of the inner and the mirrored state
   TAG_DEV static void boundary_flux(const Params& P, const double* ui, double n1, double n2, int,
                                     int, double* F) {
-    const double nn = sqrt(n1 * n1 + n2 * n2);
-    const double nx = n1 / nn, ny = n2 / nn;
+    const double inn = int_rsqrt(n1 * n1 + n2 * n2);
+    const double nx = n1 * inn, ny = n2 * inn;
     const double un = nx * ui[1] + ny * ui[2];
     const double ub[5] = {ui[0], ui[1] - 2.0 * un * nx, ui[2] - 2.0 * un * ny, ui[3], ui[4]};
     double G[4];
@@ -153,10 +147,9 @@ struct PhysIE2D {
   }
 
   TAG_DEV static void max_speeds(const Params& P, const double* u, double& l1, double& l2) {
-    const double rho = u[0];
-    const double v1 = u[1] / rho, v2 = u[2] / rho;
-    const double p = P.gm1 * u[3];
-    const double c = sqrt(P.gamma * p / rho);
+    const double irho = int_rcp(u[0]);
+    const double v1 = u[1] * irho, v2 = u[2] * irho;
+    const double c = int_sqrt(P.gamma * (P.gm1 * u[3]) * irho);
     l1 = fabs(v1) + c;
     l2 = fabs(v2) + c;
   }

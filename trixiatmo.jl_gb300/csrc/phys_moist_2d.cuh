@@ -10,8 +10,9 @@ namespace tag {
 struct PhysMoist2D {
   static constexpr int NV = 6;
   static constexpr int NA = 6;
-  // rho_qd, rho_qv, rho_ql, v1/2, v2/2, 1/T, (v1^2 + v2^2)/4 (odd stride)
-  static constexpr int NQ = 7;
+  // rho_qd/2, rho_qv/2, rho_ql/2, v1/2, v2/2, T/2, 1/(2T), (v1^2 + v2^2)/4,
+  // log2 of rho_qd, rho_qv, rho_ql and T (words), (pad: odd stride)
+  static constexpr int NQ = 13;
   static constexpr bool kLastHalved = false;
   static constexpr bool kHasSources = true;
   static constexpr bool kSurfaceNoncons = false;  // surface flux only (flux_zero)
@@ -40,38 +41,55 @@ struct PhysMoist2D {
     return q;
   }
 
-  // get_current_condition, :383-402
-  TAG_DEV static void condition(const Params& P, const double* u, double& p, double& T) {
+  // get_current_condition, :383-402: T = num / den; divisions, here and below,
+  // on the integer pipe (int_math.cuh)
+  TAG_DEV static void temperature_ratio(const Params& P, const double* u, double ri, double& num,
+                                        double& den) {
     const double rho_qd = u[0] - u[4] - u[5];
-    const double v1 = u[1] / u[0], v2 = u[2] / u[0];
-    const double rho_e = u[3] - 0.5 * (u[1] * v1 + u[2] * v2);
-    T = (rho_e - P.L_00 * u[4]) / (rho_qd * P.c_vd + u[4] * P.c_vv + u[5] * P.c_pl);
-    p = (rho_qd * P.R_d + u[4] * P.R_v) * T;
+    const double rho_e = fma(-0.5 * ri, fma(u[2], u[2], u[1] * u[1]), u[3]);
+    num = fma(-P.L_00, u[4], rho_e);
+    den = fma(u[5], P.c_pl, fma(u[4], P.c_vv, rho_qd * P.c_vd));
+  }
+  TAG_DEV static double pressure_at(const Params& P, const double* u, double T) {
+    return fma(u[4], P.R_v, (u[0] - u[4] - u[5]) * P.R_d) * T;
+  }
+  TAG_DEV static void condition(const Params& P, const double* u, double ri, double& p, double& T) {
+    double num, den;
+    temperature_ratio(P, u, ri, num, den);
+    T = int_div(num, den);
+    p = pressure_at(P, u, T);
   }
 
-  // mixture ratio of specific heats and sound speed (:921-930)
-  TAG_DEV static double sound(const Params& P, const double* u, double p) {
-    const double qv = u[4] / u[0], ql = u[5] / u[0];
-    const double qd = 1.0 - qv - ql;
-    const double gm = (qd * P.c_pd + qv * P.c_pv + ql * P.c_pl) *
-                      (1.0 / (qd * P.c_vd + qv * P.c_vv + ql * P.c_pl));
-    return sqrt(gm * p / u[0]);
+  // mixture ratio of specific heats (:921-930), of densities instead of ratios
+  TAG_DEV static double gamma_mixture(const Params& P, const double* u) {
+    const double rho_qd = u[0] - u[4] - u[5];
+    return int_div(fma(u[5], P.c_pl, fma(u[4], P.c_pv, rho_qd * P.c_pd)),
+                   fma(u[5], P.c_pl, fma(u[4], P.c_vv, rho_qd * P.c_vd)));
+  }
+  TAG_DEV static double sound(const Params& P, const double* u, double ri, double p) {
+    return int_sqrt(gamma_mixture(P, u) * p * ri);
   }
 
   TAG_DEV static void node_prims(const Params& P, const double* u, double* q, unsigned& bad) {
-    double p, T;
-    condition(P, u, p, T);
-    const double ri = 1.0 / u[0];
+    const double ri = int_rcp(u[0]);
+    double num, den;
+    temperature_ratio(P, u, ri, num, den);
+    const double T = int_div(num, den);
     const double v1 = u[1] * ri, v2 = u[2] * ri;
-    q[0] = u[0] - u[4] - u[5];
-    q[1] = u[4];
-    q[2] = u[5];
+    q[0] = 0.5 * (u[0] - u[4] - u[5]);
+    q[1] = 0.5 * u[4];
+    q[2] = 0.5 * u[5];
     q[3] = 0.5 * v1;
     q[4] = 0.5 * v2;
-    q[5] = 1.0 / T;
-    q[6] = 0.25 * (v1 * v1 + v2 * v2);
-    if (!(u[0] > 0.0)) bad |= TAG_S_NEG_DENSITY;
-    if (!(p > 0.0)) bad |= TAG_S_NEG_PRESSURE;
+    q[5] = 0.5 * T;
+    q[6] = 0.5 * int_div(den, num);
+    q[7] = 0.25 * fma(v2, v2, v1 * v1);
+    q[8] = log_word(q[0]);
+    q[9] = log_word_signed(q[1]);
+    q[10] = log_word_signed(q[2]);
+    q[11] = log_word(T);
+    if (not_positive(u[0])) bad |= TAG_S_NEG_DENSITY;
+    if (not_positive(pressure_at(P, u, T))) bad |= TAG_S_NEG_PRESSURE;
   }
 
   // flux_chandrashekar (:936-1003, R_q = 0) for one symmetric pair, on the
@@ -79,20 +97,27 @@ struct PhysMoist2D {
   TAG_DEV static void volume_pair(const Params& P, const double* a, const double* b, double n1,
                                   double n2, double* Fa, double* Fb) {
     const double v1a = a[3] + b[3], v2a = a[4] + b[4];
-    const double K = a[6] + b[6];
+    const double K = a[7] + b[7];
     const double vdn = n1 * v1a + n2 * v2a;
-    double rqd_mean, iT_mean;
-    ln_mean_pair<false>(a[0], b[0], a[5], b[5], 0.0, 0.0, 0.0, 0.0, rqd_mean, iT_mean);
-    const double rqv_mean = (a[1] != 0.0 && b[1] != 0.0) ? ln_mean_single(a[1], b[1]) : 0.0;
-    const double rql_mean = (a[2] != 0.0 && b[2] != 0.0) ? ln_mean_single(a[2], b[2]) : 0.0;
-    const double p_int = (P.R_d * (0.5 * (a[0] + b[0])) + P.R_v * (0.5 * (a[1] + b[1]))) /
-                         (0.5 * (a[5] + b[5]));
+    const double rqd_mean = (a[0] + b[0]) * ln_factor(a[0], b[0], log_difference(a[8], b[8]));
+    // inv_ln_mean of 1/T
+    const double T_mean = (a[5] + b[5]) * inv_ln_factor(a[5], b[5], log_difference(a[11], b[11]));
+    const double rqv_avg = a[1] + b[1], rql_avg = a[2] + b[2];
+    const double rqv_mean = !is_zero(a[1]) && !is_zero(b[1])
+                                ? rqv_avg * ln_factor(a[1], b[1], log_difference(a[9], b[9]))
+                                : 0.0;
+    const double rql_mean = !is_zero(a[2]) && !is_zero(b[2])
+                                ? rql_avg * ln_factor(a[2], b[2], log_difference(a[10], b[10]))
+                                : 0.0;
+    const double p_int = fma(P.R_v, rqv_avg, P.R_d * (a[0] + b[0])) * int_rcp(a[6] + b[6]);
     const double f_d = rqd_mean * vdn, f_v = rqv_mean * vdn, f_l = rql_mean * vdn;
     const double f1 = f_d + f_v + f_l;
     const double f2 = f1 * v1a + n1 * p_int;
     const double f3 = f1 * v2a + n2 * p_int;
-    const double f4 = (P.c_vd * iT_mean - K) * f_d + (P.L_00 + P.c_vv * iT_mean - K) * f_v +
-                      (P.c_pl * iT_mean - K) * f_l + v1a * f2 + v2a * f3;
+    // (c_vd T - K) f_d + (L_00 + c_vv T - K) f_v + (c_pl T - K) f_l + v.(f2, f3)
+    const double cf = fma(P.c_pl, f_l, fma(P.c_vv, f_v, P.c_vd * f_d));
+    const double f4 =
+        fma(v2a, f3, fma(v1a, f2, fma(-K, f1, fma(P.L_00, f_v, T_mean * cf))));
     Fa[0] = Fb[0] = f1;
     Fa[1] = Fb[1] = f2;
     Fa[2] = Fb[2] = f3;
@@ -103,33 +128,37 @@ struct PhysMoist2D {
 
   // flux(u, normal_direction), :63-82
   TAG_DEV static void flux(const Params& P, const double* u, double n1, double n2, double* f) {
-    double p, T;
-    condition(P, u, p, T);
-    const double v1 = u[1] / u[0], v2 = u[2] / u[0];
-    const double qv = u[4] / u[0], ql = u[5] / u[0];
-    const double vn = v1 * n1 + v2 * n2;
-    const double rvn = u[0] * vn;
-    f[0] = rvn;
-    f[1] = rvn * v1 + p * n1;
-    f[2] = rvn * v2 + p * n2;
+    double vn, p;
+    flux_at(P, u, int_rcp(u[0]), n1, n2, f, vn, p);
+  }
+  // with the caller's 1/rho; returns the normal velocity and the pressure
+  TAG_DEV static void flux_at(const Params& P, const double* u, double ri, double n1, double n2,
+                              double* f, double& vn, double& p) {
+    double T;
+    condition(P, u, ri, p, T);
+    vn = fma(u[2], n2, u[1] * n1) * ri;
+    f[0] = u[0] * vn;
+    f[1] = fma(u[1], vn, p * n1);
+    f[2] = fma(u[2], vn, p * n2);
     f[3] = (u[3] + p) * vn;
-    f[4] = rvn * qv;
-    f[5] = rvn * ql;
+    f[4] = u[4] * vn;
+    f[5] = u[5] * vn;
   }
 
   // FluxLMARS, :446-485
   TAG_DEV static void lmars(const Params& P, const double* ul, const double* ur, double n1,
                             double n2, double* F) {
     const double a = P.c_lmars;
+    const double irl = int_rcp(ul[0]), irr = int_rcp(ur[0]);
     double p_l, T_l, p_r, T_r;
-    condition(P, ul, p_l, T_l);
-    condition(P, ur, p_r, T_r);
-    const double v_l = (ul[1] / ul[0]) * n1 + (ul[2] / ul[0]) * n2;
-    const double v_r = (ur[1] / ur[0]) * n1 + (ur[2] / ur[0]) * n2;
-    const double nrm = sqrt(n1 * n1 + n2 * n2);
-    const double rho = 0.5 * (ul[0] + ur[0]);
-    const double p_int = 0.5 * (p_l + p_r) - 0.5 * a * rho * (v_r - v_l) / nrm;
-    const double v_int = 0.5 * (v_l + v_r) - 1.0 / (2.0 * a * rho) * (p_r - p_l) * nrm;
+    condition(P, ul, irl, p_l, T_l);
+    condition(P, ur, irr, p_r, T_r);
+    const double v_l = fma(ul[2], n2, ul[1] * n1) * irl;
+    const double v_r = fma(ur[2], n2, ur[1] * n1) * irr;
+    const double nsq = fma(n2, n2, n1 * n1), inorm = int_rsqrt(nsq), nrm = nsq * inorm;
+    const double rs = ul[0] + ur[0];  // 2 rho
+    const double p_int = 0.5 * (p_l + p_r) - 0.25 * a * rs * (v_r - v_l) * inorm;
+    const double v_int = 0.5 * (v_l + v_r) - int_rcp(a * rs) * (p_r - p_l) * nrm;
     const double* us = v_int > 0.0 ? ul : ur;
     const double ps = v_int > 0.0 ? p_l : p_r;
 #pragma unroll
@@ -142,15 +171,13 @@ struct PhysMoist2D {
   // flux_lax_friedrichs with max_abs_speed_naive (:893-918)
   TAG_DEV static void llf(const Params& P, const double* ul, const double* ur, double n1,
                           double n2, double* F) {
-    double fl[6], fr[6], p_l, T_l, p_r, T_r;
-    flux(P, ul, n1, n2, fl);
-    flux(P, ur, n1, n2, fr);
-    condition(P, ul, p_l, T_l);
-    condition(P, ur, p_r, T_r);
-    const double vl = (ul[1] / ul[0]) * n1 + (ul[2] / ul[0]) * n2;
-    const double vr = (ur[1] / ur[0]) * n1 + (ur[2] / ur[0]) * n2;
+    double fl[6], fr[6], vl, vr, p_l, p_r;
+    const double irl = int_rcp(ul[0]), irr = int_rcp(ur[0]);
+    flux_at(P, ul, irl, n1, n2, fl, vl, p_l);
+    flux_at(P, ur, irr, n1, n2, fr, vr, p_r);
     const double lam = fmax(fabs(vl), fabs(vr)) +
-                       fmax(sound(P, ul, p_l), sound(P, ur, p_r)) * sqrt(n1 * n1 + n2 * n2);
+                       fmax(sound(P, ul, irl, p_l), sound(P, ur, irr, p_r)) *
+                           int_sqrt(n1 * n1 + n2 * n2);
 #pragma unroll
     for (int v = 0; v < 6; ++v) F[v] = 0.5 * (fl[v] + fr[v]) - 0.5 * lam * (ur[v] - ul[v]);
   }
@@ -174,27 +201,24 @@ struct PhysMoist2D {
   // the pressure Riemann problem at the wall (Toro 2009, section 6.3.3)
   TAG_DEV static void slip_wall(const Params& P, const double* ui, double n1, double n2,
                                 double* F) {
-    const double nrm = sqrt(n1 * n1 + n2 * n2);
-    const double c = n1 / nrm, s = n2 / nrm;
-    const double vn = (c * ui[1] + s * ui[2]) / ui[0];
+    const double nsq = n1 * n1 + n2 * n2, inorm = int_rsqrt(nsq);
+    const double ri = int_rcp(ui[0]);
+    const double vn = fma(n2, ui[2], n1 * ui[1]) * (inorm * ri);
     double p, T;
-    condition(P, ui, p, T);
-    const double qv = ui[4] / ui[0], ql = ui[5] / ui[0];
-    const double qd = 1.0 - qv - ql;
-    const double gm = (qd * P.c_pd + qv * P.c_pv + ql * P.c_pl) *
-                      (1.0 / (qd * P.c_vd + qv * P.c_vv + ql * P.c_pl));
+    condition(P, ui, ri, p, T);
+    const double gm = gamma_mixture(P, ui);
     double p_star;
     if (vn <= 0.0) {
-      const double cs = sqrt(gm * p / ui[0]);
-      p_star = p * pow(1.0 + 0.5 * (gm - 1.0) * vn / cs, 2.0 * gm * (1.0 / (gm - 1.0)));
+      const double ics = int_rsqrt(gm * p * ri);
+      p_star = p * int_pow(fma(0.5 * (gm - 1.0) * vn, ics, 1.0), 2.0 * gm * int_rcp(gm - 1.0));
     } else {
-      const double A = 2.0 / ((gm + 1.0) * ui[0]);
-      const double B = p * (gm - 1.0) / (gm + 1.0);
-      p_star = p + 0.5 * vn / A * (vn + sqrt(vn * vn + 4.0 * A * (p + B)));
+      const double iA = 0.5 * (gm + 1.0) * ui[0];
+      const double B = int_div(p * (gm - 1.0), gm + 1.0);
+      p_star = p + 0.5 * vn * iA * (vn + int_sqrt(vn * vn + int_div(4.0 * (p + B), iA)));
     }
     F[0] = 0.0;
-    F[1] = p_star * c * nrm;
-    F[2] = p_star * s * nrm;
+    F[1] = p_star * n1;
+    F[2] = p_star * n2;
     F[3] = F[4] = F[5] = 0.0;
   }
 
@@ -214,13 +238,13 @@ struct PhysMoist2D {
   // phase_change_term, :405-430
   TAG_DEV static double phase_change(const Params& P, const double* u) {
     double p, T;
-    condition(P, u, p, T);
+    condition(P, u, int_rcp(u[0]), p, T);
     const double rho_qd = u[0] - u[4] - u[5];
     const double T_C = T - 273.15;
-    const double p_vs = 611.2 * exp(17.62 * T_C / (243.12 + T_C));
-    const double a = p_vs / (P.R_v * T) - u[4];
+    const double p_vs = 611.2 * int_exp(int_div(17.62 * T_C, 243.12 + T_C));
+    const double a = int_div(p_vs, P.R_v * T) - u[4];
     const double b = u[0] - u[4] - rho_qd;
-    return a + b - sqrt(a * a + b * b);
+    return a + b - int_sqrt(a * a + b * b);
   }
 
   // source_terms_geopotential (:320-340), + phase change for the moist bubble
@@ -252,7 +276,7 @@ struct PhysMoist2D {
         const double sn = sin(0.5 * (z - 9000.0) * (1.0 / (16000.0 - 9000.0)));
         tau = 0.5 * (sn * sn);
       }
-      const double v1 = u[1] / u[0], v2 = u[2] / u[0];
+      const double ri = int_rcp(u[0]), v1 = u[1] * ri, v2 = u[2] * ri;
       s[1] += -tau * u[0] * (v1 - 10.0);
       s[2] += -tau * u[0] * (v2 - 0.0);
       return;
@@ -307,11 +331,12 @@ struct PhysMoist2D {
 
   // max_abs_speeds, :921-930
   TAG_DEV static void max_speeds(const Params& P, const double* u, double& l1, double& l2) {
+    const double ri = int_rcp(u[0]);
     double p, T;
-    condition(P, u, p, T);
-    const double c = sound(P, u, p);
-    l1 = fabs(u[1] / u[0]) + c;
-    l2 = fabs(u[2] / u[0]) + c;
+    condition(P, u, ri, p, T);
+    const double c = sound(P, u, ri, p);
+    l1 = fabs(u[1] * ri) + c;
+    l2 = fabs(u[2] * ri) + c;
   }
 };
 

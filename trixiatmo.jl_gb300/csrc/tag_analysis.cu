@@ -155,7 +155,7 @@ struct An<PhysMoist2D> {
   static constexpr bool kEntropy = true, kEnergy = true;
   TAG_DEV static double entropy(const P& q, const double* u, const double*) {
     double p, T;
-    PhysMoist2D::condition(q, u, p, T);
+    PhysMoist2D::condition(q, u, int_rcp(u[0]), p, T);
     const double rho_qd = u[0] - u[4] - u[5], rho_qv = u[4], rho_ql = u[5];
     const double lT = log(T);
     const double s_d = q.c_vd * lT - q.R_d * log(rho_qd * q.R_d);
@@ -166,7 +166,7 @@ struct An<PhysMoist2D> {
   TAG_DEV static double energy_total(const P&, const double* u, const double*) { return u[3]; }
   TAG_DEV static double dsdt(const P& q, const double* u, const double* du, const double*) {
     double p, T;
-    PhysMoist2D::condition(q, u, p, T);
+    PhysMoist2D::condition(q, u, int_rcp(u[0]), p, T);
     const double v1 = u[1] / u[0], v2 = u[2] / u[0];
     const double v_square = v1 * v1 + v2 * v2;
     const double rho_qd = u[0] - u[4] - u[5], rho_qv = u[4], rho_ql = u[5];
