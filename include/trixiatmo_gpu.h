@@ -451,12 +451,11 @@ int tag_fp64_peak(double* flops_per_s);
 /* Diagnostics, no counterpart in the reference (whose ln_mean, inv_ln_mean
  * and stolarsky_mean come from Trixi, imported at src/TrixiAtmo.jl:37):
  * evaluates the device forms of those means on n host value pairs (x[q],
- * y[q]) in one kernel.  kind 0: the 2D kernels' pair form (six-coefficient
- * polynomials, logarithms beyond f2 = 1e-2); 1: the same with per-node
- * logarithms and the four-term form below f2 = 1e-4; 2: the 3D energy
- * kernel's halved form (polynomials up to f2 = 0.09); 3: the single means;
- * 4: the potential-temperature kernels' Stolarsky mean with gamma = cp / cv;
- * 5 and 6: the halved form of kind 2 with one mean's pair (x[q], y[q]) and
+ * y[q]) in one kernel.  kind 0: the element kernels' integer forms from node
+ * logarithms; 3: the interface kernels' forms of the values themselves; 1 and
+ * 2: the FP64 polynomial forms of halved values (ranges 0.01 and 0.09 of f2,
+ * logarithms beyond); 4: the potential-temperature kernels' Stolarsky mean
+ * with gamma = cp / cv; 5 and 6: kind 2 with one mean's pair (x[q], y[q]) and
  * the other's (1, 1), so that the two means take different forms
  * (5: ln_mean of the pair in out1; 6: inv_ln_mean of the pair in out2).
  * out1 = ln_mean (kind 4: the Stolarsky mean), out2 = inv_ln_mean.

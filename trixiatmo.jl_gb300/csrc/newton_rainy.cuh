@@ -25,8 +25,8 @@ constexpr int oW1 = 0, oB1 = oW1 + kMlpH * kMlpIn, oW2 = oB1 + kMlpH, oB2 = oW2 
 TAG_DEV double rainy_t_unsat(const double* u, double& e_int) {
   using C = RainyConst;
   const double rho = u[0] + u[1] + u[2];
-  e_int = u[5] - 0.5 * (u[3] * u[3] + u[4] * u[4]) / rho;
-  return (e_int - u[1] * C::ref_L) / (C::c_vd * u[0] + C::c_vv * u[1] + C::c_l * u[2]);
+  e_int = fma(-0.5 * int_rcp(rho), u[3] * u[3] + u[4] * u[4], u[5]);
+  return int_div(e_int - u[1] * C::ref_L, C::c_vd * u[0] + C::c_vv * u[1] + C::c_l * u[2]);
 }
 
 // Network inputs of a rainy state: (rho_dry, rho_moist, rho_rain, internal
@@ -84,70 +84,73 @@ struct NewtonArgs {
                      // memory; the limiter after the last stage of a step), or null
 };
 
-// Residual of the saturation system at x, given svp = e_s(x[2]).
-TAG_DEV void rainy_residual_at(const double* u, const double* x, double svp, double* r) {
+// What the saturation solve reads of a node's conserved variables: internal
+// energy, moist density and the part c_vd rho_d + c_l rho_r of the heat capacity.
+struct RainyNode {
+  double e_int, moist, cap;
+};
+TAG_DEV RainyNode rainy_node(const double* u) {
   using C = RainyConst;
-  const double rho = u[0] + u[1] + u[2];
-  const double ri = 1.0 / rho;
-  const double v1 = u[3] * ri, v2 = u[4] * ri;
-  double r1 = (C::c_vd * u[0] + C::c_vv * x[0] + C::c_l * (x[1] + u[2])) * x[2];
-  r1 += x[0] * C::ref_L;
-  r1 -= (u[5] - rho * 0.5 * (v1 * v1 + v2 * v2));
-  double r2 = fmin(svp / (C::R_v * x[2]), u[1]);
-  r2 -= x[0];
-  r2 *= 1.0e7;
-  double r3 = u[1];
-  r3 -= x[0] + x[1];
-  r3 *= 1.0e7;
-  r[0] = r1;
-  r[1] = r2;
-  r[2] = r3;
+  const double ir = int_rcp(u[0] + u[1] + u[2]);
+  return RainyNode{fma(-0.5 * ir, fma(u[4], u[4], u[3] * u[3]), u[5]), u[1],
+                   fma(C::c_l, u[2], C::c_vd * u[0])};
 }
 
-// Residual of the saturation system at x; returns e_s(x[2]), which the
-// Newton update at the same x reuses.
-TAG_DEV double rainy_residual(const double* u, const double* x, double* r) {
-  const double svp = rainy_e_s(x[2]);
-  rainy_residual_at(u, x, svp, r);
-  return svp;
+// Residual of the saturation system at an iterate and what the Newton update
+// at the same iterate reuses.  r[1] and r[2] are the reference's mass rows
+// without their factor 1e7, which the stopping criterion puts back.
+struct RainyResidual {
+  double r[3];
+  double iT, vs, heat;  // 1/T, e_s(T) / (R_v T), heat capacity
+};
+TAG_DEV RainyResidual rainy_residual_at(const RainyNode& n, const double* x, double iT,
+                                        double svp) {
+  using C = RainyConst;
+  RainyResidual q;
+  q.iT = iT;
+  q.vs = svp * (iT * kRainyInvRv);
+  q.heat = fma(C::c_l, x[1], fma(C::c_vv, x[0], n.cap));
+  q.r[0] = fma(q.heat, x[2], fma(x[0], C::ref_L, -n.e_int));
+  q.r[1] = fmin(q.vs, n.moist) - x[0];
+  q.r[2] = n.moist - (x[0] + x[1]);
+  return q;
+}
+TAG_DEV RainyResidual rainy_residual(const RainyNode& n, const double* x) {
+  const double iT = int_rcp(x[2]);
+  return rainy_residual_at(n, x, iT, rainy_e_s(x[2], iT));
 }
 
-// Newton update dx = J^{-1} r with the reference Jacobian (Cramer's rule);
-// svp = e_s(x[2]) as the residual at x returned it
-TAG_DEV void rainy_newton_step(const double* u, const double* x, const double* r, double svp,
+// Newton update dx = J^{-1} r with the reference Jacobian (Cramer's rule; the
+// two mass rows and their residuals share the factor 1e7, which cancels).
+TAG_DEV void rainy_newton_step(const RainyNode& n, const double* x, const RainyResidual& q,
                                double* dx) {
   using C = RainyConst;
-  const double svp_t = rainy_e_s_T_from(x[2], svp);
-  const double a = C::c_vv * x[2] + C::ref_L, b = C::c_l * x[2];
-  const double c = C::c_vd * u[0] + C::c_vv * x[0] + C::c_l * (x[1] + u[2]);
-  const double d = -10000000.0, e = 0.0;
-  const double f = (svp / (C::R_v * x[2]) < u[1]) ? (svp_t * x[2] - svp) / (C::R_v * x[2] * x[2]) * 1.0e7 : 0.0;
-  const double g = -10000000.0, h = -10000000.0, i = 0.0;
-  const double A = e * i - f * h, B = -(d * i - f * g), Cc = d * h - e * g;
-  const double id = 1.0 / (a * A + b * B + c * Cc);
-  dx[0] = (A * r[0] + (c * h - b * i) * r[1] + (b * f - c * e) * r[2]) * id;
-  dx[1] = (B * r[0] + (a * i - c * g) * r[1] + (c * d - a * f) * r[2]) * id;
-  dx[2] = (Cc * r[0] + (b * g - a * h) * r[1] + (a * e - b * d) * r[2]) * id;
+  const double T = x[2], c = q.heat;
+  // d(vs)/dT = vs ((c1 - 1) + c2 / T) / T below the moist density, else 0
+  const double f = q.vs < n.moist ? q.vs * q.iT * fma(kRainyC2, q.iT, kRainyC1 - 1.0) : 0.0;
+  const double a = fma(C::c_vv, T, C::ref_L), b = C::c_l * T, ab = a - b;
+  const double id = int_rcp(fma(f, ab, c));
+  const double t = fma(f, q.r[0], -c * q.r[1]);
+  dx[0] = fma(b * f, q.r[2], t) * id;
+  dx[1] = -fma(fma(a, f, c), q.r[2], t) * id;
+  dx[2] = fma(b, q.r[2], fma(ab, q.r[1], q.r[0])) * id;
 }
 
-TAG_DEV bool rainy_newton_done(const double* u, const double* r, int mode, double tol) {
-  if (mode == 0) return fmax(fabs(r[0]), fmax(fabs(r[1]), fabs(r[2]))) < tol;
-  const double rho = u[0] + u[1] + u[2];
-  const double e_int = u[5] - 0.5 * (u[3] * u[3] + u[4] * u[4]) / rho;
-  const double s2 = tol * 1.0e7 * fabs(u[1]);
-  return fabs(r[0]) < tol * fabs(e_int) && fabs(r[1]) <= s2 && fabs(r[2]) <= s2;
+TAG_DEV bool rainy_newton_done(const RainyNode& n, const double* r, int mode, double tol) {
+  // mode 0: max(|r_0|, 1e7 |r_1|, 1e7 |r_2|) < tol
+  if (mode == 0) return fmax(1.0e-7 * fabs(r[0]), fmax(fabs(r[1]), fabs(r[2]))) < 1.0e-7 * tol;
+  const double s2 = tol * fabs(n.moist);
+  return fabs(r[0]) < tol * fabs(n.e_int) && fabs(r[1]) <= s2 && fabs(r[2]) <= s2;
 }
 
 // Size of a residual in the units of the stopping criterion: max |r| for
 // mode 0; for mode 1 each component over its own scale (|E_int| for the
-// energy, 1e7 rho_moist for the two mass rows), so that a size below tol is
+// energy, rho_moist for the two mass rows), so that a size below tol is
 // convergence in both modes.
-TAG_DEV double rainy_residual_size(const double* u, const double* r, int mode) {
-  if (mode == 0) return fmax(fabs(r[0]), fmax(fabs(r[1]), fabs(r[2])));
-  const double rho = u[0] + u[1] + u[2];
-  const double e_int = u[5] - 0.5 * (u[3] * u[3] + u[4] * u[4]) / rho;
-  const double sm = 1.0e7 * fabs(u[1]);
-  return fmax(fabs(r[0]) / fabs(e_int), fmax(fabs(r[1]), fabs(r[2])) / sm);
+TAG_DEV double rainy_residual_size(const RainyNode& n, const double* r, int mode) {
+  const double m = fmax(fabs(r[1]), fabs(r[2]));
+  if (mode == 0) return fmax(fabs(r[0]), 1.0e7 * m);
+  return fmax(int_div(fabs(r[0]), fabs(n.e_int)), int_div(m, fabs(n.moist)));
 }
 
 // Snaps a converged iterate to a grid fixed by the node's state: vapour and
@@ -169,44 +172,35 @@ TAG_DEV void rainy_snap(const double* u, double* x) {
 // further updates are taken from there; if the criterion then fails, the
 // iterate before the snap is kept.  svp0 > 0 is e_s(x[2]) of the start when
 // the caller has it already (a guess computed it), else 0.
-TAG_DEV int rainy_newton_run(const double* u, double* x, int mode, double tol, int maxit,
-                             int polish, bool& converged, double svp0 = 0.0) {
-  double r[3], dx[3];
+TAG_DEV int rainy_newton_run(const double* u, const RainyNode& n, double* x, int mode, double tol,
+                             int maxit, int polish, bool& converged, double svp0 = 0.0) {
+  double dx[3];
   int it = 0;
   converged = false;
   for (; it < maxit; ++it) {
-    double svp;
-    if (it == 0 && svp0 > 0.0) {
-      svp = svp0;
-      rainy_residual_at(u, x, svp, r);
-    } else {
-      svp = rainy_residual(u, x, r);
-    }
-    if (rainy_newton_done(u, r, mode, tol)) {
+    const double iT = int_rcp(x[2]);
+    const double svp = it == 0 && svp0 > 0.0 ? svp0 : rainy_e_s(x[2], iT);
+    const RainyResidual q = rainy_residual_at(n, x, iT, svp);
+    if (rainy_newton_done(n, q.r, mode, tol)) {
       converged = true;
       break;
     }
-    rainy_newton_step(u, x, r, svp, dx);
+    rainy_newton_step(n, x, q, dx);
     x[0] -= dx[0];
     x[1] -= dx[1];
     x[2] -= dx[2];
   }
-  if (!converged) {
-    rainy_residual(u, x, r);
-    converged = rainy_newton_done(u, r, mode, tol);
-  }
+  if (!converged) converged = rainy_newton_done(n, rainy_residual(n, x).r, mode, tol);
   if (polish > 0 && converged) {
     double y[3] = {x[0], x[1], x[2]};
     rainy_snap(u, y);
     for (int p = 0; p < polish; ++p) {
-      const double svp = rainy_residual(u, y, r);
-      rainy_newton_step(u, y, r, svp, dx);
+      rainy_newton_step(n, y, rainy_residual(n, y), dx);
       y[0] -= dx[0];
       y[1] -= dx[1];
       y[2] -= dx[2];
     }
-    rainy_residual(u, y, r);
-    if (rainy_newton_done(u, r, mode, tol)) {
+    if (rainy_newton_done(n, rainy_residual(n, y).r, mode, tol)) {
       x[0] = y[0];
       x[1] = y[1];
       x[2] = y[2];
@@ -220,10 +214,9 @@ TAG_DEV int rainy_newton_run(const double* u, double* x, int mode, double tol, i
 // returns false for a saturated node.  svp = e_s(T_unsat) (0 if T_unsat <= 0).
 TAG_DEV bool rainy_closed_form_guess(const double* u, double* x, double& tu, double& e_int,
                                      double& svp) {
-  using C = RainyConst;
   tu = rainy_t_unsat(u, e_int);
   svp = tu > 0.0 ? rainy_e_s(tu) : 0.0;
-  if (tu > 0.0 && svp / (C::R_v * tu) >= u[1]) {
+  if (tu > 0.0 && svp * (int_rcp(tu) * kRainyInvRv) >= u[1]) {
     x[0] = u[1];
     x[1] = 0.0;
     x[2] = tu;
@@ -238,15 +231,15 @@ TAG_DEV bool rainy_closed_form_guess(const double* u, double* x, double& tu, dou
 // Returns true where the closed form was taken; svp = e_s(x[2]).
 TAG_DEV bool rainy_learned_guess(const float* __restrict__ P, const double* u, double* x,
                                  double& svp) {
-  using C = RainyConst;
   double e_int, tu;
   if (rainy_closed_form_guess(u, x, tu, e_int, svp)) return true;
   float xin[kMlpIn];
   mlp_inputs(u, e_int, tu, xin);
   const double T = tu + fmax((double)mlp_forward(P, xin), 0.0);
-  svp = rainy_e_s(T);
+  const double iT = int_rcp(T);
+  svp = rainy_e_s(T, iT);
   x[2] = T;
-  x[0] = fmin(svp / (C::R_v * T), u[1]);
+  x[0] = fmin(svp * (iT * kRainyInvRv), u[1]);
   x[1] = u[1] - x[0];
   return false;
 }
@@ -264,6 +257,7 @@ TAG_DEV int newton_rainy_node(const float* sp, double* __restrict__ un, const Ne
 #pragma unroll
   for (int v = 0; v < 6; ++v) s[v] = un[v];
   if (un[2] < 0.0) un[2] = 0.0;
+  const RainyNode n = rainy_node(s);
   double x[3] = {un[6], un[7], un[8]};
   conv = false;
   fallback = 0;
@@ -277,18 +271,16 @@ TAG_DEV int newton_rainy_node(const float* sp, double* __restrict__ un, const Ne
     guessed = rainy_learned_guess(sp, s, xg, svp_g);
     if (!guessed) {
       // saturated node: keep the MLP guess only where it starts closer
-      double rg[3], rw[3];
-      rainy_residual_at(s, xg, svp_g, rg);
-      rainy_residual(s, x, rw);
-      const double sg = rainy_residual_size(s, rg, a.mode);
-      guessed = isfinite(sg) && sg < rainy_residual_size(s, rw, a.mode);
+      const double sg = rainy_residual_size(
+          n, rainy_residual_at(n, xg, int_rcp(xg[2]), svp_g).r, a.mode);
+      guessed = isfinite(sg) && sg < rainy_residual_size(n, rainy_residual(n, x).r, a.mode);
     }
   } else if (a.learned == 2) {
     double tu, e_int;
     guessed = rainy_closed_form_guess(s, xg, tu, e_int, svp_g);
   }
   if (guessed) {
-    its = rainy_newton_run(s, xg, a.mode, a.tol, a.maxit_learned, a.polish, conv, svp_g);
+    its = rainy_newton_run(s, n, xg, a.mode, a.tol, a.maxit_learned, a.polish, conv, svp_g);
     if (conv && isfinite(xg[2])) {
       x[0] = xg[0];
       x[1] = xg[1];
@@ -298,7 +290,7 @@ TAG_DEV int newton_rainy_node(const float* sp, double* __restrict__ un, const Ne
       conv = false;
     }
   }
-  if (!conv) its += rainy_newton_run(s, x, a.mode, a.tol, a.maxit, a.polish, conv);
+  if (!conv) its += rainy_newton_run(s, n, x, a.mode, a.tol, a.maxit, a.polish, conv);
   un[6] = x[0];
   un[7] = x[1];
   un[8] = x[2];

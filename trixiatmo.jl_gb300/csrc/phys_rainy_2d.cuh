@@ -20,46 +20,57 @@ struct RainyConst {
 
 // saturation_vapour_pressure (:397-419),
 //   e_s(T) = ref_s_p (T / ref_temp)^c1 exp(c2 (1 / ref_temp - 1 / T)),
-// evaluated as ref_s_p exp(c1 log(T / ref_temp) + c2 (1 / ref_temp - 1 / T)):
-// one logarithm and one exponential where the power costs both again (FP64
-// transcendentals are the rainy kernels' main cost).  Relative difference to
-// the reference's form: a few ulp.
+// evaluated as ref_s_p exp(c1 ln2 (log2 T - log2 ref_temp) + c2 (1 / ref_temp - 1 / T)):
+// one logarithm and one exponential where the power costs both again, both on
+// the integer pipe (int_math.cuh).  Relative difference to the reference's
+// form: a few ulp.
 constexpr double kRainyC1 = (RainyConst::c_pv - RainyConst::c_l) / RainyConst::R_v;
 constexpr double kRainyC2 =
     (RainyConst::ref_L - (RainyConst::c_pv - RainyConst::c_l) * RainyConst::ref_temp) /
     RainyConst::R_v;
+constexpr double kRainyC1Ln2 = kRainyC1 * 0.6931471805599453;
+// log2(273.15) 2^58 and 1 / (R_v)
+constexpr i64 kRainyLog2Ref = TAG_RAINY_LOG2_REF;
+constexpr double kRainyInvRv = 1.0 / RainyConst::R_v;
 
-TAG_DEV double rainy_e_s(double T) {
+// e_s(T) with iT = 1/T
+TAG_DEV double rainy_e_s(double T, double iT) {
   using C = RainyConst;
-  return C::ref_s_p * exp(kRainyC1 * log(T / C::ref_temp) + kRainyC2 * (1.0 / C::ref_temp - 1.0 / T));
+  if (!(T > 0.0)) return C::ref_s_p * slow_exp(kRainyC1 * log(T / C::ref_temp));  // NaN for T < 0
+  return C::ref_s_p * int_exp(fma(kRainyC2, 1.0 / C::ref_temp - iT,
+                                  kRainyC1Ln2 * int_log2_ratio(T, kRainyLog2Ref)));
 }
+TAG_DEV double rainy_e_s(double T) { return rainy_e_s(T, int_rcp(T)); }
 
 // saturation_vapour_pressure_derivative (:421-446) from the value e_s = e_s(T):
 // the reference's ref_s_p / ref_temp^c1 (c1 T^(c1-1) + c2 T^(c1-2)) exp(...)
-// equals e_s(T) (c1 + c2 / T) / T
-TAG_DEV double rainy_e_s_T_from(double T, double e_s) { return e_s * (kRainyC1 + kRainyC2 / T) / T; }
+// equals e_s(T) (c1 + c2 / T) / T (iT = 1/T)
+TAG_DEV double rainy_e_s_T_from(double iT, double e_s) {
+  return e_s * fma(kRainyC2, iT, kRainyC1) * iT;
+}
 
-TAG_DEV double rainy_e_s_T(double T) { return rainy_e_s_T_from(T, rainy_e_s(T)); }
+TAG_DEV double rainy_e_s_T(double T) { return rainy_e_s_T_from(int_rcp(T), rainy_e_s(T)); }
 
 // x^(1/8) by three correctly rounded square roots (x^0.125 to a few ulp;
 // NaN for x < 0, as the power)
-TAG_DEV double rainy_root8(double x) { return sqrt(sqrt(sqrt(x))); }
+TAG_DEV double rainy_root8(double x) { return int_sqrt(int_sqrt(int_sqrt(x))); }
 
 // terminal_velocity_rain, :380-395
 TAG_DEV double rainy_v_rain(double rho_moist, double rho_rain) {
   using C = RainyConst;
   if (rho_rain > 0.0)
     return C::v_0 * 1.9386213994279082 *
-           rainy_root8(rho_rain / (C::pi * (rho_moist + rho_rain) * C::N_0));
+           rainy_root8(int_div(rho_rain, C::pi * (rho_moist + rho_rain) * C::N_0));
   return 0.0;
 }
 
 struct PhysRainy2D {
   static constexpr int NV = 9;
   static constexpr int NA = 9;
-  // rho_d, rho_m, rho_r, v1/2, v2/2, rho_vapour, rho_cloud, T, 1/T,
-  // v_rain(rho_vapour + rho_cloud, rho_r), (v1^2 + v2^2)/4
-  static constexpr int NQ = 11;
+  // rho_d/2, rho_vapour/2, rho_cloud/2, rho_r/2, v1/2, v2/2, T/2, 1/(2T),
+  // v_rain(rho_vapour + rho_cloud, rho_r)/2, (v1^2 + v2^2)/4, log2 of rho_d,
+  // rho_vapour and T (words; odd stride)
+  static constexpr int NQ = 13;
   static constexpr bool kLastHalved = false;
   static constexpr bool kHasSources = true;
   static constexpr bool kSurfaceNoncons = false;  // surface flux only (flux_zero)
@@ -82,9 +93,9 @@ struct PhysRainy2D {
     using C = RainyConst;
     const double rho = u[0] + u[1] + u[2];
     if (u[1] == 0.0 && u[2] == 0.0) {
-      const double ri = 1.0 / rho;
+      const double ri = int_rcp(rho);
       const double v1 = u[3] * ri, v2 = u[4] * ri;
-      T = (u[5] - 0.5 * (v1 * v1 + v2 * v2) * rho) / (C::c_vd * rho);
+      T = int_div(u[5] - 0.5 * (v1 * v1 + v2 * v2) * rho, C::c_vd * rho);
       rv = 0.0;
       rc = 0.0;
       return;
@@ -96,51 +107,54 @@ struct PhysRainy2D {
     if (rc < 0.0 && fabs(rc) <= 1e-15) rc = 0.0;
   }
 
+  // (R_d + R_v q_v) / (c_vd + c_vv q_v + c_l q_l), of densities instead of the
+  // ratios to the dry one
+  TAG_DEV static double gas_ratio(double rd, double rv, double rl) {
+    using C = RainyConst;
+    return int_div(fma(C::R_v, rv, C::R_d * rd), fma(C::c_l, rl, fma(C::c_vv, rv, C::c_vd * rd)));
+  }
+
   TAG_DEV static void node_prims(const Params&, const double* u, double* q, unsigned& bad) {
     double rv, rc, T;
     nlsol(u, rv, rc, T);
-    const double ri = 1.0 / (u[0] + u[1] + u[2]);
+    const double ri = int_rcp(u[0] + u[1] + u[2]);
     const double v1 = u[3] * ri, v2 = u[4] * ri;
-    q[0] = u[0];
-    q[1] = u[1];
-    q[2] = u[2];
-    q[3] = 0.5 * v1;
-    q[4] = 0.5 * v2;
-    q[5] = rv;
-    q[6] = rc;
-    q[7] = T;
-    q[8] = 1.0 / T;
-    q[9] = rainy_v_rain(rv + rc, u[2]);
-    q[10] = 0.25 * (v1 * v1 + v2 * v2);
-    if (!(u[0] > 0.0)) bad |= TAG_S_NEG_DENSITY;
-    if (!(T > 0.0)) bad |= TAG_S_NEG_PRESSURE;
+    q[0] = 0.5 * u[0];
+    q[1] = 0.5 * rv;
+    q[2] = 0.5 * rc;
+    q[3] = 0.5 * u[2];
+    q[4] = 0.5 * v1;
+    q[5] = 0.5 * v2;
+    q[6] = 0.5 * T;
+    q[7] = 0.5 * int_rcp(T);
+    q[8] = 0.5 * rainy_v_rain(rv + rc, u[2]);
+    q[9] = 0.25 * fma(v2, v2, v1 * v1);
+    q[10] = log_word_signed(u[0]);
+    q[11] = log_word_signed(rv);
+    q[12] = log_word_signed(T);
+    if (not_positive(u[0])) bad |= TAG_S_NEG_DENSITY;
+    if (not_positive(T)) bad |= TAG_S_NEG_PRESSURE;
   }
 
   // flux_ec_rain, :872-961, for one symmetric pair (no nonconservative part)
   TAG_DEV static void volume_pair(const Params&, const double* a, const double* b, double n1,
                                   double n2, double* Fa, double* Fb) {
     using C = RainyConst;
-    const double v1a = a[3] + b[3], v2a = a[4] + b[4];
-    const double K = a[10] + b[10];
+    const double v1a = a[4] + b[4], v2a = a[5] + b[5];
+    const double K = a[9] + b[9];
     const double vdn = n1 * v1a + n2 * v2a;
-    const double vrn = 0.5 * n2 * (a[9] + b[9]);
-    const double rd_avg = 0.5 * (a[0] + b[0]);
-    const double rv_avg = 0.5 * (a[5] + b[5]);
-    const double rc_avg = 0.5 * (a[6] + b[6]);
-    const double rr_avg = 0.5 * (a[2] + b[2]);
-    // ln_mean of the dry densities, inv_ln_mean of 1/T and 1/(1/T_a + 1/T_b)
-    // (= 1/(2 iT_avg), the pressure's divisor) from one shared reciprocal
-    double rd_log, iT_log, i_sum;
-    if (a[0] != 0.0 && b[0] != 0.0) {
-      ln_mean_pair<false, true>(a[0], b[0], a[8], b[8], 0.0, 0.0, 0.0, 0.0, rd_log, iT_log,
-                                &i_sum);
-    } else {
-      rd_log = 0.0;
-      iT_log = inv_ln_mean_single(a[8], b[8]);
-      i_sum = 1.0 / (a[8] + b[8]);
-    }
-    const double rv_log = (a[5] != 0.0 && b[5] != 0.0) ? ln_mean_single(a[5], b[5]) : 0.0;
-    const double p_int = (C::R_d * rd_avg + C::R_v * rv_avg) * (2.0 * i_sum);
+    const double vrn = n2 * (a[8] + b[8]);
+    const double rd_avg = a[0] + b[0], rv_avg = a[1] + b[1];
+    const double rc_avg = a[2] + b[2], rr_avg = a[3] + b[3];
+    const double rd_log = !is_zero(a[0]) && !is_zero(b[0])
+                              ? rd_avg * ln_factor(a[0], b[0], log_difference(a[10], b[10]))
+                              : 0.0;
+    const double rv_log = !is_zero(a[1]) && !is_zero(b[1])
+                              ? rv_avg * ln_factor(a[1], b[1], log_difference(a[11], b[11]))
+                              : 0.0;
+    // inv_ln_mean of 1/T
+    const double T_log = (a[6] + b[6]) * inv_ln_factor(a[6], b[6], log_difference(a[12], b[12]));
+    const double p_int = fma(C::R_v, rv_avg, C::R_d * rd_avg) * int_rcp(a[7] + b[7]);
     const double f_v = rv_log * vdn;
     const double f_c = rc_avg * vdn;
     const double f_d = rd_log * vdn;
@@ -149,8 +163,10 @@ struct PhysRainy2D {
     const double f_rho = f_d + f_m + f_r;
     const double f_m1 = f_rho * v1a + p_int * n1;
     const double f_m2 = f_rho * v2a + p_int * n2;
-    const double f_e = (C::c_vd * iT_log - K) * f_d + (C::c_vv * iT_log - K + C::ref_L) * f_v +
-                       (C::c_l * iT_log - K) * (f_c + f_r) + (v1a * f_m1 + v2a * f_m2);
+    // (c_vd T - K) f_d + (c_vv T - K + L) f_v + (c_l T - K)(f_c + f_r) + v.(f_m1, f_m2)
+    const double cf = fma(C::c_l, f_c + f_r, fma(C::c_vv, f_v, C::c_vd * f_d));
+    const double f_e =
+        fma(v2a, f_m2, fma(v1a, f_m1, fma(-K, f_rho, fma(C::ref_L, f_v, T_log * cf))));
     Fa[0] = Fb[0] = f_d;
     Fa[1] = Fb[1] = f_m;
     Fa[2] = Fb[2] = f_r;
@@ -168,7 +184,7 @@ struct PhysRainy2D {
     double rv, rc, T;
     nlsol(u, rv, rc, T);
     const double rho = u[0] + u[1] + u[2];
-    const double ri = 1.0 / rho;
+    const double ri = int_rcp(rho);
     const double v1 = u[3] * ri, v2 = u[4] * ri;
     const double vr = rainy_v_rain(u[1], u[2]);
     const double vn = v1 * n1 + v2 * n2;
@@ -192,7 +208,7 @@ struct PhysRainy2D {
     double rv, rc, T;
     nlsol(u, rv, rc, T);
     const double rho = u[0] + u[1] + u[2];
-    const double ri = 1.0 / rho;
+    const double ri = int_rcp(rho);
     const double v1 = u[3] * ri, v2 = u[4] * ri;
     const double vr = rainy_v_rain(u[1], u[2]);
     const double vn = v1 * n1 + v2 * n2;
@@ -206,10 +222,8 @@ struct PhysRainy2D {
     f[5] = (u[5] + p) * vn - (C::c_l * T + 0.5 * (v1 * v1 + v2 * v2)) * u[2] * vrn;
     f[6] = f[7] = f[8] = 0.0;
     vabs = fabs(vn) + fabs(vrn);
-    const double q_v = rv / u[0];
-    const double q_l = (rc + u[2]) / u[0];
-    const double gm = 1.0 + (C::R_d + C::R_v * q_v) / (C::c_vd + C::c_vv * q_v + C::c_l * q_l);
-    c = sqrt(gm * p * ri);
+    const double gm = 1.0 + gas_ratio(u[0], rv, rc + u[2]);
+    c = int_sqrt(gm * p * ri);
   }
 
   // speed_of_sound (:332-366) and the normal speeds of max_abs_speed_naive (:595-611)
@@ -217,12 +231,10 @@ struct PhysRainy2D {
     using C = RainyConst;
     double rv, rc, T;
     nlsol(u, rv, rc, T);
-    const double ri = 1.0 / (u[0] + u[1] + u[2]);
+    const double ri = int_rcp(u[0] + u[1] + u[2]);
     const double p = (C::R_d * u[0] + C::R_v * rv) * T;
-    const double q_v = rv / u[0];
-    const double q_l = (rc + u[2]) / u[0];
-    const double gm = 1.0 + (C::R_d + C::R_v * q_v) / (C::c_vd + C::c_vv * q_v + C::c_l * q_l);
-    return sqrt(gm * p * ri);
+    const double gm = 1.0 + gas_ratio(u[0], rv, rc + u[2]);
+    return int_sqrt(gm * p * ri);
   }
 
   // pressure(u), :328-341
@@ -238,14 +250,13 @@ struct PhysRainy2D {
   TAG_DEV static void lmars(const double* ul, const double* ur, double n1, double n2, double* F) {
     const double a = 360.0;
     const double rl = ul[0] + ul[1] + ul[2], rr = ur[0] + ur[1] + ur[2];
-    const double ril = 1.0 / rl, rir = 1.0 / rr;
     const double pl = pressure(ul), pr = pressure(ur);
-    const double vl = (ul[3] * ril) * n1 + (ul[4] * ril) * n2;
-    const double vr = (ur[3] * rir) * n1 + (ur[4] * rir) * n2;
-    const double nrm = sqrt(n1 * n1 + n2 * n2);
-    const double rho = 0.5 * (rl + rr);
-    const double p_int = 0.5 * (pl + pr) - 0.5 * a * rho * (vr - vl) / nrm;
-    const double v_int = 0.5 * (vl + vr) - 1.0 / (2.0 * a * rho) * (pr - pl) * nrm;
+    const double vl = fma(ul[4], n2, ul[3] * n1) * int_rcp(rl);
+    const double vr = fma(ur[4], n2, ur[3] * n1) * int_rcp(rr);
+    const double nsq = n1 * n1 + n2 * n2, inorm = int_rsqrt(nsq), nrm = nsq * inorm;
+    const double rs = rl + rr;  // 2 rho
+    const double p_int = 0.5 * (pl + pr) - 0.25 * a * rs * (vr - vl) * inorm;
+    const double v_int = 0.5 * (vl + vr) - int_rcp(a * rs) * (pr - pl) * nrm;
     const double* us = v_int > 0.0 ? ul : ur;
     const double ps = v_int > 0.0 ? pl : pr;
     F[0] = us[0] * v_int;
@@ -261,29 +272,26 @@ struct PhysRainy2D {
   // pressure of the Riemann problem against the wall (Toro 2009, 6.3.3)
   TAG_DEV static void slip_wall(const double* ui, double n1, double n2, double* F) {
     using C = RainyConst;
-    const double nrm = sqrt(n1 * n1 + n2 * n2);
-    const double c = n1 / nrm, s = n2 / nrm;
+    const double inorm = int_rsqrt(n1 * n1 + n2 * n2);
     const double rho = ui[0] + ui[1] + ui[2];
-    const double ri = 1.0 / rho;
-    const double vn = (c * ui[3] + s * ui[4]) * ri;
+    const double ri = int_rcp(rho);
+    const double vn = fma(n2, ui[4], n1 * ui[3]) * (inorm * ri);
     double rv, rc, T;
     nlsol(ui, rv, rc, T);
     const double p = (C::R_d * ui[0] + C::R_v * rv) * T;
-    const double q_v = rv / ui[0];
-    const double q_l = (rc + ui[2]) / ui[0];
-    const double gm = 1.0 + (C::R_d + C::R_v * q_v) / (C::c_vd + C::c_vv * q_v + C::c_l * q_l);
+    const double gm = 1.0 + gas_ratio(ui[0], rv, rc + ui[2]);
     double p_star;
     if (vn <= 0.0) {
-      const double cs = sqrt(gm * p * ri);
-      p_star = p * pow(1.0 + 0.5 * (gm - 1.0) * vn / cs, 2.0 * gm * (1.0 / (gm - 1.0)));
+      const double ics = int_rsqrt(gm * p * ri);
+      p_star = p * int_pow(fma(0.5 * (gm - 1.0) * vn, ics, 1.0), 2.0 * gm * int_rcp(gm - 1.0));
     } else {
-      const double A = 2.0 / ((gm + 1.0) * rho);
-      const double B = p * (gm - 1.0) / (gm + 1.0);
-      p_star = p + 0.5 * vn / A * (vn + sqrt(vn * vn + 4.0 * A * (p + B)));
+      const double iA = 0.5 * (gm + 1.0) * rho;
+      const double B = int_div(p * (gm - 1.0), gm + 1.0);
+      p_star = p + 0.5 * vn * iA * (vn + int_sqrt(vn * vn + int_div(4.0 * (p + B), iA)));
     }
     F[0] = F[1] = F[2] = 0.0;
-    F[3] = p_star * c * nrm;
-    F[4] = p_star * s * nrm;
+    F[3] = p_star * n1;
+    F[4] = p_star * n2;
     F[5] = F[6] = F[7] = F[8] = 0.0;
   }
 
@@ -298,7 +306,7 @@ struct PhysRainy2D {
     double fl[9], fr[9], vl, vr, cl, cr;
     flux_and_speeds(ul, n1, n2, fl, vl, cl);
     flux_and_speeds(ur, n1, n2, fr, vr, cr);
-    const double lam = fmax(vl, vr) + fmax(cl, cr) * sqrt(n1 * n1 + n2 * n2);
+    const double lam = fmax(vl, vr) + fmax(cl, cr) * int_sqrt(n1 * n1 + n2 * n2);
 #pragma unroll
     for (int v = 0; v < 9; ++v) F[v] = 0.5 * (fl[v] + fr[v]) - 0.5 * lam * (ur[v] - ul[v]);
   }
@@ -349,13 +357,14 @@ struct PhysRainy2D {
       double rv, rc, T;
       nlsol(u, rv, rc, T);
       const double rho = u[0] + u[1] + u[2];
-      const double rho_vs = rainy_e_s(T) / (C::R_v * T);
+      const double iT = int_rcp(T);
+      const double rho_vs = rainy_e_s(T, iT) * iT * kRainyInvRv;
       // rho_r^0.1875, rho_r^0.5 and rho_r^0.875 from square roots: with
       // r8 = rho_r^(1/8) and r16 = r8^(1/2), r16^3, sqrt(rho_r) and r8^7
-      const double r8 = rainy_root8(u[2]), r16 = sqrt(r8);
+      const double r8 = rainy_root8(u[2]), r16 = int_sqrt(r8);
       const double r8_2 = r8 * r8, r8_4 = r8_2 * r8_2;
       double S_ev = (3.86e-3 - 9.41e-5 * (T - C::ref_temp)) * (1.0 + 9.1 * (r16 * r16 * r16));
-      S_ev *= (rho_vs - rv) * sqrt(u[2]);
+      S_ev *= (rho_vs - rv) * int_sqrt(u[2]);
       const double S_auto = 0.001 * rc;
       const double S_acc = 1.72 * rc * (r8_4 * r8_2 * r8);
       const double S_rain = S_auto + S_acc - S_ev;
@@ -406,7 +415,7 @@ struct PhysRainy2D {
 
   // max_abs_speeds, :588-593
   TAG_DEV static void max_speeds(const Params&, const double* u, double& l1, double& l2) {
-    const double ri = 1.0 / (u[0] + u[1] + u[2]);
+    const double ri = int_rcp(u[0] + u[1] + u[2]);
     const double c = sound(u);
     l1 = fabs(u[3] * ri) + c;
     l2 = fabs(u[4] * ri) + c + fabs(rainy_v_rain(u[1], u[2]));

@@ -16,53 +16,66 @@ void set_last_error(const std::string& msg);
 
 constexpr int kMaxNodes = 8;  // n = polydeg + 1 supported up to polydeg 7
 
-// Logarithmic mean and its inverse in the form of Ranocha et al., ACM TOMS 49
-// (2023), arXiv:2112.10517: a 4-term series in f2 = ((x-y)/(x+y))^2 when
-// f2 < 1e-4, else (y-x)/log(y/x).  Trixi.ln_mean / Trixi.inv_ln_mean are the
-// reference's definitions (imported at src/TrixiAtmo.jl:37).
-TAG_DEV double ln_mean(double x, double y) {
-  const double f2 = (x * (x - 2.0 * y) + y * y) / (x * (x + 2.0 * y) + y * y);
-  if (f2 < 1.0e-4) {
-    return (x + y) * 52.5 / (105.0 + f2 * (35.0 + f2 * (21.0 + f2 * 15.0)));
-  }
-  return (y - x) / log(y / x);
+// Factors of the logarithmic means of a node pair, from the difference d of
+// their log2_fixed node logarithms (b minus a):
+//   ln_mean(xa, xb) = (xa + xb)/2 R,  inv_ln_mean(1/ya, 1/yb) = (ya + yb)/2 Q.
+// Values within a factor of two (every pair of an element that resolves its
+// stratification) take the integer series, whatever their size: no reciprocal,
+// no logarithm, no branch that splits a warp.  Beyond it d itself is the
+// logarithm: |d| >= 1, so its 2^-52 is a relative error of the same size.
+TAG_DEV double log_of_difference(i64 d) { return (double)d * 1.539095918623324e-16; }  // ln2 2^-52
+
+// (Values of opposite sign, which a moisture density may have, give NaN: the
+// logarithm of their ratio.)
+TAG_DEV bool opposite_signs(double a, double b) { return (i64)(f64_bits(a) ^ f64_bits(b)) < 0; }
+static __device__ __noinline__ double ln_factor_far(double xa, double xb, i64 d) {
+  if (opposite_signs(xa, xb)) return f64_from(0x7ff8000000000000ull);
+  return int_div(2.0 * (xb - xa), log_of_difference(d) * (xa + xb));
+}
+static __device__ __noinline__ double inv_ln_factor_far(double ya, double yb, i64 d) {
+  return int_div(2.0 * ya * yb * log_of_difference(d), (yb - ya) * (ya + yb));
+}
+TAG_DEV double ln_factor(double xa, double xb, i64 d) {
+  const u64 a = magnitude(d);
+  return series_in_range(a) ? ln_mean_factor(log_square(a)) : ln_factor_far(xa, xb, d);
+}
+TAG_DEV double inv_ln_factor(double ya, double yb, i64 d) {
+  const u64 a = magnitude(d);
+  return series_in_range(a) ? inv_ln_mean_factor(log_square(a)) : inv_ln_factor_far(ya, yb, d);
 }
 
-TAG_DEV double inv_ln_mean(double x, double y) {
-  const double f2 = (x * (x - 2.0 * y) + y * y) / (x * (x + 2.0 * y) + y * y);
-  if (f2 < 1.0e-4) {
-    return (105.0 + f2 * (35.0 + f2 * (21.0 + f2 * 15.0))) / (52.5 * (x + y));
-  }
-  return log(y / x) / (y - x);
+// The means of two values themselves (interface kernels): ln_mean(x, y), and
+// inv_ln_mean(1/x, 1/y) from the reciprocals' own values.
+TAG_DEV double ln_mean_of(double x, double y) {
+  return 0.5 * (x + y) * ln_factor(x, y, log2_fixed(y) - log2_fixed(x));
+}
+TAG_DEV double inv_ln_mean_of_reciprocals(double x, double y) {
+  return 0.5 * (x + y) * inv_ln_factor(x, y, log2_fixed(y) - log2_fixed(x));
 }
 
-// Both logarithmic means of one node pair with a single reciprocal and no
-// logarithm in the common case.  With f2 = ((y-x)/(y+x))^2 and z = sqrt(f2):
+// Node logarithms are kept among the other node quantities as raw words.
+TAG_DEV double log_word(double x) { return f64_from((u64)log2_fixed(x)); }
+// The same of |x|, with an offset that separates the signs: pairs of one sign
+// see the difference of the logarithms, pairs of two signs leave the series.
+TAG_DEV double log_word_signed(double x) {
+  const u64 b = f64_bits(x);
+  return f64_from((u64)log2_fixed(f64_from(b & 0x7fffffffffffffffull)) + ((b >> 63) << 62));
+}
+TAG_DEV bool is_zero(double x) { return (f64_bits(x) << 1) == 0; }
+TAG_DEV i64 log_difference(double wa, double wb) { return (i64)(f64_bits(wb) - f64_bits(wa)); }
+
+// FP64 forms of the two means, which the diagnostics (tag_means.cu) hold beside
+// the kernels' integer forms.  With f2 = ((y-x)/(y+x))^2 and z = sqrt(f2):
 //   ln_mean(x, y)     = (x+y)/2 * z/atanh(z) = (x+y)/2 * R(f2)
 //   inv_ln_mean(x, y) = 2/(x+y) * atanh(z)/z = 2/(x+y) * Q(f2)
-// Q(f2) = sum_k f2^k/(2k+1) and R = 1/Q.  Below kShortF2 the four-term Taylor
-// forms are exact to < 2e-17 relative.  On the wider ranges [0, F] R and Q are
-// polynomials 1 + f2 (c0 + f2 (c1 + ...)), Chebyshev economizations of their
-// Taylor series (C. Lanczos, J. Math. Phys. 17 (1938) 123-199; coefficients
-// made and checked by csrc/log_mean_series.py): six coefficients each for
-// F = kSeriesF2 = 0.01 (exact to < 5e-19 relative), nine (R) and ten (Q) for
-// F = kLongF2 = 0.09 (< 4e-18).  So they agree with the reference's definition
-// (a 4-term series below f2 = 1e-4, (y-x)/log(y/x) above) to rounding.
-//   rho_mean = ln_mean(xa, xb), inv_beta_mean = inv_ln_mean(ya, yb).
-// Beyond the series range the logarithmic form (y - x)/log(y/x) is evaluated,
-// from per-node logarithms Lx = log x, Ly = log y where the caller supplies
-// them (log(y/x) = Ly - Lx; with |y/x - 1| > 0.2 there the difference is
-// accurate to ~1e-14 relative).  Such a caller guarantees the logarithms are
-// valid whenever a pair can leave the series range (see kLogMeanRange).
+// Below kShortF2 the four-term Taylor forms are exact to < 2e-17 relative.  On
+// the wider ranges [0, F] R and Q are Chebyshev economizations of their Taylor
+// series (C. Lanczos, J. Math. Phys. 17 (1938) 123-199; coefficients made and
+// checked by csrc/log_mean_series.py): six coefficients each for F = kSeriesF2
+// (exact to < 5e-19 relative), nine (R) and ten (Q) for F = kLongF2 (< 4e-18).
 constexpr double kShortF2 = 1.0e-4;
 constexpr double kSeriesF2 = 1.0e-2;
-// An element whose node values x satisfy ((max-min)/(max+min))^2 below this
-// bound never leaves the series range (margin for rounding of f2).
-constexpr double kLogMeanRange = 0.9e-2;
 constexpr double kLongF2 = 0.09;
-// The same bound for kLongF2: a 3.75 km layer of an isothermal 250 K
-// atmosphere reaches f2 = 0.064, so tall shell elements stay in range.
-constexpr double kLongLogRange = 0.08;
 
 TAG_DEV double ln_short_R(double f2) {
   return fma(f2, fma(f2, fma(f2, -44.0 / 945.0, -4.0 / 45.0), -1.0 / 3.0), 1.0);
@@ -118,64 +131,11 @@ TAG_DEV double ln_series_Q_long(double f2) {
   return fma(r, f2, 1.0);
 }
 
-// The rare branch, kept out of line so that the common path is not predicated
-// with its extra reciprocal; the series are evaluated only for a mean that is
-// still in range.
-static __device__ __noinline__ void ln_mean_pair_log(double sx, double dx, double sy, double dy,
-                                                     double f2x, double f2y, double Lxa,
-                                                     double Lxb, double Lya, double Lyb,
-                                                     double& rho_mean, double& inv_beta_mean) {
-  const bool lx = f2x >= kSeriesF2, ly = f2y >= kSeriesF2;
-  const double nx = lx ? dx : 0.5 * sx * ln_series_R(f2x);
-  const double ex = lx ? Lxb - Lxa : 1.0;
-  const double ny = ly ? Lyb - Lya : 2.0 * ln_series_Q(f2y);
-  const double ey = ly ? dy : sy;
-  const double r2 = 1.0 / (ex * ey);
-  rho_mean = nx * ey * r2;
-  inv_beta_mean = ny * ex * r2;
-}
-
-// kNodeLogs: true when the caller supplies per-node logarithms (elements
-// whose pairs often leave the series range, e.g. tall 3D elements); false to
-// take the logarithms inside the rare branch (2D elements rarely need them).
-// kShort: take the four-term series below kShortF2.  Worth it only where a
-// warp's pairs share one direction (the 3D kernel); in the 2D kernel a warp
-// mixes horizontal and vertical pairs and the extra branch diverges.
-// inv_sum_y (optional): 1/(ya + yb), a by-product of the shared reciprocal.
-template <bool kNodeLogs, bool kShort = kNodeLogs>
-TAG_DEV void ln_mean_pair(double xa, double xb, double ya, double yb, double Lxa, double Lxb,
-                          double Lya, double Lyb, double& rho_mean, double& inv_beta_mean,
-                          double* inv_sum_y = nullptr) {
-  const double sx = xa + xb, dx = xb - xa;
-  const double sy = ya + yb, dy = yb - ya;
-  const double r = 1.0 / (sx * sy);
-  const double isx = sy * r, isy = sx * r;
-  if (inv_sum_y) *inv_sum_y = isy;
-  const double tx = dx * isx, ty = dy * isy;
-  const double f2x = tx * tx, f2y = ty * ty;
-  const double fm = fmax(f2x, f2y);
-  if (kShort && fm < kShortF2) {
-    // nearly equal values (e.g. horizontal pairs of a smooth atmosphere)
-    rho_mean = 0.5 * sx * ln_short_R(f2x);
-    inv_beta_mean = 2.0 * isy * ln_short_Q(f2y);
-  } else if (fm < kSeriesF2) {
-    rho_mean = 0.5 * sx * ln_series_R(f2x);
-    inv_beta_mean = 2.0 * isy * ln_series_Q(f2y);
-  } else if constexpr (kNodeLogs) {
-    ln_mean_pair_log(sx, dx, sy, dy, f2x, f2y, Lxa, Lxb, Lya, Lyb, rho_mean, inv_beta_mean);
-  } else {
-    rho_mean = f2x < kSeriesF2 ? 0.5 * sx * ln_series_R(f2x) : dx / log(xb / xa);
-    inv_beta_mean = f2y < kSeriesF2 ? 2.0 * isy * ln_series_Q(f2y) : log(yb / ya) / dy;
-  }
-}
-
 // Out-of-line branch of ln_mean_pair_halved for a pair with f2 at or above
-// the series range lim (kLongF2 or kSeriesF2) in either mean (elements
-// flagged by needs_logs give per-node logarithms Lxa = log(xa/2) ...;
-// kLogsInline takes log(y/x) here instead, for kernels whose elements rarely
-// need them; differences of logarithms do not see the halving).  One
+// the series range lim (kLongF2 or kSeriesF2) in either mean, from the
+// logarithms Lxa = log(xa/2) ... (differences do not see the halving).  One
 // reciprocal serves both means: rho_mean = nx/ex and inv_beta_mean = ny/ey.
-template <bool kLong, bool kLogsInline>
+template <bool kLong>
 static __device__ __noinline__ void ln_mean_pair_halved_log(double sx, double dx, double sy,
                                                             double dy, double f2x, double f2y,
                                                             double Lxa, double Lxb, double Lya,
@@ -186,8 +146,8 @@ static __device__ __noinline__ void ln_mean_pair_halved_log(double sx, double dx
   const double Rx = kLong ? ln_series_R_long(f2x) : ln_series_R(f2x);
   const double Qy = kLong ? ln_series_Q_long(f2y) : ln_series_Q(f2y);
   const double nx = lx ? 2.0 * dx : sx * Rx;
-  const double ny = ly ? (kLogsInline ? log((sy + dy) / (sy - dy)) : Lyb - Lya) : Qy;
-  const double ex = lx ? (kLogsInline ? log((sx + dx) / (sx - dx)) : Lxb - Lxa) : 1.0;
+  const double ny = ly ? Lyb - Lya : Qy;
+  const double ex = lx ? Lxb - Lxa : 1.0;
   const double ey = ly ? 2.0 * dy : sy;
   const double r2 = 1.0 / (ex * ey);
   rho_mean = nx * ey * r2;
@@ -200,13 +160,8 @@ static __device__ __noinline__ void ln_mean_pair_halved_log(double sx, double dx
 // reciprocal per pair.  Each mean takes the form its own f2 selects: the
 // four-term series below kShortF2 (when kShort), else the polynomial on
 // [0, kLongF2] (kLong) or [0, kSeriesF2]; logarithms for both once either f2
-// is beyond that range.  So a pair's result does not depend on which pairs
-// share its warp, and in a tall element's vertical lines, where the density
-// varies and the temperature hardly does, inv_ln_mean keeps its short form.
-// The branch tests compare the bit patterns of the non-negative f2 on the
-// integer pipe.  kShort pays where a warp's pairs share one direction (both
-// element kernels order their pairs so).
-template <bool kShort = true, bool kLong = true, bool kLogsInline = false>
+// is beyond that range.
+template <bool kShort = true, bool kLong = true>
 TAG_DEV void ln_mean_pair_halved(double hxa, double hxb, double hya, double hyb, double Lxa,
                                  double Lxb, double Lya, double Lyb, double& rho_mean,
                                  double& inv_beta_mean) {
@@ -219,7 +174,7 @@ TAG_DEV void ln_mean_pair_halved(double hxa, double hxb, double hya, double hyb,
   const double f2x = tx * tx, f2y = ty * ty;
   const long long bx = __double_as_longlong(f2x), by = __double_as_longlong(f2y);
   if (max(bx, by) >= __double_as_longlong(lim)) {
-    ln_mean_pair_halved_log<kLong, kLogsInline>(sx, dx, sy, dy, f2x, f2y, Lxa, Lxb, Lya, Lyb,
+    ln_mean_pair_halved_log<kLong>(sx, dx, sy, dy, f2x, f2y, Lxa, Lxb, Lya, Lyb,
                                                 rho_mean, inv_beta_mean);
     return;
   }
@@ -234,70 +189,6 @@ TAG_DEV void ln_mean_pair_halved(double hxa, double hxb, double hya, double hyb,
     Q = kLong ? ln_series_Q_long(f2y) : ln_series_Q(f2y);
   rho_mean = sx * R;
   inv_beta_mean = isy * Q;
-}
-
-// Factors of the logarithmic means of a node pair, from the difference d of
-// their log2_fixed node logarithms (b minus a):
-//   ln_mean(xa, xb) = (xa + xb)/2 R,  inv_ln_mean(1/ya, 1/yb) = (ya + yb)/2 Q.
-// Values within a factor of two (every pair of an element that resolves its
-// stratification) take the integer series, whatever their size: no reciprocal,
-// no logarithm, no branch that splits a warp.  Beyond it d itself is the
-// logarithm: |d| >= 1, so its 2^-52 is a relative error of the same size.
-TAG_DEV double log_of_difference(i64 d) { return (double)d * 1.539095918623324e-16; }  // ln2 2^-52
-
-// (Values of opposite sign, which a moisture density may have, give NaN: the
-// logarithm of their ratio.)
-TAG_DEV bool opposite_signs(double a, double b) { return (i64)(f64_bits(a) ^ f64_bits(b)) < 0; }
-static __device__ __noinline__ double ln_factor_far(double xa, double xb, i64 d) {
-  if (opposite_signs(xa, xb)) return f64_from(0x7ff8000000000000ull);
-  return int_div(2.0 * (xb - xa), log_of_difference(d) * (xa + xb));
-}
-static __device__ __noinline__ double inv_ln_factor_far(double ya, double yb, i64 d) {
-  return int_div(2.0 * ya * yb * log_of_difference(d), (yb - ya) * (ya + yb));
-}
-TAG_DEV double ln_factor(double xa, double xb, i64 d) {
-  const u64 a = magnitude(d);
-  return series_in_range(a) ? ln_mean_factor(log_square(a)) : ln_factor_far(xa, xb, d);
-}
-TAG_DEV double inv_ln_factor(double ya, double yb, i64 d) {
-  const u64 a = magnitude(d);
-  return series_in_range(a) ? inv_ln_mean_factor(log_square(a)) : inv_ln_factor_far(ya, yb, d);
-}
-
-// The means of two values themselves (interface kernels): ln_mean(x, y), and
-// inv_ln_mean(1/x, 1/y) from the reciprocals' own values.
-TAG_DEV double ln_mean_of(double x, double y) {
-  return 0.5 * (x + y) * ln_factor(x, y, log2_fixed(y) - log2_fixed(x));
-}
-TAG_DEV double inv_ln_mean_of_reciprocals(double x, double y) {
-  return 0.5 * (x + y) * inv_ln_factor(x, y, log2_fixed(y) - log2_fixed(x));
-}
-
-// Node logarithms are kept among the other node quantities as raw words.
-TAG_DEV double log_word(double x) { return f64_from((u64)log2_fixed(x)); }
-// The same of |x|, with an offset that separates the signs: pairs of one sign
-// see the difference of the logarithms, pairs of two signs leave the series.
-TAG_DEV double log_word_signed(double x) {
-  const u64 b = f64_bits(x);
-  return f64_from((u64)log2_fixed(f64_from(b & 0x7fffffffffffffffull)) + ((b >> 63) << 62));
-}
-TAG_DEV bool is_zero(double x) { return (f64_bits(x) << 1) == 0; }
-TAG_DEV i64 log_difference(double wa, double wb) { return (i64)(f64_bits(wb) - f64_bits(wa)); }
-
-// One logarithmic mean (or its inverse) with its own reciprocal: the series of
-// ln_mean_pair in the common range, the reference's (y-x)/log(y/x) outside.
-TAG_DEV double ln_mean_single(double x, double y) {
-  const double s = x + y, d = y - x;
-  const double t = d / s, f2 = t * t;
-  if (f2 < kSeriesF2) return 0.5 * s * ln_series_R(f2);
-  return d / log(y / x);
-}
-
-TAG_DEV double inv_ln_mean_single(double x, double y) {
-  const double s = x + y, d = y - x;
-  const double t = d / s, f2 = t * t;
-  if (f2 < kSeriesF2) return 2.0 * ln_series_Q(f2) / s;
-  return log(y / x) / d;
 }
 
 // !(x > 0.0) and !isfinite(x) on the integer pipe (the FP64 pipe is the
@@ -316,40 +207,6 @@ TAG_DEV bool not_finite(double x) {
 TAG_DEV double twice(double x) { return f64_from(f64_bits(x) + (1ull << 52)); }
 // x / 2 of a normal number with a normal half
 TAG_DEV double half_of(double x) { return f64_from(f64_bits(x) - (1ull << 52)); }
-
-// Whether the values of one element can push a node pair out of the series
-// range of ln_mean_pair.
-TAG_DEV bool needs_logs(double vmin, double vmax, double range = kLogMeanRange) {
-  const double t = (vmax - vmin) / (vmax + vmin);
-  return t * t >= range;
-}
-
-// needs_logs for the two positive node fields q[node * stride + ka] and
-// q[node * stride + kb] of one element, evaluated by one whole warp; the
-// minima and maxima are taken on the integer pipe (the bit patterns of
-// positive doubles order like their values).  Valid in every lane.
-TAG_DEV bool element_needs_logs(const double* q, int nodes, int stride, int ka, int kb,
-                                double range) {
-  const int lane = threadIdx.x & 31;
-  long long a0 = 0x7fefffffffffffffll, a1 = 0, b0 = 0x7fefffffffffffffll, b1 = 0;
-  for (int node = lane; node < nodes; node += 32) {
-    const long long x = __double_as_longlong(q[node * stride + ka]);
-    const long long y = __double_as_longlong(q[node * stride + kb]);
-    a0 = min(a0, x);
-    a1 = max(a1, x);
-    b0 = min(b0, y);
-    b1 = max(b1, y);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    a0 = min(a0, __shfl_xor_sync(0xffffffffu, a0, o));
-    a1 = max(a1, __shfl_xor_sync(0xffffffffu, a1, o));
-    b0 = min(b0, __shfl_xor_sync(0xffffffffu, b0, o));
-    b1 = max(b1, __shfl_xor_sync(0xffffffffu, b1, o));
-  }
-  return needs_logs(__longlong_as_double(a0), __longlong_as_double(a1), range) ||
-         needs_logs(__longlong_as_double(b0), __longlong_as_double(b1), range);
-}
 
 // Face node (i, j) of face f (0 = xi-, 1 = xi+, 2 = eta-, 3 = eta+) at index l.
 TAG_DEV void face_node(int f, int l, int n, int& i, int& j) {

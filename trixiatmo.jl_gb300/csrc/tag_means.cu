@@ -19,16 +19,17 @@ int mfail(int code, const std::string& msg) {
   return code;
 }
 
-// kind 0: ln_mean_pair (2D kernels: six-coefficient polynomials, logarithms inline)
-// kind 1: ln_mean_pair with per-node logarithms and the four-term short form
-// kind 2: ln_mean_pair_halved (3D energy kernel; halved inputs)
-// kind 3: ln_mean_single / inv_ln_mean_single
+// kind 0: the element kernels' integer forms from node logarithms (ln_factor,
+//         and inv_ln_factor of the reciprocals); kind 3: the interface kernels'
+//         forms of the values themselves
+// kinds 1, 2: the FP64 polynomial forms of halved values with per-node
+//         logarithms, ranges 0.01 (1) and 0.09 (2)
 // kind 4: Stolarsky mean of the potential-temperature kernels (out2 unused)
-// kind 5: ln_mean_pair_halved with the pair as the ln_mean pair and (1, 1) as
-//         the inv_ln_mean pair; kind 6 the other way round
-// kind 7: int_rcp(x) and int_rsqrt(y); kind 8: int_pow(x, gamma) and int_exp(y)
+// kind 5: as kind 2 with the pair as the ln_mean pair and (1, 1) as the
+//         inv_ln_mean pair; kind 6 the other way round
 // out1 = ln_mean(x, y) (kind 4: the Stolarsky mean), out2 = inv_ln_mean(x, y);
 // kinds 5 and 6 return the means of their (x, y) and (1, 1) pairs.
+// kind 7: int_rcp(x) and int_rsqrt(y); kind 8: int_pow(x, gamma) and int_exp(y)
 __global__ void k_eval_means(int kind, long n, const double* __restrict__ x,
                              const double* __restrict__ y, PhysPT2D::Params pt,
                              double* __restrict__ out1, double* __restrict__ out2) {
@@ -37,14 +38,16 @@ __global__ void k_eval_means(int kind, long n, const double* __restrict__ x,
   const double a = x[q], b = y[q];
   double m = 0.0, im = 0.0;
   if (kind == 0) {
-    ln_mean_pair<false>(a, b, a, b, 0.0, 0.0, 0.0, 0.0, m, im);
-  } else if (kind == 1) {
-    const double la = log(a), lb = log(b);
-    ln_mean_pair<true>(a, b, a, b, la, lb, la, lb, m, im);
-  } else if (kind == 2) {
+    const double ia = int_rcp(a), ib = int_rcp(b);
+    m = 0.5 * (a + b) * ln_factor(a, b, log_difference(log_word(a), log_word(b)));
+    im = 0.5 * (ia + ib) * inv_ln_factor(ia, ib, log_difference(log_word(ia), log_word(ib)));
+  } else if (kind == 1 || kind == 2) {
     const double ha = 0.5 * a, hb = 0.5 * b;
     const double la = log(ha), lb = log(hb);
-    ln_mean_pair_halved(ha, hb, ha, hb, la, lb, la, lb, m, im);
+    if (kind == 1)
+      ln_mean_pair_halved<true, false>(ha, hb, ha, hb, la, lb, la, lb, m, im);
+    else
+      ln_mean_pair_halved(ha, hb, ha, hb, la, lb, la, lb, m, im);
   } else if (kind == 5 || kind == 6) {
     const double ha = 0.5 * a, hb = 0.5 * b;
     const double la = log(ha), lb = log(hb), l1 = log(0.5);
@@ -53,8 +56,8 @@ __global__ void k_eval_means(int kind, long n, const double* __restrict__ x,
     else
       ln_mean_pair_halved(0.5, 0.5, ha, hb, l1, l1, la, lb, m, im);
   } else if (kind == 3) {
-    m = ln_mean_single(a, b);
-    im = inv_ln_mean_single(a, b);
+    m = ln_mean_of(a, b);
+    im = inv_ln_mean_of_reciprocals(int_rcp(a), int_rcp(b));
   } else if (kind == 7) {
     m = int_rcp(a);
     im = int_rsqrt(b);
