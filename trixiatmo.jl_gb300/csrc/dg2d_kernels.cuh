@@ -12,6 +12,7 @@
 // Layouts: u[e][j][i][v] (Trixi's u[v, i, j, e]); Ja[e][j][i][d][c]
 // (contravariant_vectors[c, d, i, j, e]); invJ[e][j][i]; sfv[e][face][l][NA].
 #pragma once
+#include "fixed_flux.cuh"
 #include "tag_common.cuh"
 
 namespace tag {
@@ -20,6 +21,7 @@ struct BasisDev {
   double Ds[kMaxNodes * kMaxNodes];  // Dsplit[a * n + b] (row a, column b)
   double winv0, winvN;               // 1 / w_0, 1 / w_N
   double Dh[kMaxNodes * kMaxNodes];  // D_hat[a * n + b] (weak form)
+  FxBasis fx;                        // Dsplit in fixed point
 };
 
 enum VolumeKind : int { kVolFluxDiff = 0, kVolWeak = 1 };

@@ -123,8 +123,9 @@ struct ElemSmem3D {
   static constexpr int oQ = oU + nnn * NV;
   static constexpr int oJa = oQ + nnn * NQ;       // contravariant vectors as stored
   static constexpr int oA = oJa + nnn * 9;        // accumulators [3][nnn][NA]
-  static constexpr int oL = oA + 3 * nnn * NA;    // CFL speeds [3][nnn]
-  static constexpr int per_elem = oL + 3 * nnn;
+  static constexpr int oL = oA;                   // CFL speeds [3][nnn], once the sums are used up
+  static constexpr int oF = oA + 3 * nnn * NA;    // fixed point: FxScale, field maxima
+  static constexpr int per_elem = oF + (Phys::kFixed ? kFxDoubles + (kMxCount + 1) / 2 : 0);
   static size_t bytes(int epb) { return sizeof(double) * (size_t)per_elem * epb + sizeof(BasisDev); }
 };
 
@@ -152,29 +153,91 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
     const double b = reinterpret_cast<const double*>(&basis)[t];
     smem[t] = t < kMaxNodes * kMaxNodes ? 0.5 * b : b;
   }
-  {
-    const double* ug = u + (size_t)e_first * nnn * NV;
-    for (int t = threadIdx.x; t < ne * nnn * NV; t += nthr) {
-      const int el = t / (nnn * NV), r = t % (nnn * NV);
-      base[el * S::per_elem + S::oU + r] = ug[t];
-    }
-    const double* jg = Ja + (size_t)e_first * nnn * 9;
-    for (int t = threadIdx.x; t < ne * nnn * 9; t += nthr) {
-      const int el = t / (nnn * 9), r = t % (nnn * 9);
-      base[el * S::per_elem + S::oJa + r] = jg[t];
-    }
+  if constexpr (Phys::kFixed) {
+    for (int t = threadIdx.x; t < ne * kMxCount; t += nthr)
+      reinterpret_cast<u32*>(base + t / kMxCount * S::per_elem + S::oF + kFxDoubles)[t % kMxCount] = 0;
   }
+  for (int el = 0; el < ne; ++el) {
+    double* eb = base + el * S::per_elem;
+    copy_in(eb + S::oU, u + (size_t)(e_first + el) * nnn * NV, nnn * NV);
+    copy_in(eb + S::oJa, Ja + (size_t)(e_first + el) * nnn * 9, nnn * 9);
+  }
+  copy_in_wait();
   __syncthreads();
 
-  // per-node quantities; zero the accumulators
-  for (int t = threadIdx.x; t < ne * nnn; t += nthr) {
-    const int el = t / nnn, node = t % nnn;
-    double* eb = base + el * S::per_elem;
-    Phys::node_prims(Pp, eb + S::oU + node * NV, eb + S::oQ + node * NQ, bad);
+  // per-node quantities; zero the accumulators; the maxima that the scales of
+  // the element's words are chosen from, 32 nodes per warp
+  if constexpr (Phys::kFixed) {
+    constexpr int CH = (nnn + 31) / 32, CF = (2 * nn + 31) / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = nthr >> 5;
+    for (int task = warp; task < ne * CH; task += nwarps) {
+      const int el = task / CH, node = (task % CH) * 32 + lane;
+      double* eb = base + el * S::per_elem;
+      u32* mx = reinterpret_cast<u32*>(eb + S::oF + kFxDoubles);
+      u32 m[kMxF] = {};
+      if (node < nnn) {
+        double* q = eb + S::oQ + node * NQ;
+        Phys::node_prims(Pp, eb + S::oU + node * NV, q, bad);
+        q[5] -= 0.25 * eb[S::oU + NV - 1];  // phi of the element's first node
 #pragma unroll
-    for (int d = 0; d < 3; ++d)
+        for (int d = 0; d < 3; ++d) {
+          m[kMxV] = max(m[kMxV], high_magnitude(q[1 + d]));
 #pragma unroll
-      for (int v = 0; v < NA; ++v) eb[S::oA + (d * nnn + node) * NA + v] = 0.0;
+          for (int c = 0; c < 3; ++c)
+            m[kMxN + d] = max(m[kMxN + d], high_magnitude(eb[S::oJa + node * 9 + 3 * d + c]));
+#pragma unroll
+          for (int v = 0; v < NA; ++v) eb[S::oA + (d * nnn + node) * NA + v] = 0.0;
+        }
+        // the words' products take densities as positive: bad states leave
+        m[kMxRho] = not_positive(q[0]) ? 0x7ff00000u : high_magnitude(q[0]);
+        m[kMxP] = high_magnitude(q[4]);
+        m[kMxG] = high_magnitude(q[5]);
+        m[kMxX] = not_positive(q[6]) ? 0x7ff00000u : high_magnitude(q[6]);
+      }
+#pragma unroll
+      for (int k = 0; k < kMxF; ++k) warp_max_into(mx + k, m[k]);
+    }
+    // surface fluxes of each direction's two faces
+    for (int task = warp; task < ne * 3 * CF; task += nwarps) {
+      const int el = task / (3 * CF), d = task / CF % 3, k = (task % CF) * 32 + lane;
+      u32* mx = reinterpret_cast<u32*>(base + el * S::per_elem + S::oF + kFxDoubles);
+      u32 m[3] = {};
+      if (k < 2 * nn) {
+        const double* sf = sfv + (((size_t)(e_first + el) * 6 + 2 * d) * nn + k) * NA;
+        m[0] = high_magnitude(sf[0]);
+        m[1] = max(high_magnitude(sf[1]), max(high_magnitude(sf[2]), high_magnitude(sf[3])));
+        m[2] = high_magnitude(sf[4]);
+      }
+#pragma unroll
+      for (int kind = 0; kind < 3; ++kind) warp_max_into(mx + kMxF + 3 * kind + d, m[kind]);
+    }
+    __syncthreads();
+    if (threadIdx.x < ne) {
+      double* f = base + threadIdx.x * S::per_elem + S::oF;
+      *reinterpret_cast<FxScale*>(f) =
+          fx_scale(reinterpret_cast<u32*>(f + kFxDoubles), 3, sb->fx);
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < ne * nnn; t += nthr) {
+      const int el = t / nnn, node = t % nnn;
+      double* eb = base + el * S::per_elem;
+      const FxScale& fs = *reinterpret_cast<const FxScale*>(eb + S::oF);
+      if (!fs.ok) continue;
+      fx_convert_node<3>(eb + S::oQ + node * NQ, fs);
+      double* ja = eb + S::oJa + node * 9;
+#pragma unroll
+      for (int c = 0; c < 9; ++c) ja[c] = f64_from((u64)to_fixed(ja[c], fs.sn[c / 3] - 2));
+    }
+  } else {
+    for (int t = threadIdx.x; t < ne * nnn; t += nthr) {
+      const int el = t / nnn, node = t % nnn;
+      double* eb = base + el * S::per_elem;
+      Phys::node_prims(Pp, eb + S::oU + node * NV, eb + S::oQ + node * NQ, bad);
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+#pragma unroll
+        for (int v = 0; v < NA; ++v) eb[S::oA + (d * nnn + node) * NA + v] = 0.0;
+    }
   }
   __syncthreads();
 
@@ -194,9 +257,24 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
       // line = p1 + n * p2 over the two other directions (ascending)
       const int p1 = line % n, p2 = line / n;
       double* eb = base + el * S::per_elem;
+      const FxScale& fs = *reinterpret_cast<const FxScale*>(eb + S::oF);
+      const bool fixed = Phys::kFixed && fs.ok;
+      FxShift fk{};
+      if (fixed) fk = fx_shift(fs);
       for (int r = 0; r < S::R; ++r) {
         int a, b;
         if (on && round_robin_pair(n, r, slot, a, b)) {
+          i64 Qab = 0;
+          if (fixed) {
+            // ordered so that the weight is positive
+            Qab = sb->fx.Q[a * n + b];
+            if (Qab < 0) {
+              const int c = a;
+              a = b;
+              b = c;
+              Qab = -Qab;
+            }
+          }
           int na_, nb_;
           if (d == 0) {
             na_ = (p2 * n + p1) * n + a;
@@ -210,6 +288,23 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
           }
           const double* ja_a = eb + S::oJa + na_ * 9 + 3 * d;
           const double* ja_b = eb + S::oJa + nb_ * 9 + 3 * d;
+          if (fixed) {
+            if constexpr (Phys::kFixed) {
+              const i64* wa = reinterpret_cast<const i64*>(eb + S::oQ + na_ * NQ);
+              const i64* wb = reinterpret_cast<const i64*>(eb + S::oQ + nb_ * NQ);
+              i64 Fa[NA], Fb[NA];
+              fx_energy_pair<3>(wa, wb, reinterpret_cast<const i64*>(ja_a),
+                                reinterpret_cast<const i64*>(ja_b), Qab, fk, fs.kq[d], Fa,
+                                Fb);
+              i64* ca = reinterpret_cast<i64*>(eb + S::oA + (d * nnn + na_) * NA);
+              i64* cb = reinterpret_cast<i64*>(eb + S::oA + (d * nnn + nb_) * NA);
+#pragma unroll
+              for (int v = 0; v < NA; ++v) {
+                ca[v] += Fa[v];
+                cb[v] -= Fb[v];
+              }
+            }
+          } else {
           const double nrm[3] = {ja_a[0] + ja_b[0], ja_a[1] + ja_b[1], ja_a[2] + ja_b[2]};
           double Fa[NA], Fb[NA];
           Phys::volume_pair(Pp, eb + S::oQ + na_ * NQ, eb + S::oQ + nb_ * NQ, nrm, Fa, Fb);
@@ -220,6 +315,7 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
           for (int v = 0; v < NA; ++v) {
             ca[v] = fma(dab, Fa[v], ca[v]);
             cb[v] = fma(dba, Fb[v], cb[v]);
+          }
           }
         }
         __syncwarp();
@@ -237,6 +333,18 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
           const double* sf =
               sfv + ((((size_t)(e_first + el) * 6 + 2 * d + end) * n + p2) * n + p1) * NA;
           double* c = eb + S::oA + (d * nnn + nd) * NA;
+          if (fixed) {
+            // unweighted: 1/w joins with the node's volume terms
+            i64* w64 = reinterpret_cast<i64*>(c);
+            const int sd = fx_direction_scale(fs, d) + sb->fx.sq;
+#pragma unroll
+            for (int v = 0; v < NA; ++v)
+              w64[v] += fx_surface(sf[v],
+                                   fx_kind_scale(fs, v == 0 ? 0 : v < NA - 1 ? 1 : 2) + sd +
+                                       (Phys::kLastHalved && v == NA - 1),
+                                   sb->fx.S[end]);
+            continue;
+          }
 #pragma unroll
           for (int v = 0; v < NA; ++v)
             c[v] = fma(sf[v], Phys::kLastHalved && v == NA - 1 ? half_of(w) : w, c[v]);
@@ -246,71 +354,77 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
   }
   __syncthreads();
 
-  // per (node, variable): direction sums (surface integral included),
-  // Jacobian, sources, stage update
-  for (int t = threadIdx.x; t < ne * nnn * NA; t += nthr) {
-    const int el = t / (nnn * NA), r = t % (nnn * NA);
-    const int node = r / NA, v = r % NA;
+  // per node: direction sums (surface integral included), Jacobian, sources,
+  // stage update; the new state (or the time derivative) takes the old
+  // state's place in shared memory and leaves as one block per element
+  for (int t = threadIdx.x; t < ne * nnn; t += nthr) {
+    const int el = t / nnn, node = t % nnn;
     const int e = e_first + el;
     double* eb = base + el * S::per_elem;
-    const double acc = eb[S::oA + (0 * nnn + node) * NA + v] +
-                       eb[S::oA + (1 * nnn + node) * NA + v] + eb[S::oA + (2 * nnn + node) * NA + v];
     const size_t gq = (size_t)e * nnn + node;
-    const double ij = Phys::kLastHalved && v == NA - 1 ? twice(invJ[gq]) : invJ[gq];
-    const double dv = acc * (-ij) + Phys::source(Pp, eb + S::oU + node * NV, v);
-    if (not_finite(dv)) bad |= TAG_S_NAN;
-    if (MODE == kModeRhs) {
-      du[gq * NV + v] = dv;
+    const double ij = invJ[gq];
+    double acc[NA];
+    const double* A = eb + S::oA + node * NA;
+    const FxScale& fs = *reinterpret_cast<const FxScale*>(eb + S::oF);
+    if (Phys::kFixed && fs.ok) {
+      // each direction's sum over its quadrature weight
+      const int at[3] = {node % n, node / n % n, node / nn};
+      const int sd[3] = {fx_direction_scale(fs, 0), fx_direction_scale(fs, 1),
+                         fx_direction_scale(fs, 2)};
+#pragma unroll
+      for (int v = 0; v < NA; ++v) {
+        int scale;
+        const i64 tot = fx_weighted_sum<3>(reinterpret_cast<const i64*>(A + v), nnn * NA, sb->fx.W,
+                                           at, sd, scale);
+        acc[v] = from_fixed(tot, fx_kind_scale(fs, v == 0 ? 0 : v < NA - 1 ? 1 : 2) + scale +
+                                     sb->fx.sq + sb->fx.kw);
+      }
     } else {
-      const size_t kq = gq * NA + v;
+#pragma unroll
+      for (int v = 0; v < NA; ++v) acc[v] = A[v] + A[nnn * NA + v] + A[2 * nnn * NA + v];
+    }
+    double* un = eb + S::oU + node * NV;
+    double dv[NA];
+#pragma unroll
+    for (int v = 0; v < NA; ++v) {
+      dv[v] = acc[v] * -(Phys::kLastHalved && v == NA - 1 ? twice(ij) : ij);
+      if (v == 1 || v == 2) dv[v] += Phys::source(Pp, un, v);
+      if (not_finite(dv[v])) bad |= TAG_S_NAN;
+    }
+    if (MODE == kModeRhs) {
+#pragma unroll
+      for (int v = 0; v < NV; ++v) un[v] = v < NA ? dv[v] : 0.0;
+    } else {
       const double dt = st.dt[st.member ? st.member[e] : 0];
-      const double un = stage_value(st, eb[S::oU + node * NV + v], kreg + kq, dt, dv);
-      // all reads of this node's old state (the Coriolis source) precede the
-      // barrier below; write the new value to global memory now and to
-      // shared memory after it
-      u[gq * NV + v] = un;
-      eb[S::oA + node * NA + v] = un;  // stage the new value (direction-0 slot is free)
+#pragma unroll
+      for (int v = 0; v < NA; ++v)
+        un[v] = stage_value(st, un[v], kreg + gq * NA + v, dt, dv[v]);
     }
   }
-  if (MODE == kModeRhs) {
-    for (int t = threadIdx.x; t < ne * nnn * (NV - NA); t += nthr) {
-      const int el = t / (nnn * (NV - NA)), r = t % (nnn * (NV - NA));
-      const int node = r / (NV - NA), v = NA + r % (NV - NA);
-      du[((size_t)(e_first + el) * nnn + node) * NV + v] = 0.0;
-    }
-  }
+  __syncthreads();
+  for (int el = 0; el < ne; ++el)
+    copy_out((MODE == kModeRhs ? du : u) + (size_t)(e_first + el) * nnn * NV,
+             base + el * S::per_elem + S::oU, nnn * NV);
   if (MODE == kModeStage && st.max_speed != nullptr) {
-    __syncthreads();
     for (int t = threadIdx.x; t < ne * nnn; t += nthr) {
       const int el = t / nnn, node = t % nnn;
       double* eb = base + el * S::per_elem;
-      double un[NV];
-#pragma unroll
-      for (int v = 0; v < NA; ++v) un[v] = eb[S::oA + node * NA + v];
-#pragma unroll
-      for (int v = NA; v < NV; ++v) un[v] = eb[S::oU + node * NV + v];
       double lam[3];
-      Phys::max_speeds(Pp, un, lam);
-      const double* ja = eb + S::oJa + node * 9;
-      const double ij = fabs(invJ[(size_t)(e_first + el) * nnn + node]);
+      Phys::max_speeds(Pp, eb + S::oU + node * NV, lam);
+      const size_t gq = (size_t)(e_first + el) * nnn + node;
+      const double* ja = Phys::kFixed ? Ja + gq * 9 : eb + S::oJa + node * 9;
+      const double ij = fabs(invJ[gq]);
 #pragma unroll
       for (int d = 0; d < 3; ++d)
         eb[S::oL + d * nnn + node] =
             fabs(ja[3 * d] * lam[0] + ja[3 * d + 1] * lam[1] + ja[3 * d + 2] * lam[2]) * ij;
     }
+    // the step's result to the registered sink (host memory over the host link)
+    if (st.sink != nullptr)
+      for (int el = 0; el < ne; ++el)
+        copy_out(st.sink + (size_t)(e_first + el) * nnn * NV, base + el * S::per_elem + S::oU,
+                 nnn * NV);
     __syncthreads();
-    // the step's result to the registered sink (host memory over the host
-    // link): each element's state is one contiguous block, stored by
-    // consecutive threads at consecutive addresses
-    if (st.sink != nullptr) {
-      double* o = st.sink + (size_t)e_first * nnn * NV;
-      for (int t = threadIdx.x; t < ne * nnn * NV; t += nthr) {
-        const int el = t / (nnn * NV), r = t % (nnn * NV);
-        const int node = r / NV, v = r % NV;
-        const double* eb = base + el * S::per_elem;
-        o[t] = v < NA ? eb[S::oA + node * NA + v] : eb[S::oU + node * NV + v];
-      }
-    }
     // one warp per element: the per-direction maxima over its nodes on the
     // integer pipe (the speeds are non-negative, and the bit patterns of
     // non-negative doubles order like their values), then summed

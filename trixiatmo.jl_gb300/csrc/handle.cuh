@@ -37,6 +37,13 @@ struct Ops;
 // Threads of an element-kernel CTA: `items` work items split `div` ways,
 // rounded up to whole warps.
 inline int cta_threads(int items, int div) { return ((items + div - 1) / div + 31) / 32 * 32; }
+// Tiles of the 3D kernels: div 1 to 3 as above; 4 to 6 the same rounded up to
+// whole groups of four warps, one for each of the SM's sub-partitions (their
+// registers are separate, so an odd warp can cost a CTA's place on all four).
+inline int tile_threads(int items, int div) {
+  const int t = cta_threads(items, div > 3 ? div - 3 : div);
+  return div > 3 ? (t + 127) / 128 * 128 : t;
+}
 
 struct tag_handle_s {
   int eq = 0, n = 0, nelem = 0, nif = 0, nbd = 0, nv = 0, na = 0;
@@ -102,7 +109,7 @@ struct tag_handle_s {
   bool speed_valid = false;
   int epb = 0;
   // threads of a CTA = its elements' work items / tile_div, rounded up to
-  // whole warps (1 or 2: one or two items per thread and phase)
+  // whole warps (one to three items per thread and phase; 3D: tile_threads)
   int tile_div = 1;
   const Ops* ops = nullptr;
   // analysis (allocated by the first analysis call)

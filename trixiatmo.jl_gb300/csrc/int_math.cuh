@@ -100,6 +100,12 @@ TAG_HD i64 smulhi64(i64 a, i64 b) {
   return (i64)(((__int128)a * b) >> 64);
 #endif
 }
+// High word of an unsigned product without the low words' part: the error is
+// in [-3, 0] and -1.25 on average.
+TAG_HD u64 umul_high(u64 a, u64 b) {
+  const u32 ah = (u32)(a >> 32), al = (u32)a, bh = (u32)(b >> 32), bl = (u32)b;
+  return (u64)ah * bh + mulhi32(ah, bl) + mulhi32(al, bh);
+}
 // (a b) >> 32 of a 64-bit and a 32-bit word
 TAG_HD u64 mulhi64x32(u64 a, u32 b) {
   return (u64)(u32)(a >> 32) * b + mulhi32((u32)a, b);
@@ -392,48 +398,71 @@ TAG_HD double int_log2_ratio(double x, i64 ref_q58) {
 // by the OR of their magnitudes.
 TAG_HD u64 magnitude(i64 d) { return d < 0 ? 0ull - (u64)d : (u64)d; }
 TAG_HD bool series_in_range(u64 a) { return (u32)(a >> 32) < (1u << 20); }
-TAG_HD u64 log_square(u64 a) { return mulhi64(a << 12, a << 12); }
+TAG_HD u64 log_square(u64 a) { return umul_high(a << 12, a << 12); }
 
 // 1 - c for c (Q0.64) below 1/2, rounded to 53 bits: numbers just below 1 are
 // spaced by 2^-53, so the subtraction is one of the bit patterns.
 TAG_HD double one_minus(u64 c) { return f64_from(0x3ff0000000000000ull - ((c + 1024u) >> 11)); }
 
-// tanh(x)/x at x = d ln2 / 2: ln_mean(u, v) = (u + v)/2 times it, with
+// 1 - tanh(x)/x (Q0.64) at x = d ln2 / 2: ln_mean(u, v) = (u + v)/2 tanh(x)/x, with
 // d = log2(v) - log2(u) (ln_mean = (u + v)/2 t/atanh(t) and t = tanh(x)).
 // Taylor series in z, the first seven terms in integers, six more in binary32
 // (below 2^-35 together).  No reciprocal and no branch on the size of d.
-TAG_HD double ln_mean_factor(u64 z) {
+TAG_HD u64 ln_mean_deficit(u64 z) {
   const float zf = (float)(u32)(z >> 32) * 2.3283064365386963e-10f;
   const float P = fmaf(zf, -fmaf(zf, -fmaf(zf, -fmaf(zf, -TAG_LN_B4, TAG_LN_B3), TAG_LN_B2),
                                  TAG_LN_B1), TAG_LN_B0);
-  u64 p = (u64)f32_to_int(P * 2.305843009213694e18f) << 3;  // Q.61 -> Q.64
-  p = TAG_LN_A6 - mulhi64(z, p);
-  p = TAG_LN_A5 - mulhi64(z, p);
-  p = TAG_LN_A4 - mulhi64(z, p);
-  p = TAG_LN_A3 - mulhi64(z, p);
-  p = TAG_LN_A2 - mulhi64(z, p);
-  p = TAG_LN_A1 - mulhi64(z, p);
-  p = TAG_LN_A0 - mulhi64(z, p);
-  return one_minus(mulhi64(z, p));
+  // the small coefficients in 32-bit words (the tail and A6 in Q.61, the product
+  // under A4 in Q.56): below 2^-57 of the result at z = 1
+  const u32 zh = (u32)(z >> 32);
+  const u32 p6 = (u32)(TAG_LN_A6 >> 3) - mulhi32(zh, (u32)f32_to_int(P * 2.305843009213694e18f));
+  u64 p = TAG_LN_A5 - ((u64)mulhi32(zh, p6) << 3);
+  p = TAG_LN_A4 - ((u64)mulhi32(zh, (u32)(p >> 8)) << 8);
+  p = TAG_LN_A3 - umul_high(z, p);
+  p = TAG_LN_A2 - umul_high(z, p);
+  p = TAG_LN_A1 - umul_high(z, p);
+  p = TAG_LN_A0 - umul_high(z, p);
+  return umul_high(z, p);
 }
 
-// x/sinh(x) at x = d ln2: inv_ln_mean(1/u, 1/v) = (u + v)/2 times it (with
+// 1 - x/sinh(x) (Q0.64) at x = d ln2: inv_ln_mean(1/u, 1/v) = (u + v)/2 x/sinh(x) (with
 // r = v/u: log(r)/(1/u - 1/v) = u v log(r)/(v - u), and (u + v)(v - u)/(2 u v)
 // = sinh(log r)).  So the mean of reciprocals needs no reciprocal.
-TAG_HD double inv_ln_mean_factor(u64 z) {
+TAG_HD u64 inv_ln_mean_deficit(u64 z) {
   const float zf = (float)(u32)(z >> 32) * 2.3283064365386963e-10f;
   const float P = fmaf(zf, -fmaf(zf, -fmaf(zf, -fmaf(zf, -TAG_INV_B4, TAG_INV_B3), TAG_INV_B2),
                                  TAG_INV_B1), TAG_INV_B0);
-  u64 p = (u64)f32_to_int(P * 2.305843009213694e18f) << 3;
-  p = TAG_INV_A6 - mulhi64(z, p);
-  p = TAG_INV_A5 - mulhi64(z, p);
-  p = TAG_INV_A4 - mulhi64(z, p);
-  p = TAG_INV_A3 - mulhi64(z, p);
-  p = TAG_INV_A2 - mulhi64(z, p);
-  p = TAG_INV_A1 - mulhi64(z, p);
-  p = TAG_INV_A0 - mulhi64(z, p);
-  return one_minus(mulhi64(z, p));
+  // the small coefficients in 32-bit words (the tail and A6 in Q.61, the product
+  // under A4 in Q.56): below 2^-57 of the result at z = 1
+  const u32 zh = (u32)(z >> 32);
+  const u32 p6 = (u32)(TAG_INV_A6 >> 3) - mulhi32(zh, (u32)f32_to_int(P * 2.305843009213694e18f));
+  u64 p = TAG_INV_A5 - ((u64)mulhi32(zh, p6) << 3);
+  p = TAG_INV_A4 - ((u64)mulhi32(zh, (u32)(p >> 8)) << 8);
+  p = TAG_INV_A3 - umul_high(z, p);
+  p = TAG_INV_A2 - umul_high(z, p);
+  p = TAG_INV_A1 - umul_high(z, p);
+  p = TAG_INV_A0 - umul_high(z, p);
+  return umul_high(z, p);
 }
+
+// The same for z below 2^-11 (values within 1.5 %: the horizontal pairs of a
+// smooth atmosphere): three terms, the inner two in 32-bit words (error below
+// 2^-57); 40 instructions instead of 85.
+constexpr u64 kShortZ = 1ull << 53;
+TAG_HD u64 short_deficit(u64 z, u64 a0, u32 a1_q39, u32 a2_q40) {
+  const u32 zn = (u32)(z >> 21);                             // z 2^11 in Q0.32
+  const u32 p1 = a1_q39 - (mulhi32(zn, a2_q40) >> 12);       // a1 - z a2, Q.39
+  return umul_high(z, a0 - (((u64)zn * p1) >> 18));          // a0 - z p1, Q.64
+}
+TAG_HD u64 ln_mean_deficit_short(u64 z) {
+  return short_deficit(z, TAG_LN_A0, (u32)(TAG_LN_A1 >> 25), (u32)(TAG_LN_A2 >> 24));
+}
+TAG_HD u64 inv_ln_mean_deficit_short(u64 z) {
+  return short_deficit(z, TAG_INV_A0, (u32)(TAG_INV_A1 >> 25), (u32)(TAG_INV_A2 >> 24));
+}
+
+TAG_HD double ln_mean_factor(u64 z) { return one_minus(ln_mean_deficit(z)); }
+TAG_HD double inv_ln_mean_factor(u64 z) { return one_minus(inv_ln_mean_deficit(z)); }
 
 // A mean's factor 1 - z (a0 + z (a1 + ...)) with coefficients of run-time
 // parameters, in the same form (any signs; seven Q0.63 words, six binary32).
@@ -443,7 +472,7 @@ struct EvenSeries {
   float b[6];
   int ok;
 };
-TAG_HD double even_factor(const EvenSeries& s, u64 z) {
+TAG_HD u64 even_deficit(const EvenSeries& s, u64 z) {
   const i64 zq = (i64)(z >> 1);  // Q0.63
   const float zf = (float)(u32)(z >> 32) * 2.3283064365386963e-10f;
   float P = s.b[5];
@@ -452,8 +481,9 @@ TAG_HD double even_factor(const EvenSeries& s, u64 z) {
   i64 p = (i64)f32_to_int(P * 1.152921504606847e18f) << 3;  // Q.60 -> Q.63
 #pragma unroll
   for (int k = 6; k >= 0; --k) p = s.a[k] + (smulhi64(zq, p) << 1);
-  return one_minus((u64)(smulhi64(zq, p) << 2));
+  return (u64)(smulhi64(zq, p) << 2);
 }
+TAG_HD double even_factor(const EvenSeries& s, u64 z) { return one_minus(even_deficit(s, z)); }
 
 // The Stolarsky mean S(u, v) = (g-1)/g (v^g - u^g)/(v^(g-1) - u^(g-1)) is
 // (u + v)/2 times sinh(g x) (g-1)/g / (sinh((g-1) x) cosh(x)), x = log(v/u)/2:

@@ -19,7 +19,7 @@ struct OpsImpl3D {
                      double) {
     const int epb = h->epb > 0 ? h->epb : 1;
     const int blocks = (h->nelem + epb - 1) / epb;
-    const int threads = std::min(cap(), cta_threads(epb * S::TPE, h->tile_div));
+    const int threads = std::min(cap(), tile_threads(epb * S::TPE, h->tile_div));
     const size_t smem = S::bytes(epb);
     StageArgs st{};
     st.member = h->d_member;
@@ -64,7 +64,7 @@ struct OpsImpl3D {
     static int c = 1024;
     return c;
   }
-  static int max_threads() { return cap(); }
+  static int max_threads() { return 1024; }  // of a tile; the kernel strides over its work
   static size_t smem_bytes(int epb) { return S::bytes(epb); }
   static const Ops* get() {
     static const Ops ops{&interface, &element, &max_speed, &load_state, &init, &smem_bytes,

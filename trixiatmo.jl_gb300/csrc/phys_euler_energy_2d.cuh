@@ -16,6 +16,7 @@ struct PhysEnergy2D {
   static constexpr int NQ = 9;
   // volume_pair returns half the energy flux (the kernel doubles the node sums)
   static constexpr bool kLastHalved = true;
+  static constexpr bool kFixed = false;  // volume integral in FP64
   static constexpr bool kHasSources = false;
   static constexpr bool kSurfaceNoncons = false;  // surface flux only (flux_zero)
 

@@ -11,11 +11,12 @@ namespace tag {
 struct PhysEnergy3D {
   static constexpr int NV = 6;
   static constexpr int NA = 5;
-  // rho/2, v1/2, v2/2, v3/2, p/2, phi/4, theta = (p/rho) / (4 (gamma - 1)),
+  // rho/2, v1/2, v2/2, v3/2, p/2, phi/4 (less the first node's), theta = (p/rho) / (4 (gamma - 1)),
   // log2(rho), log2(p/rho) (log2_fixed words; odd stride)
   static constexpr int NQ = 9;
   // volume_pair returns half the energy flux (the kernel doubles the node sums)
   static constexpr bool kLastHalved = true;
+  static constexpr bool kFixed = true;  // volume integral in words (fixed_flux.cuh)
   static constexpr bool kHasSources = true;  // Coriolis, added per (node, variable)
 
   struct Params {
@@ -66,7 +67,8 @@ struct PhysEnergy3D {
   //   f1 (v_a.v_b / 4 + mean(p/rho) / (2 (gamma - 1)) +- g) + (p_a vn_b + p_b vn_a) / 4.
   // The FP64 pipe bounds the kernel, so the reciprocal and the two series of
   // the means go to the integer pipe (int_math.cuh): the right-hand side of
-  // the 2,654,208-node shell at polydeg 5 went from 3.48 to 2.37 ms.
+  // the 2,654,208-node shell at polydeg 5 went from 3.48 to 2.32 ms.  Elements
+  // in range take fx_energy_pair (fixed_flux.cuh) instead of this form.
   TAG_DEV static void volume_pair(const Params& P, const double* qa, const double* qb,
                                   const double* nrm, double* Fa, double* Fb) {
     const double R = ln_factor(qa[0], qb[0], log_difference(qa[7], qb[7]));

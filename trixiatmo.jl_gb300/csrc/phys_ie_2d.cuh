@@ -18,6 +18,7 @@ struct PhysIE2D {
   // log2(rho), log2(p/rho) (log2_fixed words), pad (odd stride)
   static constexpr int NQ = 9;
   static constexpr bool kLastHalved = false;
+  static constexpr bool kFixed = false;  // volume integral in FP64
   static constexpr bool kHasSources = false;
   static constexpr bool kSurfaceNoncons = true;
 

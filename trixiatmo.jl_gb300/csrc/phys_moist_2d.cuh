@@ -14,6 +14,7 @@ struct PhysMoist2D {
   // log2 of rho_qd, rho_qv, rho_ql and T (words), (pad: odd stride)
   static constexpr int NQ = 13;
   static constexpr bool kLastHalved = false;
+  static constexpr bool kFixed = false;  // volume integral in FP64
   static constexpr bool kHasSources = true;
   static constexpr bool kSurfaceNoncons = false;  // surface flux only (flux_zero)
 

@@ -22,6 +22,7 @@ struct PhysPT2D {
   // log2(rho_theta) (log2_fixed words; odd stride)
   static constexpr int NQ = 9;
   static constexpr bool kLastHalved = false;
+  static constexpr bool kFixed = false;  // volume integral in FP64
   // MountainWaveSetup's Rayleigh damping when set (Params::mountain)
   static constexpr bool kHasSources = true;
   // surface flux (FluxLMARS(c), flux_zero) or (flux_ec, a nonconservative

@@ -19,6 +19,7 @@ struct PhysPT3D {
   // value (phys_pt_2d.cuh), log2(rho), log2(rho_theta), (pad: odd stride)
   static constexpr int NQ = 11;
   static constexpr bool kLastHalved = false;
+  static constexpr bool kFixed = false;  // volume integral in FP64
   static constexpr bool kHasSources = true;  // Coriolis, per (node, variable)
 
   struct Params {

@@ -72,6 +72,7 @@ struct PhysRainy2D {
   // rho_vapour and T (words; odd stride)
   static constexpr int NQ = 13;
   static constexpr bool kLastHalved = false;
+  static constexpr bool kFixed = false;  // volume integral in FP64
   static constexpr bool kHasSources = true;
   static constexpr bool kSurfaceNoncons = false;  // surface flux only (flux_zero)
 

@@ -63,6 +63,7 @@ void load_basis(BasisDev& b, const double* dsplit_colmajor, const double* w, int
     for (int c = 0; c < n; ++c) b.Ds[a * n + c] = dsplit_colmajor[a + n * c];
   b.winv0 = 1.0 / w[0];
   b.winvN = 1.0 / w[n - 1];
+  load_fixed_basis(b.fx, b.Ds, w, n);
   // D_hat = -M^{-1} D^T M from D_split = 2 D - M^{-1} B:
   //   D[a][c] = (Ds[a][c] + (M^{-1} B)[a][c]) / 2,  D_hat[a][c] = -D[c][a] w_c / w_a
   for (int a = 0; a < n; ++a)
@@ -147,7 +148,7 @@ int build_graph(tag_handle h) {
 // Times the element kernel (rhs mode, on the state `u`) for candidate tiles
 // and keeps the fastest: elements per CTA (the shared-memory tile, each
 // element's state, metric terms and accumulators staged once) times threads
-// per CTA (one or two work items per thread and phase).  The trial launches'
+// per CTA (one to three work items per thread and phase).  The trial launches'
 // status bits are discarded.
 int autotune(tag_handle h, const double* u) {
   if (h->epb > 0) return TAG_OK;
@@ -162,11 +163,13 @@ int autotune(tag_handle h, const double* u) {
   int best = 1, best_div = 1;
   float best_ms = 1e30f;
   const int cands[] = {1, 2, 3, 4, 6, 8, 12, 16};
-  for (int trial = 0; trial < 16; ++trial) {
-    const int c = cands[trial >> 1], div = 1 + (trial & 1);
+  const int ndiv = h->dim == 3 ? 6 : 2;
+  for (int trial = 0; trial < 8 * ndiv; ++trial) {
+    const int c = cands[trial / ndiv], div = 1 + trial % ndiv;
     if ((size_t)h->ops->smem_bytes(c) > (size_t)max_smem) continue;
     if (c * h->ops->threads_per_element > h->ops->max_threads() && c > 1) continue;
-    if (div == 2 && c * h->ops->threads_per_element < 128) continue;
+    const int share = (div - 1) % 3 + 1;  // work items per thread
+    if (share > 1 && c * h->ops->threads_per_element < 64 * share) continue;
     h->epb = c;
     h->tile_div = div;
     double* uu = const_cast<double*>(u);
@@ -1486,7 +1489,8 @@ int tag_get_cta_threads(tag_handle h, int32_t* threads) {
   if (!h || !threads) return fail(TAG_E_INVALID, "null argument");
   const int epb = h->epb > 0 ? h->epb : 1;
   *threads = h->ops ? std::min(h->ops->max_threads(),
-                               cta_threads(epb * h->ops->threads_per_element, h->tile_div))
+                               (h->dim == 3 ? tile_threads : cta_threads)(
+                                   epb * h->ops->threads_per_element, h->tile_div))
                     : 0;
   return TAG_OK;
 }

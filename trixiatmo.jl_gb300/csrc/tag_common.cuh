@@ -219,6 +219,29 @@ TAG_DEV void face_node(int f, int l, int n, int& i, int& j) {
   }
 }
 
+// Block copies of `count` doubles by the threads of a CTA.  copy_in is
+// asynchronous (wait with copy_in_wait before the barrier): 16 bytes per
+// instruction where both sides allow it, 8 otherwise; no registers between.
+TAG_DEV void copy_in(double* smem, const double* __restrict__ g, int count) {
+  const u32 s = (u32)__cvta_generic_to_shared(smem);
+  if (((((size_t)g) | s | (count * 8u)) & 15u) == 0) {
+    for (int t = threadIdx.x; t < count / 2; t += blockDim.x)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s + 16 * t), "l"(g + 2 * t));
+  } else {
+    for (int t = threadIdx.x; t < count; t += blockDim.x)
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(s + 8 * t), "l"(g + t));
+  }
+}
+TAG_DEV void copy_in_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+TAG_DEV void copy_out(double* __restrict__ g, const double* smem, int count) {
+  if (((((size_t)g) | (size_t)smem | (count * 8u)) & 15u) == 0) {
+    for (int t = threadIdx.x; t < count / 2; t += blockDim.x)
+      reinterpret_cast<double2*>(g)[t] = reinterpret_cast<const double2*>(smem)[t];
+  } else {
+    for (int t = threadIdx.x; t < count; t += blockDim.x) g[t] = smem[t];
+  }
+}
+
 // Atomic max of a non-negative double stored as its IEEE bit pattern.
 TAG_DEV void atomic_max_nonneg(double* addr, double v) {
   atomicMax(reinterpret_cast<unsigned long long*>(addr),

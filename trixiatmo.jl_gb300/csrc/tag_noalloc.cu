@@ -137,7 +137,7 @@ int launch_noalloc(const tag_config* cfg, const PhysEnergy2D::Params& P, const B
   if (rc) return rc;
   int epb = 1;
   while (epb < 16 && S::bytes(epb + 1) <= 48 * 1024 && (epb + 1) * S::TPE <= 1024) ++epb;
-  const int threads = std::min(cap, epb * S::TPE);
+  const int threads = std::min(cap, (epb * S::TPE + 31) / 32 * 32);  // whole warps
   StageArgs st{};
   k_element<Phys, n, kModeRhs><<<(nelem + epb - 1) / epb, threads, S::bytes(epb), s>>>(
       P, basis, const_cast<double*>(u), du, nullptr, cfg->contravariant_vectors,
@@ -199,6 +199,7 @@ int tag_rhs_noalloc(const tag_config* cfg, const double* u, double* du, void* st
     for (int c = 0; c < n; ++c) basis.Ds[a * n + c] = cfg->derivative_split[a + n * c];
   basis.winv0 = 1.0 / cfg->weights[0];
   basis.winvN = 1.0 / cfg->weights[n - 1];
+  load_fixed_basis(basis.fx, basis.Ds, cfg->weights, n);
   switch (n) {
     case 2: rc = launch_noalloc<2>(cfg, P, basis, u, du, s, sfv, status); break;
     case 3: rc = launch_noalloc<3>(cfg, P, basis, u, du, s, sfv, status); break;
