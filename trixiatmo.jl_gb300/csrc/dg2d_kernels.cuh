@@ -185,7 +185,8 @@ struct ElemSmem {
   static constexpr int oC = oJa + nn * 4;        // slots [2][nn][n - 1][NA], one per partner
   static constexpr int oL = oC + 2 * nn * (n - 1) * NA;  // CFL speeds [2][nn]
   static constexpr int oS = oL + 2 * nn;          // sources [nn][NA]
-  static constexpr int per_elem = oS + (Phys::kHasSources ? nn * NA : 0);
+  static constexpr int oF = oS + (Phys::kHasSources ? nn * NA : 0);  // fixed point: FxScale
+  static constexpr int per_elem = (oF + (Phys::kFixed ? kFxDoubles : 0) + 1) / 2 * 2;
   static size_t bytes(int epb) { return sizeof(double) * (size_t)per_elem * epb + sizeof(BasisDev); }
 };
 
@@ -208,21 +209,15 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
   unsigned bad = 0;
 
   // --- phase 0: basis + element data to shared memory
-  for (int t = threadIdx.x; t < (int)(sizeof(BasisDev) / sizeof(double)); t += nthr)
-    smem[t] = reinterpret_cast<const double*>(&basis)[t];
-  {
-    const double* ug = u + (size_t)e_first * nn * NV;
-    for (int t = threadIdx.x; t < ne * nn * NV; t += nthr) {
-      const int el = t / (nn * NV), r = t % (nn * NV);
-      base[el * S::per_elem + S::oU + r] = ug[t];
-    }
-    // contravariant vectors are kept halved: the pair normal is the sum
-    const double* jg = Ja + (size_t)e_first * nn * 4;
-    for (int t = threadIdx.x; t < ne * nn * 4; t += nthr) {
-      const int el = t / (nn * 4), r = t % (nn * 4);
-      base[el * S::per_elem + S::oJa + r] = 0.5 * jg[t];
-    }
+  // (the pair normal is the sum of two contravariant vectors, twice the average
+  // the two-point fluxes take; they are linear in it, so D_split is halved)
+  for (int t = threadIdx.x; t < (int)(sizeof(BasisDev) / sizeof(double)); t += nthr) {
+    const double b = reinterpret_cast<const double*>(&basis)[t];
+    smem[t] = t < kMaxNodes * kMaxNodes ? 0.5 * b : b;
   }
+  copy_in_blocks(base + S::oU, S::per_elem, u + (size_t)e_first * nn * NV, nn * NV, ne);
+  copy_in_blocks(base + S::oJa, S::per_elem, Ja + (size_t)e_first * nn * 4, nn * 4, ne);
+  copy_in_wait();
   __syncthreads();
 
   // --- phase 1: per-node primitives
@@ -230,8 +225,63 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
     const int el = t / nn, node = t % nn;
     double* eb = base + el * S::per_elem;
     Phys::node_prims(Pp, eb + S::oU + node * NV, eb + S::oQ + node * NQ, bad);
+    if constexpr (Phys::kFixed)
+      eb[S::oQ + node * NQ + 4] -= 0.25 * eb[S::oU + NV - 1];  // phi of the first node
   }
   __syncthreads();
+
+  // --- phase 1b (fixed point): one warp per element takes the maxima of the
+  //     node values, metric terms and surface fluxes and chooses the scales;
+  //     then node values and metric terms become words in place
+  if constexpr (Phys::kFixed) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = nthr >> 5;
+    for (int el = warp; el < ne; el += nwarps) {
+      double* eb = base + el * S::per_elem;
+      u32 m[kMxCount] = {};
+      for (int node = lane; node < nn; node += 32) {
+        const double *q = eb + S::oQ + node * NQ, *ja = eb + S::oJa + node * 4;
+        m[kMxV] = max(m[kMxV], max(high_magnitude(q[1]), high_magnitude(q[2])));
+        // the words' products take densities as positive: bad states leave
+        m[kMxRho] = max(m[kMxRho], not_positive(q[0]) ? 0x7ff00000u : high_magnitude(q[0]));
+        m[kMxP] = max(m[kMxP], high_magnitude(q[3]));
+        m[kMxG] = max(m[kMxG], high_magnitude(q[4]));
+        m[kMxX] = max(m[kMxX], not_positive(q[5]) ? 0x7ff00000u : high_magnitude(q[5]));
+        m[kMxN] = max(m[kMxN], max(high_magnitude(ja[0]), high_magnitude(ja[1])));
+        m[kMxN + 1] = max(m[kMxN + 1], max(high_magnitude(ja[2]), high_magnitude(ja[3])));
+      }
+      for (int k = lane; k < 4 * n; k += 32) {
+        const double* sf = sfv + ((size_t)(e_first + el) * 4 * n + k) * NA;
+        const u32 a = high_magnitude(sf[0]), c = high_magnitude(sf[3]),
+                  b = max(high_magnitude(sf[1]), high_magnitude(sf[2]));
+        const bool second = k >= 2 * n;
+        m[kMxF] = max(m[kMxF], second ? 0u : a);
+        m[kMxF + 1] = max(m[kMxF + 1], second ? a : 0u);
+        m[kMxF + 3] = max(m[kMxF + 3], second ? 0u : b);
+        m[kMxF + 4] = max(m[kMxF + 4], second ? b : 0u);
+        m[kMxF + 6] = max(m[kMxF + 6], second ? 0u : c);
+        m[kMxF + 7] = max(m[kMxF + 7], second ? c : 0u);
+      }
+#pragma unroll
+      for (int k = 0; k < kMxCount; ++k) {
+        const bool used = k < kMxN + 2 || (k >= kMxF && (k - kMxF) % 3 < 2);
+        if (used) m[k] = __reduce_max_sync(0xffffffffu, m[k]);
+      }
+      const FxScale s = fx_scale(m, 2, sb->fx);
+      if (lane == 0) *reinterpret_cast<FxScale*>(eb + S::oF) = s;
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < ne * nn; t += nthr) {
+      const int el = t / nn, node = t % nn;
+      double* eb = base + el * S::per_elem;
+      const FxScale& fs = *reinterpret_cast<const FxScale*>(eb + S::oF);
+      if (!fs.ok) continue;
+      fx_convert_node<2>(eb + S::oQ + node * NQ, fs);
+      double* ja = eb + S::oJa + node * 4;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) ja[c] = f64_from((u64)to_fixed(ja[c], fs.sn[c / 2] - 2));
+    }
+    __syncthreads();
+  }
 
   // --- phase 2 (weak form): contravariant fluxes per node,
   //     F~_d = f(u, Ja^d) into slot 0 of direction d
@@ -240,9 +290,9 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
       const int el = t / (nn * 2), r = t % (nn * 2);
       const int node = r >> 1, d = r & 1;
       double* eb = base + el * S::per_elem;
-      const double* ja = eb + S::oJa + node * 4 + 2 * d;  // halved
+      const double* ja = eb + S::oJa + node * 4 + 2 * d;
       double F[NA];
-      Phys::flux(Pp, eb + S::oU + node * NV, 2.0 * ja[0], 2.0 * ja[1], F);
+      Phys::flux(Pp, eb + S::oU + node * NV, ja[0], ja[1], F);
 #pragma unroll
       for (int v = 0; v < NA; ++v) eb[S::oC + (d * nn + node) * (n - 1) * NA + v] = F[v];
     }
@@ -265,13 +315,31 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
     double* eb = base + el * S::per_elem;
     const double* ja_a = eb + S::oJa + na_ * 4 + 2 * d;
     const double* ja_b = eb + S::oJa + nb_ * 4 + 2 * d;
-    const double n1 = ja_a[0] + ja_b[0];
-    const double n2 = ja_a[1] + ja_b[1];
+    double* ca = eb + S::oC + ((d * nn + na_) * (n - 1) + b - 1) * NA;  // b > a
+    double* cb = eb + S::oC + ((d * nn + nb_) * (n - 1) + a) * NA;
+    if constexpr (Phys::kFixed) {
+      const FxScale& fs = *reinterpret_cast<const FxScale*>(eb + S::oF);
+      if (fs.ok) {
+        // the pair ordered so that the weight is positive; words to be summed
+        const i64 Qab = sb->fx.Q[a * n + b];
+        const bool turn = Qab < 0;
+        const int p = turn ? nb_ : na_, q = turn ? na_ : nb_;
+        i64 Fa[NA], Fb[NA];
+        Phys::fixed_pair(Pp, eb + S::oQ + p * NQ, eb + S::oQ + q * NQ, turn ? ja_b : ja_a,
+                         turn ? ja_a : ja_b, turn ? -Qab : Qab, fx_shift(fs), fs.kq[d], Fa, Fb);
+        double *cp = turn ? cb : ca, *cq = turn ? ca : cb;
+#pragma unroll
+        for (int v = 0; v < NA; ++v) {
+          cp[v] = f64_from((u64)Fa[v]);
+          cq[v] = f64_from((u64)-Fb[v]);
+        }
+        continue;
+      }
+    }
+    const double n1 = ja_a[0] + ja_b[0], n2 = ja_a[1] + ja_b[1];
     double Fa[NA], Fb[NA];
     Phys::volume_pair(Pp, eb + S::oQ + na_ * NQ, eb + S::oQ + nb_ * NQ, n1, n2, Fa, Fb);
     // raw pair fluxes; the D_split weights are applied in the slot reduction
-    double* ca = eb + S::oC + ((d * nn + na_) * (n - 1) + b - 1) * NA;  // b > a
-    double* cb = eb + S::oC + ((d * nn + nb_) * (n - 1) + a) * NA;
 #pragma unroll
     for (int v = 0; v < NA; ++v) {
       ca[v] = Fa[v];
@@ -303,7 +371,31 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
     const int i = node % n, j = node / n;
     const int e = e_first + el;
     double* eb = base + el * S::per_elem;
+    const double* se = sfv + (size_t)e * 4 * n * NA + v;
+    const bool halved = VOL == kVolFluxDiff && Phys::kLastHalved && v == NA - 1;
+    const FxScale& fs = *reinterpret_cast<const FxScale*>(eb + S::oF);
     double acc = 0.0;
+    if (VOL == kVolFluxDiff && Phys::kFixed && fs.ok) {
+      // sums of words and unweighted surface fluxes, then 1/w per direction
+      const int kind = v == 0 ? 0 : v < NA - 1 ? 1 : 2;
+      const int ks = fx_kind_scale(fs, kind) + sb->fx.sq;
+      const int sd[2] = {fx_direction_scale(fs, 0), fx_direction_scale(fs, 1)}, at[2] = {i, j};
+      i64 A[2] = {0, 0};
+#pragma unroll
+      for (int d = 0; d < 2; ++d) {
+        const double* c = eb + S::oC + (d * nn + node) * (n - 1) * NA + v;
+#pragma unroll
+        for (int s = 0; s < n - 1; ++s) A[d] += (i64)f64_bits(c[s * NA]);
+        if (at[d] == 0 || at[d] == n - 1) {
+          const int end = at[d] == 0 ? 0 : 1;
+          A[d] += fx_surface(se[((2 * d + end) * n + at[1 - d]) * NA], ks + sd[d] + (halved ? 1 : 0),
+                             sb->fx.S[end]);
+        }
+      }
+      int scale;
+      const i64 tot = fx_weighted_sum<2>(A, 1, sb->fx.W, at, sd, scale);
+      acc = from_fixed(tot, ks + scale + sb->fx.kw);
+    } else {
     if constexpr (VOL == kVolFluxDiff) {
       // slot s of node a holds the flux with partner s (s < a) or s + 1
 #pragma unroll
@@ -325,8 +417,6 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
     }
     // surface terms: one multiply-add per direction (a node lies on at most
     // one of a direction's two faces)
-    const double* se = sfv + (size_t)e * 4 * n * NA + v;
-    const bool halved = VOL == kVolFluxDiff && Phys::kLastHalved && v == NA - 1;
     if (i == 0 || i == n - 1) {
       const double w = i == 0 ? sb->winv0 : sb->winvN;
       acc = fma(se[((i == 0 ? 0 : 1) * n + j) * NA], halved ? half_of(w) : w, acc);
@@ -334,6 +424,7 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
     if (j == 0 || j == n - 1) {
       const double w = j == 0 ? sb->winv0 : sb->winvN;
       acc = fma(se[((j == 0 ? 2 : 3) * n + i) * NA], halved ? half_of(w) : w, acc);
+    }
     }
     const size_t gq = (size_t)e * nn + node;
     const double ij = halved ? twice(invJ[gq]) : invJ[gq];
@@ -378,8 +469,9 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
       double* eb = base + el * S::per_elem;
       double l1, l2;
       Phys::max_speeds(Pp, eb + S::oU + node * NV, l1, l2);
-      const double* ja = eb + S::oJa + node * 4;  // halved
-      const double ij = 2.0 * fabs(invJ[(size_t)(e_first + el) * nn + node]);
+      const size_t gq = (size_t)(e_first + el) * nn + node;
+      const double* ja = Phys::kFixed ? Ja + gq * 4 : eb + S::oJa + node * 4;
+      const double ij = fabs(invJ[gq]);
       eb[S::oL + node] = fabs(ja[0] * l1 + ja[1] * l2) * ij;
       eb[S::oL + nn + node] = fabs(ja[2] * l1 + ja[3] * l2) * ij;
     }

@@ -290,12 +290,9 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
           const double* ja_b = eb + S::oJa + nb_ * 9 + 3 * d;
           if (fixed) {
             if constexpr (Phys::kFixed) {
-              const i64* wa = reinterpret_cast<const i64*>(eb + S::oQ + na_ * NQ);
-              const i64* wb = reinterpret_cast<const i64*>(eb + S::oQ + nb_ * NQ);
               i64 Fa[NA], Fb[NA];
-              fx_energy_pair<3>(wa, wb, reinterpret_cast<const i64*>(ja_a),
-                                reinterpret_cast<const i64*>(ja_b), Qab, fk, fs.kq[d], Fa,
-                                Fb);
+              Phys::fixed_pair(Pp, eb + S::oQ + na_ * NQ, eb + S::oQ + nb_ * NQ, ja_a, ja_b, Qab,
+                               fk, fs.kq[d], Fa, Fb);
               i64* ca = reinterpret_cast<i64*>(eb + S::oA + (d * nnn + na_) * NA);
               i64* cb = reinterpret_cast<i64*>(eb + S::oA + (d * nnn + nb_) * NA);
 #pragma unroll

@@ -3,7 +3,7 @@
 // State u = (rho, rho_v1, rho_v2, rho_e, phi); phi = g z is passive (zero flux,
 // zero time derivative), so kernels evolve NA = 4 active variables.
 #pragma once
-#include "tag_common.cuh"
+#include "fixed_flux.cuh"
 
 namespace tag {
 
@@ -11,12 +11,12 @@ struct PhysEnergy2D {
   static constexpr int NV = 5;  // stored variables per node
   static constexpr int NA = 4;  // variables with nonzero du
   // per-node quantities kept in shared memory (odd stride: no bank conflicts):
-  // rho/2, v1/2, v2/2, p/2, phi/4, theta = (p/rho) / (4 (gamma - 1)),
+  // rho/2, v1/2, v2/2, p/2, phi/4 (less the first node's), theta = (p/rho) / (4 (gamma - 1)),
   // log2(rho), log2(p/rho) (log2_fixed words), (pad)
   static constexpr int NQ = 9;
   // volume_pair returns half the energy flux (the kernel doubles the node sums)
   static constexpr bool kLastHalved = true;
-  static constexpr bool kFixed = false;  // volume integral in FP64
+  static constexpr bool kFixed = true;  // volume integral in words (fixed_flux.cuh)
   static constexpr bool kHasSources = false;
   static constexpr bool kSurfaceNoncons = false;  // surface flux only (flux_zero)
 
@@ -66,6 +66,7 @@ struct PhysEnergy2D {
   // momentum fluxes of the two sides are f1 v + n (p_avg +- 2 rho_mean g), and
   // half the energy fluxes
   //   f1 (v_a.v_b / 4 + mean(p/rho) / (2 (gamma - 1)) +- g) + (p_a vn_b + p_b vn_a) / 4.
+  // Elements in range take fx_energy_pair (fixed_flux.cuh) instead.
   TAG_DEV static void volume_pair(const Params& P, const double* qa, const double* qb,
                                   double n1, double n2, double* Fa, double* Fb) {
     const double R = ln_factor(qa[0], qb[0], log_difference(qa[6], qb[6]));
@@ -91,6 +92,14 @@ struct PhysEnergy2D {
     const double e = fma(f1, x, fma(qa[3], vnb, qb[3] * vna));
     Fa[3] = fma(f1, g, e);
     Fb[3] = fma(-f1, g, e);
+  }
+
+  TAG_DEV static void fixed_pair(const Params&, const double* qa, const double* qb,
+                                 const double* na, const double* nb, i64 Q, const FxShift& k,
+                                 int kq, i64* Fa, i64* Fb) {
+    fx_energy_pair<2>(reinterpret_cast<const i64*>(qa), reinterpret_cast<const i64*>(qb),
+                      reinterpret_cast<const i64*>(na), reinterpret_cast<const i64*>(nb), Q, k, kq,
+                      Fa, Fb);
   }
 
   // FluxLMARS (:397-430) between states ul, ur for the (unnormalised) normal n:

@@ -4,7 +4,7 @@
 // State u = (rho, rho_v1, rho_v2, rho_v3, rho_e, phi); phi is passive, so
 // kernels evolve NA = 5 active variables.
 #pragma once
-#include "tag_common.cuh"
+#include "fixed_flux.cuh"
 
 namespace tag {
 
@@ -97,6 +97,14 @@ struct PhysEnergy3D {
     const double e = fma(f1, x, fma(qa[4], vnb, qb[4] * vna));
     Fa[4] = fma(f1, g, e);
     Fb[4] = fma(-f1, g, e);
+  }
+
+  TAG_DEV static void fixed_pair(const Params&, const double* qa, const double* qb,
+                                 const double* na, const double* nb, i64 Q, const FxShift& k,
+                                 int kq, i64* Fa, i64* Fb) {
+    fx_energy_pair<3>(reinterpret_cast<const i64*>(qa), reinterpret_cast<const i64*>(qb),
+                      reinterpret_cast<const i64*>(na), reinterpret_cast<const i64*>(nb), Q, k, kq,
+                      Fa, Fb);
   }
 
   // FluxLMARS (3D, :430-466) for the (unnormalised) normal n:

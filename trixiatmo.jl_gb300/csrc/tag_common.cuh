@@ -232,6 +232,26 @@ TAG_DEV void copy_in(double* smem, const double* __restrict__ g, int count) {
       asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(s + 8 * t), "l"(g + t));
   }
 }
+// The same for `ne` blocks, consecutive in g and `stride` doubles apart in
+// shared memory.
+TAG_DEV void copy_in_blocks(double* smem, int stride, const double* __restrict__ g, int count,
+                            int ne) {
+  const u32 s = (u32)__cvta_generic_to_shared(smem);
+  if (((((size_t)g) | s | (count * 8u) | (stride * 8u)) & 15u) == 0) {
+    const int c2 = count / 2;
+    for (int t = threadIdx.x; t < ne * c2; t += blockDim.x) {
+      const int el = t / c2, r = t - el * c2;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s + 8 * stride * el + 16 * r),
+                   "l"(g + 2 * t));
+    }
+  } else {
+    for (int t = threadIdx.x; t < ne * count; t += blockDim.x) {
+      const int el = t / count, r = t - el * count;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(s + 8 * (stride * el + r)),
+                   "l"(g + t));
+    }
+  }
+}
 TAG_DEV void copy_in_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 TAG_DEV void copy_out(double* __restrict__ g, const double* smem, int count) {
   if (((((size_t)g) | (size_t)smem | (count * 8u)) & 15u) == 0) {
