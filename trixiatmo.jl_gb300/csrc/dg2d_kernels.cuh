@@ -183,8 +183,9 @@ struct ElemSmem {
   static constexpr int oQ = oU + nn * NV;
   static constexpr int oJa = oQ + nn * NQ;
   static constexpr int oC = oJa + nn * 4;        // slots [2][nn][n - 1][NA], one per partner
-  static constexpr int oL = oC + 2 * nn * (n - 1) * NA;  // CFL speeds [2][nn]
-  static constexpr int oS = oL + 2 * nn;          // sources [nn][NA]
+  static constexpr int oL = oC;                  // CFL speeds [2][nn], once the slots are used up
+  static constexpr int sizeC = 2 * nn * (n - 1) * NA;
+  static constexpr int oS = oC + (sizeC > 2 * nn + 9 ? sizeC : 2 * nn + 9);  // sources [nn][NA]
   static constexpr int oF = oS + (Phys::kHasSources ? nn * NA : 0);  // fixed point: FxScale
   static constexpr int per_elem = (oF + (Phys::kFixed ? kFxDoubles : 0) + 1) / 2 * 2;
   static size_t bytes(int epb) { return sizeof(double) * (size_t)per_elem * epb + sizeof(BasisDev); }
@@ -230,8 +231,8 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
   }
   __syncthreads();
 
-  // --- phase 1b (fixed point): one warp per element takes the maxima of the
-  //     node values, metric terms and surface fluxes and chooses the scales;
+  // --- phase 1b (fixed point): a warp takes an element's maxima of the node
+  //     values, metric terms and surface fluxes, a thread chooses its scales,
   //     then node values and metric terms become words in place
   if constexpr (Phys::kFixed) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = nthr >> 5;
@@ -266,8 +267,17 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
         const bool used = k < kMxN + 2 || (k >= kMxF && (k - kMxF) % 3 < 2);
         if (used) m[k] = __reduce_max_sync(0xffffffffu, m[k]);
       }
-      const FxScale s = fx_scale(m, 2, sb->fx);
-      if (lane == 0) *reinterpret_cast<FxScale*>(eb + S::oF) = s;
+      // (the pair slots are not in use yet)
+      if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < kMxCount; ++k) reinterpret_cast<u32*>(eb + S::oC)[k] = m[k];
+      }
+    }
+    __syncthreads();
+    for (int el = threadIdx.x; el < ne; el += nthr) {
+      double* eb = base + el * S::per_elem;
+      *reinterpret_cast<FxScale*>(eb + S::oF) =
+          fx_scale(reinterpret_cast<const u32*>(eb + S::oC), 2, sb->fx);
     }
     __syncthreads();
     for (int t = threadIdx.x; t < ne * nn; t += nthr) {

@@ -155,6 +155,20 @@ TAG_HD float fx_fraction(u32 hi, int s) {
   return m * pow2f((int)(hi >> 20) - 1023 - s);
 }
 
+// The largest k with x 2^k <= top (x > 0; 120 for x = 0), and a bound x of scale s
+// brought under top by raising s.
+TAG_HD int fx_room(float x, float top) {
+  if (!(x > 1e-30f)) return x == x ? 120 : 0;
+  // by the exponents of x and top, one less where x's significand is larger
+  const u32 bx = f32_bits(x), bt = f32_bits(top);
+  return (int)(bt >> 23) - (int)(bx >> 23) - ((bx & 0x7fffffu) > (bt & 0x7fffffu) ? 1 : 0);
+}
+TAG_HD void fx_fit(float& x, int& s, float top) {
+  const int k = min(0, fx_room(x, top));
+  x *= pow2f(k);
+  s -= k;
+}
+
 // Scales of an element from its maxima mx (kMxF + 3 kind + d: surface fluxes of
 // the mass, the momentum and the transported scalar on direction d's faces) in
 // `dims` directions.  Each is the smallest that bounds the words derived from it
@@ -182,40 +196,26 @@ TAG_HD FxScale fx_scale(const u32* mx, int dims, const FxBasis& b) {
   const float rho = 2.0f * fx_fraction(mx[kMxRho], s.sr), v = fx_fraction(mx[kMxV], s.sv),
               g = 2.0f * fx_fraction(mx[kMxG], s.sg);
   // x = mean(scalar) + v.v
-  float x = 1.0f;
-  for (s.sx = max(e[kMxX] + 2, 2 * s.sv);; ++s.sx) {
-    x = 2.0f * fx_fraction(mx[kMxX], s.sx) + D * v * v * pow2f(2 * s.sv - s.sx);
-    if (!(x > top)) break;
-  }
+  s.sx = max(e[kMxX] + 2, 2 * s.sv);
+  float x = 2.0f * fx_fraction(mx[kMxX], s.sx) + D * v * v * pow2f(2 * s.sv - s.sx);
+  fx_fit(x, s.sx, top);
   // pressure sum +- 2 rho_mean g
-  float p = 1.0f, pp = 1.0f;
   s.sp = max(max(e[kMxP] + 2, s.sr + s.sg + 1), s.sr + 2 * s.sv);
   for (int d = 0; d < dims; ++d) s.sp = max(s.sp, e[kMxF + 3 + d] + 4 - s.sn[d] - b.sq);
-  for (;; ++s.sp) {
-    p = fx_fraction(mx[kMxP], s.sp);
-    pp = 2.0f * p + rho * g * pow2f(s.sr + s.sg + 1 - s.sp);
-    if (!(pp > top)) break;
-  }
-  // h = rho_mean x + (p +- 2 rho_mean g) / 2
-  float h = 1.0f;
+  float pp = 2.0f * fx_fraction(mx[kMxP], s.sp) + rho * g * pow2f(s.sr + s.sg + 1 - s.sp);
+  fx_fit(pp, s.sp, top);
+  const float p = fx_fraction(mx[kMxP], s.sp);
+  // h = rho_mean x + (p +- 2 rho_mean g) / 2, shifted left by jh
   s.sh = max(s.sr + s.sx, s.sp - 1);
-  for (int d = 0; d < dims; ++d) s.sh = max(s.sh, e[kMxF + 6 + d] + 3 - s.sv - s.sn[d] - b.sq);
-  for (;; ++s.sh) {
-    h = rho * x * pow2f(s.sr + s.sx - s.sh) + pp * pow2f(s.sp - 1 - s.sh);
-    if (!(h > top)) break;
-  }
-  s.jh = 0;
-  while (s.jh < 8 && 2.0f * h <= top) {
-    h *= 2.0f;
-    ++s.jh;
-  }
+  int fluxes = -10000;  // surface fluxes to 1/16
+  for (int d = 0; d < dims; ++d)
+    fluxes = max(fluxes, e[kMxF + 6 + d] + 3 - s.sv - s.sn[d] - b.sq);
+  s.sh = max(s.sh, fluxes);
+  float h = rho * x * pow2f(s.sr + s.sx - s.sh) + pp * pow2f(s.sp - 1 - s.sh);
+  fx_fit(h, s.sh, top);
+  s.jh = max(0, min(min(fx_room(h, top), s.sh - fluxes), 8));
+  h *= pow2f(s.jh);
   s.sh -= s.jh;
-  for (int d = 0; d < dims; ++d)  // surface fluxes to 1/16
-    while (s.jh > 0 && e[kMxF + 6 + d] + 3 > s.sh + s.sv + s.sn[d] + b.sq) {
-      h *= 0.5f;
-      --s.jh;
-      ++s.sh;
-    }
   for (int d = 0; d < dims; ++d) {
     const float n = 2.0f * fx_fraction(mx[kMxN + d], s.sn[d]);
     const float vn = D * 2.0f * v * n;  // per unit of Q
@@ -228,10 +228,8 @@ TAG_HD FxScale fx_scale(const u32* mx, int dims, const FxBasis& b) {
     most = fmaxf(most, b.row * vn * (h + p * pow2f(s.sp - 1 - s.sh)) +
                            0.5f * fx_fraction(mx[kMxF + 6 + d], s.sh + s.sv + sd));
     most = fmaxf(most, b.one * n);
-    while (s.kq[d] < 12 && 2.0f * most <= top) {
-      most *= 2.0f;
-      ++s.kq[d];
-    }
+    s.kq[d] = max(0, min(fx_room(most, top), 12));
+    most *= pow2f(s.kq[d]);
     if (!(most <= 0.49f)) s.ok = 0;
   }
   return s;

@@ -124,7 +124,7 @@ int stage_sequence(tag_handle h) {
 }
 
 int build_graph(tag_handle h) {
-  const int key = h->epb * 8 + h->tile_div;
+  const int key = h->epb * 16 + h->tile_div;
   if (h->graph && h->graph_epb == key && h->graph_sink == h->sink) return TAG_OK;
   if (h->graph) {
     cudaGraphExecDestroy(h->graph);
@@ -162,14 +162,18 @@ int autotune(tag_handle h, const double* u) {
   TAG_CUDA(cudaEventCreate(&b));
   int best = 1, best_div = 1;
   float best_ms = 1e30f;
-  const int cands[] = {1, 2, 3, 4, 6, 8, 12, 16};
-  const int ndiv = h->dim == 3 ? 6 : 2;
-  for (int trial = 0; trial < 8 * ndiv; ++trial) {
-    const int c = cands[trial / ndiv], div = 1 + trial % ndiv;
+  // (elements per CTA, tile_div): every element count with one to three items
+  // per thread (3D also in whole groups of four warps)
+  std::vector<std::pair<int, int>> tiles;
+  for (int c : {1, 2, 3, 4, 6, 8, 12, 16})
+    for (int div = 1; div <= (h->dim == 3 ? 6 : 3); ++div) {
+      const int share = (div - 1) % 3 + 1;  // work items per thread
+      if (c * h->ops->threads_per_element > h->ops->max_threads() && c > 1) continue;
+      if (share > 1 && c * h->ops->threads_per_element < 64 * share) continue;
+      tiles.push_back({c, div});
+    }
+  for (const auto& [c, div] : tiles) {
     if ((size_t)h->ops->smem_bytes(c) > (size_t)max_smem) continue;
-    if (c * h->ops->threads_per_element > h->ops->max_threads() && c > 1) continue;
-    const int share = (div - 1) % 3 + 1;  // work items per thread
-    if (share > 1 && c * h->ops->threads_per_element < 64 * share) continue;
     h->epb = c;
     h->tile_div = div;
     double* uu = const_cast<double*>(u);
@@ -1488,10 +1492,10 @@ int tag_set_tile(tag_handle h, int32_t epb, int32_t items_per_thread) {
 int tag_get_cta_threads(tag_handle h, int32_t* threads) {
   if (!h || !threads) return fail(TAG_E_INVALID, "null argument");
   const int epb = h->epb > 0 ? h->epb : 1;
-  *threads = h->ops ? std::min(h->ops->max_threads(),
-                               (h->dim == 3 ? tile_threads : cta_threads)(
-                                   epb * h->ops->threads_per_element, h->tile_div))
-                    : 0;
+  const int items = h->ops ? epb * h->ops->threads_per_element : 0, div = h->tile_div;
+  *threads = !h->ops ? 0
+                     : std::min(h->ops->max_threads(), h->dim == 3 ? tile_threads(items, div)
+                                                                   : cta_threads(items, div));
   return TAG_OK;
 }
 
