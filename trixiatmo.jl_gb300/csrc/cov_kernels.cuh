@@ -23,10 +23,13 @@
 
 namespace tag {
 
-// packed per-node element data
+// packed per-node element data: area element, contravariant metric, covariant
+// metric (standard form: the first two are the contractions Gamma^i : G_con of
+// the pressure source), bottom topography, the geometric source's coefficients
+// of hv^1 v^1, hv^1 v^2 and hv^2 v^2 in both components, f J and 1/J
 enum CovPack : int {
   kPJ = 0, kPGc11, kPGc12, kPGc22, kPGv11, kPGv12, kPGv22, kPHs,
-  kPC111, kPC112, kPC122, kPC211, kPC212, kPC222, kPF, kPInvJ, kPack = 16
+  kPS100, kPS101, kPS111, kPS200, kPS201, kPS211, kPFJ, kPInvJ, kPack = 16
 };
 
 TAG_DEV int cov_find_group(const CovGroups& G, int blk, bool iface) {
@@ -36,22 +39,49 @@ TAG_DEV int cov_find_group(const CovGroups& G, int blk, bool iface) {
   return lo;
 }
 
-// packs aux (26), the Coriolis parameter f = 2 Omega z / |x| and 1/J per node
+// packs aux (26), the Coriolis parameter f = 2 Omega z / |x| times J and 1/J per
+// node.  The geometric source is a contraction of hv (x) v with geometry alone:
+//   standard: Gamma^i : (hv (x) v + g h^2/2 G_con);
+//   split: (Gamma^i : T - G_con^ij w_j) / 2 with w_j = Gamma^k_jl (G_cov T)_kl,
+// so its six coefficients are formed here, once, instead of 60 operations per
+// node and stage.
 __global__ void k_cov_pack(const double* __restrict__ aux, const double* __restrict__ xyz,
-                           long nodes, double omega, double* __restrict__ pk) {
+                           long nodes, double omega, int split, double* __restrict__ pk) {
   const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= nodes) return;
   const double* a = aux + q * 26;
   double* p = pk + q * kPack;
-  p[kPJ] = a[12];
-  p[kPGc11] = a[16]; p[kPGc12] = a[17]; p[kPGc22] = a[18];
-  p[kPGv11] = a[13]; p[kPGv12] = a[14]; p[kPGv22] = a[15];
+  const double J = a[12], v11 = a[13], v12 = a[14], v22 = a[15];
+  const double c11 = a[16], c12 = a[17], c22 = a[18];
+  const double g111 = a[20], g112 = a[21], g122 = a[22], g211 = a[23], g212 = a[24], g222 = a[25];
+  p[kPJ] = J;
+  p[kPGc11] = c11; p[kPGc12] = c12; p[kPGc22] = c22;
+  p[kPGv11] = v11; p[kPGv12] = v12; p[kPGv22] = v22;
   p[kPHs] = a[19];
-#pragma unroll
-  for (int k = 0; k < 6; ++k) p[kPC111 + k] = a[20 + k];
+  // symmetric parts Gamma^i : T
+  double s1[3] = {g111, 2.0 * g112, g122}, s2[3] = {g211, 2.0 * g212, g222};
+  if (split) {
+    const double w1[3] = {g111 * v11 + g211 * v12,
+                          (g111 * v12 + g112 * v11) + (g211 * v22 + g212 * v12),
+                          g112 * v12 + g212 * v22};
+    const double w2[3] = {g112 * v11 + g212 * v12,
+                          (g112 * v12 + g122 * v11) + (g212 * v22 + g222 * v12),
+                          g122 * v12 + g222 * v22};
+    for (int k = 0; k < 3; ++k) {
+      s1[k] = 0.5 * (s1[k] - (c11 * w1[k] + c12 * w2[k]));
+      s2[k] = 0.5 * (s2[k] - (c12 * w1[k] + c22 * w2[k]));
+    }
+  } else {
+    p[kPGv11] = g111 * c11 + 2.0 * g112 * c12 + g122 * c22;
+    p[kPGv12] = g211 * c11 + 2.0 * g212 * c12 + g222 * c22;
+  }
+  for (int k = 0; k < 3; ++k) {
+    p[kPS100 + k] = s1[k];
+    p[kPS200 + k] = s2[k];
+  }
   const double* x = xyz + q * 3;
-  p[kPF] = 2.0 * omega * x[2] / sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
-  p[kPInvJ] = 1.0 / a[12];
+  p[kPFJ] = 2.0 * omega * x[2] / sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]) * J;
+  p[kPInvJ] = 1.0 / J;
 }
 
 // ---- pointwise physics on packed data -----------------------------------------
@@ -77,34 +107,24 @@ TAG_DEV void cov_flux(const CovParams& P, const double* u, double ih, const doub
   f[2] = J * (u[2] * vo + cov_gcon(p, 1, o) * gt);
 }
 
-// source_terms_geometric_coriolis (standard or split), after apply_jacobian
+// source_terms_geometric_coriolis (standard or split), after apply_jacobian,
+// from the coefficients of k_cov_pack
 TAG_DEV void cov_source(const CovParams& P, const double* u, double ih, const double* p,
                         double* s) {
   const double hv0 = u[1], hv1 = u[2];
   const double v0 = hv0 * ih, v1 = hv1 * ih;
-  const double T00 = hv0 * v0, T01 = hv0 * v1, T10 = hv1 * v0, T11 = hv1 * v1;
-  double sg0, sg1;
+  const double T00 = hv0 * v0, T01 = hv0 * v1, T11 = hv1 * v1;
+  double sg0 = fma(p[kPS111], T11, fma(p[kPS101], T01, p[kPS100] * T00));
+  double sg1 = fma(p[kPS211], T11, fma(p[kPS201], T01, p[kPS200] * T00));
   if (!P.split) {
     const double gt = 0.5 * P.g * u[0] * u[0];
-    sg0 = p[kPC111] * (T00 + gt * p[kPGc11]) + p[kPC112] * (T01 + gt * p[kPGc12]) +
-          p[kPC112] * (T10 + gt * p[kPGc12]) + p[kPC122] * (T11 + gt * p[kPGc22]);
-    sg1 = p[kPC211] * (T00 + gt * p[kPGc11]) + p[kPC212] * (T01 + gt * p[kPGc12]) +
-          p[kPC212] * (T10 + gt * p[kPGc12]) + p[kPC222] * (T11 + gt * p[kPGc22]);
-  } else {
-    // C = G_cov T, w_i = (Gamma^1 C[0,:])_i + (Gamma^2 C[1,:])_i
-    const double C00 = p[kPGv11] * T00 + p[kPGv12] * T10, C01 = p[kPGv11] * T01 + p[kPGv12] * T11;
-    const double C10 = p[kPGv12] * T00 + p[kPGv22] * T10, C11 = p[kPGv12] * T01 + p[kPGv22] * T11;
-    const double w0 = (p[kPC111] * C00 + p[kPC112] * C01) + (p[kPC211] * C10 + p[kPC212] * C11);
-    const double w1 = (p[kPC112] * C00 + p[kPC122] * C01) + (p[kPC212] * C10 + p[kPC222] * C11);
-    const double s0 = p[kPC111] * T00 + p[kPC112] * T01 + p[kPC112] * T10 + p[kPC122] * T11;
-    const double s1 = p[kPC211] * T00 + p[kPC212] * T01 + p[kPC212] * T10 + p[kPC222] * T11;
-    sg0 = 0.5 * (s0 - (p[kPGc11] * w0 + p[kPGc12] * w1));
-    sg1 = 0.5 * (s1 - (p[kPGc12] * w0 + p[kPGc22] * w1));
+    sg0 = fma(gt, p[kPGv11], sg0);
+    sg1 = fma(gt, p[kPGv12], sg1);
   }
-  const double fJ = p[kPF] * p[kPJ];
+  const double f0 = p[kPFJ] * hv0, f1 = p[kPFJ] * hv1;
   s[0] = 0.0;
-  s[1] = -(sg0 + fJ * (p[kPGc12] * hv0 - p[kPGc11] * hv1));
-  s[2] = -(sg1 + fJ * (p[kPGc22] * hv0 - p[kPGc12] * hv1));
+  s[1] = -fma(p[kPGc12], f0, fma(-p[kPGc11], f1, sg0));
+  s[2] = -fma(p[kPGc22], f0, fma(-p[kPGc12], f1, sg1));
 }
 
 // ---- interface fluxes ------------------------------------------------------------
@@ -165,7 +185,7 @@ TAG_DEV void cov_surface(const CovParams& P, const double* a, const double* c, d
   }
   if (P.surf_diss) {
     const double goo = o ? w.gc22 : w.gc11;
-    const double lam = fmax(fabs(vao) + sqrt(goo * a[0] * P.g), fabs(vco) + sqrt(goo * c[0] * P.g));
+    const double lam = fmax(fabs(vao) + int_sqrt(goo * a[0] * P.g), fabs(vco) + int_sqrt(goo * c[0] * P.g));
     const double s = -0.5 * J * lam;
     F[0] += s * (c[0] - a[0]);
     F[1] += s * (c[1] - a[1]);
@@ -230,7 +250,7 @@ TAG_DEV void cov_interface_body(const CovParams& P, const CovGroup& G, int lblk,
   double rt[3], lt[3], Fp[3], Fs[3];
   cov_transform(ur, ar, al, rt);
   cov_transform(ul, al, ar, lt);
-  const double ihl = 1.0 / ul[0], ihr = 1.0 / ur[0];
+  const double ihl = int_rcp(ul[0]), ihr = int_rcp(ur[0]);
   cov_side_flux(P, ul, rt, ihl, ihr, al, f0, Fp);
   cov_side_flux(P, ur, lt, ihr, ihl, ar, f1, Fs);
   double* s0 = sfv + G.sf0 + ((long)(e0 - G.e0) * 4 + f0) * n * 3 + l * 3;
@@ -293,6 +313,7 @@ TAG_DEV void cov_element_body(const CovParams& P, const CovGroup& G, int lblk,
   const int i = node % n, j = node / n;
   const long gq = G.node0 + (long)(el_first + el) * nn + node;
   double ui[3], ih = 0.0;  // ih = 1/h, shared by the fluxes and the source
+  const bool regrouped = VK == 1 && P.split && P.vol_sym <= 1;
   double* qn = q + threadIdx.x * kCovQ;
   const double* __restrict__ pg = pk + gq * kPack;  // re-read where needed (L1 hit)
   if (act) {
@@ -301,7 +322,7 @@ TAG_DEV void cov_element_body(const CovParams& P, const CovGroup& G, int lblk,
     double p[kPack];
 #pragma unroll
     for (int k = 0; k < kPack; ++k) p[k] = __ldg(pg + k);
-    ih = 1.0 / ui[0];
+    ih = int_rcp(ui[0]);
     if constexpr (VK == 0) {
       cov_flux(P, ui, ih, p, 0, qn);
       cov_flux(P, ui, ih, p, 1, qn + 3);
@@ -313,13 +334,21 @@ TAG_DEV void cov_element_body(const CovParams& P, const CovGroup& G, int lblk,
       qn[3] = p[kPGv12] * v1 + p[kPGv22] * v2;
       qn[4] = p[kPJ] * ui[1];
       qn[5] = p[kPJ] * ui[2];
-      qn[6] = ui[0];
-      qn[7] = p[kPHs];
-      qn[8] = p[kPJ];
-      qn[9] = p[kPGc11];
-      qn[10] = p[kPGc12];
-      qn[11] = p[kPGc22];
-      qn[12] = 0.5 * P.g * ui[0] * ui[0];
+      if (regrouped) {
+        qn[6] = ui[0] + p[kPHs];
+        qn[7] = v1 * qn[4];
+        qn[8] = v2 * qn[4];
+        qn[9] = v1 * qn[5];
+        qn[10] = v2 * qn[5];
+      } else {
+        qn[6] = ui[0];
+        qn[7] = p[kPHs];
+        qn[8] = p[kPJ];
+        qn[9] = p[kPGc11];
+        qn[10] = p[kPGc12];
+        qn[11] = p[kPGc22];
+        qn[12] = 0.5 * P.g * ui[0] * ui[0];
+      }
     }
   }
   __syncthreads();
@@ -336,68 +365,68 @@ TAG_DEV void cov_element_body(const CovParams& P, const CovGroup& G, int lblk,
 #pragma unroll
         for (int v = 0; v < 3; ++v) acc[v] = fma(d2, F2[v], fma(d1, F1[v], acc[v]));
       }
-    } else if (P.split && P.vol_sym <= 1) {
+    } else if (regrouped) {
       // Split form with flux_central or flux_ec (and flux_nonconservative_ec):
       // every pair flux is a sum of products of a node-a factor and a node-b
-      // factor, so each line sum sum_b D_ab f(a, b) is formed from a few
-      // contractions sum_b D_ab x_b of node-b quantities (the pair terms of
-      // covariant_shallow_water_split.jl:100-215 regrouped; 10 instead of
-      // ~33 FP64 operations per partner node).  b = a is left out of the
-      // symmetric part and kept in the nonconservative part, as in the
-      // pairwise form.
+      // factor, so each line sum sum_b D_ab f(a, b) is formed from contractions
+      // sum_b D_ab x_b of node-b quantities (the pair terms of
+      // covariant_shallow_water_split.jl:100-215 regrouped; with the products
+      // v J hv formed per node, eight multiply-adds per partner node).  b = a is
+      // left out of the symmetric part and kept in the nonconservative part, as
+      // in the pairwise form.
       const double* qa = qn;
-      const double h_a = ui[0], hs_a = qa[7], J_a = qa[8];
-      const double gh = P.g * h_a;
+      const double gh = P.g * ui[0];
+      const double gc11 = __ldg(pg + kPGc11), gc12 = __ldg(pg + kPGc12),
+                   gc22 = __ldg(pg + kPGc22), hs_a = __ldg(pg + kPHs);
       double nc1 = 0.0, nc2 = 0.0;
 #pragma unroll
       for (int d = 0; d < 2; ++d) {
         const double hvo_a = d ? ui[2] : ui[1];
         const double Jhvo_a = d ? qa[5] : qa[4];
-        const double gco0 = d ? qa[10] : qa[9], gco1 = d ? qa[11] : qa[10];
         const int a = d ? j : i;
-        double SD = 0.0, A1 = 0.0, A2 = 0.0, A3 = 0.0, A4 = 0.0, A5 = 0.0;
+        double A1 = 0.0, A2 = 0.0, A3 = 0.0, A4 = 0.0, A5 = 0.0;
         double B2 = 0.0, B3 = 0.0, BH = 0.0;
 #pragma unroll
         for (int b = 0; b < n; ++b) {
           const double* qb = eq + (d ? b * n + i : j * n + b) * kCovQ;
           const double Dab = sb->Ds[a * n + b];
           if (b != a) {
-            const double Jb = d ? qb[5] : qb[4];
-            SD += Dab;
-            A1 = fma(Dab, Jb, A1);
+            A1 = fma(Dab, qb[4 + d], A1);
             A2 = fma(Dab, qb[0], A2);
-            A3 = fma(Dab, qb[0] * Jb, A3);
+            A3 = fma(Dab, qb[7 + 2 * d], A3);
             A4 = fma(Dab, qb[1], A4);
-            A5 = fma(Dab, qb[1] * Jb, A5);
+            A5 = fma(Dab, qb[8 + 2 * d], A5);
           }
           if (P.vol_nc) {
             B2 = fma(Dab, qb[2], B2);
             B3 = fma(Dab, qb[3], B3);
-            BH = fma(Dab, qb[6] + qb[7], BH);
+            BH = fma(Dab, qb[6], BH);
           }
         }
-        acc[0] += 0.5 * (Jhvo_a * SD + A1);
+        const double SD = sb->Dsum[a];  // the row of D_split without b = a
+        const double m = fma(Jhvo_a, SD, A1);
+        acc[0] = fma(0.5, m, acc[0]);
         if (P.vol_sym == 1) {
           // flux_ec: f = m (1, (v_a + v_b) / 2), m = (J hv_a + J hv_b) / 2
-          acc[1] += 0.25 * ((qa[0] * Jhvo_a) * SD + qa[0] * A1 + Jhvo_a * A2 + A3);
-          acc[2] += 0.25 * ((qa[1] * Jhvo_a) * SD + qa[1] * A1 + Jhvo_a * A4 + A5);
+          acc[1] = fma(0.25, fma(qa[0], m, fma(Jhvo_a, A2, A3)), acc[1]);
+          acc[2] = fma(0.25, fma(qa[1], m, fma(Jhvo_a, A4, A5)), acc[2]);
         } else {
           // flux_central of the split fluxes: (J hv v_a + J hv v_b) / 2
-          acc[1] += 0.5 * ((Jhvo_a * qa[0]) * SD + A3);
-          acc[2] += 0.5 * ((Jhvo_a * qa[1]) * SD + A5);
+          acc[1] = fma(0.5, fma(qa[7 + 2 * d], SD, A3), acc[1]);
+          acc[2] = fma(0.5, fma(qa[8 + 2 * d], SD, A5), acc[2]);
         }
         if (P.vol_nc) {
           const double Daa = sb->Ds[a * n + a];
-          const double Sall = SD + Daa;
           const double B0 = fma(Daa, qa[0], A2), B1 = fma(Daa, qa[1], A4);
           const double half_m = 0.5 * hvo_a;
-          const double ph = gh * (BH - hs_a * Sall);
-          nc1 += J_a * (half_m * (qa[9] * B2 + qa[10] * B3 - B0) + gco0 * ph);
-          nc2 += J_a * (half_m * (qa[10] * B2 + qa[11] * B3 - B1) + gco1 * ph);
+          const double ph = gh * fma(-hs_a, SD + Daa, BH);
+          nc1 = fma(d ? gc12 : gc11, ph, fma(half_m, fma(gc11, B2, fma(gc12, B3, -B0)), nc1));
+          nc2 = fma(d ? gc22 : gc12, ph, fma(half_m, fma(gc12, B2, fma(gc22, B3, -B1)), nc2));
         }
       }
-      acc[1] += 0.5 * nc1;
-      acc[2] += 0.5 * nc2;
+      const double hJ = 0.5 * __ldg(pg + kPJ);
+      acc[1] = fma(hJ, nc1, acc[1]);
+      acc[2] = fma(hJ, nc2, acc[2]);
     } else {
       const double* qa = qn;
       const double h_a = ui[0], hs_a = qa[7], J_a = qa[8];
@@ -448,12 +477,16 @@ TAG_DEV void cov_element_body(const CovParams& P, const CovGroup& G, int lblk,
       acc[2] += 0.5 * nc2;
     }
     const double* se = sfv + G.sf0 + (long)(el_first + el) * 4 * n * 3;
+    // one multiply-add per direction (a node lies on at most one of its faces)
+    if (i == 0 || i == n - 1) {
+      const double w = i == 0 ? sb->winv0 : sb->winvN;
 #pragma unroll
-    for (int v = 0; v < 3; ++v) {
-      if (i == 0) acc[v] += se[(0 * n + j) * 3 + v] * sb->winv0;
-      if (i == n - 1) acc[v] += se[(1 * n + j) * 3 + v] * sb->winvN;
-      if (j == 0) acc[v] += se[(2 * n + i) * 3 + v] * sb->winv0;
-      if (j == n - 1) acc[v] += se[(3 * n + i) * 3 + v] * sb->winvN;
+      for (int v = 0; v < 3; ++v) acc[v] = fma(se[((i == 0 ? 0 : 1) * n + j) * 3 + v], w, acc[v]);
+    }
+    if (j == 0 || j == n - 1) {
+      const double w = j == 0 ? sb->winv0 : sb->winvN;
+#pragma unroll
+      for (int v = 0; v < 3; ++v) acc[v] = fma(se[((j == 0 ? 2 : 3) * n + i) * 3 + v], w, acc[v]);
     }
     double s[3];
     {
@@ -468,9 +501,9 @@ TAG_DEV void cov_element_body(const CovParams& P, const CovGroup& G, int lblk,
 #pragma unroll
     for (int v = 0; v < 3; ++v) {
       dv[v] = acc[v] * fac + s[v];
-      if (!isfinite(dv[v])) bad |= TAG_S_NAN;
+      if (not_finite(dv[v])) bad |= TAG_S_NAN;
     }
-    if (!(ui[0] > 0.0)) bad |= TAG_S_NEG_DENSITY;
+    if (not_positive(ui[0])) bad |= TAG_S_NEG_DENSITY;
     if (MODE == kModeRhs) {
 #pragma unroll
       for (int v = 0; v < 3; ++v) du[gq * 3 + v] = dv[v];
@@ -504,19 +537,31 @@ TAG_DEV void cov_element_body(const CovParams& P, const CovGroup& G, int lblk,
     // CFL speeds of the updated state, scaled by n: dt = cfl 2 / (n max_e(l1 + l2))
     __syncthreads();
     if (act) {
-      const double ihn = 1.0 / un[0];
-      qn[0] = fabs(un[1] * ihn) + sqrt(__ldg(pg + kPGc11) * un[0] * P.g);
-      qn[1] = fabs(un[2] * ihn) + sqrt(__ldg(pg + kPGc22) * un[0] * P.g);
+      const double ihn = int_rcp(un[0]);
+      qn[0] = fabs(un[1] * ihn) + int_sqrt(__ldg(pg + kPGc11) * un[0] * P.g);
+      qn[1] = fabs(un[2] * ihn) + int_sqrt(__ldg(pg + kPGc22) * un[0] * P.g);
+    }
+    // maxima over the rows, then over the element's rows
+    __syncthreads();
+    if (act && i == 0) {
+      double m1 = 0.0, m2 = 0.0;
+#pragma unroll
+      for (int k = 0; k < n; ++k) {
+        m1 = fmax(m1, qn[k * kCovQ]);
+        m2 = fmax(m2, qn[k * kCovQ + 1]);
+      }
+      qn[2] = m1;
+      qn[3] = m2;
     }
     __syncthreads();
-    if (threadIdx.x < ne) {
-      const double* eq = q + threadIdx.x * nn * kCovQ;
+    if (act && node == 0) {
       double m1 = 0.0, m2 = 0.0;
-      for (int k = 0; k < nn; ++k) {
-        m1 = fmax(m1, eq[k * kCovQ]);
-        m2 = fmax(m2, eq[k * kCovQ + 1]);
+#pragma unroll
+      for (int k = 0; k < n; ++k) {
+        m1 = fmax(m1, qn[k * n * kCovQ + 2]);
+        m2 = fmax(m2, qn[k * n * kCovQ + 3]);
       }
-      const int e = G.e0 + el_first + threadIdx.x;
+      const int e = G.e0 + el_first + el;
       atomic_max_nonneg(st.max_speed + (st.member ? st.member[e] : 0), n * (m1 + m2));
     }
   }
@@ -551,13 +596,15 @@ __global__ void __launch_bounds__(256, 3) k_cov_element(CovParams P, const CovGr
   if (bad) atomicOr(status, bad);
 }
 
-// scaled CFL speed n max_e(l1 + l2) of a host-set state, per member
+// scaled CFL speed n max_e(l1 + l2) of a host-set state, per member: one warp
+// per element (blockDim a multiple of 32), the lanes stride over its nodes
 __global__ void k_cov_max_speed(CovParams P, const CovGroups* __restrict__ GG,
                                 const double* __restrict__ u, const double* __restrict__ pk,
                                 const int* __restrict__ member, double* __restrict__ max_speed,
                                 int nelem) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nelem) return;
+  const int lane = threadIdx.x & 31;
+  const int e = (int)(((long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (e >= nelem) return;  // warp-uniform
   int gi = 0;
   for (int k = 1; k < GG->count; ++k)
     if (GG->g[k].e0 <= e) gi = k;
@@ -565,13 +612,19 @@ __global__ void k_cov_max_speed(CovParams P, const CovGroups* __restrict__ GG,
   const int n = G.n, nn = n * n;
   const long q0 = G.node0 + (long)(e - G.e0) * nn;
   double m1 = 0.0, m2 = 0.0;
-  for (int node = 0; node < nn; ++node) {
+  for (int node = lane; node < nn; node += 32) {
     const double* uq = u + (q0 + node) * 3;
     const double* p = pk + (q0 + node) * kPack;
-    m1 = fmax(m1, fabs(uq[1] / uq[0]) + sqrt(p[kPGc11] * uq[0] * P.g));
-    m2 = fmax(m2, fabs(uq[2] / uq[0]) + sqrt(p[kPGc22] * uq[0] * P.g));
+    const double ih = int_rcp(uq[0]);
+    m1 = fmax(m1, fabs(uq[1] * ih) + int_sqrt(p[kPGc11] * uq[0] * P.g));
+    m2 = fmax(m2, fabs(uq[2] * ih) + int_sqrt(p[kPGc22] * uq[0] * P.g));
   }
-  atomic_max_nonneg(max_speed + (member ? member[e] : 0), n * (m1 + m2));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    m1 = fmax(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+    m2 = fmax(m2, __shfl_xor_sync(0xffffffffu, m2, o));
+  }
+  if (lane == 0) atomic_max_nonneg(max_speed + (member ? member[e] : 0), n * (m1 + m2));
 }
 
 }  // namespace tag

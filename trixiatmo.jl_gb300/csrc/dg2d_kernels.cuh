@@ -22,6 +22,7 @@ struct BasisDev {
   double winv0, winvN;               // 1 / w_0, 1 / w_N
   double Dh[kMaxNodes * kMaxNodes];  // D_hat[a * n + b] (weak form)
   FxBasis fx;                        // Dsplit in fixed point
+  double Dsum[kMaxNodes];            // row sums of Dsplit without the diagonal
 };
 
 enum VolumeKind : int { kVolFluxDiff = 0, kVolWeak = 1 };

@@ -64,6 +64,9 @@ void load_basis(BasisDev& b, const double* dsplit_colmajor, const double* w, int
   b.winv0 = 1.0 / w[0];
   b.winvN = 1.0 / w[n - 1];
   load_fixed_basis(b.fx, b.Ds, w, n);
+  for (int a = 0; a < n; ++a)
+    for (int c = 0; c < n; ++c)
+      if (c != a) b.Dsum[a] += b.Ds[a * n + c];
   // D_hat = -M^{-1} D^T M from D_split = 2 D - M^{-1} B:
   //   D[a][c] = (Ds[a][c] + (M^{-1} B)[a][c]) / 2,  D_hat[a][c] = -D[c][a] w_c / w_a
   for (int a = 0; a < n; ++a)
@@ -246,7 +249,7 @@ int cov_element(tag_handle h, int mode, double* u, double* du, int stage, bool l
 }
 
 int cov_max_speed(tag_handle h, const double* u) {
-  k_cov_max_speed<<<(h->nelem + 127) / 128, 128, 0, h->stream>>>(
+  k_cov_max_speed<<<(h->nelem + 7) / 8, 256, 0, h->stream>>>(  // a warp per element
       h->p_cov, h->d_groups, u, h->d_pk, h->d_member, h->d_mscal + 2 * h->nmembers, h->nelem);
   TAG_CUDA(cudaGetLastError());
   return TAG_OK;
@@ -443,7 +446,7 @@ int create_cov(const tag_config* cfgs, int m, tag_handle* out) {
   if (cudaMallocHost(&h->h_pin, sizeof(double) * (3 * m + 2)) != cudaSuccess)
     return cleanup(fail(TAG_E_CUDA, "pinned alloc failed"));
   k_cov_pack<<<(unsigned)((nodes + 255) / 256), 256, 0, h->stream>>>(h->d_aux, h->d_xy, nodes,
-                                                                      omega, h->d_pk);
+                                                                      omega, P.split, h->d_pk);
   if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(h->stream) != cudaSuccess)
     return cleanup(fail(TAG_E_CUDA, "upload failed"));
   {
