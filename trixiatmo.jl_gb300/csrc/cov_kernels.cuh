@@ -85,26 +85,25 @@ __global__ void k_cov_pack(const double* __restrict__ aux, const double* __restr
 }
 
 // ---- pointwise physics on packed data -----------------------------------------
-TAG_DEV double cov_gcon(const double* p, int i, int j) {
-  return (i == 0 && j == 0) ? p[kPGc11] : (i == 1 && j == 1) ? p[kPGc22] : p[kPGc12];
-}
-
-// contravariant flux component o of one node (standard or split form); ih = 1/h
-TAG_DEV void cov_flux(const CovParams& P, const double* u, double ih, const double* p, int o,
-                      double* f) {
-  const double J = p[kPJ];
-  const double m = J * u[1 + o];
-  if (P.split) {
-    f[0] = m;
-    f[1] = m * (u[1] * ih);
-    f[2] = m * (u[2] * ih);
-    return;
+// contravariant fluxes of one node (standard or split form) in both directions,
+// F[0..2] and F[3..5]: the momentum part is the symmetric J (hv (x) v), plus
+// J G_con g h^2/2 in the standard form; ih = 1/h
+TAG_DEV void cov_flux(const CovParams& P, const double* u, double ih, const double* p, double* F) {
+  const double m1 = p[kPJ] * u[1], m2 = p[kPJ] * u[2];
+  const double v1 = u[1] * ih, v2 = u[2] * ih;
+  double T11 = m1 * v1, T12 = m1 * v2, T22 = m2 * v2;
+  if (!P.split) {
+    const double gt = p[kPJ] * (0.5 * P.g * u[0] * u[0]);
+    T11 = fma(p[kPGc11], gt, T11);
+    T12 = fma(p[kPGc12], gt, T12);
+    T22 = fma(p[kPGc22], gt, T22);
   }
-  const double vo = u[1 + o] * ih;
-  const double gt = 0.5 * P.g * u[0] * u[0];
-  f[0] = m;
-  f[1] = J * (u[1] * vo + cov_gcon(p, 0, o) * gt);
-  f[2] = J * (u[2] * vo + cov_gcon(p, 1, o) * gt);
+  F[0] = m1;
+  F[1] = T11;
+  F[2] = T12;
+  F[3] = m2;
+  F[4] = T12;
+  F[5] = T22;
 }
 
 // source_terms_geometric_coriolis (standard or split), after apply_jacobian,
@@ -128,158 +127,194 @@ TAG_DEV void cov_source(const CovParams& P, const double* u, double ih, const do
 }
 
 // ---- interface fluxes ------------------------------------------------------------
-// Geometry of one side of an interface node (the reference's aux layout: A
-// column-major at 0..5, the contravariant basis column-major at 6..11, J at
-// 12, G_11 G_12 G_22 at 13..15, G^11 G^12 G^22 at 16..18).
-struct CovSide {
-  double A[6], Ac[6], J, gv11, gv12, gv22, gc11, gc12, gc22;
+// Geometry of the two sides of an interface node, packed once per handle from
+// the reference's aux layout (A column-major at 0..5, the contravariant basis
+// column-major at 6..11, J at 12, G_11 G_12 G_22 at 13..15, G^11 G^12 G^22 at
+// 16..18) for the face normal o of the side:
+//   M: the other side's (hv^1, hv^2) in this side's basis, row-major;
+//   J with the face's outward sign, G^{1o}, G^{2o}, sqrt(g G^{oo});
+//   E = G_con G_cov - 1 (rounding of the stored metric), row-major.
+// In place of 19 numbers of either node: 76 instead of 160 FP64 operations per
+// interface node (the FP64 pipe is the bound).  Arrays of kIfSide values per side, the
+// interface nodes contiguous, so a warp's loads are coalesced.
+enum CovIfPack : int {
+  kIM = 0, kIJ = 4, kIG1, kIG2, kISpeed, kIE = 8, kIfSide = 12, kIfPack = 2 * kIfSide
 };
 
-TAG_DEV void cov_load_side(const double* __restrict__ a, CovSide& s) {
-#pragma unroll
-  for (int k = 0; k < 6; ++k) {
-    s.A[k] = a[k];
-    s.Ac[k] = a[6 + k];
-  }
-  s.J = a[12];
-  s.gv11 = a[13]; s.gv12 = a[14]; s.gv22 = a[15];
-  s.gc11 = a[16]; s.gc12 = a[17]; s.gc22 = a[18];
+struct CovIfNode {
+  int e0, e1, f0, f1, l1;
+  long q0, q1;  // nodes of the two sides
+};
+TAG_DEV CovIfNode cov_if_node(const CovGroup& G, int n, int k, int l,
+                              const int* __restrict__ if_e, const int* __restrict__ if_f,
+                              const int* __restrict__ if_flip) {
+  CovIfNode r;
+  const int kk = G.if0 + k;
+  r.e0 = if_e[2 * kk];
+  r.e1 = if_e[2 * kk + 1];
+  r.f0 = if_f[2 * kk];
+  r.f1 = if_f[2 * kk + 1];
+  r.l1 = if_flip[kk] ? n - 1 - l : l;
+  int i0, j0, i1, j1;
+  face_node(r.f0, l, n, i0, j0);
+  face_node(r.f1, r.l1, n, i1, j1);
+  r.q0 = G.node0 + (long)(r.e0 - G.e0) * n * n + j0 * n + i0;
+  r.q1 = G.node0 + (long)(r.e1 - G.e0) * n * n + j1 * n + i1;
+  return r;
 }
 
-// state of another node in the contravariant basis of `to`
-TAG_DEV void cov_transform(const double* u, const CovSide& from, const CovSide& to, double* s) {
-  double gl[3];
-#pragma unroll
-  for (int r = 0; r < 3; ++r) gl[r] = from.A[r] * u[1] + from.A[3 + r] * u[2];
-  s[0] = u[0];
-#pragma unroll
-  for (int r = 0; r < 2; ++r) s[1 + r] = to.Ac[r] * gl[0] + to.Ac[2 + r] * gl[1] + to.Ac[4 + r] * gl[2];
+// one side: `mine` and `other` aux rows, face f of `mine`
+TAG_DEV void cov_pack_side(const double* mine, const double* other, int f, double g,
+                           double* __restrict__ p, long stride) {
+  const int o = f >> 1;
+  for (int r = 0; r < 2; ++r)
+    for (int c = 0; c < 2; ++c)
+      p[(kIM + 2 * r + c) * stride] = mine[6 + r] * other[3 * c] + mine[8 + r] * other[3 * c + 1] +
+                                      mine[10 + r] * other[3 * c + 2];
+  const double v11 = mine[13], v12 = mine[14], v22 = mine[15];
+  const double c11 = mine[16], c12 = mine[17], c22 = mine[18];
+  p[kIJ * stride] = f & 1 ? mine[12] : -mine[12];
+  p[kIG1 * stride] = o ? c12 : c11;
+  p[kIG2 * stride] = o ? c22 : c12;
+  p[kISpeed * stride] = sqrt(g * (o ? c22 : c11));
+  p[(kIE + 0) * stride] = fma(c11, v11, fma(c12, v12, -1.0));
+  p[(kIE + 1) * stride] = fma(c11, v12, c12 * v22);
+  p[(kIE + 2) * stride] = fma(c12, v11, c22 * v12);
+  p[(kIE + 3) * stride] = fma(c12, v12, fma(c22, v22, -1.0));
 }
 
-// surface flux (+ 0.5 nonconservative) along o of left state a and right
-// state c, both sides' geometry `w` (the reference passes aux_vars_ll twice);
-// iha = 1 / a[0], ihc = 1 / c[0]
-TAG_DEV void cov_surface(const CovParams& P, const double* a, const double* c, double iha,
-                         double ihc, const CovSide& w, int o, double* F) {
-  const double J = w.J;
-  const double gco0 = o ? w.gc12 : w.gc11;  // G^{1o}
-  const double gco1 = o ? w.gc22 : w.gc12;  // G^{2o}
-  const double ao = o ? a[2] : a[1], co = o ? c[2] : c[1];
-  const double va1 = a[1] * iha, va2 = a[2] * iha, vc1 = c[1] * ihc, vc2 = c[2] * ihc;
-  const double vao = o ? va2 : va1, vco = o ? vc2 : vc1;
+// grid as k_cov_interface
+__global__ void k_cov_pack_interfaces(double g, const CovGroups* __restrict__ GG,
+                                      const double* __restrict__ aux,
+                                      const int* __restrict__ if_e, const int* __restrict__ if_f,
+                                      const int* __restrict__ if_flip, long nodes,
+                                      double* __restrict__ ipk) {
+  const CovGroup& G = GG->g[cov_find_group(*GG, blockIdx.x, true)];
+  const int t = (blockIdx.x - G.iblk0) * blockDim.x + threadIdx.x;
+  const int n = G.n;
+  if (t >= G.nif * n) return;
+  const CovIfNode r = cov_if_node(G, n, t / n, t % n, if_e, if_f, if_flip);
+  double* p = ipk + G.ifnode0 + t;
+  cov_pack_side(aux + r.q0 * 26, aux + r.q1 * 26, r.f0, g, p, nodes);
+  cov_pack_side(aux + r.q1 * 26, aux + r.q0 * 26, r.f1, g, p + kIfSide * nodes, nodes);
+}
+
+// Outward surface flux (+ 0.5 nonconservative) of one side, face f, in its own
+// basis and with its own geometry p[kIfSide] for both states (the reference
+// passes aux_vars_ll twice).  mine, w: this side's state and the other's in this
+// side's basis; their reciprocals and square roots of h; hph = g h h' / 2.
+TAG_DEV void cov_side_flux(const CovParams& P, const double* mine, const double* w, double ihm,
+                           double ihw, double sqm, double sqw, double hph, int f,
+                           const double* p, double* F) {
+  const bool second = f >> 1, plus = f & 1;
+  // a: left state, c: right state along the face's direction
+  const double a0 = plus ? mine[0] : w[0], c0 = plus ? w[0] : mine[0];
+  const double a1 = plus ? mine[1] : w[1], c1 = plus ? w[1] : mine[1];
+  const double a2 = plus ? mine[2] : w[2], c2 = plus ? w[2] : mine[2];
+  const double iha = plus ? ihm : ihw, ihc = plus ? ihw : ihm;
+  const double va1 = a1 * iha, va2 = a2 * iha, vc1 = c1 * ihc, vc2 = c2 * ihc;
+  const double ao = second ? a2 : a1, co = second ? c2 : c1;
+  const double vao = second ? va2 : va1, vco = second ? vc2 : vc1;
+  const double g1 = p[kIG1], g2 = p[kIG2];
+  double F0 = 0.5 * (ao + co), F1, F2;
   if (P.surf_sym == 1) {
-    const double m = 0.5 * (J * ao + J * co);
-    F[0] = m;
-    F[1] = 0.5 * (va1 + vc1) * m;
-    F[2] = 0.5 * (va2 + vc2) * m;
-  } else if (P.split) {
-    const double ma = J * ao, mc = J * co;
-    F[0] = 0.5 * (ma + mc);
-    F[1] = 0.5 * (ma * va1 + mc * vc1);
-    F[2] = 0.5 * (ma * va2 + mc * vc2);
+    const double hm = 0.5 * F0;
+    F1 = (va1 + vc1) * hm;
+    F2 = (va2 + vc2) * hm;
   } else {
-    const double ga = 0.5 * P.g * a[0] * a[0], gc = 0.5 * P.g * c[0] * c[0];
-    F[0] = 0.5 * (J * ao + J * co);
-    F[1] = 0.5 * (J * (a[1] * vao + gco0 * ga) + J * (c[1] * vco + gco0 * gc));
-    F[2] = 0.5 * (J * (a[2] * vao + gco1 * ga) + J * (c[2] * vco + gco1 * gc));
+    F1 = 0.5 * fma(ao, va1, co * vc1);
+    F2 = 0.5 * fma(ao, va2, co * vc2);
+    if (!P.split) {
+      const double gt = 0.25 * P.g * fma(a0, a0, c0 * c0);
+      F1 = fma(g1, gt, F1);
+      F2 = fma(g2, gt, F2);
+    }
   }
   if (P.surf_diss) {
-    const double goo = o ? w.gc22 : w.gc11;
-    const double lam = fmax(fabs(vao) + int_sqrt(goo * a[0] * P.g), fabs(vco) + int_sqrt(goo * c[0] * P.g));
-    const double s = -0.5 * J * lam;
-    F[0] += s * (c[0] - a[0]);
-    F[1] += s * (c[1] - a[1]);
-    F[2] += s * (c[2] - a[2]);
+    const double s = -0.5 * fmax(fma(plus ? sqm : sqw, p[kISpeed], fabs(vao)),
+                                 fma(plus ? sqw : sqm, p[kISpeed], fabs(vco)));
+    F0 = fma(s, c0 - a0, F0);
+    F1 = fma(s, c1 - a1, F1);
+    F2 = fma(s, c2 - a2, F2);
   }
-  if (P.surf_nc == 1) {
-    // flux_nonconservative_ec with both geometries `w` (no topography jump)
-    const double vcv0 = w.gv11 * vc1 + w.gv12 * vc2;
-    const double vcv1 = w.gv12 * vc1 + w.gv22 * vc2;
-    const double half_m = 0.5 * ao;
-    const double ph = P.g * a[0] * c[0];
-    F[1] += 0.5 * (J * (half_m * (w.gc11 * vcv0 + w.gc12 * vcv1 - vc1) + gco0 * ph));
-    F[2] += 0.5 * (J * (half_m * (w.gc12 * vcv0 + w.gc22 * vcv1 - vc2) + gco1 * ph));
-  } else if (P.surf_nc == 2) {
-    const double ph = P.g * a[0] * c[0];
-    F[1] += 0.5 * (J * (gco0 * ph));
-    F[2] += 0.5 * (J * (gco1 * ph));
+  if (P.surf_nc) {
+    F1 = fma(g1, hph, F1);
+    F2 = fma(g2, hph, F2);
+    if (P.surf_nc == 1) {
+      // flux_nonconservative_ec with one geometry (no topography jump): the
+      // velocity term is hv_a^o / 2 (G_con G_cov - 1) v_c
+      const double q = 0.25 * ao;
+      F1 = fma(q, fma(p[kIE], vc1, p[kIE + 1] * vc2), F1);
+      F2 = fma(q, fma(p[kIE + 2], vc1, p[kIE + 3] * vc2), F2);
+    }
   }
-}
-
-// outward flux of one side (face f of its element)
-// ih_mine = 1 / mine[0], ih_other = 1 / other_in_mine[0] (the transformation
-// keeps h), each computed once per interface node
-TAG_DEV void cov_side_flux(const CovParams& P, const double* mine, const double* other_in_mine,
-                           double ih_mine, double ih_other, const CovSide& w, int f, double* F) {
-  const int o = f >> 1;
-  if ((f & 1) == 0) {
-    cov_surface(P, other_in_mine, mine, ih_other, ih_mine, w, o, F);
-    F[0] = -F[0];
-    F[1] = -F[1];
-    F[2] = -F[2];
-  } else {
-    cov_surface(P, mine, other_in_mine, ih_mine, ih_other, w, o, F);
-  }
+  const double J = p[kIJ];
+  F[0] = J * F0;
+  F[1] = J * F1;
+  F[2] = J * F2;
 }
 
 template <int n>
-TAG_DEV void cov_interface_body(const CovParams& P, const CovGroup& G, int lblk, const double* u,
-                                const double* aux, const int* if_e, const int* if_f,
-                                const int* if_flip, double* sfv) {
+TAG_DEV void cov_interface_body(const CovParams& P, const CovGroup& G, int lblk,
+                                const double* __restrict__ u, const double* __restrict__ ipk,
+                                long nodes, const int* __restrict__ if_e,
+                                const int* __restrict__ if_f, const int* __restrict__ if_flip,
+                                double* __restrict__ sfv) {
   const int t = lblk * blockDim.x + threadIdx.x;
   const int k = t / n, l = t % n;
   if (k >= G.nif) return;
-  const int kk = G.if0 + k;
-  const int e0 = if_e[2 * kk], e1 = if_e[2 * kk + 1];
-  const int f0 = if_f[2 * kk], f1 = if_f[2 * kk + 1];
-  const int l1 = if_flip[kk] ? n - 1 - l : l;
-  int i0, j0, i1, j1;
-  face_node(f0, l, n, i0, j0);
-  face_node(f1, l1, n, i1, j1);
-  const long q0 = G.node0 + (long)(e0 - G.e0) * n * n + j0 * n + i0;
-  const long q1 = G.node0 + (long)(e1 - G.e0) * n * n + j1 * n + i1;
-  double ul[3], ur[3];
+  double p[kIfPack];
+#pragma unroll
+  for (int j = 0; j < kIfPack; ++j)
+    p[j] = (j % kIfSide < kIE || P.surf_nc == 1) ? __ldg(ipk + j * nodes + G.ifnode0 + t) : 0.0;
+  const CovIfNode r = cov_if_node(G, n, k, l, if_e, if_f, if_flip);
+  double ul[3], ur[3], rt[3], lt[3], Fl[3], Fr[3];
 #pragma unroll
   for (int v = 0; v < 3; ++v) {
-    ul[v] = u[q0 * 3 + v];
-    ur[v] = u[q1 * 3 + v];
+    ul[v] = u[r.q0 * 3 + v];
+    ur[v] = u[r.q1 * 3 + v];
   }
-  CovSide al, ar;
-  cov_load_side(aux + q0 * 26, al);
-  cov_load_side(aux + q1 * 26, ar);
-  double rt[3], lt[3], Fp[3], Fs[3];
-  cov_transform(ur, ar, al, rt);
-  cov_transform(ul, al, ar, lt);
+  const double* pr = p + kIfSide;
+  rt[0] = ur[0];
+  rt[1] = fma(p[kIM], ur[1], p[kIM + 1] * ur[2]);
+  rt[2] = fma(p[kIM + 2], ur[1], p[kIM + 3] * ur[2]);
+  lt[0] = ul[0];
+  lt[1] = fma(pr[kIM], ul[1], pr[kIM + 1] * ul[2]);
+  lt[2] = fma(pr[kIM + 2], ul[1], pr[kIM + 3] * ul[2]);
   const double ihl = int_rcp(ul[0]), ihr = int_rcp(ur[0]);
-  cov_side_flux(P, ul, rt, ihl, ihr, al, f0, Fp);
-  cov_side_flux(P, ur, lt, ihr, ihl, ar, f1, Fs);
-  double* s0 = sfv + G.sf0 + ((long)(e0 - G.e0) * 4 + f0) * n * 3 + l * 3;
-  double* s1 = sfv + G.sf0 + ((long)(e1 - G.e0) * 4 + f1) * n * 3 + l1 * 3;
+  const double sql = P.surf_diss ? int_sqrt(ul[0]) : 0.0;
+  const double sqr = P.surf_diss ? int_sqrt(ur[0]) : 0.0;
+  const double hph = P.surf_nc ? 0.5 * P.g * ul[0] * ur[0] : 0.0;
+  cov_side_flux(P, ul, rt, ihl, ihr, sql, sqr, hph, r.f0, p, Fl);
+  cov_side_flux(P, ur, lt, ihr, ihl, sqr, sql, hph, r.f1, pr, Fr);
+  double* s0 = sfv + G.sf0 + ((long)(r.e0 - G.e0) * 4 + r.f0) * n * 3 + l * 3;
+  double* s1 = sfv + G.sf0 + ((long)(r.e1 - G.e0) * 4 + r.f1) * n * 3 + r.l1 * 3;
 #pragma unroll
   for (int v = 0; v < 3; ++v) {
-    s0[v] = Fp[v];
-    s1[v] = Fs[v];
+    s0[v] = Fl[v];
+    s1[v] = Fr[v];
   }
 }
 
-__global__ void __launch_bounds__(256) k_cov_interface(CovParams P, const CovGroups* __restrict__ GG,
-                                                       const double* __restrict__ u,
-                                                       const double* __restrict__ aux,
-                                                       const int* __restrict__ if_e,
-                                                       const int* __restrict__ if_f,
-                                                       const int* __restrict__ if_flip,
-                                                       double* __restrict__ sfv) {
+// 128-thread CTAs (the interface node counts fill the SMs evenly: 43,200 nodes
+// are 169 CTAs of 256 on 152 SMs)
+constexpr int kCovIfThreads = 128;
+__global__ void __launch_bounds__(kCovIfThreads)
+    k_cov_interface(CovParams P, const CovGroups* __restrict__ GG, const double* __restrict__ u,
+                    const double* __restrict__ ipk, long nodes, const int* __restrict__ if_e,
+                    const int* __restrict__ if_f, const int* __restrict__ if_flip,
+                    double* __restrict__ sfv) {
   const int gi = cov_find_group(*GG, blockIdx.x, true);
   const CovGroup& G = GG->g[gi];
   const int lblk = blockIdx.x - G.iblk0;
   switch (G.n) {
-    case 4: cov_interface_body<4>(P, G, lblk, u, aux, if_e, if_f, if_flip, sfv); break;
-    case 6: cov_interface_body<6>(P, G, lblk, u, aux, if_e, if_f, if_flip, sfv); break;
-    case 8: cov_interface_body<8>(P, G, lblk, u, aux, if_e, if_f, if_flip, sfv); break;
-    case 2: cov_interface_body<2>(P, G, lblk, u, aux, if_e, if_f, if_flip, sfv); break;
-    case 3: cov_interface_body<3>(P, G, lblk, u, aux, if_e, if_f, if_flip, sfv); break;
-    case 5: cov_interface_body<5>(P, G, lblk, u, aux, if_e, if_f, if_flip, sfv); break;
-    case 7: cov_interface_body<7>(P, G, lblk, u, aux, if_e, if_f, if_flip, sfv); break;
+    case 4: cov_interface_body<4>(P, G, lblk, u, ipk, nodes, if_e, if_f, if_flip, sfv); break;
+    case 6: cov_interface_body<6>(P, G, lblk, u, ipk, nodes, if_e, if_f, if_flip, sfv); break;
+    case 8: cov_interface_body<8>(P, G, lblk, u, ipk, nodes, if_e, if_f, if_flip, sfv); break;
+    case 2: cov_interface_body<2>(P, G, lblk, u, ipk, nodes, if_e, if_f, if_flip, sfv); break;
+    case 3: cov_interface_body<3>(P, G, lblk, u, ipk, nodes, if_e, if_f, if_flip, sfv); break;
+    case 5: cov_interface_body<5>(P, G, lblk, u, ipk, nodes, if_e, if_f, if_flip, sfv); break;
+    case 7: cov_interface_body<7>(P, G, lblk, u, ipk, nodes, if_e, if_f, if_flip, sfv); break;
     default: break;
   }
 }
@@ -324,8 +359,7 @@ TAG_DEV void cov_element_body(const CovParams& P, const CovGroup& G, int lblk,
     for (int k = 0; k < kPack; ++k) p[k] = __ldg(pg + k);
     ih = int_rcp(ui[0]);
     if constexpr (VK == 0) {
-      cov_flux(P, ui, ih, p, 0, qn);
-      cov_flux(P, ui, ih, p, 1, qn + 3);
+      cov_flux(P, ui, ih, p, qn);
     } else {
       const double v1 = ui[1] * ih, v2 = ui[2] * ih;
       qn[0] = v1;

@@ -25,6 +25,7 @@ struct CovGroup {
   int epb;       // elements per CTA
   int blk0;      // first CTA of the group in the element launch
   int iblk0;     // first CTA of the group in the interface launch
+  long ifnode0;  // first node of interface if0 in the packed interface geometry
   int basis;     // offset of the group's BasisDev in the basis array
 };
 

@@ -57,7 +57,8 @@ struct tag_handle_s {
   CovGroups h_groups{};
   CovGroups* d_groups = nullptr;
   BasisDev* d_bases = nullptr;
-  double *d_aux = nullptr, *d_pk = nullptr;
+  double *d_aux = nullptr, *d_pk = nullptr, *d_ipk = nullptr;
+  long cov_if_nodes = 0;  // interface nodes packed in d_ipk
   int cov_blocks = 0, cov_iblocks = 0, cov_threads = 0;
   size_t cov_smem = 0;
   PhysEnergy2D::Params p_energy{};

@@ -220,9 +220,9 @@ __global__ void k_fp64_probe(double* out, int iters, double seed) {
 // ---- covariant equations (element groups of possibly different degree) ------
 int cov_interface(tag_handle h, const double* u) {
   if (h->cov_iblocks == 0) return TAG_OK;
-  k_cov_interface<<<h->cov_iblocks, 256, 0, h->stream>>>(h->p_cov, h->d_groups, u, h->d_aux,
-                                                         h->d_if_e, h->d_if_f, h->d_if_flip,
-                                                         h->d_sfv);
+  k_cov_interface<<<h->cov_iblocks, kCovIfThreads, 0, h->stream>>>(
+      h->p_cov, h->d_groups, u, h->d_ipk, h->cov_if_nodes, h->d_if_e, h->d_if_f, h->d_if_flip,
+      h->d_sfv);
   TAG_CUDA(cudaGetLastError());
   return TAG_OK;
 }
@@ -350,6 +350,7 @@ int create_cov(const tag_config* cfgs, int m, tag_handle* out) {
   long node_off = 0, sf_off = 0;
   int e_off = 0, if_off = 0, blk = 0, iblk = 0;
   size_t smem = 0;
+  long if_nodes = 0;
   for (int k = 0; k < m; ++k) {
     const tag_config* c = &cfgs[k];
     const int n = c->polydeg + 1, nn = n * n;
@@ -393,7 +394,9 @@ int create_cov(const tag_config* cfgs, int m, tag_handle* out) {
     g.blk0 = blk;
     blk += (g.ne + g.epb - 1) / g.epb;
     g.iblk0 = iblk;
-    iblk += (g.nif * g.n + 255) / 256;
+    iblk += (g.nif * g.n + kCovIfThreads - 1) / kCovIfThreads;
+    g.ifnode0 = if_nodes;
+    if_nodes += (long)g.nif * g.n;
     smem = std::max(smem, sizeof(double) * (size_t)g.epb * cov_elem_doubles(g.n));
   }
   tag_handle h = new tag_handle_s();
@@ -432,6 +435,9 @@ int create_cov(const tag_config* cfgs, int m, tag_handle* out) {
   if ((rc = upload(&h->d_xy, xyz.data(), xyz.size(), h->stream))) return cleanup(rc);
   if ((rc = upload(&h->d_pk, (const double*)nullptr, (size_t)nodes * kPack, h->stream)))
     return cleanup(rc);
+  h->cov_if_nodes = if_nodes;
+  if ((rc = upload(&h->d_ipk, (const double*)nullptr, (size_t)if_nodes * kIfPack, h->stream)))
+    return cleanup(rc);
   if ((rc = upload(&h->d_sfv, (const double*)nullptr, (size_t)sf, h->stream))) return cleanup(rc);
   if ((rc = upload(&h->d_if_e, ie.data(), ie.size(), h->stream))) return cleanup(rc);
   if ((rc = upload(&h->d_if_f, ifc.data(), ifc.size(), h->stream))) return cleanup(rc);
@@ -447,6 +453,9 @@ int create_cov(const tag_config* cfgs, int m, tag_handle* out) {
     return cleanup(fail(TAG_E_CUDA, "pinned alloc failed"));
   k_cov_pack<<<(unsigned)((nodes + 255) / 256), 256, 0, h->stream>>>(h->d_aux, h->d_xy, nodes,
                                                                       omega, P.split, h->d_pk);
+  if (iblk > 0)
+    k_cov_pack_interfaces<<<iblk, kCovIfThreads, 0, h->stream>>>(
+        P.g, h->d_groups, h->d_aux, h->d_if_e, h->d_if_f, h->d_if_flip, if_nodes, h->d_ipk);
   if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(h->stream) != cudaSuccess)
     return cleanup(fail(TAG_E_CUDA, "upload failed"));
   {
@@ -893,6 +902,7 @@ int tag_destroy(tag_handle h) {
   if (h->d_an_rng) cudaFree(h->d_an_rng);
   if (h->d_aux) cudaFree(h->d_aux);
   if (h->d_pk) cudaFree(h->d_pk);
+  if (h->d_ipk) cudaFree(h->d_ipk);
   if (h->d_groups) cudaFree(h->d_groups);
   if (h->d_bases) cudaFree(h->d_bases);
   if (h->d_mlp) cudaFree(h->d_mlp);
