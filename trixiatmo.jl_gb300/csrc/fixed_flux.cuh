@@ -285,8 +285,12 @@ TAG_DEV i64 fx_weighted_sum(const i64* A, int stride, const i64* W, const int* n
 }
 
 // c with factor = 1 - c (Q0.64) of a logarithmic mean of two words of one scale
-// from the difference of the logarithms; the far branch divides in FP64.
+// from the difference of the logarithms; beyond a factor of 256 the far branch
+// divides in FP64.
 static __device__ __noinline__ u64 fx_far_deficit(i64 a, i64 b, i64 d, int inverse) {
+  const u64 m = magnitude(d);
+  if (middle_range(m))
+    return inverse ? inv_ln_mean_deficit_middle(m) : ln_mean_deficit_middle(m);
   const double x = (double)a, y = (double)b;
   const double f = inverse ? inv_ln_factor_far(x, y, d) : ln_factor_far(x, y, d);
   return f < 1.0 && f > 0.0 ? (u64)((1.0 - f) * 18446744073709551616.0) : 0;

@@ -7,8 +7,9 @@
 //
 // The Stolarsky mean S(x, y) = (gamma-1)/gamma (y^g - x^g) / (y^(g-1) - x^(g-1))
 // (Winters et al. 2020) is (x+y)/2 times an even function of log(y/x), evaluated
-// as its series on the integer pipe for values within a factor of two
-// (int_math.cuh); beyond that, and for gamma outside (1, 2), from powers.
+// as its series on the integer pipe for values within a factor of two and from
+// exponentials of the logarithms' difference up to 256 (int_math.cuh); beyond
+// that, and for gamma outside (1, 2), from powers.
 #pragma once
 #include "tag_common.cuh"
 
@@ -34,6 +35,7 @@ struct PhysPT2D {
     double sc[8];                        // Stolarsky series in f^2 (gamma outside (1, 2))
     EvenSeries stol;                     // Stolarsky factor of the logarithms' difference
     u64 gamma_q61;                       // gamma as int_pow takes it
+    u64 stol_q64;                        // 2 (gamma - 1) / gamma, 0: no middle range
     int volume;                          // 0 flux_tec, 1 flux_ec, 2 flux_etec,
                                          // 3 flux_kennedy_gruber (3D only)
     int nc;                              // 0 waruszewski, 1 artiano, 2 souza
@@ -56,6 +58,10 @@ struct PhysPT2D {
     q.stol_fac = (q.gamma - 1.0) / q.gamma;
     q.stol = stolarsky_series(q.gamma);
     q.gamma_q61 = pow_exponent(q.gamma);
+    // (stolarsky_deficit_middle's range)
+    q.stol_q64 = q.gamma >= 1.3 && q.gamma <= 1.9
+                     ? (u64)ldexpl(2.0L * ((long double)q.gamma - 1.0L) / q.gamma, 64)
+                     : 0;
     q.nc = (int)p[4];
     q.volume = (int)p[5];
     q.surface = (int)p[6];
@@ -107,9 +113,14 @@ struct PhysPT2D {
     if (not_positive(u[3])) bad |= TAG_S_NEG_PRESSURE;
   }
 
-  // Stolarsky mean over the arithmetic mean, from the values themselves: the
-  // series in f^2 where they nearly agree, else powers
-  static __device__ __noinline__ double stolarsky_factor_far(const Params& P, double x, double y) {
+  // Stolarsky mean over the arithmetic mean beyond a factor of two: up to 256
+  // from the logarithms' difference (a: its magnitude), else from the values
+  // themselves, the series in f^2 where they nearly agree (gamma outside (1, 2)),
+  // else powers
+  static __device__ __noinline__ double stolarsky_factor_far(const Params& P, double x, double y,
+                                                             u64 a) {
+    if (P.stol.ok && P.stol_q64 && middle_range(a))
+      return middle_factor(stolarsky_deficit_middle(a, P.gamma_q61, P.stol_q64));
     const double s = x + y, d = y - x;
     const double t = d / s, f2 = t * t;
     if (f2 < 1e-2) {
@@ -124,7 +135,7 @@ struct PhysPT2D {
   TAG_DEV static double stolarsky_factor(const Params& P, double x, double y, i64 d) {
     const u64 a = magnitude(d);
     return series_in_range(a) && P.stol.ok ? even_factor(P.stol, log_square(a))
-                                           : stolarsky_factor_far(P, x, y);
+                                           : stolarsky_factor_far(P, x, y, a);
   }
   TAG_DEV static double stolarsky(const Params& P, double x, double y) {
     return 0.5 * (x + y) * stolarsky_factor(P, x, y, log2_fixed(y) - log2_fixed(x));

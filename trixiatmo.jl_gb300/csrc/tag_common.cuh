@@ -21,8 +21,9 @@ constexpr int kMaxNodes = 8;  // n = polydeg + 1 supported up to polydeg 7
 //   ln_mean(xa, xb) = (xa + xb)/2 R,  inv_ln_mean(1/ya, 1/yb) = (ya + yb)/2 Q.
 // Values within a factor of two (every pair of an element that resolves its
 // stratification) take the integer series, whatever their size: no reciprocal,
-// no logarithm, no branch that splits a warp.  Beyond it d itself is the
-// logarithm: |d| >= 1, so its 2^-52 is a relative error of the same size.
+// no logarithm, no branch that splits a warp.  Up to a factor of 256 (vertical
+// pairs of elements some 5 km tall and more, edges of clouds) an exponential of d
+// and a reciprocal in words; beyond, d itself is the logarithm of the definition.
 TAG_DEV double log_of_difference(i64 d) { return (double)d * 1.539095918623324e-16; }  // ln2 2^-52
 
 // (Values of opposite sign, which a moisture density may have, give NaN: the
@@ -30,9 +31,13 @@ TAG_DEV double log_of_difference(i64 d) { return (double)d * 1.539095918623324e-
 TAG_DEV bool opposite_signs(double a, double b) { return (i64)(f64_bits(a) ^ f64_bits(b)) < 0; }
 static __device__ __noinline__ double ln_factor_far(double xa, double xb, i64 d) {
   if (opposite_signs(xa, xb)) return f64_from(0x7ff8000000000000ull);
+  const u64 a = magnitude(d);
+  if (middle_range(a)) return middle_factor(ln_mean_deficit_middle(a));
   return int_div(2.0 * (xb - xa), log_of_difference(d) * (xa + xb));
 }
 static __device__ __noinline__ double inv_ln_factor_far(double ya, double yb, i64 d) {
+  const u64 a = magnitude(d);
+  if (middle_range(a)) return middle_factor(inv_ln_mean_deficit_middle(a));
   return int_div(2.0 * ya * yb * log_of_difference(d), (yb - ya) * (ya + yb));
 }
 TAG_DEV double ln_factor(double xa, double xb, i64 d) {
