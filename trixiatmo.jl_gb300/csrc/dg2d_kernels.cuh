@@ -242,7 +242,8 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
       u32 m[kMxCount] = {};
       for (int node = lane; node < nn; node += 32) {
         const double *q = eb + S::oQ + node * NQ, *ja = eb + S::oJa + node * 4;
-        m[kMxV] = max(m[kMxV], max(high_magnitude(q[1]), high_magnitude(q[2])));
+        m[kMxV] = max(m[kMxV], high_magnitude(q[1]));
+        m[kMxV + 1] = max(m[kMxV + 1], high_magnitude(q[2]));
         // the words' products take densities as positive: bad states leave
         m[kMxRho] = max(m[kMxRho], not_positive(q[0]) ? 0x7ff00000u : high_magnitude(q[0]));
         m[kMxP] = max(m[kMxP], high_magnitude(q[3]));
@@ -265,7 +266,7 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
       }
 #pragma unroll
       for (int k = 0; k < kMxCount; ++k) {
-        const bool used = k < kMxN + 2 || (k >= kMxF && (k - kMxF) % 3 < 2);
+        const bool used = k < kMxRho ? k < 2 : k < kMxN || (k - kMxN) % 3 < 2;
         if (used) m[k] = __reduce_max_sync(0xffffffffu, m[k]);
       }
       // (the pair slots are not in use yet)

@@ -181,7 +181,7 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
         q[5] -= 0.25 * eb[S::oU + NV - 1];  // phi of the element's first node
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-          m[kMxV] = max(m[kMxV], high_magnitude(q[1 + d]));
+          m[kMxV + d] = high_magnitude(q[1 + d]);
 #pragma unroll
           for (int c = 0; c < 3; ++c)
             m[kMxN + d] = max(m[kMxN + d], high_magnitude(eb[S::oJa + node * 9 + 3 * d + c]));
