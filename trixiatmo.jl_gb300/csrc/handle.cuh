@@ -37,6 +37,16 @@ struct Ops;
 // Threads of an element-kernel CTA: `items` work items split `div` ways,
 // rounded up to whole warps.
 inline int cta_threads(int items, int div) { return ((items + div - 1) / div + 31) / 32 * 32; }
+// Threads of an interface-kernel CTA for `total` interface nodes: the largest of
+// 256 to 32 that still gives each of the 152 SMs a CTA.  A small mesh's few CTAs
+// of 256 would queue eight warps on one SM's FP64 pipe and leave the others idle:
+// 60 x 8 elements, polydeg 3 (3,936 nodes): 80 stages 1.68 ms with 16 CTAs of
+// 256, 1.60 ms with 123 of 32; dry 64 x 32 elements, 100 stages: 2.17 -> 2.01 ms.
+inline int interface_threads(long total) {
+  int t = 256;
+  while (t > 32 && total <= 152L * t) t /= 2;
+  return t;
+}
 // Tiles of the 3D kernels: div 1 to 3 as above; 4 to 6 the same rounded up to
 // whole groups of four warps, one for each of the SM's sub-partitions (their
 // registers are separate, so an odd warp can cost a CTA's place on all four).

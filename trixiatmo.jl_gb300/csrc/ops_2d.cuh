@@ -51,7 +51,7 @@ struct OpsImpl {
   static int interface(tag_handle h, const double* u) {
     const int total = (h->nif + h->nbd) * n;
     if (total == 0) return TAG_OK;
-    const int threads = 256;
+    const int threads = interface_threads(total);
     if (h->need_bvals && !h->bvals_set)
       return fail(TAG_E_INVALID, "Dirichlet boundary faces without states (tag_set_boundary_values)");
     k_interface<Phys, n><<<(total + threads - 1) / threads, threads, 0, h->stream>>>(

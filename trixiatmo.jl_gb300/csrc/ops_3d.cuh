@@ -9,7 +9,8 @@ struct OpsImpl3D {
   static int interface(tag_handle h, const double* u) {
     const int total = (h->nif + h->nbd) * n * n;
     if (total == 0) return TAG_OK;
-    k_interface3d<Phys, n><<<(total + 255) / 256, 256, 0, h->stream>>>(
+    const int threads = interface_threads(total);
+    k_interface3d<Phys, n><<<(total + threads - 1) / threads, threads, 0, h->stream>>>(
         params_of<Phys>(h), u, h->d_Ja, h->d_invJ, h->d_if_e, h->d_if_f, h->d_if_flip, h->nif,
         h->d_bd_e, h->d_bd_f, h->nbd, h->d_sfv);
     TAG_CUDA(cudaGetLastError());
