@@ -256,10 +256,9 @@ TAG_DEV void cov_side_flux(const CovParams& P, const double* mine, const double*
 
 template <int n>
 TAG_DEV void cov_interface_body(const CovParams& P, const CovGroup& G, int lblk,
-                                const double* __restrict__ u, const double* __restrict__ ipk,
-                                long nodes, const int* __restrict__ if_e,
-                                const int* __restrict__ if_f, const int* __restrict__ if_flip,
-                                double* __restrict__ sfv) {
+                                const double* u, const double* __restrict__ ipk, long nodes,
+                                const int* __restrict__ if_e, const int* __restrict__ if_f,
+                                const int* __restrict__ if_flip, double* __restrict__ sfv) {
   const int t = lblk * blockDim.x + threadIdx.x;
   const int k = t / n, l = t % n;
   if (k >= G.nif) return;
@@ -269,6 +268,7 @@ TAG_DEV void cov_interface_body(const CovParams& P, const CovGroup& G, int lblk,
     p[j] = (j % kIfSide < kIE || P.surf_nc == 1) ? __ldg(ipk + j * nodes + G.ifnode0 + t) : 0.0;
   const CovIfNode r = cov_if_node(G, n, k, l, if_e, if_f, if_flip);
   double ul[3], ur[3], rt[3], lt[3], Fl[3], Fr[3];
+  wait_for_previous();
 #pragma unroll
   for (int v = 0; v < 3; ++v) {
     ul[v] = u[r.q0 * 3 + v];
@@ -287,6 +287,7 @@ TAG_DEV void cov_interface_body(const CovParams& P, const CovGroup& G, int lblk,
   const double hph = P.surf_nc ? 0.5 * P.g * ul[0] * ur[0] : 0.0;
   cov_side_flux(P, ul, rt, ihl, ihr, sql, sqr, hph, r.f0, p, Fl);
   cov_side_flux(P, ur, lt, ihr, ihl, sqr, sql, hph, r.f1, pr, Fr);
+  release_next();
   double* s0 = sfv + G.sf0 + ((long)(r.e0 - G.e0) * 4 + r.f0) * n * 3 + l * 3;
   double* s1 = sfv + G.sf0 + ((long)(r.e1 - G.e0) * 4 + r.f1) * n * 3 + r.l1 * 3;
 #pragma unroll
@@ -300,7 +301,7 @@ TAG_DEV void cov_interface_body(const CovParams& P, const CovGroup& G, int lblk,
 // are 169 CTAs of 256 on 152 SMs)
 constexpr int kCovIfThreads = 128;
 __global__ void __launch_bounds__(kCovIfThreads)
-    k_cov_interface(CovParams P, const CovGroups* __restrict__ GG, const double* __restrict__ u,
+    k_cov_interface(CovParams P, const CovGroups* __restrict__ GG, const double* u,
                     const double* __restrict__ ipk, long nodes, const int* __restrict__ if_e,
                     const int* __restrict__ if_f, const int* __restrict__ if_flip,
                     double* __restrict__ sfv) {
@@ -331,9 +332,9 @@ __host__ __device__ constexpr int cov_elem_doubles(int n) { return n * n * kCovQ
 // parameter so that each volume kind gets its own register allocation
 template <int n, int MODE, int VK>
 TAG_DEV void cov_element_body(const CovParams& P, const CovGroup& G, int lblk,
-                              const BasisDev* __restrict__ bases, double* __restrict__ u,
+                              const BasisDev* __restrict__ bases, double* u,
                               double* __restrict__ du, double* __restrict__ kreg,
-                              const double* __restrict__ pk, const double* __restrict__ sfv,
+                              const double* __restrict__ pk, const double* sfv,
                               StageArgs st, double* smem, unsigned& bad) {
   constexpr int nn = n * n;
   BasisDev* sb = reinterpret_cast<BasisDev*>(smem);
@@ -352,11 +353,12 @@ TAG_DEV void cov_element_body(const CovParams& P, const CovGroup& G, int lblk,
   double* qn = q + threadIdx.x * kCovQ;
   const double* __restrict__ pg = pk + gq * kPack;  // re-read where needed (L1 hit)
   if (act) {
-#pragma unroll
-    for (int v = 0; v < 3; ++v) ui[v] = u[gq * 3 + v];
     double p[kPack];
 #pragma unroll
     for (int k = 0; k < kPack; ++k) p[k] = __ldg(pg + k);
+    wait_for_previous();
+#pragma unroll
+    for (int v = 0; v < 3; ++v) ui[v] = u[gq * 3 + v];
     ih = int_rcp(ui[0]);
     if constexpr (VK == 0) {
       cov_flux(P, ui, ih, p, qn);
@@ -386,6 +388,7 @@ TAG_DEV void cov_element_body(const CovParams& P, const CovGroup& G, int lblk,
     }
   }
   __syncthreads();
+  release_next();
   double un[3] = {0.0, 0.0, 0.0};
   if (act) {
     const double* eq = q + el * nn * kCovQ;
@@ -606,11 +609,10 @@ TAG_DEV void cov_element_body(const CovParams& P, const CovGroup& G, int lblk,
 template <int MODE, int VK>
 __global__ void __launch_bounds__(256, 3) k_cov_element(CovParams P, const CovGroups* __restrict__ GG,
                                                      const BasisDev* __restrict__ bases,
-                                                     double* __restrict__ u,
-                                                     double* __restrict__ du,
+                                                     double* u, double* __restrict__ du,
                                                      double* __restrict__ kreg,
                                                      const double* __restrict__ pk,
-                                                     const double* __restrict__ sfv, StageArgs st,
+                                                     const double* sfv, StageArgs st,
                                                      unsigned* __restrict__ status) {
   extern __shared__ double smem[];
   const int gi = cov_find_group(*GG, blockIdx.x, false);

@@ -75,7 +75,7 @@ TAG_DEV double stage_value(const StageArgs& st, double uo, double* __restrict__ 
 // ---------------------------------------------------------------------------
 template <class Phys, int n>
 __global__ void __launch_bounds__(256) k_interface(
-    typename Phys::Params P, const double* __restrict__ u, const double* __restrict__ Ja,
+    typename Phys::Params P, const double* u, const double* __restrict__ Ja,
     const double* __restrict__ invJ, const int* __restrict__ if_e, const int* __restrict__ if_f,
     const int* __restrict__ if_flip, int nif, const int* __restrict__ bd_e,
     const int* __restrict__ bd_f, const int* __restrict__ bd_kind, int nbd,
@@ -92,17 +92,19 @@ __global__ void __launch_bounds__(256) k_interface(
     face_node(f1, l1, n, i1, j1);
     const size_t q0 = ((size_t)e0 * n + j0) * n + i0;
     const size_t q1 = ((size_t)e1 * n + j1) * n + i1;
+    const double s = ((invJ[q0] < 0.0) ? -1.0 : 1.0) * ((f0 & 1) ? 1.0 : -1.0);
+    const double n1 = s * Ja[q0 * 4 + 2 * (f0 >> 1)];
+    const double n2 = s * Ja[q0 * 4 + 2 * (f0 >> 1) + 1];
+    wait_for_previous();
     double ul[NV], ur[NV];
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
       ul[v] = u[q0 * NV + v];
       ur[v] = u[q1 * NV + v];
     }
-    const double s = ((invJ[q0] < 0.0) ? -1.0 : 1.0) * ((f0 & 1) ? 1.0 : -1.0);
-    const double n1 = s * Ja[q0 * 4 + 2 * (f0 >> 1)];
-    const double n2 = s * Ja[q0 * 4 + 2 * (f0 >> 1) + 1];
     double F[NA];
     Phys::surface_flux(P, ul, ur, n1, n2, F);
+    release_next();
     double* s0 = sfv + (((size_t)e0 * 4 + f0) * n + l) * NA;
     double* s1 = sfv + (((size_t)e1 * 4 + f1) * n + l1) * NA;
     if constexpr (Phys::kSurfaceNoncons) {
@@ -131,12 +133,13 @@ __global__ void __launch_bounds__(256) k_interface(
     int i, j;
     face_node(f, l, n, i, j);
     const size_t q = ((size_t)e * n + j) * n + i;
-    double ui[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) ui[v] = u[q * NV + v];
     const double sj = (invJ[q] < 0.0) ? -1.0 : 1.0;
     double n1 = sj * Ja[q * 4 + 2 * (f >> 1)];
     double n2 = sj * Ja[q * 4 + 2 * (f >> 1) + 1];
+    wait_for_previous();
+    double ui[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) ui[v] = u[q * NV + v];
     double F[NA];
     // StructuredMesh walls: normal in the +xi/+eta sense, states ordered by
     // the face parity inside boundary_flux, result turned outward here
@@ -196,7 +199,7 @@ template <class Phys, int n, int MODE, int VOL = kVolFluxDiff>
 __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double* __restrict__ u,
                           double* __restrict__ du, double* __restrict__ kreg,
                           const double* __restrict__ Ja, const double* __restrict__ invJ,
-                          const double* __restrict__ sfv, int nelem, int epb, StageArgs st,
+                          const double* sfv, int nelem, int epb, StageArgs st,
                           unsigned* __restrict__ status) {
   using S = ElemSmem<Phys, n>;
   constexpr int NV = Phys::NV, NA = Phys::NA, NQ = Phys::NQ;
@@ -217,8 +220,9 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
     const double b = reinterpret_cast<const double*>(&basis)[t];
     smem[t] = t < kMaxNodes * kMaxNodes ? 0.5 * b : b;
   }
-  copy_in_blocks(base + S::oU, S::per_elem, u + (size_t)e_first * nn * NV, nn * NV, ne);
   copy_in_blocks(base + S::oJa, S::per_elem, Ja + (size_t)e_first * nn * 4, nn * 4, ne);
+  wait_for_previous();
+  copy_in_blocks(base + S::oU, S::per_elem, u + (size_t)e_first * nn * NV, nn * NV, ne);
   copy_in_wait();
   __syncthreads();
 
@@ -374,6 +378,7 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
     }
   }
   __syncthreads();
+  release_next();
 
   // --- phase 3: per (node, variable): slot sums, surface integral, Jacobian,
   //     sources, stage update
@@ -585,6 +590,7 @@ __global__ void __launch_bounds__(MaxSpeedTile<n>::T) k_max_speed(
 // max_speed) (or the fixed dt); reset the speed accumulator for the step's
 // last stage.  max_speed starts at nextfloat(0) like the reference.
 static __global__ void k_begin_step(MemberScalars s, const StepCtl* ctl, int nmembers, int n) {
+  release_next();
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m >= nmembers) return;
   s.t[m] += s.dt[m];

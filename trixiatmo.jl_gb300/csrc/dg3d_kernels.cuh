@@ -53,7 +53,7 @@ TAG_DEV bool round_robin_pair(int n, int r, int s, int& a, int& b) {
 
 template <class Phys, int n>
 __global__ void __launch_bounds__(256) k_interface3d(
-    typename Phys::Params P, const double* __restrict__ u, const double* __restrict__ Ja,
+    typename Phys::Params P, const double* u, const double* __restrict__ Ja,
     const double* __restrict__ invJ, const int* __restrict__ if_e, const int* __restrict__ if_f,
     const int* __restrict__ if_o, int nif, const int* __restrict__ bd_e,
     const int* __restrict__ bd_f, int nbd, double* __restrict__ sfv) {
@@ -71,16 +71,18 @@ __global__ void __launch_bounds__(256) k_interface3d(
     const size_t q0 = (((size_t)e0 * n + k0) * n + j0) * n + i0;
     const size_t q1 = (((size_t)e1 * n + k1) * n + j1) * n + i1;
     double ul[NV], ur[NV], nrm[3];
+    const double s = ((invJ[q0] < 0.0) ? -1.0 : 1.0) * ((f0 & 1) ? 1.0 : -1.0);
+#pragma unroll
+    for (int c = 0; c < 3; ++c) nrm[c] = s * Ja[(q0 * 3 + (f0 >> 1)) * 3 + c];
+    wait_for_previous();
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
       ul[v] = u[q0 * NV + v];
       ur[v] = u[q1 * NV + v];
     }
-    const double s = ((invJ[q0] < 0.0) ? -1.0 : 1.0) * ((f0 & 1) ? 1.0 : -1.0);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) nrm[c] = s * Ja[(q0 * 3 + (f0 >> 1)) * 3 + c];
     double F[NA];
     Phys::surface_flux(P, ul, ur, nrm, F);
+    release_next();
     double* a0 = sfv + ((((size_t)e0 * 6 + f0) * n + l2) * n + l1) * NA;
     double* a1 = sfv + ((((size_t)e1 * 6 + f1) * n + s2) * n + s1) * NA;
 #pragma unroll
@@ -97,11 +99,12 @@ __global__ void __launch_bounds__(256) k_interface3d(
     face_node3d(f, l1, l2, n, i, j, k);
     const size_t q = (((size_t)e * n + k) * n + j) * n + i;
     double ui[NV], nrm[3];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) ui[v] = u[q * NV + v];
     const double s = ((invJ[q] < 0.0) ? -1.0 : 1.0) * ((f & 1) ? 1.0 : -1.0);
 #pragma unroll
     for (int c = 0; c < 3; ++c) nrm[c] = s * Ja[(q * 3 + (f >> 1)) * 3 + c];
+    wait_for_previous();
+#pragma unroll
+    for (int v = 0; v < NV; ++v) ui[v] = u[q * NV + v];
     double F[NA];
     Phys::boundary_flux(P, ui, nrm, F);
     double* a0 = sfv + ((((size_t)e * 6 + f) * n + l2) * n + l1) * NA;
@@ -133,7 +136,7 @@ template <class Phys, int n, int MODE>
 __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, double* __restrict__ u,
                             double* __restrict__ du, double* __restrict__ kreg,
                             const double* __restrict__ Ja, const double* __restrict__ invJ,
-                            const double* __restrict__ sfv, int nelem, int epb, StageArgs st,
+                            const double* sfv, int nelem, int epb, StageArgs st,
                             unsigned* __restrict__ status) {
   using S = ElemSmem3D<Phys, n>;
   constexpr int NV = Phys::NV, NA = Phys::NA, NQ = Phys::NQ;
@@ -157,11 +160,11 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
     for (int t = threadIdx.x; t < ne * kMxCount; t += nthr)
       reinterpret_cast<u32*>(base + t / kMxCount * S::per_elem + S::oF + kFxDoubles)[t % kMxCount] = 0;
   }
-  for (int el = 0; el < ne; ++el) {
-    double* eb = base + el * S::per_elem;
-    copy_in(eb + S::oU, u + (size_t)(e_first + el) * nnn * NV, nnn * NV);
-    copy_in(eb + S::oJa, Ja + (size_t)(e_first + el) * nnn * 9, nnn * 9);
-  }
+  for (int el = 0; el < ne; ++el)
+    copy_in(base + el * S::per_elem + S::oJa, Ja + (size_t)(e_first + el) * nnn * 9, nnn * 9);
+  wait_for_previous();
+  for (int el = 0; el < ne; ++el)
+    copy_in(base + el * S::per_elem + S::oU, u + (size_t)(e_first + el) * nnn * NV, nnn * NV);
   copy_in_wait();
   __syncthreads();
 
@@ -350,6 +353,7 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
     }
   }
   __syncthreads();
+  release_next();
 
   // per node: direction sums (surface integral included), Jacobian, sources,
   // stage update; the new state (or the time derivative) takes the old

@@ -47,6 +47,32 @@ inline int interface_threads(long total) {
   while (t > 32 && total <= 152L * t) t /= 2;
   return t;
 }
+// Meshes whose stages are overlapped launches: a stage is two dependent kernels
+// of 5 to 13 us each on a mesh this small, and the gap between them and the
+// loads of geometry are a fifth of it.  Measured, launches in order against
+// overlapped: 10 to 20 steps of 3,840 nodes (potential temperature) 1.60 -> 1.37
+// ms, 15,840 (dry) 1.87 -> 1.77 ms, shallow water 24,576 nodes 0.93 -> 0.87 ms;
+// above, CTAs that start early fill the SMs unevenly: 32,768 nodes 1.97 -> 2.01
+// ms, 131,072 nodes 4.65 -> 5.07 ms.
+constexpr long kOverlapNodes = 24576;
+
+// Launches a kernel that, with `overlap`, may start before the stream's previous
+// kernel has ended (it waits for it by wait_for_previous).
+template <class Kernel, class... Args>
+cudaError_t launch_overlapped(bool overlap, Kernel kernel, int blocks, int threads, size_t smem,
+                              cudaStream_t stream, Args&&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3(blocks);
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = stream;
+  c.attrs = &attr;
+  c.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&c, kernel, std::forward<Args>(args)...);
+}
 // Tiles of the 3D kernels: div 1 to 3 as above; 4 to 6 the same rounded up to
 // whole groups of four warps, one for each of the SM's sub-partitions (their
 // registers are separate, so an odd warp can cost a CTA's place on all four).
@@ -117,6 +143,7 @@ struct tag_handle_s {
   double* sink = nullptr;
   double* graph_sink = nullptr;
   bool capturing_steps = false;
+  bool overlap() const { return nodes <= kOverlapNodes; }
   bool speed_valid = false;
   int epb = 0;
   // threads of a CTA = its elements' work items / tile_div, rounded up to

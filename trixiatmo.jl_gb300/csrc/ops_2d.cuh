@@ -54,10 +54,10 @@ struct OpsImpl {
     const int threads = interface_threads(total);
     if (h->need_bvals && !h->bvals_set)
       return fail(TAG_E_INVALID, "Dirichlet boundary faces without states (tag_set_boundary_values)");
-    k_interface<Phys, n><<<(total + threads - 1) / threads, threads, 0, h->stream>>>(
+    TAG_CUDA(launch_overlapped(
+        h->overlap(), k_interface<Phys, n>, (total + threads - 1) / threads, threads, 0, h->stream,
         params_of<Phys>(h), u, h->d_Ja, h->d_invJ, h->d_if_e, h->d_if_f, h->d_if_flip, h->nif,
-        h->d_bd_e, h->d_bd_f, h->d_bd_kind, h->nbd, h->d_sfv, h->d_bvals);
-    TAG_CUDA(cudaGetLastError());
+        h->d_bd_e, h->d_bd_f, h->d_bd_kind, h->nbd, h->d_sfv, h->d_bvals));
     return TAG_OK;
   }
   static int element(tag_handle h, int mode, double* u, double* du, int stage, bool last,
@@ -76,15 +76,14 @@ struct OpsImpl {
       st.dt = h->d_mscal + h->nmembers;
       st.max_speed = last ? h->d_mscal + 2 * h->nmembers : nullptr;
       st.sink = last && h->capturing_steps ? h->sink : nullptr;
-      k_element<Phys, n, kModeStage, VOL><<<blocks, threads, smem, h->stream>>>(
-          params_of<Phys>(h), h->basis, u, du, h->d_k, h->d_Ja, h->d_invJ, h->d_sfv, h->nelem,
-          epb, st, h->d_status);
+      TAG_CUDA(launch_overlapped(h->overlap(), k_element<Phys, n, kModeStage, VOL>, blocks, threads,
+                                 smem, h->stream, params_of<Phys>(h), h->basis, u, du, h->d_k,
+                                 h->d_Ja, h->d_invJ, h->d_sfv, h->nelem, epb, st, h->d_status));
     } else {
-      k_element<Phys, n, kModeRhs, VOL><<<blocks, threads, smem, h->stream>>>(
-          params_of<Phys>(h), h->basis, u, du, h->d_k, h->d_Ja, h->d_invJ, h->d_sfv, h->nelem,
-          epb, st, h->d_status);
+      TAG_CUDA(launch_overlapped(h->overlap(), k_element<Phys, n, kModeRhs, VOL>, blocks, threads,
+                                 smem, h->stream, params_of<Phys>(h), h->basis, u, du, h->d_k,
+                                 h->d_Ja, h->d_invJ, h->d_sfv, h->nelem, epb, st, h->d_status));
     }
-    TAG_CUDA(cudaGetLastError());
     return TAG_OK;
   }
   static int max_speed(tag_handle h, const double* u) {

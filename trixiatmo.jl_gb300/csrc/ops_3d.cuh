@@ -10,10 +10,10 @@ struct OpsImpl3D {
     const int total = (h->nif + h->nbd) * n * n;
     if (total == 0) return TAG_OK;
     const int threads = interface_threads(total);
-    k_interface3d<Phys, n><<<(total + threads - 1) / threads, threads, 0, h->stream>>>(
-        params_of<Phys>(h), u, h->d_Ja, h->d_invJ, h->d_if_e, h->d_if_f, h->d_if_flip, h->nif,
-        h->d_bd_e, h->d_bd_f, h->nbd, h->d_sfv);
-    TAG_CUDA(cudaGetLastError());
+    TAG_CUDA(launch_overlapped(
+        h->overlap(), k_interface3d<Phys, n>, (total + threads - 1) / threads, threads, 0,
+        h->stream, params_of<Phys>(h), u, h->d_Ja, h->d_invJ, h->d_if_e, h->d_if_f, h->d_if_flip,
+        h->nif, h->d_bd_e, h->d_bd_f, h->nbd, h->d_sfv));
     return TAG_OK;
   }
   static int element(tag_handle h, int mode, double* u, double* du, int stage, bool last,
@@ -29,15 +29,14 @@ struct OpsImpl3D {
       st.dt = h->d_mscal + h->nmembers;
       st.max_speed = last ? h->d_mscal + 2 * h->nmembers : nullptr;
       st.sink = last && h->capturing_steps ? h->sink : nullptr;
-      k_element3d<Phys, n, kModeStage><<<blocks, threads, smem, h->stream>>>(
-          params_of<Phys>(h), h->basis, u, du, h->d_k, h->d_Ja, h->d_invJ, h->d_sfv, h->nelem,
-          epb, st, h->d_status);
+      TAG_CUDA(launch_overlapped(h->overlap(), k_element3d<Phys, n, kModeStage>, blocks, threads,
+                                 smem, h->stream, params_of<Phys>(h), h->basis, u, du, h->d_k,
+                                 h->d_Ja, h->d_invJ, h->d_sfv, h->nelem, epb, st, h->d_status));
     } else {
-      k_element3d<Phys, n, kModeRhs><<<blocks, threads, smem, h->stream>>>(
-          params_of<Phys>(h), h->basis, u, du, h->d_k, h->d_Ja, h->d_invJ, h->d_sfv, h->nelem,
-          epb, st, h->d_status);
+      TAG_CUDA(launch_overlapped(h->overlap(), k_element3d<Phys, n, kModeRhs>, blocks, threads,
+                                 smem, h->stream, params_of<Phys>(h), h->basis, u, du, h->d_k,
+                                 h->d_Ja, h->d_invJ, h->d_sfv, h->nelem, epb, st, h->d_status));
     }
-    TAG_CUDA(cudaGetLastError());
     return TAG_OK;
   }
   static int max_speed(tag_handle h, const double* u) { return speeds(h, u, nullptr); }

@@ -213,6 +213,15 @@ TAG_DEV double twice(double x) { return f64_from(f64_bits(x) + (1ull << 52)); }
 // x / 2 of a normal number with a normal half
 TAG_DEV double half_of(double x) { return f64_from(f64_bits(x) - (1ull << 52)); }
 
+// Programmatic dependent launch (launch_overlapped): a kernel lets the next one
+// of its stream start once all its CTAs are past their main work (earlier, the
+// next one's CTAs would fill the SMs unevenly), and that one loads what no kernel
+// writes (geometry, indices, operators) before it waits for this one's end.  A launch without the attribute is unaffected.  What
+// the previous kernels write is read after the wait, and through pointers
+// without __restrict__, whose loads the compiler may not move across it.
+TAG_DEV void release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+TAG_DEV void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Face node (i, j) of face f (0 = xi-, 1 = xi+, 2 = eta-, 3 = eta+) at index l.
 TAG_DEV void face_node(int f, int l, int n, int& i, int& j) {
   if (f < 2) {
