@@ -876,10 +876,10 @@ TRAFFIC_PER_DOF = {"shell": 281.26,      # k_element3d, stage mode, full shell
                    "swe": 214.71,         # k_cov_element weak form, 8 of the SWE members
                    "swe_ec": 215.20}      # k_cov_element split EC form, the same 8 members
 # FP64 operations the element kernel executes per DOF (DFMA counted as 2), from
-# the same ncu captures (smsp__sass_thread_inst_executed_op_{dfma,dadd,dmul}),
-# beside the algorithmic count: the kernel computes per-node quantities once
-# where the reference's formulas recompute them per pair
-EXECUTED_FLOPS_PER_DOF = {"shell": 950.7, "ensemble": 368.7}
+# ncu (smsp__sass_thread_inst_executed_op_{dfma,dadd,dmul}; profiles/pipes_gb300.md),
+# beside the algorithmic count: the volume integral is evaluated in 64-bit words
+# on the integer pipe
+EXECUTED_FLOPS_PER_DOF = {"shell": 57.1, "ensemble": 41.7}
 
 
 def executed_roofline(workload, dofs, ms_el, peak_fp64):
