@@ -321,7 +321,7 @@ __global__ void __launch_bounds__(kCovIfThreads)
 }
 
 // ---- element kernel --------------------------------------------------------------
-// One thread per node (epb * n^2 <= 256 threads).  Shared memory per node:
+// One thread per node (epb n^2 of 128 or 256 threads).  Shared memory per node:
 // flux differencing: v1, v2, (G_cov v)_1, (G_cov v)_2, J hv^1, J hv^2, h, h_s, J,
 // G^11, G^12, G^22, g h^2 / 2 (13 doubles, an odd stride); weak form: the two
 // contravariant fluxes.
@@ -604,7 +604,8 @@ TAG_DEV void cov_element_body(const CovParams& P, const CovGroup& G, int lblk,
   }
 }
 
-// 256 threads and at least three CTAs per SM: up to 85 registers, which the
+// At most 256 threads (128 on small meshes, chosen with the groups) and at least three
+// CTAs per SM: up to 85 registers, which the
 // FP64-latency-bound body uses for independent operations in flight
 template <int MODE, int VK>
 __global__ void __launch_bounds__(256, 3) k_cov_element(CovParams P, const CovGroups* __restrict__ GG,

@@ -388,8 +388,24 @@ int create_cov(const tag_config* cfgs, int m, tag_handle* out) {
     e_off += c->nelements;
     if_off += c->ninterfaces;
   }
+  // Element CTAs of 128 threads where they lower the threads of the fullest SM:
+  // the FP64 pipe that bounds the kernel is the SM's own, and 338 CTAs of 256 on
+  // 152 SMs leave it 26 % idle behind those with three.  10 steps of 5,400 elements
+  // of degree 3: 1.75 ms with 256, 1.65 ms with 128.  From eight CTAs per SM on
+  // the two hardly differ; n = 6 and 7 fill 256 better (2,400 elements of degree 5:
+  // 1.79 against 1.81 ms).
+  const auto fullest = [&G](int threads) {
+    int ctas = 0;
+    for (int k = 0; k < G.count; ++k) {
+      const int epb = std::max(1, threads / (G.g[k].n * G.g[k].n));
+      ctas += (G.g[k].ne + epb - 1) / epb;
+    }
+    return (ctas + 151) / 152 * threads;
+  };
+  const int cov_threads = fullest(256) < 8 * 256 && fullest(128) < fullest(256) ? 128 : 256;
   for (int k = 0; k < G.count; ++k) {
     CovGroup& g = G.g[k];
+    g.epb = std::max(1, cov_threads / (g.n * g.n));
     g.blk0 = blk;
     blk += (g.ne + g.epb - 1) / g.epb;
     g.iblk0 = iblk;
@@ -417,7 +433,7 @@ int create_cov(const tag_config* cfgs, int m, tag_handle* out) {
   h->h_groups = G;
   h->cov_blocks = blk;
   h->cov_iblocks = iblk;
-  h->cov_threads = 256;
+  h->cov_threads = cov_threads;
   h->cov_smem = smem + sizeof(BasisDev);
   h->epb = 1;  // tiling is per group; no autotuning
   h->ops = &kCovOps;
