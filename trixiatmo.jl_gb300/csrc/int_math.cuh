@@ -298,12 +298,18 @@ TAG_HD u64 exp2_fraction(u64 g) {
 }
 
 TAG_SLOW i64 slow_log2_fixed(double x) {
-  // subnormals are scaled up; zeros, negative values, infinities and NaN (bad
-  // states, flagged by the callers) give 0
-  if (!(x > 0.0) || f64_exponent(f64_bits(x)) == 0x7ffu) return 0;
-  const u64 b = f64_bits(x * 18014398509481984.0);  // 2^54
-  const i64 e = (i64)f64_exponent(b) - 1023 - 54;
-  return e * (1ll << 52) + (log2_significand(significand(b)) >> 11);
+  // Subnormals are scaled up.  Values that have no logarithm (bad states, and
+  // partial densities below zero) get words that keep them out of the means'
+  // series beside any other value: negative ones the word of |x| and 2^62 (1024
+  // octaves), zeros -1536 octaves.  Infinities and NaN give 0; they make the
+  // means non-finite by themselves.
+  if (x == 0.0) return -(1536ll << 52);
+  if (x != x || f64_exponent(f64_bits(x)) == 0x7ffu) return 0;
+  const double m = x < 0.0 ? -x : x;
+  const u64 b = f64_bits(m < 1.0 ? m * 18014398509481984.0 : m);  // 2^54
+  const i64 e = (i64)f64_exponent(b) - 1023 - (m < 1.0 ? 54 : 0);
+  return e * (1ll << 52) + ((log2_significand(significand(b)) + 1024) >> 11) +
+         (x < 0.0 ? 1ll << 62 : 0);
 }
 
 // log2(x) as Q11.52 for normal positive x (absolute error < 2^-53): the node

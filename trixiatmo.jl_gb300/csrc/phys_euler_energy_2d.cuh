@@ -49,7 +49,7 @@ struct PhysEnergy2D {
     q[2] = u[2] * hir;
     q[3] = 0.5 * p;
     q[4] = 0.25 * u[4];
-    q[5] = pr * P.quarter_inv_gm1;
+    q[5] = invertible(pr * P.quarter_inv_gm1);
     q[6] = log_word(rho);
     q[7] = log_word(pr);
     if (not_positive(rho)) bad |= TAG_S_NEG_DENSITY;

@@ -50,7 +50,7 @@ struct PhysEnergy3D {
     q[3] = u[3] * hir;
     q[4] = 0.5 * p;
     q[5] = 0.25 * u[5];
-    q[6] = pr * P.quarter_inv_gm1;
+    q[6] = invertible(pr * P.quarter_inv_gm1);
     q[7] = log_word(rho);
     q[8] = log_word(pr);
     if (not_positive(rho)) bad |= TAG_S_NEG_DENSITY;

@@ -45,7 +45,7 @@ struct PhysIE2D {
     q[2] = u[2] * hir;
     q[3] = 0.5 * p;
     q[4] = 0.5 * u[4];
-    q[5] = 0.5 * pr * P.inv_gm1;
+    q[5] = invertible(0.5 * pr * P.inv_gm1);
     q[6] = log_word(rho);
     q[7] = log_word(pr);
     if (not_positive(rho)) bad |= TAG_S_NEG_DENSITY;

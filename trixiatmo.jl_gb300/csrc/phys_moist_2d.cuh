@@ -82,10 +82,10 @@ struct PhysMoist2D {
     q[2] = 0.5 * u[5];
     q[3] = 0.5 * v1;
     q[4] = 0.5 * v2;
-    q[5] = 0.5 * T;
+    q[5] = invertible(0.5 * T);
     q[6] = 0.5 * int_div(den, num);
     q[7] = 0.25 * fma(v2, v2, v1 * v1);
-    q[8] = log_word(q[0]);
+    q[8] = log_word_signed(q[0]);
     q[9] = log_word_signed(q[1]);
     q[10] = log_word_signed(q[2]);
     q[11] = log_word(T);
@@ -100,7 +100,9 @@ struct PhysMoist2D {
     const double v1a = a[3] + b[3], v2a = a[4] + b[4];
     const double K = a[7] + b[7];
     const double vdn = n1 * v1a + n2 * v2a;
-    const double rqd_mean = (a[0] + b[0]) * ln_factor(a[0], b[0], log_difference(a[8], b[8]));
+    // (two nodes without dry air: no value, as their pressure's gas would be missing)
+    const double rqd_mean =
+        invertible(a[0] + b[0]) * ln_factor(a[0], b[0], log_difference(a[8], b[8]));
     // inv_ln_mean of 1/T
     const double T_mean = (a[5] + b[5]) * inv_ln_factor(a[5], b[5], log_difference(a[11], b[11]));
     const double rqv_avg = a[1] + b[1], rql_avg = a[2] + b[2];

@@ -94,7 +94,9 @@ struct PhysPT2D {
   // the third mean's half node value (volume 3: flux_kennedy_gruber's theta)
   TAG_DEV static double third_value(const Params& P, double rho, double rho_theta, double irho) {
     if (P.volume == 0) return 0.0;
-    return P.volume == 2 ? 0.5 * rho * int_rcp(rho_theta) : 0.5 * rho_theta * irho;
+    if (P.volume == 2) return 0.5 * rho * int_rcp(rho_theta);
+    const double x = 0.5 * rho_theta * irho;
+    return P.volume == 1 ? invertible(x) : x;
   }
 
   TAG_DEV static void node_prims(const Params& P, const double* u, double* q, unsigned& bad) {
@@ -105,7 +107,7 @@ struct PhysPT2D {
     q[2] = u[2] * hir;
     q[3] = 0.5 * pressure(P, u[3]);
     q[4] = 0.5 * u[4];
-    q[5] = 0.5 * u[3];
+    q[5] = invertible(0.5 * u[3]);
     q[6] = third_value(P, rho, u[3], irho);
     q[7] = log_word(rho);
     q[8] = log_word(u[3]);
@@ -119,6 +121,7 @@ struct PhysPT2D {
   // else powers
   static __device__ __noinline__ double stolarsky_factor_far(const Params& P, double x, double y,
                                                              u64 a) {
+    if (opposite_signs(x, y)) return quiet_nan();
     if (P.stol.ok && P.stol_q64 && middle_range(a))
       return middle_factor(stolarsky_deficit_middle(a, P.gamma_q61, P.stol_q64));
     const double s = x + y, d = y - x;

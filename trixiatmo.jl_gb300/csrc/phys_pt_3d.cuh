@@ -49,7 +49,7 @@ struct PhysPT3D {
     q[3] = u[3] * hir;
     q[4] = 0.5 * PhysPT2D::pressure(P, u[4]);
     q[5] = 0.5 * u[5];
-    q[6] = 0.5 * u[4];
+    q[6] = invertible(0.5 * u[4]);
     q[7] = PhysPT2D::third_value(P, rho, u[4], irho);
     q[8] = log_word(rho);
     q[9] = log_word(u[4]);

@@ -126,7 +126,7 @@ struct PhysRainy2D {
     q[3] = 0.5 * u[2];
     q[4] = 0.5 * v1;
     q[5] = 0.5 * v2;
-    q[6] = 0.5 * T;
+    q[6] = invertible(0.5 * T);
     q[7] = 0.5 * int_rcp(T);
     q[8] = 0.5 * rainy_v_rain(rv + rc, u[2]);
     q[9] = 0.25 * fma(v2, v2, v1 * v1);

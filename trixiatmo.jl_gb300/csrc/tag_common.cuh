@@ -26,16 +26,23 @@ constexpr int kMaxNodes = 8;  // n = polydeg + 1 supported up to polydeg 7
 // and a reciprocal in words; beyond, d itself is the logarithm of the definition.
 TAG_DEV double log_of_difference(i64 d) { return (double)d * 1.539095918623324e-16; }  // ln2 2^-52
 
-// (Values of opposite sign, which a moisture density may have, give NaN: the
-// logarithm of their ratio.)
+// Values of opposite sign, which partial densities and bad states may have, give
+// NaN: the logarithm of their ratio.  Beside a zero the mean is 0 and its inverse
+// has no value.
 TAG_DEV bool opposite_signs(double a, double b) { return (i64)(f64_bits(a) ^ f64_bits(b)) < 0; }
+TAG_DEV bool is_zero(double x) { return (f64_bits(x) << 1) == 0; }
+TAG_DEV double quiet_nan() { return f64_from(0x7ff8000000000000ull); }
+// A node value whose inverse is averaged: NaN in place of zero.
+TAG_DEV double invertible(double x) { return is_zero(x) ? quiet_nan() : x; }
 static __device__ __noinline__ double ln_factor_far(double xa, double xb, i64 d) {
-  if (opposite_signs(xa, xb)) return f64_from(0x7ff8000000000000ull);
+  if (opposite_signs(xa, xb)) return quiet_nan();
+  if (is_zero(xa) || is_zero(xb)) return 0.0;
   const u64 a = magnitude(d);
   if (middle_range(a)) return middle_factor(ln_mean_deficit_middle(a));
   return int_div(2.0 * (xb - xa), log_of_difference(d) * (xa + xb));
 }
 static __device__ __noinline__ double inv_ln_factor_far(double ya, double yb, i64 d) {
+  if (opposite_signs(ya, yb) || is_zero(ya) || is_zero(yb)) return quiet_nan();
   const u64 a = magnitude(d);
   if (middle_range(a)) return middle_factor(inv_ln_mean_deficit_middle(a));
   return int_div(2.0 * ya * yb * log_of_difference(d), (yb - ya) * (ya + yb));
@@ -60,13 +67,12 @@ TAG_DEV double inv_ln_mean_of_reciprocals(double x, double y) {
 
 // Node logarithms are kept among the other node quantities as raw words.
 TAG_DEV double log_word(double x) { return f64_from((u64)log2_fixed(x)); }
-// The same of |x|, with an offset that separates the signs: pairs of one sign
-// see the difference of the logarithms, pairs of two signs leave the series.
+// The same where values below zero are common: log2_fixed's words of negative
+// values without its out-of-line branch.
 TAG_DEV double log_word_signed(double x) {
   const u64 b = f64_bits(x);
   return f64_from((u64)log2_fixed(f64_from(b & 0x7fffffffffffffffull)) + ((b >> 63) << 62));
 }
-TAG_DEV bool is_zero(double x) { return (f64_bits(x) << 1) == 0; }
 TAG_DEV i64 log_difference(double wa, double wb) { return (i64)(f64_bits(wb) - f64_bits(wa)); }
 
 // FP64 forms of the two means, which the diagnostics (tag_means.cu) hold beside
