@@ -190,8 +190,9 @@ struct ElemSmem {
   static constexpr int oL = oC;                  // CFL speeds [2][nn], once the slots are used up
   static constexpr int sizeC = 2 * nn * (n - 1) * NA;
   static constexpr int oS = oC + (sizeC > 2 * nn + 9 ? sizeC : 2 * nn + 9);  // sources [nn][NA]
-  static constexpr int oF = oS + (Phys::kHasSources ? nn * NA : 0);  // fixed point: FxScale
-  static constexpr int per_elem = (oF + (Phys::kFixed ? kFxDoubles : 0) + 1) / 2 * 2;
+  // fixed point: FxScale (16-byte aligned)
+  static constexpr int oF = (oS + (Phys::kHasSources ? nn * NA : 0) + 1) / 2 * 2;
+  static constexpr int per_elem = oF + (Phys::kFixed ? kFxDoubles<2> : 0);
   static size_t bytes(int epb) { return sizeof(double) * (size_t)per_elem * epb + sizeof(BasisDev); }
 };
 
@@ -244,35 +245,23 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
     for (int el = warp; el < ne; el += nwarps) {
       double* eb = base + el * S::per_elem;
       u32 m[kMxCount] = {};
-      for (int node = lane; node < nn; node += 32) {
-        const double *q = eb + S::oQ + node * NQ, *ja = eb + S::oJa + node * 4;
-        m[kMxV] = max(m[kMxV], high_magnitude(q[1]));
-        m[kMxV + 1] = max(m[kMxV + 1], high_magnitude(q[2]));
-        // the words' products take densities as positive: bad states leave
-        m[kMxRho] = max(m[kMxRho], not_positive(q[0]) ? 0x7ff00000u : high_magnitude(q[0]));
-        m[kMxP] = max(m[kMxP], high_magnitude(q[3]));
-        m[kMxG] = max(m[kMxG], high_magnitude(q[4]));
-        m[kMxX] = max(m[kMxX], not_positive(q[5]) ? 0x7ff00000u : high_magnitude(q[5]));
-        m[kMxN] = max(m[kMxN], max(high_magnitude(ja[0]), high_magnitude(ja[1])));
-        m[kMxN + 1] = max(m[kMxN + 1], max(high_magnitude(ja[2]), high_magnitude(ja[3])));
-      }
+      for (int node = lane; node < nn; node += 32)
+        fx_node_maxima<2>(eb + S::oQ + node * NQ, eb + S::oJa + node * 4,
+                          [&m](int k, u32 x) { m[k] = max(m[k], x); });
       for (int k = lane; k < 4 * n; k += 32) {
         const double* sf = sfv + ((size_t)(e_first + el) * 4 * n + k) * NA;
-        const u32 a = high_magnitude(sf[0]), c = high_magnitude(sf[3]),
-                  b = max(high_magnitude(sf[1]), high_magnitude(sf[2]));
         const bool second = k >= 2 * n;
-        m[kMxF] = max(m[kMxF], second ? 0u : a);
-        m[kMxF + 1] = max(m[kMxF + 1], second ? a : 0u);
-        m[kMxF + 3] = max(m[kMxF + 3], second ? 0u : b);
-        m[kMxF + 4] = max(m[kMxF + 4], second ? b : 0u);
-        m[kMxF + 6] = max(m[kMxF + 6], second ? 0u : c);
-        m[kMxF + 7] = max(m[kMxF + 7], second ? c : 0u);
+#pragma unroll
+        for (int v = 0; v < NA; ++v) {
+          const u32 a = high_magnitude(sf[v]);
+          u32 &m0 = m[fx_face_max<2>(v, 0)], &m1 = m[fx_face_max<2>(v, 1)];
+          m0 = max(m0, second ? 0u : a);
+          m1 = max(m1, second ? a : 0u);
+        }
       }
 #pragma unroll
-      for (int k = 0; k < kMxCount; ++k) {
-        const bool used = k < kMxRho ? k < 2 : k < kMxN || (k - kMxN) % 3 < 2;
-        if (used) m[k] = __reduce_max_sync(0xffffffffu, m[k]);
-      }
+      for (int k = 0; k < kMxCount; ++k)
+        if (fx_used(k, 2)) m[k] = __reduce_max_sync(0xffffffffu, m[k]);
       // (the pair slots are not in use yet)
       if (lane == 0) {
 #pragma unroll
@@ -280,21 +269,21 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
       }
     }
     __syncthreads();
-    for (int el = threadIdx.x; el < ne; el += nthr) {
-      double* eb = base + el * S::per_elem;
-      *reinterpret_cast<FxScale*>(eb + S::oF) =
-          fx_scale(reinterpret_cast<const u32*>(eb + S::oC), 2, sb->fx);
+    for (int t = threadIdx.x; t < 2 * ne; t += nthr) {
+      double* eb = base + (t >> 1) * S::per_elem;
+      fx_scale<2>(reinterpret_cast<const u32*>(eb + S::oC), sb->fx, t & 1,
+                  *reinterpret_cast<FxScale<2>*>(eb + S::oF));
     }
     __syncthreads();
     for (int t = threadIdx.x; t < ne * nn; t += nthr) {
       const int el = t / nn, node = t % nn;
       double* eb = base + el * S::per_elem;
-      const FxScale& fs = *reinterpret_cast<const FxScale*>(eb + S::oF);
+      const FxScale<2>& fs = *reinterpret_cast<const FxScale<2>*>(eb + S::oF);
       if (!fs.ok) continue;
       fx_convert_node<2>(eb + S::oQ + node * NQ, fs);
       double* ja = eb + S::oJa + node * 4;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) ja[c] = f64_from((u64)to_fixed(ja[c], fs.sn[c / 2] - 2));
+      for (int c = 0; c < 4; ++c) ja[c] = f64_from((u64)to_fixed(ja[c], fs.sn[c / 2][c % 2] - 2));
     }
     __syncthreads();
   }
@@ -334,15 +323,15 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
     double* ca = eb + S::oC + ((d * nn + na_) * (n - 1) + b - 1) * NA;  // b > a
     double* cb = eb + S::oC + ((d * nn + nb_) * (n - 1) + a) * NA;
     if constexpr (Phys::kFixed) {
-      const FxScale& fs = *reinterpret_cast<const FxScale*>(eb + S::oF);
+      const FxScale<2>& fs = *reinterpret_cast<const FxScale<2>*>(eb + S::oF);
       if (fs.ok) {
         // the pair ordered so that the weight is positive; words to be summed
-        const i64 Qab = sb->fx.Q[a * n + b];
-        const bool turn = Qab < 0;
+        const u64 Qab = sb->fx.Q[a * n + b];
+        const bool turn = Qab & 1;
         const int p = turn ? nb_ : na_, q = turn ? na_ : nb_;
         i64 Fa[NA], Fb[NA];
         Phys::fixed_pair(Pp, eb + S::oQ + p * NQ, eb + S::oQ + q * NQ, turn ? ja_b : ja_a,
-                         turn ? ja_a : ja_b, turn ? -Qab : Qab, fx_shift(fs), fs.kq[d], Fa, Fb);
+                         turn ? ja_a : ja_b, Qab, fs.k[d], Fa, Fb);
         double *cp = turn ? cb : ca, *cq = turn ? ca : cb;
 #pragma unroll
         for (int v = 0; v < NA; ++v) {
@@ -390,13 +379,11 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
     double* eb = base + el * S::per_elem;
     const double* se = sfv + (size_t)e * 4 * n * NA + v;
     const bool halved = VOL == kVolFluxDiff && Phys::kLastHalved && v == NA - 1;
-    const FxScale& fs = *reinterpret_cast<const FxScale*>(eb + S::oF);
+    const FxScale<2>& fs = *reinterpret_cast<const FxScale<2>*>(eb + S::oF);
     double acc = 0.0;
     if (VOL == kVolFluxDiff && Phys::kFixed && fs.ok) {
       // sums of words and unweighted surface fluxes, then 1/w per direction
-      const int kind = v == 0 ? 0 : v < NA - 1 ? 1 : 2;
-      const int ks = fx_kind_scale(fs, kind) + sb->fx.sq;
-      const int sd[2] = {fx_direction_scale(fs, 0), fx_direction_scale(fs, 1)}, at[2] = {i, j};
+      const int sd[2] = {fs.sum[0][v], fs.sum[1][v]}, at[2] = {i, j};
       i64 A[2] = {0, 0};
 #pragma unroll
       for (int d = 0; d < 2; ++d) {
@@ -405,13 +392,13 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
         for (int s = 0; s < n - 1; ++s) A[d] += (i64)f64_bits(c[s * NA]);
         if (at[d] == 0 || at[d] == n - 1) {
           const int end = at[d] == 0 ? 0 : 1;
-          A[d] += fx_surface(se[((2 * d + end) * n + at[1 - d]) * NA], ks + sd[d] + (halved ? 1 : 0),
+          A[d] += fx_surface(se[((2 * d + end) * n + at[1 - d]) * NA], sd[d] + (halved ? 1 : 0),
                              sb->fx.S[end]);
         }
       }
       int scale;
       const i64 tot = fx_weighted_sum<2>(A, 1, sb->fx.W, at, sd, scale);
-      acc = from_fixed(tot, ks + scale + sb->fx.kw);
+      acc = fx_zero(fs, v) ? 0.0 : from_fixed(tot, scale + sb->fx.kw);
     } else {
     if constexpr (VOL == kVolFluxDiff) {
       // slot s of node a holds the flux with partner s (s < a) or s + 1

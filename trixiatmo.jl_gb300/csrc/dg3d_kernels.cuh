@@ -127,8 +127,9 @@ struct ElemSmem3D {
   static constexpr int oJa = oQ + nnn * NQ;       // contravariant vectors as stored
   static constexpr int oA = oJa + nnn * 9;        // accumulators [3][nnn][NA]
   static constexpr int oL = oA;                   // CFL speeds [3][nnn], once the sums are used up
-  static constexpr int oF = oA + 3 * nnn * NA;    // fixed point: FxScale, field maxima
-  static constexpr int per_elem = oF + (Phys::kFixed ? kFxDoubles + (kMxCount + 1) / 2 : 0);
+  // fixed point: FxScale (16-byte aligned), field maxima
+  static constexpr int oF = (oA + 3 * nnn * NA + 1) / 2 * 2;
+  static constexpr int per_elem = oF + (Phys::kFixed ? kFxDoubles<3> + (kMxCount + 3) / 4 * 2 : 0);
   static size_t bytes(int epb) { return sizeof(double) * (size_t)per_elem * epb + sizeof(BasisDev); }
 };
 
@@ -158,7 +159,8 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
   }
   if constexpr (Phys::kFixed) {
     for (int t = threadIdx.x; t < ne * kMxCount; t += nthr)
-      reinterpret_cast<u32*>(base + t / kMxCount * S::per_elem + S::oF + kFxDoubles)[t % kMxCount] = 0;
+      reinterpret_cast<u32*>(base + t / kMxCount * S::per_elem + S::oF +
+                             kFxDoubles<3>)[t % kMxCount] = 0;
   }
   for (int el = 0; el < ne; ++el)
     copy_in(base + el * S::per_elem + S::oJa, Ja + (size_t)(e_first + el) * nnn * 9, nnn * 9);
@@ -176,60 +178,50 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
     for (int task = warp; task < ne * CH; task += nwarps) {
       const int el = task / CH, node = (task % CH) * 32 + lane;
       double* eb = base + el * S::per_elem;
-      u32* mx = reinterpret_cast<u32*>(eb + S::oF + kFxDoubles);
-      u32 m[kMxF] = {};
+      u32* mx = reinterpret_cast<u32*>(eb + S::oF + kFxDoubles<3>);
+      u32 m[kMxFm] = {};
       if (node < nnn) {
         double* q = eb + S::oQ + node * NQ;
         Phys::node_prims(Pp, eb + S::oU + node * NV, q, bad);
         q[5] -= 0.25 * eb[S::oU + NV - 1];  // phi of the element's first node
+        fx_node_maxima<3>(q, eb + S::oJa + node * 9, [&m](int k, u32 x) { m[k] = x; });
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          m[kMxV + d] = high_magnitude(q[1 + d]);
-#pragma unroll
-          for (int c = 0; c < 3; ++c)
-            m[kMxN + d] = max(m[kMxN + d], high_magnitude(eb[S::oJa + node * 9 + 3 * d + c]));
+        for (int d = 0; d < 3; ++d)
 #pragma unroll
           for (int v = 0; v < NA; ++v) eb[S::oA + (d * nnn + node) * NA + v] = 0.0;
-        }
-        // the words' products take densities as positive: bad states leave
-        m[kMxRho] = not_positive(q[0]) ? 0x7ff00000u : high_magnitude(q[0]);
-        m[kMxP] = high_magnitude(q[4]);
-        m[kMxG] = high_magnitude(q[5]);
-        m[kMxX] = not_positive(q[6]) ? 0x7ff00000u : high_magnitude(q[6]);
       }
 #pragma unroll
-      for (int k = 0; k < kMxF; ++k) warp_max_into(mx + k, m[k]);
+      for (int k = 0; k < kMxFm; ++k) warp_max_into(mx + k, m[k]);
     }
     // surface fluxes of each direction's two faces
     for (int task = warp; task < ne * 3 * CF; task += nwarps) {
       const int el = task / (3 * CF), d = task / CF % 3, k = (task % CF) * 32 + lane;
-      u32* mx = reinterpret_cast<u32*>(base + el * S::per_elem + S::oF + kFxDoubles);
-      u32 m[3] = {};
+      u32* mx = reinterpret_cast<u32*>(base + el * S::per_elem + S::oF + kFxDoubles<3>);
+      u32 m[NA] = {};
       if (k < 2 * nn) {
         const double* sf = sfv + (((size_t)(e_first + el) * 6 + 2 * d) * nn + k) * NA;
-        m[0] = high_magnitude(sf[0]);
-        m[1] = max(high_magnitude(sf[1]), max(high_magnitude(sf[2]), high_magnitude(sf[3])));
-        m[2] = high_magnitude(sf[4]);
+#pragma unroll
+        for (int v = 0; v < NA; ++v) m[v] = high_magnitude(sf[v]);
       }
 #pragma unroll
-      for (int kind = 0; kind < 3; ++kind) warp_max_into(mx + kMxF + 3 * kind + d, m[kind]);
+      for (int v = 0; v < NA; ++v) warp_max_into(mx + fx_face_max<3>(v, d), m[v]);
     }
     __syncthreads();
-    if (threadIdx.x < ne) {
-      double* f = base + threadIdx.x * S::per_elem + S::oF;
-      *reinterpret_cast<FxScale*>(f) =
-          fx_scale(reinterpret_cast<u32*>(f + kFxDoubles), 3, sb->fx);
+    for (int t = threadIdx.x; t < 3 * ne; t += nthr) {
+      double* f = base + t / 3 * S::per_elem + S::oF;
+      fx_scale<3>(reinterpret_cast<const u32*>(f + kFxDoubles<3>), sb->fx, t % 3,
+                  *reinterpret_cast<FxScale<3>*>(f));
     }
     __syncthreads();
     for (int t = threadIdx.x; t < ne * nnn; t += nthr) {
       const int el = t / nnn, node = t % nnn;
       double* eb = base + el * S::per_elem;
-      const FxScale& fs = *reinterpret_cast<const FxScale*>(eb + S::oF);
+      const FxScale<3>& fs = *reinterpret_cast<const FxScale<3>*>(eb + S::oF);
       if (!fs.ok) continue;
       fx_convert_node<3>(eb + S::oQ + node * NQ, fs);
       double* ja = eb + S::oJa + node * 9;
 #pragma unroll
-      for (int c = 0; c < 9; ++c) ja[c] = f64_from((u64)to_fixed(ja[c], fs.sn[c / 3] - 2));
+      for (int c = 0; c < 9; ++c) ja[c] = f64_from((u64)to_fixed(ja[c], fs.sn[c / 3][c % 3] - 2));
     }
   } else {
     for (int t = threadIdx.x; t < ne * nnn; t += nthr) {
@@ -260,22 +252,21 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
       // line = p1 + n * p2 over the two other directions (ascending)
       const int p1 = line % n, p2 = line / n;
       double* eb = base + el * S::per_elem;
-      const FxScale& fs = *reinterpret_cast<const FxScale*>(eb + S::oF);
+      const FxScale<3>& fs = *reinterpret_cast<const FxScale<3>*>(eb + S::oF);
       const bool fixed = Phys::kFixed && fs.ok;
       FxShift fk{};
-      if (fixed) fk = fx_shift(fs);
+      if (fixed) fk = fs.k[d];
       for (int r = 0; r < S::R; ++r) {
         int a, b;
         if (on && round_robin_pair(n, r, slot, a, b)) {
-          i64 Qab = 0;
+          u64 Qab = 0;
           if (fixed) {
             // ordered so that the weight is positive
             Qab = sb->fx.Q[a * n + b];
-            if (Qab < 0) {
+            if (Qab & 1) {
               const int c = a;
               a = b;
               b = c;
-              Qab = -Qab;
             }
           }
           int na_, nb_;
@@ -295,7 +286,7 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
             if constexpr (Phys::kFixed) {
               i64 Fa[NA], Fb[NA];
               Phys::fixed_pair(Pp, eb + S::oQ + na_ * NQ, eb + S::oQ + nb_ * NQ, ja_a, ja_b, Qab,
-                               fk, fs.kq[d], Fa, Fb);
+                               fk, Fa, Fb);
               i64* ca = reinterpret_cast<i64*>(eb + S::oA + (d * nnn + na_) * NA);
               i64* cb = reinterpret_cast<i64*>(eb + S::oA + (d * nnn + nb_) * NA);
 #pragma unroll
@@ -336,12 +327,9 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
           if (fixed) {
             // unweighted: 1/w joins with the node's volume terms
             i64* w64 = reinterpret_cast<i64*>(c);
-            const int sd = fx_direction_scale(fs, d) + sb->fx.sq;
 #pragma unroll
             for (int v = 0; v < NA; ++v)
-              w64[v] += fx_surface(sf[v],
-                                   fx_kind_scale(fs, v == 0 ? 0 : v < NA - 1 ? 1 : 2) + sd +
-                                       (Phys::kLastHalved && v == NA - 1),
+              w64[v] += fx_surface(sf[v], fs.sum[d][v] + (Phys::kLastHalved && v == NA - 1),
                                    sb->fx.S[end]);
             continue;
           }
@@ -366,19 +354,17 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
     const double ij = invJ[gq];
     double acc[NA];
     const double* A = eb + S::oA + node * NA;
-    const FxScale& fs = *reinterpret_cast<const FxScale*>(eb + S::oF);
+    const FxScale<3>& fs = *reinterpret_cast<const FxScale<3>*>(eb + S::oF);
     if (Phys::kFixed && fs.ok) {
       // each direction's sum over its quadrature weight
       const int at[3] = {node % n, node / n % n, node / nn};
-      const int sd[3] = {fx_direction_scale(fs, 0), fx_direction_scale(fs, 1),
-                         fx_direction_scale(fs, 2)};
 #pragma unroll
       for (int v = 0; v < NA; ++v) {
+        const int sd[3] = {fs.sum[0][v], fs.sum[1][v], fs.sum[2][v]};
         int scale;
         const i64 tot = fx_weighted_sum<3>(reinterpret_cast<const i64*>(A + v), nnn * NA, sb->fx.W,
                                            at, sd, scale);
-        acc[v] = from_fixed(tot, fx_kind_scale(fs, v == 0 ? 0 : v < NA - 1 ? 1 : 2) + scale +
-                                     sb->fx.sq + sb->fx.kw);
+        acc[v] = fx_zero(fs, v) ? 0.0 : from_fixed(tot, scale + sb->fx.kw);
       }
     } else {
 #pragma unroll

@@ -5,21 +5,23 @@
 // FP64 operation occupies an SM for 20 cycles per warp (measured 1.57 per clock);
 // the product hmul below takes 3.4, a sum 1.
 //
-// Words: m stands for m 2^(s - 64) with one exponent s per field and element,
-// chosen from the element's largest values so that every intermediate stays in
-// (-1/2, 1/2): |m| < 2^63 without a run-time test.  A node field below 1/4 of its
-// scale keeps 62 bits relative to the element's largest value; a product rounds
-// at 2^-64 of its scale, which the bounds of fx_scale place near the result.
+// Words: m stands for m 2^(s - 64) with one exponent s per field, component and
+// element, chosen from the element's largest values so that every intermediate
+// stays in (-1/2, 1/2): |m| < 2^63 without a run-time test.  A node field below 1/4
+// of its scale keeps 62 bits relative to the element's largest value; a product
+// rounds at 2^-64 of its scale, which the bounds of fx_scale place near the result.
 //
 // Weights: with the quadrature weights w, Q_ab = w_a Dsplit_ab is antisymmetric,
 // so one product Q_ab n serves both nodes of a pair, the surface fluxes join the
 // sums unweighted, and 1/w_a is applied once per node and direction.  Sums of
 // words are exact and independent of their order.
 //
-// Measured on the shell at polydeg 5 (2,654,208 nodes): the element kernel 2.15
-// ms in FP64 (its pipe 90 % busy) and 0.93 ms in words (issue slots 55 %, integer
-// pipes 50 % busy); its error against extended precision is 0.4 to 0.8 of the
-// FP64 form's.
+// Measured on the shell at polydeg 5 (2,654,208 nodes): right-hand side 2.32 ms
+// with the FP64 form (its pipe 90 % busy), 1.11 ms in words.  Of that 0.04 ms are the
+// scales by component.  With one scale per direction the horizontal momentum of
+// flat elements lost up to eight places: its error against extended precision, over
+// the FP64 form's, was 3 in elements 170 times as wide as tall and 320 at 20,000;
+// it is 0.6 to 1.1 now at every width.
 //
 // Elements whose values leave the scales' range (infinities, NaN, magnitudes
 // beyond 2^+-150) take the FP64 form.
@@ -45,10 +47,8 @@ TAG_HD i64 hmul_raw(i64 a, i64 b) {
   return (i64)(umul_high(offset_word(a), offset_word(b)) - kOffset) - (a >> 1) - (b >> 1);
 }
 TAG_HD i64 hmul(i64 a, i64 b) { return hmul_raw(a, b) + 1; }
-// for b >= 0 (1 low)
-TAG_HD i64 hmul_pos(i64 a, i64 b) {
-  return (i64)umul_high(offset_word(a), (u64)b) - (b >> 1) + 1;
-}
+// for b >= 0, with all 64 places for b (1 low)
+TAG_HD i64 hmul_pos(i64 a, u64 b) { return (i64)(umul_high(offset_word(a), b) - (b >> 1)) + 1; }
 
 // x < 2^e as a word of scale e + 2: x 2^(62 - e), towards zero.
 TAG_HD i64 to_fixed(double x, int e) {
@@ -64,26 +64,23 @@ TAG_HD i64 to_fixed(double x, int e) {
 TAG_HD double from_fixed(i64 m, int s) {
   if (m == 0) return 0.0;
   const u64 a = magnitude(m);
-#ifdef __CUDA_ARCH__
-  const int lz = __clzll((i64)a);
-#else
-  const int lz = __builtin_clzll(a);
-#endif
+  const int lz = leading_zeros(a);
   const u64 r = ((u64)(1021 + s - lz) << 52) + round53(a << lz);
   return f64_from(r | ((u64)m & 0x8000000000000000ull));
 }
 
 // Basis in words (FxBasis::ok: the operator is antisymmetric, as it is on
-// Legendre-Gauss-Lobatto nodes): Q[a n + b] = w_a Dsplit_ab / 2 2^(64 - sq), each
-// below 1/2 and a row's magnitudes summing to at most 1; W[a] = 2^(64 - kw) / w_a
+// Legendre-Gauss-Lobatto nodes): Q[a n + b] = |w_a Dsplit_ab| / 2 2^(64 - sq), each
+// below 1, with the sign in the last place (1: negative); W[a] = 2^(64 - kw) / w_a
 // below 1/2.
 struct FxBasis {
-  i64 Q[64];
+  u64 Q[64];
   i64 W[8];
-  float one, row;  // the largest |Q_ab| and row sum, as fractions of 2^sq
-  int S[2];        // relative change of the first and last node's weight, times 2^63
-  int sq, kw, ok, pad;  // (a multiple of 16 bytes)
+  float row;  // the largest row sum of |Q|, over 2^sq
+  int S[2];   // relative change of the first and last node's weight, times 2^63
+  int sq, kw, ok, pad[2];  // (a multiple of 16 bytes)
 };
+static_assert(sizeof(FxBasis) % 16 == 0, "16-byte aligned");
 
 inline void load_fixed_basis(FxBasis& f, const double* Ds, const double* w, int n) {
   std::memset(&f, 0, sizeof(f));
@@ -102,9 +99,8 @@ inline void load_fixed_basis(FxBasis& f, const double* Ds, const double* w, int 
   }
   f.ok = row > 0.0 && skew <= 1e-12 * row && std::isfinite(row) && std::isfinite(winv);
   if (!f.ok) return;
-  f.sq = std::max(std::ilogb(row) + 1, std::ilogb(one) + 2);
+  f.sq = std::ilogb(one) + 1;
   f.kw = std::ilogb(winv) + 2;
-  f.one = (float)std::ldexp(one, -f.sq) * 1.00001f;
   f.row = (float)std::ldexp(row, -f.sq) * 1.00001f;
   // The weights and the operator are rounded by themselves, so w_a Dsplit_ab and
   // -w_b Dsplit_ba differ in their last places: the weights are adjusted to the
@@ -124,7 +120,7 @@ inline void load_fixed_basis(FxBasis& f, const double* Ds, const double* w, int 
     for (int b = 0; b < n; ++b) {
       if (b == a) continue;
       const long double q = 0.25L * (ww[a] * Ds[a * n + b] - ww[b] * Ds[b * n + a]);
-      f.Q[a * n + b] = (i64)llroundl(ldexpl(q, 64 - f.sq));
+      f.Q[a * n + b] = (u64)llroundl(ldexpl(fabsl(q), 63 - f.sq)) << 1 | (q < 0 ? 1 : 0);
     }
     f.W[a] = (i64)llroundl(ldexpl(1.0L / ww[a], 64 - f.kw));
   }
@@ -133,26 +129,76 @@ inline void load_fixed_basis(FxBasis& f, const double* Ds, const double* w, int 
 }
 
 // Largest magnitudes of an element's fields, as high words of the doubles
-// (their order is the values'), and the scales chosen from them.
-// Velocities by component, so that sums of components and normal velocities are
-// bounded by their own values: a place or two of every word.  (Shell elements
-// 15 km tall, whose density falls by e^2, need it: without, their energy error at
-// polydeg 7 was 1.35 of the FP64 form's, now 0.8.)
+// (their order is the values'), and the scales chosen from them.  Velocities,
+// contravariant vectors and the surface fluxes of momentum by component: the
+// vertical face of a flat element can be thousands of times its lateral ones,
+// and a component that is small or zero must not be rounded at the largest one's
+// scale (kMxN, kMxFv: 3 direction + component).
 enum FxMax : int {
-  kMxV = 0, kMxRho = kMxV + 3, kMxP, kMxX, kMxG, kMxN, kMxF = kMxN + 3, kMxCount = kMxF + 9
+  kMxV = 0, kMxRho = kMxV + 3, kMxP, kMxX, kMxG, kMxN, kMxFm = kMxN + 9, kMxFv = kMxFm + 3,
+  kMxFe = kMxFv + 9, kMxCount = kMxFe + 3
 };
+// (in a system of `dims` directions)
+TAG_HD constexpr bool fx_used(int k, int dims) {
+  const int r = k < kMxRho ? k : k < kMxN ? 0 : k < kMxFm ? k - kMxN : k < kMxFv ? k - kMxFm
+                : k < kMxFe ? k - kMxFv : k - kMxFe;
+  return r / 3 < dims && r % 3 < dims;
+}
 
-struct FxScale {
-  int sv, sr, sp, sx, sg;  // velocities (halved), density, pressure, transported scalar's node
-                           // value, geopotential differences
-  int sh;                  // the scalar's flux over the normal velocity (rho x + p/2)
-  int jh;                  // left shift of that sum
-  int sn[3], kq[3];        // contravariant vectors per direction; left shift of Q n
-  int ok;
+// Shifts that bring a pair's terms to their sums' scales, four to a word (a pair
+// reads them all, and registers bound the warps in flight): of the weighted normal
+// for the normal velocity and of the transported momentum for the momentum's sum,
+// both by component (right); of v.v by component; of 2 rho_mean g, of rho_mean x
+// and p/2 in h (right), of h itself (left).
+struct alignas(16) FxShift {
+  u32 n, t, v, hxpj;
 };
-constexpr int kFxDoubles = (sizeof(FxScale) + 7) / 8;  // its place in shared memory
+TAG_HD int fx_byte(u32 w, int k) {
+#ifdef __CUDA_ARCH__
+  return (int)__byte_perm(w, 0u, 0x4440u + k);
+#else
+  return (int)(w >> (8 * k)) & 255;
+#endif
+}
+template <int D>
+struct alignas(16) FxScale {
+  FxShift k[D];          // by direction
+  int sn[D][3];          // scales: contravariant vectors by direction and component,
+  int sum[D][5];         // each variable's sums by direction,
+  int sv[3];             // velocities (halved),
+  int sr, sp, sx, sg;    // density, pressure, transported scalar's node value, geopotential
+  int ok;
+  int zero[2], pad[2];   // at rest: the sums of mass and of the transported scalar are 0
+};
+// Whether variable v's sums are exactly 0 (their words are products of roundings).
+template <int D>
+TAG_HD bool fx_zero(const FxScale<D>& s, int v) {
+  return (v == 0 && s.zero[0]) || (v == D + 1 && s.zero[1]);
+}
+template <int D>
+constexpr int kFxDoubles = sizeof(FxScale<D>) / 8;  // its place in shared memory
+static_assert(kFxDoubles<2> % 2 == 0 && kFxDoubles<3> % 2 == 0, "16-byte aligned");
 
 TAG_HD u32 high_magnitude(double x) { return (u32)(f64_bits(x) >> 32) & 0x7fffffffu; }
+
+// A node's values and contravariant vectors into the maxima by up(FxMax, magnitude).
+// The words' products take densities as positive: bad states leave.
+template <int D, class Up>
+TAG_HD void fx_node_maxima(const double* q, const double* ja, Up up) {
+#pragma unroll
+  for (int c = 0; c < D; ++c) up(kMxV + c, high_magnitude(q[1 + c]));
+  up(kMxRho, not_positive(q[0]) ? 0x7ff00000u : high_magnitude(q[0]));
+  up(kMxP, high_magnitude(q[D + 1]));
+  up(kMxG, high_magnitude(q[D + 2]));
+  up(kMxX, not_positive(q[D + 3]) ? 0x7ff00000u : high_magnitude(q[D + 3]));
+#pragma unroll
+  for (int k = 0; k < D * D; ++k) up(kMxN + 3 * (k / D) + k % D, high_magnitude(ja[k]));
+}
+// Place of the surface flux of variable v on direction d's faces.
+template <int D>
+TAG_HD constexpr int fx_face_max(int v, int d) {
+  return v == 0 ? kMxFm + d : v == D + 1 ? kMxFe + d : kMxFv + 3 * d + v - 1;
+}
 
 // 2^k, and an upper bound of a high word's double over 2^s
 TAG_HD float pow2f(int k) { return f32_from((u32)(127 + max(-100, min(k, 100))) << 23); }
@@ -175,118 +221,146 @@ TAG_HD void fx_fit(float& x, int& s, float top) {
   s -= k;
 }
 
-// Scales of an element from its maxima mx (kMxF + 3 kind + d: surface fluxes of
-// the mass, the momentum and the transported scalar on direction d's faces) in
-// `dims` directions.  Each is the smallest that bounds the words derived from it
-// by 1/2, the bounds being products of the maxima themselves.
-TAG_HD FxScale fx_scale(const u32* mx, int dims, const FxBasis& b) {
-  const float top = 0.48f;
-  bool ok = b.ok != 0;
-  int e[kMxCount];  // value < 2^e
-  for (int k = 0; k < kMxCount; ++k) {
-    const int x = (int)(mx[k] >> 20) - 1022;
-    ok = ok && x <= 150;  // infinities and NaN have x = 1025
-    e[k] = x < -150 ? -150 : x;
+// Scales of an element of D directions from its maxima: each is the smallest that
+// bounds the words derived from it by 1/2, the bounds being products of the maxima
+// themselves.  One call per direction d (the calls share no results, so that a
+// thread each can take them); d = 0 also fills the common part.
+//
+// The weighted normals and the normal velocities of single pairs take the whole
+// word: they are what cancels where the wind blows along an element's faces.  The
+// room for the sums over a row of Q is left in density, pressure and h.
+template <int D>
+TAG_HD void fx_scale(const u32* mx, const FxBasis& b, int d, FxScale<D>& s) {
+  const float top = 0.48f, top_n = 0.49f;
+  // value < 2^e
+  const auto e = [mx](int k) { return max((int)(mx[k] >> 20) - 1022, -150); };
+  // velocities: the sums of a node's components and of two nodes' values fit a word
+  int sv[D], most_v = -1000;
+  float v[D], sum_v = 0.0f;
+#pragma unroll
+  for (int c = 0; c < D; ++c) {
+    sv[c] = e(kMxV + c) + 2;
+    v[c] = fx_fraction(mx[kMxV + c], sv[c]);
+    sum_v += v[c];
   }
-  FxScale s;
-  s.ok = ok ? 1 : 0;
-  s.sr = e[kMxRho] + 2;
-  s.sg = e[kMxG] + 2;
-  int ev = -150;
-  for (int c = 0; c < dims; ++c) ev = max(ev, e[kMxV + c]);
-  // so that the sums of a node's components and of two nodes' values fit a word
-  s.sv = ev + 2;
-  float sum = 0.0f, most_v = 0.0f;
-  for (int c = 0; c < dims; ++c) {
-    const float f = fx_fraction(mx[kMxV + c], s.sv);
-    sum += f;
-    most_v = fmaxf(most_v, f);
+#pragma unroll
+  for (int c = 0; c < D; ++c) {
+    if (!(sum_v <= top)) {
+      v[c] *= 0.5f;
+      sum_v -= v[c];
+      sv[c] += 1;
+    }
+    most_v = max(most_v, sv[c]);
   }
-  if (!(fmaxf(sum, 2.0f * most_v) <= 0.49f)) s.sv = ev + 3;
-  for (int d = 0; d < 3; ++d) {
-    s.sn[d] = d < dims ? e[kMxN + d] + 3 : 0;
-    s.kq[d] = 0;
+  // Scales sN of the weighted normals Q n by component (n: of a pair, per unit of Q)
+  // and svn of the normal velocity; vn is that of a pair, per unit of Q, and most_vn
+  // the largest of all directions'.
+  int sN[D], svn = 0;
+  float vn = 0.0f, most_vn = 0.0f;
+#pragma unroll
+  for (int dd = 0; dd < D; ++dd) {
+    float n[D], sum = 0.0f;
+    int sn[D], top_s = -10000;
+#pragma unroll
+    for (int c = 0; c < D; ++c) {
+      const u32 m = mx[kMxN + 3 * dd + c];
+      sn[c] = e(kMxN + 3 * dd + c) + 2;
+      n[c] = 2.0f * fx_fraction(m, sn[c]);
+      if (!(n[c] <= top_n)) {
+        n[c] *= 0.5f;
+        sn[c] += 1;
+      }
+      sn[c] += b.sq;
+      top_s = max(top_s, sn[c] + sv[c]);
+    }
+#pragma unroll
+    for (int c = 0; c < D; ++c) sum += 2.0f * v[c] * n[c] * pow2f(sn[c] + sv[c] - top_s);
+    most_vn = fmaxf(most_vn, sum);
+    if (dd == d) {
+#pragma unroll
+      for (int c = 0; c < D; ++c) sN[c] = sn[c];
+      svn = top_s;
+      vn = sum;
+    }
   }
-  for (int d = 0; d < dims; ++d)  // surface mass fluxes to 1/16
-    s.sv = max(s.sv, e[kMxF + d] + 4 - s.sr - s.sn[d] - b.sq);
-  const float rho = 2.0f * fx_fraction(mx[kMxRho], s.sr),
-              g = 2.0f * fx_fraction(mx[kMxG], s.sg);
-  float v = 0.0f, v1 = 0.0f, vv = 0.0f;  // largest component, their sum, sum of squares
-  for (int c = 0; c < dims; ++c) {
-    const float f = fx_fraction(mx[kMxV + c], s.sv);
-    v = fmaxf(v, f);
-    v1 += f;
-    vv += f * f;
-  }
+  // density: a row's mass fluxes to 0.36, surface fluxes to 1/8
+  int sr = e(kMxRho) + 2;
+  float rho = 2.0f * fx_fraction(mx[kMxRho], sr);
+  fx_fit(rho, sr, fminf(top, 0.36f / (b.row * fmaxf(most_vn, 1e-6f))));
   // x = mean(scalar) + v.v
-  s.sx = max(e[kMxX] + 2, 2 * s.sv);
-  float x = 2.0f * fx_fraction(mx[kMxX], s.sx) + vv * pow2f(2 * s.sv - s.sx);
-  fx_fit(x, s.sx, top);
-  // pressure sum +- 2 rho_mean g
-  s.sp = max(max(e[kMxP] + 2, s.sr + s.sg + 1), s.sr + 2 * s.sv);
-  for (int d = 0; d < dims; ++d) s.sp = max(s.sp, e[kMxF + 3 + d] + 4 - s.sn[d] - b.sq);
-  float pp = 2.0f * fx_fraction(mx[kMxP], s.sp) + rho * g * pow2f(s.sr + s.sg + 1 - s.sp);
-  fx_fit(pp, s.sp, top);
-  const float p = fx_fraction(mx[kMxP], s.sp);
-  // h = rho_mean x + (p +- 2 rho_mean g) / 2, shifted left by jh
-  s.sh = max(s.sr + s.sx, s.sp - 1);
-  int fluxes = -10000;  // surface fluxes to 1/16
-  for (int d = 0; d < dims; ++d)
-    fluxes = max(fluxes, e[kMxF + 6 + d] + 3 - s.sv - s.sn[d] - b.sq);
-  s.sh = max(s.sh, fluxes);
-  float h = rho * x * pow2f(s.sr + s.sx - s.sh) + pp * pow2f(s.sp - 1 - s.sh);
-  fx_fit(h, s.sh, top);
-  s.jh = max(0, min(min(fx_room(h, top), s.sh - fluxes), 8));
-  h *= pow2f(s.jh);
-  s.sh -= s.jh;
-  for (int d = 0; d < dims; ++d) {
-    const float n = 2.0f * fx_fraction(mx[kMxN + d], s.sn[d]);
-    const float vn = 2.0f * v1 * n;  // per unit of Q
-    const float mass = rho * vn;
-    const int sd = s.sn[d] + b.sq;
-    float most = b.one * vn;
-    most = fmaxf(most, b.row * mass + fx_fraction(mx[kMxF + d], s.sr + s.sv + sd));
-    most = fmaxf(most, b.row * (n * pp + 2.0f * mass * v * pow2f(s.sr + 2 * s.sv - s.sp)) +
-                           fx_fraction(mx[kMxF + 3 + d], s.sp + sd));
-    most = fmaxf(most, b.row * vn * (h + p * pow2f(s.sp - 1 - s.sh)) +
-                           0.5f * fx_fraction(mx[kMxF + 6 + d], s.sh + s.sv + sd));
-    most = fmaxf(most, b.one * n);
-    s.kq[d] = max(0, min(fx_room(most, top), 12));
-    most *= pow2f(s.kq[d]);
-    if (!(most <= 0.49f)) s.ok = 0;
+  int sx = max(e(kMxX) + 2, 2 * most_v);
+  float x = 2.0f * fx_fraction(mx[kMxX], sx);
+#pragma unroll
+  for (int c = 0; c < D; ++c) x += v[c] * v[c] * pow2f(2 * sv[c] - sx);
+  fx_fit(x, sx, top);
+  // pressure sum +- 2 rho_mean g: a row's pressure fluxes to 0.24, its transported
+  // momentum to 0.1
+  const int sg = e(kMxG) + 2;
+  const float g = 2.0f * fx_fraction(mx[kMxG], sg);
+  int sp = max(max(e(kMxP) + 2, sr + sg + 1), sr + 2 * most_v + 1);
+  float pp = 2.0f * fx_fraction(mx[kMxP], sp) + rho * g * pow2f(sr + sg + 1 - sp);
+  fx_fit(pp, sp, fminf(top, 0.24f / (top_n * b.row)));
+  if (d == 0) {
+    u32 all = 0;
+#pragma unroll
+    for (int k = 0; k < kMxCount; ++k)
+      if (fx_used(k, D)) all = max(all, mx[k]);
+    // (infinities and NaN have the exponent 1025)
+    s.ok = b.ok != 0 && (int)(all >> 20) - 1022 <= 150;
+    u32 mass = 0, scalar = 0;
+#pragma unroll
+    for (int c = 0; c < D; ++c) {
+      s.sv[c] = sv[c];
+      mass |= mx[kMxV + c] | mx[kMxFm + c];
+      scalar |= mx[kMxV + c] | mx[kMxFe + c];
+    }
+    s.zero[0] = mass == 0;
+    s.zero[1] = scalar == 0;
+    s.sr = sr;
+    s.sp = sp;
+    s.sx = sx;
+    s.sg = sg;
   }
-  return s;
+  // surface fluxes to 1/8
+  const int own = svn;
+  svn = max(svn, e(kMxFm + d) + 3 - sr);
+#pragma unroll
+  for (int c = 0; c < D; ++c) {
+    sN[c] = max(sN[c], e(kMxFv + 3 * d + c) + 3 - sp);
+    svn = max(svn, sN[c] + sv[c]);
+  }
+  vn *= pow2f(own - svn);
+  // h = rho_mean x + (p +- 2 rho_mean g) / 2, shifted left by kj: by what a row of it with
+  // the pressures' difference and the surface fluxes leave
+  int sh = max(sr + sx, sp - 1);
+  const float h = rho * x * pow2f(sr + sx - sh) + pp * pow2f(sp - 1 - sh);
+  const float row_h = b.row * vn * (h + fx_fraction(mx[kMxP], sp) * pow2f(sp - 1 - sh)) +
+                      0.5f * fx_fraction(mx[kMxFe + d], sh + svn);
+  const int room = min(min(fx_room(h, top), fx_room(row_h, top)), 8), kj = max(room, 0);
+  sh -= room;
+  FxShift k{};
+#pragma unroll
+  for (int c = 0; c < D; ++c) {
+    sN[c] = max(sN[c], sr + svn + sv[c] - sp);
+    k.n |= (u32)min(svn - sv[c] - sN[c], 63) << (8 * c);
+    k.t |= (u32)min(sN[c] + sp - sr - svn - sv[c], 63) << (8 * c);
+    k.v |= (u32)min(sx - 2 * sv[c], 63) << (8 * c);
+    s.sn[d][c] = sN[c] - b.sq;
+    s.sum[d][1 + c] = sN[c] + sp;
+  }
+  k.hxpj = (u32)min(sp - sr - sg - 1, 63) | (u32)min(sh + kj - sr - sx, 63) << 8 |
+           (u32)min(sh + kj - sp + 1, 63) << 16 | (u32)kj << 24;
+  s.k[d] = k;
+  s.sum[d][0] = sr + svn;
+  s.sum[d][D + 1] = sh + svn;
 }
 
-// Scale of the sums of kind 0 mass, 1 momentum, 2 transported scalar in
-// direction d (without the basis' part).
-TAG_HD int fx_kind_scale(const FxScale& s, int kind) {
-  return kind == 0 ? s.sr + s.sv : kind == 1 ? s.sp : s.sh + s.sv;
-}
-TAG_HD int fx_direction_scale(const FxScale& s, int d) { return s.sn[d] - s.kq[d]; }
-
-// Shifts that bring a pair's terms to their sums' scales, taken of an operand
-// before the product (which rounds; a shift of the product would truncate).
-struct FxShift {
-  int t, h, v, x, p, j;  // f v, 2 rho_mean g, v.v, rho_mean x and p/2 in h, h itself (left)
-};
-TAG_HD FxShift fx_shift(const FxScale& s) {
-  FxShift k;
-  k.t = min(s.sp - s.sr - 2 * s.sv, 63);
-  k.h = min(s.sp - s.sr - s.sg - 1, 63);
-  k.v = min(s.sx - 2 * s.sv, 63);
-  k.x = min(s.sh + s.jh - s.sr - s.sx, 63);
-  k.p = min(s.sh + s.jh - s.sp + 1, 63);
-  k.j = s.jh;
-  return k;
-}
-
-// The sum over the D directions of A[d stride] W_d (words of scales sd[d] + one
-// common part, W_d >= 0), as a word whose scale is the common part + `scale`.
+// The sum over the D directions of A[d stride] W_d (words of scales sd[d], W_d >=
+// 0), as a word of scale `scale`.
 // The sums are cancelled ones: they are brought to the coarsest direction's
 // scale and then up to the word's top before the products.
 template <int D>
-TAG_DEV i64 fx_weighted_sum(const i64* A, int stride, const i64* W, const int* node, const int* sd,
+TAG_HD i64 fx_weighted_sum(const i64* A, int stride, const i64* W, const int* node, const int* sd,
                             int& scale) {
   int top = sd[0];
 #pragma unroll
@@ -299,7 +373,7 @@ TAG_DEV i64 fx_weighted_sum(const i64* A, int stride, const i64* W, const int* n
     all |= (u64)(a[d] ^ (a[d] >> 63));
   }
   // three leading zeros: three terms below 1/8 (a sum may need two places down)
-  const int lz = __clzll((i64)all), up = max(lz - 3, 0), down = max(3 - lz, 0);
+  const int lz = leading_zeros(all), up = max(lz - 3, 0), down = max(3 - lz, 0);
   i64 tot = 0;
 #pragma unroll
   for (int d = 0; d < D; ++d) tot += hmul_pos((a[d] >> down) << up, W[node[d]]);
@@ -310,7 +384,7 @@ TAG_DEV i64 fx_weighted_sum(const i64* A, int stride, const i64* W, const int* n
 // c with factor = 1 - c (Q0.64) of a logarithmic mean of two words of one scale
 // from the difference of the logarithms; beyond a factor of 256 the far branch
 // divides in FP64.
-static __device__ __noinline__ u64 fx_far_deficit(i64 a, i64 b, i64 d, int inverse) {
+TAG_SLOW u64 fx_far_deficit(i64 a, i64 b, i64 d, int inverse) {
   const u64 m = magnitude(d);
   if (middle_range(m))
     return inverse ? inv_ln_mean_deficit_middle(m) : ln_mean_deficit_middle(m);
@@ -319,90 +393,89 @@ static __device__ __noinline__ u64 fx_far_deficit(i64 a, i64 b, i64 d, int inver
   return f < 1.0 && f > 0.0 ? (u64)((1.0 - f) * 18446744073709551616.0) : 0;
 }
 // The two means of a pair, each c by the form that fits its own difference.
-TAG_DEV u64 fx_ln_deficit(i64 a, i64 b, i64 d) {
+TAG_HD u64 fx_ln_deficit(i64 a, i64 b, i64 d) {
   const u64 m = magnitude(d);
   if (!series_in_range(m)) return fx_far_deficit(a, b, d, 0);
   const u64 z = log_square(m);
   return z < kShortZ ? ln_mean_deficit_short(z) : ln_mean_deficit(z);
 }
-TAG_DEV u64 fx_inv_ln_deficit(i64 a, i64 b, i64 d) {
+TAG_HD u64 fx_inv_ln_deficit(i64 a, i64 b, i64 d) {
   const u64 m = magnitude(d);
   if (!series_in_range(m)) return fx_far_deficit(a, b, d, 1);
   const u64 z = log_square(m);
   return z < kShortZ ? inv_ln_mean_deficit_short(z) : inv_ln_mean_deficit(z);
 }
 // s (1 - c) of a positive sum
-TAG_DEV i64 fx_reduce(i64 s, u64 c) { return s - (i64)umul_high((u64)s, c) - 1; }
+TAG_HD i64 fx_reduce(i64 s, u64 c) { return s - (i64)umul_high((u64)s, c) - 1; }
 
 // Node values of one element's words: rho/2, the halved velocities, p/2, the
 // geopotential's quarter relative to the element's first node, the transported
 // scalar's node value, then two logarithm words that are kept.  The velocities
 // are stored with their offset (a sum of two offset words is the plain sum).
 template <int D>
-TAG_DEV void fx_convert_node(double* q, const FxScale& s) {
+TAG_HD void fx_convert_node(double* q, const FxScale<D>& s) {
   i64* w = reinterpret_cast<i64*>(q);
   w[0] = to_fixed(q[0], s.sr - 2);
 #pragma unroll
-  for (int k = 1; k <= D; ++k) w[k] = (i64)offset_word(to_fixed(q[k], s.sv - 2));
+  for (int c = 0; c < D; ++c) w[1 + c] = (i64)offset_word(to_fixed(q[1 + c], s.sv[c] - 2));
   w[D + 1] = to_fixed(q[D + 1], s.sp - 2);
   w[D + 2] = to_fixed(q[D + 2], s.sg - 2);
   w[D + 3] = to_fixed(q[D + 3], s.sx - 2);
 }
 
 // The pair flux of the energy equations (volume_pair of PhysEnergy2D / 3D) in
-// words, weighted by Q_ab >= 0 (the caller orders the pair so): node a adds Fa,
+// words, weighted by Q_ab > 0 (the caller orders the pair so): node a adds Fa,
 // node b subtracts Fb.  The scalar's
 // flux is regrouped as
 //   vn (rho_mean x + (p +- 2 rho_mean g) / 2) + (p_a - p_b)(vn_b - vn_a) / 2,
 // whose factor of vn is one word near its top.  27 (3D) or 20 (2D) products.
 template <int D>
-TAG_DEV void fx_energy_pair(const i64* qa, const i64* qb, const i64* na, const i64* nb, i64 Q,
-                            const FxShift& k, int kq, i64* Fa, i64* Fb) {
+TAG_HD void fx_energy_pair(const i64* qa, const i64* qb, const i64* na, const i64* nb, u64 Q,
+                           const FxShift& k, i64* Fa, i64* Fb) {
   const i64 rho = fx_reduce(qa[0] + qb[0], fx_ln_deficit(qa[0], qb[0], qb[D + 4] - qa[D + 4]));
   i64 x = fx_reduce(qa[D + 3] + qb[D + 3],
                     fx_inv_ln_deficit(qa[D + 3], qb[D + 3], qb[D + 5] - qa[D + 5]));
   // normal velocities of both nodes and v_a.v_b: each product's offset terms
   // are collected, halves of the components' sums for the velocities
-  i64 nq[D], hq = 0;
+  i64 nq[D], v[D], hq = 0;
   u64 ua = 0, ub = 0;
-  u64 va = 0, vb = 0, vv = 0;
+  u64 va = 0, vb = 0;
 #pragma unroll
-  for (int d = 0; d < D; ++d) {
-    nq[d] = hmul_pos(na[d] + nb[d], Q) << kq;
-    const u64 nw = offset_word(nq[d]), wa = (u64)qa[1 + d], wb = (u64)qb[1 + d];
+  for (int c = 0; c < D; ++c) {
+    nq[c] = hmul_pos(na[c] + nb[c], Q);
+    const i64 nv = nq[c] >> fx_byte(k.n, c);
+    const u64 nw = offset_word(nv), wa = (u64)qa[1 + c], wb = (u64)qb[1 + c];
     va += umul_high(nw, wa);
     vb += umul_high(nw, wb);
-    vv += umul_high(wa, wb);
-    hq += nq[d] >> 1;
-    ua += offset_word(qa[1 + d]);
-    ub += offset_word(qb[1 + d]);
+    hq += nv >> 1;
+    ua += offset_word(qa[1 + c]);
+    ub += offset_word(qb[1 + c]);
+    v[c] = (i64)(wa + wb);
+    x += (i64)(umul_high(wa, wb) - (u64)(v[c] >> 1) - (kOffset - 1)) >> fx_byte(k.v, c);
   }
   const i64 sa = (i64)ua >> 1, sb = (i64)ub >> 1;
   constexpr u64 kDot = D * kOffset - D;  // modulo 2^64; the sums themselves fit
   const i64 vna = (i64)(va - kDot - (u64)(hq + sa)), vnb = (i64)(vb - kDot - (u64)(hq + sb));
-  x += (i64)(vv - kDot - (u64)(sa + sb)) >> k.v;
   const i64 vn = vna + vnb, f1 = hmul_pos(vn, rho);
-  const i64 h = hmul_pos((qb[D + 2] - qa[D + 2]) >> k.h, rho), p = qa[D + 1] + qb[D + 1];
+  const int kx = fx_byte(k.hxpj, 1), kp = fx_byte(k.hxpj, 2), kj = fx_byte(k.hxpj, 3);
+  const i64 h = hmul_pos((qb[D + 2] - qa[D + 2]) >> fx_byte(k.hxpj, 0), rho), p = qa[D + 1] + qb[D + 1];
   const i64 pp = p + h, pm = p - h;
-  const u64 wp = offset_word(pp), wm = offset_word(pm);
-  const i64 fs = f1 >> k.t;
-  const u64 c = (u64)(fs >> 1) + 2 * kOffset - 2;
-  const u64 cp = c + (u64)(pp >> 1), cm = c + (u64)(pm >> 1) + 1;
-  const u64 wf = offset_word(fs);
+  const u64 wf = offset_word(f1), wp = offset_word(pp), wm = offset_word(pm);
+  const u64 cf = kOffset - 1 + (u64)(f1 >> 1);
+  const u64 cp = kOffset - 1 + (u64)(pp >> 1), cm = kOffset - 1 + (u64)(pm >> 1);
   Fa[0] = f1;
   Fb[0] = f1;
 #pragma unroll
-  for (int d = 0; d < D; ++d) {
-    const i64 v = (i64)((u64)qa[1 + d] + (u64)qb[1 + d]);
-    const u64 t = umul_high(wf, offset_word(v)) - (u64)((v >> 1) + (nq[d] >> 1));
-    const u64 nw = offset_word(nq[d]);
-    Fa[1 + d] = (i64)(t + umul_high(nw, wp) - cp);
-    Fb[1 + d] = (i64)(t + umul_high(nw, wm) - cm);
+  for (int c = 0; c < D; ++c) {
+    const i64 t = (i64)(umul_high(wf, offset_word(v[c])) - (u64)(v[c] >> 1) - cf) >> fx_byte(k.t, c);
+    const u64 nw = offset_word(nq[c]), base = (u64)(t - (nq[c] >> 1));
+    Fa[1 + c] = (i64)(base + umul_high(nw, wp) - cp);
+    Fb[1 + c] = (i64)(base + umul_high(nw, wm) - cm);
   }
-  const i64 rx = hmul_pos(x, rho) >> k.x;
-  const i64 w = hmul_raw(((qa[D + 1] - qb[D + 1]) >> k.p) << k.j, vnb - vna);
-  Fa[D + 1] = hmul_raw(vn, (rx + (pp >> k.p)) << k.j) + w + 2;
-  Fb[D + 1] = hmul_raw(vn, (rx + (pm >> k.p)) << k.j) + w + 1;
+  const i64 rx = hmul_pos(x, rho) >> kx;
+  const i64 w = hmul_raw(((qa[D + 1] - qb[D + 1]) >> kp) << kj, vnb - vna);
+  Fa[D + 1] = hmul_raw(vn, (rx + (pp >> kp)) << kj) + w + 2;
+  Fb[D + 1] = hmul_raw(vn, (rx + (pm >> kp)) << kj) + w + 1;
 }
 
 // A surface flux below half of its sum's scale 2^s as a word of that scale, with

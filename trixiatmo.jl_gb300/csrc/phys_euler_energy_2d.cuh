@@ -39,7 +39,7 @@ struct PhysEnergy2D {
 
   // cons2prim (:527-536), once per node, the reciprocal and both logarithms
   // on the integer pipe; flags bad states.
-  TAG_DEV static void node_prims(const Params& P, const double* u, double* q, unsigned& bad) {
+  TAG_HD static void node_prims(const Params& P, const double* u, double* q, unsigned& bad) {
     const double rho = u[0];
     const double ir = int_rcp(rho), hir = 0.5 * ir;
     const double p = P.gm1 * fma(-hir, fma(u[2], u[2], u[1] * u[1]), u[3]);
@@ -67,8 +67,8 @@ struct PhysEnergy2D {
   // half the energy fluxes
   //   f1 (v_a.v_b / 4 + mean(p/rho) / (2 (gamma - 1)) +- g) + (p_a vn_b + p_b vn_a) / 4.
   // Elements in range take fx_energy_pair (fixed_flux.cuh) instead.
-  TAG_DEV static void volume_pair(const Params& P, const double* qa, const double* qb,
-                                  double n1, double n2, double* Fa, double* Fb) {
+  TAG_HD static void volume_pair(const Params& P, const double* qa, const double* qb,
+                                 double n1, double n2, double* Fa, double* Fb) {
     const double R = ln_factor(qa[0], qb[0], log_difference(qa[6], qb[6]));
     const double Q = inv_ln_factor(qa[5], qb[5], log_difference(qa[7], qb[7]));
     const double rho_mean = (qa[0] + qb[0]) * R;
@@ -94,12 +94,12 @@ struct PhysEnergy2D {
     Fb[3] = fma(-f1, g, e);
   }
 
-  TAG_DEV static void fixed_pair(const Params&, const double* qa, const double* qb,
-                                 const double* na, const double* nb, i64 Q, const FxShift& k,
-                                 int kq, i64* Fa, i64* Fb) {
+  TAG_HD static void fixed_pair(const Params&, const double* qa, const double* qb,
+                                const double* na, const double* nb, u64 Q, const FxShift& k,
+                                i64* Fa, i64* Fb) {
     fx_energy_pair<2>(reinterpret_cast<const i64*>(qa), reinterpret_cast<const i64*>(qb),
-                      reinterpret_cast<const i64*>(na), reinterpret_cast<const i64*>(nb), Q, k, kq,
-                      Fa, Fb);
+                      reinterpret_cast<const i64*>(na), reinterpret_cast<const i64*>(nb), Q, k, Fa,
+                      Fb);
   }
 
   // FluxLMARS (:397-430) between states ul, ur for the (unnormalised) normal n:

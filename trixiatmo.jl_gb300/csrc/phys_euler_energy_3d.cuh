@@ -38,7 +38,7 @@ struct PhysEnergy3D {
 
   // cons2prim (:568-578) once per node, the reciprocal and both logarithms on
   // the integer pipe.
-  TAG_DEV static void node_prims(const Params& P, const double* u, double* q, unsigned& bad) {
+  TAG_HD static void node_prims(const Params& P, const double* u, double* q, unsigned& bad) {
     const double rho = u[0];
     const double ir = int_rcp(rho), hir = 0.5 * ir;
     const double m2 = fma(u[3], u[3], fma(u[2], u[2], u[1] * u[1]));
@@ -69,8 +69,8 @@ struct PhysEnergy3D {
   // the means go to the integer pipe (int_math.cuh): the right-hand side of
   // the 2,654,208-node shell at polydeg 5 went from 3.48 to 2.32 ms.  Elements
   // in range take fx_energy_pair (fixed_flux.cuh) instead of this form.
-  TAG_DEV static void volume_pair(const Params& P, const double* qa, const double* qb,
-                                  const double* nrm, double* Fa, double* Fb) {
+  TAG_HD static void volume_pair(const Params& P, const double* qa, const double* qb,
+                                 const double* nrm, double* Fa, double* Fb) {
     const double R = ln_factor(qa[0], qb[0], log_difference(qa[7], qb[7]));
     const double Q = inv_ln_factor(qa[6], qb[6], log_difference(qa[8], qb[8]));
     const double rho_mean = (qa[0] + qb[0]) * R;
@@ -99,12 +99,12 @@ struct PhysEnergy3D {
     Fb[4] = fma(-f1, g, e);
   }
 
-  TAG_DEV static void fixed_pair(const Params&, const double* qa, const double* qb,
-                                 const double* na, const double* nb, i64 Q, const FxShift& k,
-                                 int kq, i64* Fa, i64* Fb) {
+  TAG_HD static void fixed_pair(const Params&, const double* qa, const double* qb,
+                                const double* na, const double* nb, u64 Q, const FxShift& k,
+                                i64* Fa, i64* Fb) {
     fx_energy_pair<3>(reinterpret_cast<const i64*>(qa), reinterpret_cast<const i64*>(qb),
-                      reinterpret_cast<const i64*>(na), reinterpret_cast<const i64*>(nb), Q, k, kq,
-                      Fa, Fb);
+                      reinterpret_cast<const i64*>(na), reinterpret_cast<const i64*>(nb), Q, k, Fa,
+                      Fb);
   }
 
   // FluxLMARS (3D, :430-466) for the (unnormalised) normal n:

@@ -24,56 +24,56 @@ constexpr int kMaxNodes = 8;  // n = polydeg + 1 supported up to polydeg 7
 // no logarithm, no branch that splits a warp.  Up to a factor of 256 (vertical
 // pairs of elements some 5 km tall and more, edges of clouds) an exponential of d
 // and a reciprocal in words; beyond, d itself is the logarithm of the definition.
-TAG_DEV double log_of_difference(i64 d) { return (double)d * 1.539095918623324e-16; }  // ln2 2^-52
+TAG_HD double log_of_difference(i64 d) { return (double)d * 1.539095918623324e-16; }  // ln2 2^-52
 
 // Values of opposite sign, which partial densities and bad states may have, give
 // NaN: the logarithm of their ratio.  Beside a zero the mean is 0 and its inverse
 // has no value.
-TAG_DEV bool opposite_signs(double a, double b) { return (i64)(f64_bits(a) ^ f64_bits(b)) < 0; }
-TAG_DEV bool is_zero(double x) { return (f64_bits(x) << 1) == 0; }
-TAG_DEV double quiet_nan() { return f64_from(0x7ff8000000000000ull); }
+TAG_HD bool opposite_signs(double a, double b) { return (i64)(f64_bits(a) ^ f64_bits(b)) < 0; }
+TAG_HD bool is_zero(double x) { return (f64_bits(x) << 1) == 0; }
+TAG_HD double quiet_nan() { return f64_from(0x7ff8000000000000ull); }
 // A node value whose inverse is averaged: NaN in place of zero.
-TAG_DEV double invertible(double x) { return is_zero(x) ? quiet_nan() : x; }
-static __device__ __noinline__ double ln_factor_far(double xa, double xb, i64 d) {
+TAG_HD double invertible(double x) { return is_zero(x) ? quiet_nan() : x; }
+TAG_SLOW double ln_factor_far(double xa, double xb, i64 d) {
   if (opposite_signs(xa, xb)) return quiet_nan();
   if (is_zero(xa) || is_zero(xb)) return 0.0;
   const u64 a = magnitude(d);
   if (middle_range(a)) return middle_factor(ln_mean_deficit_middle(a));
   return int_div(2.0 * (xb - xa), log_of_difference(d) * (xa + xb));
 }
-static __device__ __noinline__ double inv_ln_factor_far(double ya, double yb, i64 d) {
+TAG_SLOW double inv_ln_factor_far(double ya, double yb, i64 d) {
   if (opposite_signs(ya, yb) || is_zero(ya) || is_zero(yb)) return quiet_nan();
   const u64 a = magnitude(d);
   if (middle_range(a)) return middle_factor(inv_ln_mean_deficit_middle(a));
   return int_div(2.0 * ya * yb * log_of_difference(d), (yb - ya) * (ya + yb));
 }
-TAG_DEV double ln_factor(double xa, double xb, i64 d) {
+TAG_HD double ln_factor(double xa, double xb, i64 d) {
   const u64 a = magnitude(d);
   return series_in_range(a) ? ln_mean_factor(log_square(a)) : ln_factor_far(xa, xb, d);
 }
-TAG_DEV double inv_ln_factor(double ya, double yb, i64 d) {
+TAG_HD double inv_ln_factor(double ya, double yb, i64 d) {
   const u64 a = magnitude(d);
   return series_in_range(a) ? inv_ln_mean_factor(log_square(a)) : inv_ln_factor_far(ya, yb, d);
 }
 
 // The means of two values themselves (interface kernels): ln_mean(x, y), and
 // inv_ln_mean(1/x, 1/y) from the reciprocals' own values.
-TAG_DEV double ln_mean_of(double x, double y) {
+TAG_HD double ln_mean_of(double x, double y) {
   return 0.5 * (x + y) * ln_factor(x, y, log2_fixed(y) - log2_fixed(x));
 }
-TAG_DEV double inv_ln_mean_of_reciprocals(double x, double y) {
+TAG_HD double inv_ln_mean_of_reciprocals(double x, double y) {
   return 0.5 * (x + y) * inv_ln_factor(x, y, log2_fixed(y) - log2_fixed(x));
 }
 
 // Node logarithms are kept among the other node quantities as raw words.
-TAG_DEV double log_word(double x) { return f64_from((u64)log2_fixed(x)); }
+TAG_HD double log_word(double x) { return f64_from((u64)log2_fixed(x)); }
 // The same where values below zero are common: log2_fixed's words of negative
 // values without its out-of-line branch.
-TAG_DEV double log_word_signed(double x) {
+TAG_HD double log_word_signed(double x) {
   const u64 b = f64_bits(x);
   return f64_from((u64)log2_fixed(f64_from(b & 0x7fffffffffffffffull)) + ((b >> 63) << 62));
 }
-TAG_DEV i64 log_difference(double wa, double wb) { return (i64)(f64_bits(wb) - f64_bits(wa)); }
+TAG_HD i64 log_difference(double wa, double wb) { return (i64)(f64_bits(wb) - f64_bits(wa)); }
 
 // FP64 forms of the two means, which the diagnostics (tag_means.cu) hold beside
 // the kernels' integer forms.  With f2 = ((y-x)/(y+x))^2 and z = sqrt(f2):
@@ -205,19 +205,16 @@ TAG_DEV void ln_mean_pair_halved(double hxa, double hxb, double hya, double hyb,
 // !(x > 0.0) and !isfinite(x) on the integer pipe (the FP64 pipe is the
 // element kernels' bottleneck): IEEE bit patterns of positive doubles order
 // like their values, and an exponent field of all ones is an infinity or NaN.
-TAG_DEV bool not_positive(double x) {
-  return (unsigned long long)__double_as_longlong(x) - 1ull >= 0x7ff0000000000000ull;
-}
-TAG_DEV bool not_finite(double x) {
-  return ((unsigned long long)__double_as_longlong(x) & 0x7ff0000000000000ull) ==
-         0x7ff0000000000000ull;
+TAG_HD bool not_positive(double x) { return f64_bits(x) - 1ull >= 0x7ff0000000000000ull; }
+TAG_HD bool not_finite(double x) {
+  return (f64_bits(x) & 0x7ff0000000000000ull) == 0x7ff0000000000000ull;
 }
 
 // 2 x of a normal number with a normal double (an exponent increment on the
 // integer pipe); zero becomes 2^-1022, which any product or sum absorbs.
-TAG_DEV double twice(double x) { return f64_from(f64_bits(x) + (1ull << 52)); }
+TAG_HD double twice(double x) { return f64_from(f64_bits(x) + (1ull << 52)); }
 // x / 2 of a normal number with a normal half
-TAG_DEV double half_of(double x) { return f64_from(f64_bits(x) - (1ull << 52)); }
+TAG_HD double half_of(double x) { return f64_from(f64_bits(x) - (1ull << 52)); }
 
 // Programmatic dependent launch (launch_overlapped): a kernel lets the next one
 // of its stream start once all its CTAs are past their main work (earlier, the
