@@ -279,6 +279,22 @@ def test_words_are_no_less_precise_than_fp64(host, D, n, width, wind, tilt):
     assert np.all(words[~some] == 0)
 
 
+@pytest.mark.parametrize("n", range(2, 9))
+def test_end_fluxes_have_their_exact_weight(host, n):
+    """An element at rest takes its mass fluxes through the faces over the end weight 2 / (n (n - 1)):
+    one rounding, and 2^-60 of the largest for the words (four places of scale)."""
+    rng = np.random.default_rng(n)
+    u, ja, sf = flat_element(2, n, 4, 0.0, rng)
+    sf[:] = 0
+    sf[:, 0] = rng.uniform(0.5, 1, len(sf))
+    ok, ew, _, _ = host(2, n, u, ja, sf)
+    limit = 0.5 * np.spacing(sf.reshape(4, n, 4)[..., 0] * (n * (n - 1) / 2)) + n * n * 2.0 ** -60
+    assert ok
+    for f in range(4):
+        inner = end_nodes(2, n, f)[1:-1]  # the corners have a second face
+        assert np.all(np.abs(ew[inner, 0]) <= limit[f, 1:-1])
+
+
 @pytest.mark.parametrize("D,n", [(2, 2), (2, 5), (2, 8), (3, 3)])
 def test_words_do_not_overflow(host, D, n):
     rng = np.random.default_rng(10 * D + n)

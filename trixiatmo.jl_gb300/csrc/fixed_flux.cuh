@@ -106,8 +106,10 @@ inline void load_fixed_basis(FxBasis& f, const double* Ds, const double* w, int 
   // -w_b Dsplit_ba differ in their last places: the weights are adjusted to the
   // least sum of those relative differences squared (by a few 1e-16), and the
   // mean of the two is taken, so that Q_ab / w_a is as near Dsplit_ab as one
-  // antisymmetric matrix can be.  The surface fluxes, whose weight stays 1/w, are
-  // scaled by the change (S).
+  // antisymmetric matrix can be.  The surface fluxes, whose weight stays the
+  // rounded 1/w of the FP64 form (the end weights are 2 / (n (n - 1)): the quotient is
+  // the exact integer, which the rounded weight's own inverse is not), are scaled by
+  // the change (S).
   long double ww[8];
   for (int a = 0; a < n; ++a) {
     long double r = 0.0L;
@@ -124,8 +126,8 @@ inline void load_fixed_basis(FxBasis& f, const double* Ds, const double* w, int 
     }
     f.W[a] = (i64)llroundl(ldexpl(1.0L / ww[a], 64 - f.kw));
   }
-  f.S[0] = (int)lroundl(ldexpl(ww[0] / w[0] - 1.0L, 63));
-  f.S[1] = (int)lroundl(ldexpl(ww[n - 1] / w[n - 1] - 1.0L, 63));
+  f.S[0] = (int)lroundl(ldexpl(ww[0] * (1.0 / w[0]) - 1.0L, 63));
+  f.S[1] = (int)lroundl(ldexpl(ww[n - 1] * (1.0 / w[n - 1]) - 1.0L, 63));
 }
 
 // Largest magnitudes of an element's fields, as high words of the doubles
