@@ -221,7 +221,7 @@ def exact(D, n, u, ja, sf, op=None):
     return acc, np.maximum(size, np.abs(acc))
 
 
-def flat_element(D, n, width, wind, rng, tilt=0.0, scatter=0.0, height=1000.0):
+def flat_element(D, n, width, wind, rng, tilt=0.0, scatter=0.0, height=1000.0, octaves=None):
     """Node values, contravariant vectors and the end fluxes of the element's own traces: `width`
     heights wide, hydrostatic, wind along it and 1/width of that across."""
     x = 0.5 * (1 + lobatto(n))
@@ -233,7 +233,8 @@ def flat_element(D, n, width, wind, rng, tilt=0.0, scatter=0.0, height=1000.0):
     ja[:, range(D), range(D)] = np.prod(size) / 2 ** (D - 1) / size
     ja[:, D - 1, 0] = -tilt * ja[:, D - 1, D - 1] * rng.uniform(0.5, 1, N)
     T = rng.uniform(220, 300) * (1 + 1e-3 * rng.uniform(-1, 1, N))
-    p = 1e5 * np.exp(-G * z / (287 * T.mean())) * np.exp2(scatter * rng.uniform(-1, 1, N))
+    fall = G * height / (287 * T.mean()) if octaves is None else octaves * np.log(2)
+    p = 1e5 * np.exp(-fall * z / height) * np.exp2(scatter * rng.uniform(-1, 1, N))
     rho = p / (287 * T) * np.exp2(scatter * rng.uniform(-1, 1, N))
     v = wind * rng.uniform(-1, 1, (N, D))
     v[:, D - 1] /= width
@@ -277,6 +278,23 @@ def test_words_are_no_less_precise_than_fp64(host, D, n, width, wind, tilt):
     some = fp64 > 0  # at rest the fluxes of mass and energy vanish
     assert np.all(words[some] <= 1.25 * fp64[some]), words / fp64
     assert np.all(words[~some] == 0)
+
+
+@pytest.mark.parametrize("D,n", [(2, 3), (2, 4), (2, 6), (3, 4)])
+@pytest.mark.parametrize("octaves", [1, 2, 3, 4, 6, 8, 12, 16])
+def test_thin_nodes_of_tall_elements(host, D, n, octaves):
+    """Isothermal elements whose density falls by 2^octaves: up to 3 are taken in words, from 4 on in
+    FP64, and no row of nodes loses more than a binary place to the FP64 form."""
+    words, fp64 = [], []
+    for seed in range(40 if D == 2 else 6):
+        u, ja, sf = flat_element(D, n, 20, 20.0, np.random.default_rng(seed), octaves=octaves)
+        ok, ew, ef, _ = host(D, n, u, ja, sf)
+        assert ok if octaves <= 3 else not ok
+        if not ok:
+            return
+        words.append((ew ** 2).reshape(n, -1, D + 2).mean(1))
+        fp64.append((ef ** 2).reshape(n, -1, D + 2).mean(1))
+    assert np.all(np.mean(words, 0) <= 4 * np.mean(fp64, 0))
 
 
 @pytest.mark.parametrize("n", range(2, 9))

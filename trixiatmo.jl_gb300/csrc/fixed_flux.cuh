@@ -24,7 +24,7 @@
 // it is 0.6 to 1.1 now at every width.
 //
 // Elements whose values leave the scales' range (infinities, NaN, magnitudes
-// beyond 2^+-150) take the FP64 form.
+// beyond 2^+-150) or spread too far (kMaxSpread) take the FP64 form.
 #pragma once
 #include <algorithm>
 #include <cmath>
@@ -135,9 +135,11 @@ inline void load_fixed_basis(FxBasis& f, const double* Ds, const double* w, int 
 // contravariant vectors and the surface fluxes of momentum by component: the
 // vertical face of a flat element can be thousands of times its lateral ones,
 // and a component that is small or zero must not be rounded at the largest one's
-// scale (kMxN, kMxFv: 3 direction + component).
+// scale (kMxN, kMxFv: 3 direction + component).  kMx...Low: the smallest density,
+// pressure and transported scalar, as the largest of kHighInf less the high word.
+constexpr u32 kHighInf = 0x7ff00000u;
 enum FxMax : int {
-  kMxV = 0, kMxRho = kMxV + 3, kMxP, kMxX, kMxG, kMxN, kMxFm = kMxN + 9, kMxFv = kMxFm + 3,
+  kMxV = 0, kMxRho = kMxV + 3, kMxP, kMxX, kMxRhoLow, kMxPLow, kMxXLow, kMxG, kMxN, kMxFm = kMxN + 9, kMxFv = kMxFm + 3,
   kMxFe = kMxFv + 9, kMxCount = kMxFe + 3
 };
 // (in a system of `dims` directions)
@@ -189,10 +191,16 @@ template <int D, class Up>
 TAG_HD void fx_node_maxima(const double* q, const double* ja, Up up) {
 #pragma unroll
   for (int c = 0; c < D; ++c) up(kMxV + c, high_magnitude(q[1 + c]));
-  up(kMxRho, not_positive(q[0]) ? 0x7ff00000u : high_magnitude(q[0]));
-  up(kMxP, high_magnitude(q[D + 1]));
+  const u32 rho = not_positive(q[0]) ? kHighInf : high_magnitude(q[0]);
+  const u32 p = not_positive(q[D + 1]) ? kHighInf : high_magnitude(q[D + 1]);
+  const u32 x = not_positive(q[D + 3]) ? kHighInf : high_magnitude(q[D + 3]);
+  up(kMxRho, rho);
+  up(kMxP, p);
+  up(kMxX, x);
+  up(kMxRhoLow, kHighInf - rho);
+  up(kMxPLow, kHighInf - p);
+  up(kMxXLow, kHighInf - x);
   up(kMxG, high_magnitude(q[D + 2]));
-  up(kMxX, not_positive(q[D + 3]) ? 0x7ff00000u : high_magnitude(q[D + 3]));
 #pragma unroll
   for (int k = 0; k < D * D; ++k) up(kMxN + 3 * (k / D) + k % D, high_magnitude(ja[k]));
 }
@@ -208,6 +216,15 @@ TAG_HD float fx_fraction(u32 hi, int s) {
   const float m = f32_from(0x3f800000u + ((hi & 0xfffffu) << 3) + 8u);  // [1, 2]
   return m * pow2f((int)(hi >> 20) - 1023 - s);
 }
+
+// Half octaves that density, pressure or temperature may spread over within an
+// element.  The words are rounded at the scale of an element's largest values, FP64
+// numbers at their own, so the least dense nodes lose what the spread takes.  Error of
+// the thinnest row of nodes against extended precision, over the FP64 form's, in an
+// isothermal atmosphere at polydegs 3 and 5: up to 1.04 at 2^3 (15 km in one element),
+// 1.6 at 2^4, 2.6 at 2^5, 6 at 2^6, 26 at 2^8; of the whole element 0.6 to 1.06 at
+// every spread.
+constexpr u32 kMaxSpread = 7;
 
 // The largest k with x 2^k <= top (x > 0; 120 for x = 0), and a bound x of scale s
 // brought under top by raising s.
@@ -303,12 +320,14 @@ TAG_HD void fx_scale(const u32* mx, const FxBasis& b, int d, FxScale<D>& s) {
   float pp = 2.0f * fx_fraction(mx[kMxP], sp) + rho * g * pow2f(sr + sg + 1 - sp);
   fx_fit(pp, sp, fminf(top, 0.24f / (top_n * b.row)));
   if (d == 0) {
-    u32 all = 0;
+    u32 all = 0, spread = 0;
 #pragma unroll
     for (int k = 0; k < kMxCount; ++k)
-      if (fx_used(k, D)) all = max(all, mx[k]);
-    // (infinities and NaN have the exponent 1025)
-    s.ok = b.ok != 0 && (int)(all >> 20) - 1022 <= 150;
+      if (fx_used(k, D) && (k < kMxRhoLow || k > kMxXLow)) all = max(all, mx[k]);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) spread = max(spread, mx[kMxRho + k] + mx[kMxRhoLow + k] - kHighInf);
+    // (infinities and NaN have the exponent 1025; high words order like logarithms)
+    s.ok = b.ok != 0 && (int)(all >> 20) - 1022 <= 150 && spread <= kMaxSpread << 19;
     u32 mass = 0, scalar = 0;
 #pragma unroll
     for (int c = 0; c < D; ++c) {
