@@ -95,8 +95,8 @@ struct PhysMoist2D {
 
   // flux_chandrashekar (:936-1003, R_q = 0) for one symmetric pair, on the
   // half-valued node quantities of node_prims and the averaged normal.
-  TAG_DEV static void volume_pair(const Params& P, const double* a, const double* b, double n1,
-                                  double n2, double* Fa, double* Fb) {
+  TAG_HD static void volume_pair(const Params& P, const double* a, const double* b, double n1,
+                                 double n2, double* Fa, double* Fb) {
     const double v1a = a[3] + b[3], v2a = a[4] + b[4];
     const double K = a[7] + b[7];
     const double vdn = n1 * v1a + n2 * v2a;
@@ -112,7 +112,7 @@ struct PhysMoist2D {
     const double rql_mean = !is_zero(a[2]) && !is_zero(b[2])
                                 ? rql_avg * ln_factor(a[2], b[2], log_difference(a[10], b[10]))
                                 : 0.0;
-    const double p_int = fma(P.R_v, rqv_avg, P.R_d * (a[0] + b[0])) * int_rcp(a[6] + b[6]);
+    const double p_int = int_div(fma(P.R_v, rqv_avg, P.R_d * (a[0] + b[0])), a[6] + b[6]);
     const double f_d = rqd_mean * vdn, f_v = rqv_mean * vdn, f_l = rql_mean * vdn;
     const double f1 = f_d + f_v + f_l;
     const double f2 = f1 * v1a + n1 * p_int;

@@ -138,8 +138,8 @@ struct PhysRainy2D {
   }
 
   // flux_ec_rain, :872-961, for one symmetric pair (no nonconservative part)
-  TAG_DEV static void volume_pair(const Params&, const double* a, const double* b, double n1,
-                                  double n2, double* Fa, double* Fb) {
+  TAG_HD static void volume_pair(const Params&, const double* a, const double* b, double n1,
+                                 double n2, double* Fa, double* Fb) {
     using C = RainyConst;
     const double v1a = a[4] + b[4], v2a = a[5] + b[5];
     const double K = a[9] + b[9];
@@ -155,7 +155,7 @@ struct PhysRainy2D {
                               : 0.0;
     // inv_ln_mean of 1/T
     const double T_log = (a[6] + b[6]) * inv_ln_factor(a[6], b[6], log_difference(a[12], b[12]));
-    const double p_int = fma(C::R_v, rv_avg, C::R_d * rd_avg) * int_rcp(a[7] + b[7]);
+    const double p_int = int_div(fma(C::R_v, rv_avg, C::R_d * rd_avg), a[7] + b[7]);
     const double f_v = rv_log * vdn;
     const double f_c = rc_avg * vdn;
     const double f_d = rd_log * vdn;
