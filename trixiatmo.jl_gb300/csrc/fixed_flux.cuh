@@ -77,10 +77,17 @@ struct FxBasis {
   u64 Q[64];
   i64 W[8];
   float row;  // the largest row sum of |Q|, over 2^sq
-  int S[2];   // relative change of the first and last node's weight, times 2^63
-  int sq, kw, ok, pad[2];  // (a multiple of 16 bytes)
+  // the density's and the pressures' sums that leave a row room: mass fluxes to 0.36 for
+  // normal velocities of 2 kTopV kTopN per unit of Q, pressure fluxes to 0.24
+  float top_rho, top_p;
+  int S[2];  // relative change of the first and last node's weight, times 2^63
+  int sq, kw, ok;  // (a multiple of 16 bytes)
 };
 static_assert(sizeof(FxBasis) % 16 == 0, "16-byte aligned");
+
+constexpr float kTop = 0.48f;   // bound of a word
+constexpr float kTopV = 0.48f;  // of the sum of a node's velocity components
+constexpr float kTopN = 0.49f;  // of two nodes' contravariant vectors
 
 inline void load_fixed_basis(FxBasis& f, const double* Ds, const double* w, int n) {
   std::memset(&f, 0, sizeof(f));
@@ -102,6 +109,8 @@ inline void load_fixed_basis(FxBasis& f, const double* Ds, const double* w, int 
   f.sq = std::ilogb(one) + 1;
   f.kw = std::ilogb(winv) + 2;
   f.row = (float)std::ldexp(row, -f.sq) * 1.00001f;
+  f.top_rho = std::fmin(kTop, 0.36f / (2.0f * kTopV * kTopN * f.row));
+  f.top_p = std::fmin(kTop, 0.24f / (kTopN * f.row));
   // The weights and the operator are rounded by themselves, so w_a Dsplit_ab and
   // -w_b Dsplit_ba differ in their last places: the weights are adjusted to the
   // least sum of those relative differences squared (by a few 1e-16), and the
@@ -250,114 +259,68 @@ TAG_HD void fx_fit(float& x, int& s, float top) {
 // room for the sums over a row of Q is left in density, pressure and h.
 template <int D>
 TAG_HD void fx_scale(const u32* mx, const FxBasis& b, int d, FxScale<D>& s) {
-  const float top = 0.48f, top_n = 0.49f;
   // value < 2^e
   const auto e = [mx](int k) { return max((int)(mx[k] >> 20) - 1022, -150); };
   // velocities: the sums of a node's components and of two nodes' values fit a word
   int sv[D], most_v = -1000;
   float v[D], sum_v = 0.0f;
+  u32 mass = 0, scalar = 0;
 #pragma unroll
   for (int c = 0; c < D; ++c) {
-    sv[c] = e(kMxV + c) + 2;
-    v[c] = fx_fraction(mx[kMxV + c], sv[c]);
+    const u32 m = mx[kMxV + c];
+    sv[c] = max((int)(m >> 20) - 1022, -150) + 2;
+    v[c] = fx_fraction(m, sv[c]);
     sum_v += v[c];
+    mass |= m | mx[kMxFm + c];
+    scalar |= m | mx[kMxFe + c];
   }
 #pragma unroll
   for (int c = 0; c < D; ++c) {
-    if (!(sum_v <= top)) {
+    if (!(sum_v <= kTopV)) {
       v[c] *= 0.5f;
       sum_v -= v[c];
       sv[c] += 1;
     }
     most_v = max(most_v, sv[c]);
   }
-  // Scales sN of the weighted normals Q n by component (n: of a pair, per unit of Q)
-  // and svn of the normal velocity; vn is that of a pair, per unit of Q, and most_vn
-  // the largest of all directions'.
-  int sN[D], svn = 0;
-  float vn = 0.0f, most_vn = 0.0f;
-#pragma unroll
-  for (int dd = 0; dd < D; ++dd) {
-    float n[D], sum = 0.0f;
-    int sn[D], top_s = -10000;
-#pragma unroll
-    for (int c = 0; c < D; ++c) {
-      const u32 m = mx[kMxN + 3 * dd + c];
-      sn[c] = e(kMxN + 3 * dd + c) + 2;
-      n[c] = 2.0f * fx_fraction(m, sn[c]);
-      if (!(n[c] <= top_n)) {
-        n[c] *= 0.5f;
-        sn[c] += 1;
-      }
-      sn[c] += b.sq;
-      top_s = max(top_s, sn[c] + sv[c]);
-    }
-#pragma unroll
-    for (int c = 0; c < D; ++c) sum += 2.0f * v[c] * n[c] * pow2f(sn[c] + sv[c] - top_s);
-    most_vn = fmaxf(most_vn, sum);
-    if (dd == d) {
-#pragma unroll
-      for (int c = 0; c < D; ++c) sN[c] = sn[c];
-      svn = top_s;
-      vn = sum;
-    }
-  }
-  // density: a row's mass fluxes to 0.36, surface fluxes to 1/8
+  // density sum
   int sr = e(kMxRho) + 2;
   float rho = 2.0f * fx_fraction(mx[kMxRho], sr);
-  fx_fit(rho, sr, fminf(top, 0.36f / (b.row * fmaxf(most_vn, 1e-6f))));
+  fx_fit(rho, sr, b.top_rho);
   // x = mean(scalar) + v.v
   int sx = max(e(kMxX) + 2, 2 * most_v);
   float x = 2.0f * fx_fraction(mx[kMxX], sx);
 #pragma unroll
   for (int c = 0; c < D; ++c) x += v[c] * v[c] * pow2f(2 * sv[c] - sx);
-  fx_fit(x, sx, top);
-  // pressure sum +- 2 rho_mean g: a row's pressure fluxes to 0.24, its transported
-  // momentum to 0.1
+  fx_fit(x, sx, kTop);
+  // pressure sum +- 2 rho_mean g; a row's transported momentum to 0.1
   const int sg = e(kMxG) + 2;
-  const float g = 2.0f * fx_fraction(mx[kMxG], sg);
   int sp = max(max(e(kMxP) + 2, sr + sg + 1), sr + 2 * most_v + 1);
-  float pp = 2.0f * fx_fraction(mx[kMxP], sp) + rho * g * pow2f(sr + sg + 1 - sp);
-  fx_fit(pp, sp, fminf(top, 0.24f / (top_n * b.row)));
-  if (d == 0) {
-    u32 all = 0, spread = 0;
-#pragma unroll
-    for (int k = 0; k < kMxCount; ++k)
-      if (fx_used(k, D) && (k < kMxRhoLow || k > kMxXLow)) all = max(all, mx[k]);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) spread = max(spread, mx[kMxRho + k] + mx[kMxRhoLow + k] - kHighInf);
-    // (infinities and NaN have the exponent 1025; high words order like logarithms)
-    s.ok = b.ok != 0 && (int)(all >> 20) - 1022 <= 150 && spread <= kMaxSpread << 19;
-    u32 mass = 0, scalar = 0;
-#pragma unroll
-    for (int c = 0; c < D; ++c) {
-      s.sv[c] = sv[c];
-      mass |= mx[kMxV + c] | mx[kMxFm + c];
-      scalar |= mx[kMxV + c] | mx[kMxFe + c];
-    }
-    s.zero[0] = mass == 0;
-    s.zero[1] = scalar == 0;
-    s.sr = sr;
-    s.sp = sp;
-    s.sx = sx;
-    s.sg = sg;
-  }
-  // surface fluxes to 1/8
-  const int own = svn;
-  svn = max(svn, e(kMxFm + d) + 3 - sr);
+  float pp = 2.0f * fx_fraction(mx[kMxP], sp) +
+             rho * (2.0f * fx_fraction(mx[kMxG], sg)) * pow2f(sr + sg + 1 - sp);
+  fx_fit(pp, sp, b.top_p);
+  // This direction's weighted normals Q n: scale sN by component; surface fluxes to 1/8.
+  // The normal velocity: scale svn; vn: of a pair per unit of Q.
+  int sN[D], svn = e(kMxFm + d) + 3 - sr;
+  float vn = 0.0f;
 #pragma unroll
   for (int c = 0; c < D; ++c) {
-    sN[c] = max(sN[c], e(kMxFv + 3 * d + c) + 3 - sp);
+    const u32 m = mx[kMxN + 3 * d + c];
+    sN[c] = max((int)(m >> 20) - 1022, -150) + 2;
+    if (!(2.0f * fx_fraction(m, sN[c]) <= kTopN)) sN[c] += 1;
+    sN[c] = max(sN[c] + b.sq, e(kMxFv + 3 * d + c) + 3 - sp);
     svn = max(svn, sN[c] + sv[c]);
   }
-  vn *= pow2f(own - svn);
+#pragma unroll
+  for (int c = 0; c < D; ++c)
+    vn += 4.0f * v[c] * fx_fraction(mx[kMxN + 3 * d + c], svn - sv[c] - b.sq);
   // h = rho_mean x + (p +- 2 rho_mean g) / 2, shifted left by kj: by what a row of it with
   // the pressures' difference and the surface fluxes leave
   int sh = max(sr + sx, sp - 1);
   const float h = rho * x * pow2f(sr + sx - sh) + pp * pow2f(sp - 1 - sh);
   const float row_h = b.row * vn * (h + fx_fraction(mx[kMxP], sp) * pow2f(sp - 1 - sh)) +
                       0.5f * fx_fraction(mx[kMxFe + d], sh + svn);
-  const int room = min(min(fx_room(h, top), fx_room(row_h, top)), 8), kj = max(room, 0);
+  const int room = min(fx_room(fmaxf(h, row_h), kTop), 8), kj = max(room, 0);
   sh -= room;
   FxShift k{};
 #pragma unroll
@@ -374,6 +337,26 @@ TAG_HD void fx_scale(const u32* mx, const FxBasis& b, int d, FxScale<D>& s) {
   s.k[d] = k;
   s.sum[d][0] = sr + svn;
   s.sum[d][D + 1] = sh + svn;
+  if (d == 0) {
+    u32 all = 0, spread = 0;
+#pragma unroll
+    for (int k = 0; k < kMxCount; ++k)
+      if (fx_used(k, D)) all = max(all, mx[k]);
+#pragma unroll
+    for (int f = 0; f < 3; ++f)
+      spread = max(spread, mx[kMxRho + f] + mx[kMxRhoLow + f] - kHighInf);
+    // (infinities and NaN have the exponent 1025; high words order like logarithms; the
+    // Low entries of values above 2^-150 are in the range, too)
+    s.ok = b.ok != 0 && (int)(all >> 20) - 1022 <= 150 && spread <= kMaxSpread << 19;
+#pragma unroll
+    for (int c = 0; c < D; ++c) s.sv[c] = sv[c];
+    s.sr = sr;
+    s.sp = sp;
+    s.sx = sx;
+    s.sg = sg;
+    s.zero[0] = mass == 0;
+    s.zero[1] = scalar == 0;
+  }
 }
 
 // The sum over the D directions of A[d stride] W_d (words of scales sd[d], W_d >=
