@@ -424,7 +424,8 @@ int tag_set_elements_per_block(tag_handle h, int32_t epb);
 int tag_get_elements_per_block(tag_handle h, int32_t* epb);
 /* Fixes the tile: epb elements per CTA, 1 or 2 work items per thread and phase. */
 int tag_set_tile(tag_handle h, int32_t epb, int32_t items_per_thread);
-/* Threads per CTA of the element kernel for the current tile (measurement). */
+/* Threads per CTA that the element kernel is launched with for the current tile
+ * (measurement). */
 int tag_get_cta_threads(tag_handle h, int32_t* threads);
 
 /* Geometry of the cubed-sphere shell built on the device: what TrixiAtmo's

@@ -147,7 +147,8 @@ struct tag_handle_s {
   bool speed_valid = false;
   int epb = 0;
   // threads of a CTA = its elements' work items / tile_div, rounded up to
-  // whole warps (one to three items per thread and phase; 3D: tile_threads)
+  // whole warps (one to three items per thread and phase; 3D: tile_threads), and
+  // no more than the kernel's registers allow (Ops::launch_threads)
   int tile_div = 1;
   const Ops* ops = nullptr;
   // analysis (allocated by the first analysis call)
@@ -170,7 +171,8 @@ struct Ops {
   int (*init)(int max_smem);
   size_t (*smem_bytes)(int epb);
   int threads_per_element;
-  int (*max_threads)();  // per-CTA thread limit of the element kernels (registers)
+  int (*max_threads)();  // a tile's largest number of work items for one CTA
+  int (*launch_threads)(tag_handle h);  // threads that an element kernel's CTA is launched with
 };
 
 // The launchers of each system for n nodes per direction (null: not built).

@@ -64,7 +64,7 @@ struct OpsImpl {
                      double t) {
     const int epb = h->epb > 0 ? h->epb : 4;
     const int blocks = (h->nelem + epb - 1) / epb;
-    const int threads = std::min(cap(), cta_threads(epb * S::TPE, h->tile_div));
+    const int threads = launch_threads(h);
     const size_t smem = S::bytes(epb);
     StageArgs st{};
     st.member = h->d_member;
@@ -109,10 +109,13 @@ struct OpsImpl {
     return c;
   }
   static int max_threads() { return cap(); }
+  static int launch_threads(tag_handle h) {
+    return std::min(cap(), cta_threads((h->epb > 0 ? h->epb : 4) * S::TPE, h->tile_div));
+  }
   static size_t smem_bytes(int epb) { return S::bytes(epb); }
   static const Ops* get() {
     static const Ops ops{&interface, &element, &max_speed, nullptr, &init, &smem_bytes,
-                         S::TPE, &max_threads};
+                         S::TPE, &max_threads, &launch_threads};
     return &ops;
   }
 };

@@ -20,7 +20,7 @@ struct OpsImpl3D {
                      double) {
     const int epb = h->epb > 0 ? h->epb : 1;
     const int blocks = (h->nelem + epb - 1) / epb;
-    const int threads = std::min(cap(), tile_threads(epb * S::TPE, h->tile_div));
+    const int threads = launch_threads(h);
     const size_t smem = S::bytes(epb);
     StageArgs st{};
     st.member = h->d_member;
@@ -65,10 +65,13 @@ struct OpsImpl3D {
     return c;
   }
   static int max_threads() { return 1024; }  // of a tile; the kernel strides over its work
+  static int launch_threads(tag_handle h) {
+    return std::min(cap(), tile_threads((h->epb > 0 ? h->epb : 1) * S::TPE, h->tile_div));
+  }
   static size_t smem_bytes(int epb) { return S::bytes(epb); }
   static const Ops* get() {
     static const Ops ops{&interface, &element, &max_speed, &load_state, &init, &smem_bytes,
-                         S::TPE, &max_threads};
+                         S::TPE, &max_threads, &launch_threads};
     return &ops;
   }
 };

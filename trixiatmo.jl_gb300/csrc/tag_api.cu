@@ -268,9 +268,10 @@ int cov_init(int max_smem) {
 
 size_t cov_smem_bytes(int) { return 0; }
 int cov_max_threads() { return 256; }
+int cov_launch_threads(tag_handle h) { return h->cov_threads; }
 
 const Ops kCovOps{&cov_interface, &cov_element, &cov_max_speed, nullptr, &cov_init,
-                  &cov_smem_bytes, 256, &cov_max_threads};
+                  &cov_smem_bytes, 256, &cov_max_threads, &cov_launch_threads};
 
 // Flux options of a covariant member configuration; returns the reason it is
 // rejected, or null.
@@ -1519,11 +1520,7 @@ int tag_set_tile(tag_handle h, int32_t epb, int32_t items_per_thread) {
 
 int tag_get_cta_threads(tag_handle h, int32_t* threads) {
   if (!h || !threads) return fail(TAG_E_INVALID, "null argument");
-  const int epb = h->epb > 0 ? h->epb : 1;
-  const int items = h->ops ? epb * h->ops->threads_per_element : 0, div = h->tile_div;
-  *threads = !h->ops ? 0
-                     : std::min(h->ops->max_threads(), h->dim == 3 ? tile_threads(items, div)
-                                                                   : cta_threads(items, div));
+  *threads = h->ops ? h->ops->launch_threads(h) : 0;
   return TAG_OK;
 }
 
