@@ -418,12 +418,17 @@ void* tag_stream(tag_handle h);
  * autotuner, run on the first step or rhs call, times the element kernel for
  * elements per CTA in {1, 2, 3, 4, 6, 8, 12, 16} (the shared-memory tile: each
  * element's state, metric terms and accumulators staged once) and, for each,
- * one or two work items per thread and phase (the CTA width), and keeps the
- * fastest; setting a value here fixes the tile with one item per thread. */
+ * one to three work items per thread and phase (the CTA width; in 3D also
+ * those widths rounded up to whole groups of four warps), and keeps the
+ * fastest; setting a value here fixes the tile with one item per thread.
+ * Results do not depend on the tile. */
 int tag_set_elements_per_block(tag_handle h, int32_t epb);
 int tag_get_elements_per_block(tag_handle h, int32_t* epb);
-/* Fixes the tile: epb elements per CTA, 1 or 2 work items per thread and phase. */
+/* Fixes the tile: epb elements per CTA, 1 to 3 work items per thread and phase;
+ * in 3D, 4 to 6 are 1 to 3 items with the CTA in whole groups of four warps. */
 int tag_set_tile(tag_handle h, int32_t epb, int32_t items_per_thread);
+/* The current tile as tag_set_tile takes it (epb 0: not chosen yet). */
+int tag_get_tile(tag_handle h, int32_t* epb, int32_t* items_per_thread);
 /* Threads per CTA that the element kernel is launched with for the current tile
  * (measurement). */
 int tag_get_cta_threads(tag_handle h, int32_t* threads);

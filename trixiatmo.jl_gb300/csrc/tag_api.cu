@@ -7,6 +7,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -166,14 +167,17 @@ int autotune(tag_handle h, const double* u) {
   int best = 1, best_div = 1;
   float best_ms = 1e30f;
   // (elements per CTA, tile_div): every element count with one to three items
-  // per thread (3D also in whole groups of four warps)
+  // per thread (3D also in whole groups of four warps), each launch once
   std::vector<std::pair<int, int>> tiles;
+  std::set<std::pair<int, int>> launches;
   for (int c : {1, 2, 3, 4, 6, 8, 12, 16})
     for (int div = 1; div <= (h->dim == 3 ? 6 : 3); ++div) {
       const int share = (div - 1) % 3 + 1;  // work items per thread
       if (c * h->ops->threads_per_element > h->ops->max_threads() && c > 1) continue;
       if (share > 1 && c * h->ops->threads_per_element < 64 * share) continue;
-      tiles.push_back({c, div});
+      h->epb = c;
+      h->tile_div = div;
+      if (launches.insert({c, h->ops->launch_threads(h)}).second) tiles.push_back({c, div});
     }
   for (const auto& [c, div] : tiles) {
     if ((size_t)h->ops->smem_bytes(c) > (size_t)max_smem) continue;
@@ -1510,11 +1514,18 @@ int tag_get_elements_per_block(tag_handle h, int32_t* epb) {
 }
 
 int tag_set_tile(tag_handle h, int32_t epb, int32_t items_per_thread) {
-  if (!h || epb < 1 || items_per_thread < 1 || items_per_thread > 2)
+  if (!h || epb < 1 || items_per_thread < 1 || items_per_thread > (h->dim == 3 ? 6 : 3))
     return fail(TAG_E_INVALID, "bad argument");
   int rc = tag_set_elements_per_block(h, epb);
   if (rc) return rc;
   h->tile_div = items_per_thread;
+  return TAG_OK;
+}
+
+int tag_get_tile(tag_handle h, int32_t* epb, int32_t* items_per_thread) {
+  if (!h || !epb || !items_per_thread) return fail(TAG_E_INVALID, "null argument");
+  *epb = h->epb;
+  *items_per_thread = h->tile_div;
   return TAG_OK;
 }
 

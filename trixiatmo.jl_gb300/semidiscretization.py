@@ -693,8 +693,15 @@ class SemidiscretizationHyperbolic:
         return v.value
 
     def set_tile(self, epb, items_per_thread=1):
-        """Fixes the element kernel's tile (otherwise autotuned)."""
+        """Fixes the element kernel's tile (otherwise autotuned): elements per CTA and 1 to 3 work
+        items per thread (3D: 4 to 6 are those in whole groups of four warps)."""
         _lib.check(self._L.tag_set_tile(self._h, int(epb), int(items_per_thread)))
+
+    def tile(self):
+        """The current tile, as `set_tile` takes it (elements per CTA 0: not chosen yet)."""
+        epb, items = ctypes.c_int32(), ctypes.c_int32()
+        _lib.check(self._L.tag_get_tile(self._h, ctypes.byref(epb), ctypes.byref(items)))
+        return epb.value, items.value
 
     def cta_threads(self):
         """Threads per CTA of the element kernel for the current tile."""
