@@ -459,8 +459,9 @@ int tag_fp64_peak(double* flops_per_s);
  * evaluates the device forms of those means on n host value pairs (x[q],
  * y[q]) in one kernel.  kind 0: the element kernels' integer forms from node
  * logarithms; 3: the interface kernels' forms of the values themselves; 1 and
- * 2: the FP64 polynomial forms of halved values (ranges 0.01 and 0.09 of f2,
- * logarithms beyond); 4: the potential-temperature kernels' Stolarsky mean
+ * 2: FP64 polynomial forms of halved values (ranges 0.01 and 0.09 of f2,
+ * logarithms beyond), which no right-hand side takes: the forms that the
+ * integer ones are held against; 4: the potential-temperature kernels' Stolarsky mean
  * with gamma = cp / cv; 5 and 6: kind 2 with one mean's pair (x[q], y[q]) and
  * the other's (1, 1), so that the two means take different forms
  * (5: ln_mean of the pair in out1; 6: inv_ln_mean of the pair in out2).

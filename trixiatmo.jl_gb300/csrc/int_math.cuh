@@ -3,9 +3,9 @@
 //
 // Why: GB300 issues 2 FP64 operations per SM and clock (a measured DFMA stream
 // reaches 1.57), but 128 32-bit ones; a warp's FP64 instruction takes the pipe
-// for 16 cycles, in which four sub-partitions issue 64 others.  The element and
-// interface kernels keep the FP64 pipe 75-89 % busy and issue only 6-11
-// instructions per FP64 one.  Measured in FP64-operation times on this chip,
+// for 16 cycles, in which four sub-partitions issue 64 others.  With CUDA's FP64
+// functions the element and interface kernels kept that pipe 75-89 % busy and
+// issued only 6-11 instructions per FP64 one.  Measured in FP64-operation times on this chip,
 // 1/x costs 4.5, a/b 7.1, sqrt 7.5, rsqrt 4.7, exp 16, log 31 and pow 78; the
 // forms below take the FP64 pipe for none of them.  The integer pipe multiplies
 // 32 x 32 -> 64 bits at 22 per SM and clock: a 64-bit high product costs 0.2

@@ -1,5 +1,5 @@
-"""Coefficients of the polynomial forms of the logarithmic mean used by the
-device code (tag_common.cuh).
+"""Coefficients of the FP64 polynomial forms of the logarithmic mean in
+tag_common.cuh, against which the kernels' integer forms are held.
 
 With f = ((y - x)/(y + x))^2 and z = sqrt(f),
     ln_mean(x, y)     = (x + y)/2 * R(f),   R(f) = z / atanh(z),

@@ -1,7 +1,7 @@
-// tag_eval_means: evaluates the device forms of the logarithmic and Stolarsky
-// means (the kernels' own inline functions) on arrays of value pairs, so that
-// they can be checked directly against exact values on both sides of every
-// branch threshold.  Diagnostics only: no kernel of the right-hand side calls
+// tag_eval_means: evaluates device forms of the logarithmic and Stolarsky means
+// (kinds 0, 3, 4, 7 and 8 the kernels' own inline functions, the others FP64 forms
+// to hold them against) on arrays of value pairs, so that they can be checked
+// directly against exact values on both sides of every branch threshold.  Diagnostics only: no kernel of the right-hand side calls
 // this path.
 #include <cuda_runtime.h>
 
