@@ -62,7 +62,7 @@ int element(const double* par, int n, const double* Ds, const double* w, const d
     for (int k = 0; k < face * NA; ++k)
       up(fx_face_max<D>(k % NA, f / 2), high_magnitude(sf[f * face * NA + k]));
   FxScale<D> s;
-  for (int d = 0; d < D; ++d) fx_scale<D>(mx, b, d, s);
+  for (int d = 0; d < fx_groups(D); ++d) fx_scale<D>(mx, b, d, s);
 
   for (int d = 0; d < D; ++d)
     for (int i = 0; i < N; ++i)
@@ -93,7 +93,7 @@ int element(const double* par, int n, const double* Ds, const double* w, const d
   for (int i = 0; i < N; ++i) {
     fx_convert_node<D>(&q[i * NQ], s);
     for (int k = 0; k < D * D; ++k)
-      ja[i * D * D + k] = f64_from((u64)to_fixed(ja[i * D * D + k], s.sn[k / D][k % D] - 2));
+      ja[i * D * D + k] = f64_from((u64)to_fixed(ja[i * D * D + k], s.sn[fx_group(D, k / D)][k % D] - 2));
   }
   for (int d = 0; d < D; ++d) {
     for (int i = 0; i < N; ++i)
@@ -103,7 +103,7 @@ int element(const double* par, int n, const double* Ds, const double* w, const d
         i64 Fa[NA], Fb[NA];
         if (Q & 1) std::swap(a, c);
         Phys::fixed_pair(P, &q[a * NQ], &q[c * NQ], &ja[(a * D + d) * D], &ja[(c * D + d) * D], Q,
-                         s.k[d], Fa, Fb);
+                         s.k[fx_group(D, d)], Fa, Fb);
         for (int v = 0; v < NA; ++v) {
           A[(d * N + a) * NA + v] += Fa[v];
           A[(d * N + c) * NA + v] -= Fb[v];
@@ -113,14 +113,14 @@ int element(const double* par, int n, const double* Ds, const double* w, const d
       for (int k = 0; k < face; ++k)
         for (int v = 0; v < NA; ++v)
           A[(d * N + node(2 * d + e, k)) * NA + v] +=
-              fx_surface(sf[((2 * d + e) * face + k) * NA + v], s.sum[d][v] + (v == NA - 1), b.S[e]);
+              fx_surface(sf[((2 * d + e) * face + k) * NA + v], s.sum[fx_group(D, d)][v] + (v == NA - 1), b.S[e]);
   }
   for (int i = 0; i < N; ++i)
     for (int v = 0; v < NA; ++v) {
       int pos[D], sd[D], scale;
       for (int d = 0; d < D; ++d) {
         pos[d] = at(i, d);
-        sd[d] = s.sum[d][v];
+        sd[d] = s.sum[fx_group(D, d)][v];
       }
       const i64 t = fx_weighted_sum<D>(&A[i * NA + v], N * NA, b.W, pos, sd, scale);
       words[i * NA + v] =

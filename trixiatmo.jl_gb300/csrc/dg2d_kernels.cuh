@@ -250,14 +250,9 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
                           [&m](int k, u32 x) { m[k] = max(m[k], x); });
       for (int k = lane; k < 4 * n; k += 32) {
         const double* sf = sfv + ((size_t)(e_first + el) * 4 * n + k) * NA;
-        const bool second = k >= 2 * n;
 #pragma unroll
-        for (int v = 0; v < NA; ++v) {
-          const u32 a = high_magnitude(sf[v]);
-          u32 &m0 = m[fx_face_max<2>(v, 0)], &m1 = m[fx_face_max<2>(v, 1)];
-          m0 = max(m0, second ? 0u : a);
-          m1 = max(m1, second ? a : 0u);
-        }
+        for (int v = 0; v < NA; ++v)
+          m[fx_face_max<2>(v, 0)] = max(m[fx_face_max<2>(v, 0)], high_magnitude(sf[v]));
       }
 #pragma unroll
       for (int k = 0; k < kMxCount; ++k)
@@ -269,9 +264,9 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
       }
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < 2 * ne; t += nthr) {
-      double* eb = base + (t >> 1) * S::per_elem;
-      fx_scale<2>(reinterpret_cast<const u32*>(eb + S::oC), sb->fx, t & 1,
+    for (int el = threadIdx.x; el < ne; el += nthr) {
+      double* eb = base + el * S::per_elem;
+      fx_scale<2>(reinterpret_cast<const u32*>(eb + S::oC), sb->fx, 0,
                   *reinterpret_cast<FxScale<2>*>(eb + S::oF));
     }
     __syncthreads();
@@ -283,7 +278,7 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
       fx_convert_node<2>(eb + S::oQ + node * NQ, fs);
       double* ja = eb + S::oJa + node * 4;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) ja[c] = f64_from((u64)to_fixed(ja[c], fs.sn[c / 2][c % 2] - 2));
+      for (int c = 0; c < 4; ++c) ja[c] = f64_from((u64)to_fixed(ja[c], fs.sn[0][c % 2] - 2));
     }
     __syncthreads();
   }
@@ -331,7 +326,7 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
         const int p = turn ? nb_ : na_, q = turn ? na_ : nb_;
         i64 Fa[NA], Fb[NA];
         Phys::fixed_pair(Pp, eb + S::oQ + p * NQ, eb + S::oQ + q * NQ, turn ? ja_b : ja_a,
-                         turn ? ja_a : ja_b, Qab, fs.k[d], Fa, Fb);
+                         turn ? ja_a : ja_b, Qab, fs.k[0], Fa, Fb);
         double *cp = turn ? cb : ca, *cq = turn ? ca : cb;
 #pragma unroll
         for (int v = 0; v < NA; ++v) {
@@ -383,7 +378,7 @@ __global__ void k_element(typename Phys::Params Pp, const BasisDev basis, double
     double acc = 0.0;
     if (VOL == kVolFluxDiff && Phys::kFixed && fs.ok) {
       // sums of words and unweighted surface fluxes, then 1/w per direction
-      const int sd[2] = {fs.sum[0][v], fs.sum[1][v]}, at[2] = {i, j};
+      const int sd[2] = {fs.sum[0][v], fs.sum[0][v]}, at[2] = {i, j};
       i64 A[2] = {0, 0};
 #pragma unroll
       for (int d = 0; d < 2; ++d) {

@@ -134,11 +134,11 @@ struct ElemSmem3D {
 };
 
 template <class Phys, int n, int MODE>
-__global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, double* __restrict__ u,
-                            double* __restrict__ du, double* __restrict__ kreg,
-                            const double* __restrict__ Ja, const double* __restrict__ invJ,
-                            const double* sfv, int nelem, int epb, StageArgs st,
-                            unsigned* __restrict__ status) {
+TAG_DEV void element3d_body(const typename Phys::Params& Pp, const BasisDev& basis,
+                            double* __restrict__ u, double* __restrict__ du,
+                            double* __restrict__ kreg, const double* __restrict__ Ja,
+                            const double* __restrict__ invJ, const double* sfv, int nelem, int epb,
+                            const StageArgs& st, unsigned* __restrict__ status) {
   using S = ElemSmem3D<Phys, n>;
   constexpr int NV = Phys::NV, NA = Phys::NA, NQ = Phys::NQ;
   constexpr int nn = S::nn, nnn = S::nnn;
@@ -450,6 +450,35 @@ __global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, doub
     }
   }
   if (bad) atomicOr(status, bad);
+}
+
+template <class Phys, int n, int MODE>
+__global__ void k_element3d(typename Phys::Params Pp, const BasisDev basis, double* __restrict__ u,
+                            double* __restrict__ du, double* __restrict__ kreg,
+                            const double* __restrict__ Ja, const double* __restrict__ invJ,
+                            const double* sfv, int nelem, int epb, StageArgs st,
+                            unsigned* __restrict__ status) {
+  element3d_body<Phys, n, MODE>(Pp, basis, u, du, kreg, Ja, invJ, sfv, nelem, epb, st, status);
+}
+// The stage kernels in words, held to 80 registers (no spills): three CTAs of eight
+// warps share an SM, where the 96 that the compiler takes by itself leave two.  Shell of
+// 2,654,208 nodes, polydeg 5: a stage 1.18 ms with 96 and 1.00 ms with 80.  Right-hand
+// sides, which keep less, are faster without the bound (1.114 against 1.131 ms); up to
+// polydeg 3 they take it, too, because their times choose the stages' tile (coarse shell
+// run 1.43 against 1.38 ms).
+template <class Phys, int n, int MODE>
+__global__ void __launch_bounds__(768) k_element3d_words(
+    typename Phys::Params Pp, const BasisDev basis, double* __restrict__ u, double* __restrict__ du,
+    double* __restrict__ kreg, const double* __restrict__ Ja, const double* __restrict__ invJ,
+    const double* sfv, int nelem, int epb, StageArgs st, unsigned* __restrict__ status) {
+  element3d_body<Phys, n, MODE>(Pp, basis, u, du, kreg, Ja, invJ, sfv, nelem, epb, st, status);
+}
+template <class Phys, int n, int MODE>
+constexpr auto element3d_kernel() {
+  if constexpr (Phys::kFixed && (MODE == kModeStage || n <= 4))
+    return &k_element3d_words<Phys, n, MODE>;
+  else
+    return &k_element3d<Phys, n, MODE>;
 }
 
 // One warp per element (a 3D element has up to 512 nodes): the lanes stride

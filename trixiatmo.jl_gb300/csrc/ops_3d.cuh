@@ -29,11 +29,11 @@ struct OpsImpl3D {
       st.dt = h->d_mscal + h->nmembers;
       st.max_speed = last ? h->d_mscal + 2 * h->nmembers : nullptr;
       st.sink = last && h->capturing_steps ? h->sink : nullptr;
-      TAG_CUDA(launch_overlapped(h->overlap(), k_element3d<Phys, n, kModeStage>, blocks, threads,
+      TAG_CUDA(launch_overlapped(h->overlap(), element3d_kernel<Phys, n, kModeStage>(), blocks, threads,
                                  smem, h->stream, params_of<Phys>(h), h->basis, u, du, h->d_k,
                                  h->d_Ja, h->d_invJ, h->d_sfv, h->nelem, epb, st, h->d_status));
     } else {
-      TAG_CUDA(launch_overlapped(h->overlap(), k_element3d<Phys, n, kModeRhs>, blocks, threads,
+      TAG_CUDA(launch_overlapped(h->overlap(), element3d_kernel<Phys, n, kModeRhs>(), blocks, threads,
                                  smem, h->stream, params_of<Phys>(h), h->basis, u, du, h->d_k,
                                  h->d_Ja, h->d_invJ, h->d_sfv, h->nelem, epb, st, h->d_status));
     }
@@ -53,11 +53,11 @@ struct OpsImpl3D {
     return TAG_OK;
   }
   static int init(int max_smem) {
-    TAG_CUDA(cudaFuncSetAttribute(k_element3d<Phys, n, kModeStage>,
+    TAG_CUDA(cudaFuncSetAttribute(element3d_kernel<Phys, n, kModeStage>(),
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
-    TAG_CUDA(cudaFuncSetAttribute(k_element3d<Phys, n, kModeRhs>,
+    TAG_CUDA(cudaFuncSetAttribute(element3d_kernel<Phys, n, kModeRhs>(),
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
-    return launch_thread_cap(k_element3d<Phys, n, kModeStage>, k_element3d<Phys, n, kModeRhs>,
+    return launch_thread_cap(element3d_kernel<Phys, n, kModeStage>(), element3d_kernel<Phys, n, kModeRhs>(),
                              cap());
   }
   static int& cap() {
