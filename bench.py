@@ -402,8 +402,7 @@ def run_swe(args):
     fl = sum(6 * k * k * (N + 1) ** 2 * ALGORITHMIC_OPS[f"swe_{args.swe_variant}_{N}"]["element"]
              for k, N, _, _ in specs)
     peak_fp64, peak_src, probe_fp64 = fp64_roofline_peak(tg, clock_info)
-    achieved_tf = fl / (ms_el * 1e-3) / 1e12
-    traffic = TRAFFIC_PER_DOF.get("swe" if args.swe_variant == "weak" else "swe_ec")
+    capture = CAPTURED["swe" if args.swe_variant == "weak" else "swe_ec"]
     cpu = None if args.no_cpu else cpu_oracle_rate_swe(tg, args, eq)[0]
     line = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": 1, "steps": args.steps,
@@ -417,18 +416,12 @@ def run_swe(args):
                    "dofs": dofs, "elements": ens.nelements, "members": M,
                    "degree_runs": int(ens._H.nmembers), "build_seconds": t_build,
                    "l2": "inputs larger than L2 (u + k + packed metric data)"},
-        "roofline": {"bound": "fp64", "achieved": achieved_tf, "peak": peak_fp64 / 1e12,
-                     "unit": "TFLOP/s", "frac": achieved_tf / (peak_fp64 / 1e12),
-                     "traffic": (traffic * dofs) if traffic else None,
-                     "traffic_source": "ncu dram__bytes_read+write per DOF of a capture, "
-                                       "scaled by DOF" if traffic else None,
+        "roofline": {**fp64_roofline(capture, dofs, ms_el, fl, peak_fp64, probe_fp64),
                      "kernel": "k_cov_element (volume + surface + Jacobian + sources + RK stage)",
-                     "peak_source": peak_src, "fma_stream_tflops": probe_fp64 / 1e12,
-                     "frac_of_fma_stream": achieved_tf / (probe_fp64 / 1e12),
+                     "peak_source": peak_src,
                      "hbm_achieved_gbs": gbs, "hbm_peak_gbs": hbm_peak,
                      "hbm_frac": gbs / hbm_peak, "hbm_peak_source": hbm_src,
                      "ms_element": ms_el, "ms_interface": ms_if,
-                     "flops_per_launch": fl, "flops_source": FLOPS_SOURCE,
                      "bytes_per_launch": by},
         "ensemble_vs_sequential": {"sequential_rate": seq_value, "speedup": value / seq_value},
         "latency_ms": {"p50": float(np.percentile(lat, 50)), "p99": float(np.percentile(lat, 99)),
@@ -781,9 +774,8 @@ def run_ours(args):
         hbm_peak, hbm_src = float(peaks["hbm_gbs"]), "measured"
     except (OSError, KeyError, ValueError):
         hbm_peak, hbm_src = 6800.0, "fallback"
-    achieved_tf = fl / (ms_el * 1e-3) / 1e12
     achieved_gbs = by / (ms_el * 1e-3) / 1e9
-    traffic = TRAFFIC_PER_DOF.get(args.workload)
+    capture = CAPTURED[args.workload]
 
     # end to end through the C ABI with pinned host buffers: per step, H2D of
     # the state, one RK step (5 stages), D2H of the state.  The last stage's
@@ -833,21 +825,14 @@ def run_ours(args):
                        "elements_per_cta": semi.elements_per_block(),
                        "threads_per_cta": semi.cta_threads(), "l2": l2_note,
                        "parallelism": f"replicas x{world}"},
-            "roofline": {"bound": "fp64", "achieved": achieved_tf, "peak": peak_fp64 / 1e12,
-                         "unit": "TFLOP/s", "frac": achieved_tf / (peak_fp64 / 1e12),
-                         "traffic": (traffic * dofs) if traffic else None,
-                         "traffic_source": "ncu dram__bytes_read+write per DOF of a capture, "
-                                           "scaled by DOF" if traffic else None,
+            "roofline": {**fp64_roofline(capture, dofs, ms_el, fl, peak_fp64, probe_fp64),
                          "kernel": "element kernel (volume + surface + Jacobian + sources + "
                                    "RK stage)",
-                         "peak_source": peak_src, "fma_stream_tflops": probe_fp64 / 1e12,
-                         "frac_of_fma_stream": achieved_tf / (probe_fp64 / 1e12),
+                         "peak_source": peak_src,
                          "hbm_achieved_gbs": achieved_gbs, "hbm_peak_gbs": hbm_peak,
                          "hbm_frac": achieved_gbs / hbm_peak, "hbm_peak_source": hbm_src,
                          "ms_element": ms_el, "ms_interface": ms_if,
-                         "flops_per_launch": fl, "flops_source": FLOPS_SOURCE,
-                         "bytes_per_launch": by,
-                         "executed": executed_roofline(args.workload, dofs, ms_el, peak_fp64)},
+                         "bytes_per_launch": by},
             "e2e": {"value": e2e, "unit": UNIT, "h2d_bytes_per_step": int(u0.nbytes),
                     "d2h_bytes_per_step": int(u0.nbytes),
                     "d2h": "stored into the pinned buffer by the last stage's element kernel"},
@@ -869,26 +854,40 @@ def run_ours(args):
         torch.distributed.destroy_process_group()
 
 
-# DRAM bytes per DOF of the element kernel from ncu captures (read + write),
-# used to report `traffic` for the full-size launch.
-TRAFFIC_PER_DOF = {"shell": 281.26,      # k_element3d, stage mode, full shell
-                   "ensemble": 205.42,    # k_element 2D, stage mode, 128-member ensemble
-                   "swe": 214.71,         # k_cov_element weak form, 8 of the SWE members
-                   "swe_ec": 215.20}      # k_cov_element split EC form, the same 8 members
-# FP64 operations the element kernel executes per DOF (DFMA counted as 2), from
-# ncu (smsp__sass_thread_inst_executed_op_{dfma,dadd,dmul}; profiles/pipes_gb300.md),
-# beside the algorithmic count: the volume integral is evaluated in 64-bit words
-# on the integer pipe
-EXECUTED_FLOPS_PER_DOF = {"shell": 57.1, "ensemble": 41.7}
+# The element kernel's stage launch in ncu captures (profiles/pipes_gb300.md).
+# "traffic": dram__bytes_read + write per DOF of this workload's own launch (two
+# metrics, one pass).  "fp64": FP64 operations executed per DOF
+# (smsp__sass_thread_inst_executed_op_{dfma,dadd,dmul}, DFMA counted as 2), on
+# 663,552 shell nodes, 1,048,576 bubble nodes and the first 8 of the SWE members.
+# "bound": the energy kernels evaluate their pair fluxes in 64-bit words on the
+# integer pipe and fill neither it nor the FP64 pipe; the SWE kernels keep the
+# FP64 pipe 88-91 % busy.
+CAPTURED = {
+    "shell": {"traffic": 280.3, "fp64": 57.0, "bound": "latency (issue slots 54 %, FP64 pipe 20 %)"},
+    "ensemble": {"traffic": 210.7, "fp64": 41.7,
+                 "bound": "latency (issue slots 55 %, FP64 pipe 29 %)"},
+    "swe": {"traffic": 234.8, "fp64": 164.4, "bound": "fp64"},
+    "swe_ec": {"traffic": 234.8, "fp64": 373.6, "bound": "fp64"},
+}
 
 
-def executed_roofline(workload, dofs, ms_el, peak_fp64):
-    f = EXECUTED_FLOPS_PER_DOF.get(workload)
-    if not f:
-        return None
-    tf = f * dofs / (ms_el * 1e-3) / 1e12
-    return {"flops_per_dof": f, "achieved": tf, "frac": tf / (peak_fp64 / 1e12),
-            "source": "ncu FP64 thread instructions of the element kernel (profiles/)"}
+def fp64_roofline(capture, dofs, ms_el, formula_flops, peak_fp64, probe_fp64):
+    """The FP64 operations that the element kernel executes, against the pipe;
+    beside it the formulas' operation count over the same time, which is no
+    roofline: most of it runs as integer words or is regrouped away."""
+    achieved = capture["fp64"] * dofs / (ms_el * 1e-3) / 1e12
+    formula = formula_flops / (ms_el * 1e-3) / 1e12
+    return {"bound": capture["bound"], "achieved": achieved, "peak": peak_fp64 / 1e12,
+            "unit": "TFLOP/s", "frac": achieved / (peak_fp64 / 1e12),
+            "fma_stream_tflops": probe_fp64 / 1e12,
+            "frac_of_fma_stream": achieved / (probe_fp64 / 1e12),
+            "flops_per_launch": capture["fp64"] * dofs,
+            "flops_source": "ncu FP64 thread instructions per DOF of a capture, scaled by DOF",
+            "formula_work": {"flops_per_launch": formula_flops, "tflops": formula,
+                             "ratio_to_fp64_peak": formula / (peak_fp64 / 1e12),
+                             "flops_source": FLOPS_SOURCE},
+            "traffic": capture["traffic"] * dofs,
+            "traffic_source": "ncu dram__bytes_read+write per DOF of a capture, scaled by DOF"}
 
 
 def main():
